@@ -726,3 +726,21 @@ def test_sample_frequencies():
     expect = torch.softmax(row.double().cpu(), 0) * draws
     chi2 = float(((counts - expect) ** 2 / expect).sum())
     assert chi2 < 31.26                                         # df = 11, p = 0.001
+
+
+@pytest.mark.parametrize("n,k", [(16, 2048), (17, 2052), (2400, 4100), (5, 260), (4750, 516)])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6, 8, 9, 200, 257])
+def test_gemm_fp32_rows_and_tiles_give_the_same_bits(m, n, k):
+    """Both kernels of the float32 product sum in the same order: a row is the same bits alone, in a few rows and in
+    many, with a last tile, run or stage that is not whole; one that is not on 16 bytes goes element by element."""
+    g = torch.Generator(device=DEV).manual_seed(m * 31 + n + k)
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    got = ops().linear(x, w)
+    want = x.double() @ w.double().t()
+    # sqrt(k) * 2^-24 of products near one, and as much for the largest of m * n
+    assert float((got - want).abs().max()) < 4e-6 * (k ** 0.5) * 4
+    assert torch.equal(ops().linear(x[-1:].contiguous(), w), got[-1:])
+    many = torch.cat([x, torch.zeros(1500, k, device=DEV)])
+    assert torch.equal(ops().linear(many, w)[:m], got)
+    off = torch.empty(n * k + 1, device=DEV)[1:].view(n, k).copy_(w)
+    assert torch.equal(ops().linear(x, off), got)
