@@ -744,3 +744,36 @@ def test_gemm_fp32_rows_and_tiles_give_the_same_bits(m, n, k):
     assert torch.equal(ops().linear(many, w)[:m], got)
     off = torch.empty(n * k + 1, device=DEV)[1:].view(n, k).copy_(w)
     assert torch.equal(ops().linear(x, off), got)
+
+
+@pytest.mark.parametrize("nq,nkv,d,dv,page,window,in_keys", [
+    (8, 2, 30, 30, 16, None, False), (12, 2, 64, 36, 16, 40, False), (4, 1, 640, 512, 16, None, True), (5, 1, 320, 320, 8, None, False),
+    (18, 2, 20, 22, 16, 300, False)])
+def test_attention_fp32_wide_and_element_by_element(nq, nkv, d, dv, page, window, in_keys):
+    """float32 attention where the tiles come in pieces of 16 bytes (two buffers, or one where two do not fit) and where
+    a head size is no multiple of four; more and fewer query heads a kv head than a block has warps."""
+    seqs, prefixes, news = [1, 31, 32, 33, 257], [0, 30, 5, 0, 200], [1, 2, 33, 65, 31]
+    g = torch.Generator(device=DEV).manual_seed(d + dv)
+    width = max(-(-s // page) for s in seqs + [p + n for p, n in zip(prefixes, news)])
+    row = nkv * (d if in_keys else d + dv)
+    cache = torch.randn(len(seqs) * width + 1, page * row, device=DEV, generator=g)
+    table = (torch.randperm(len(seqs) * width, device=DEV, generator=g) + 1).view(len(seqs), width).to(torch.int32)
+    opts = dict(dv=dv, values_in_keys=in_keys)
+    for decode in (True, False):
+        n = len(seqs) if decode else sum(news)
+        q = torch.randn(n, nq * d, device=DEV, generator=g)
+        got, want = torch.zeros(n, nq * dv, device=DEV), torch.zeros(n, nq * dv, device=DEV)
+        if decode:
+            seq_t = torch.tensor(seqs, device=DEV, dtype=torch.int32)
+            ref.attention_decode(q, cache, table, seq_t, want, None, 1, nq, nkv, d, page, d ** -0.5, window, **opts)
+            for splits in (1, 3):
+                scratch = torch.full((max(ops().decode_scratch_floats(n, nq, dv, splits), 1),), float("nan"), device=DEV)
+                ops().attention_decode(q, cache, table, seq_t, got.zero_(), scratch, splits, nq, nkv, d, page, d ** -0.5, window, **opts)
+                torch.testing.assert_close(got, want, **tol(torch.float32))
+        else:
+            cu = torch.tensor([0] + list(torch.tensor(news).cumsum(0)), device=DEV, dtype=torch.int32)
+            pre = torch.tensor(prefixes, device=DEV, dtype=torch.int32)
+            tiles = _tiles_of(news, ops().prefill_tile_rows(torch.float32, d))
+            ref.attention_prefill(q, cache, table, cu, pre, *tiles, want, nq, nkv, d, page, d ** -0.5, window, **opts)
+            ops().attention_prefill(q, cache, table, cu, pre, *tiles, got, nq, nkv, d, page, d ** -0.5, window, **opts)
+            torch.testing.assert_close(got, want, **tol(torch.float32))
