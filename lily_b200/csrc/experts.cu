@@ -20,6 +20,7 @@
 // Each output number of the products is summed over k in a fixed order, so a pair's result does not depend on what
 // else is in the batch.  Router, softmax and the weighted sum are float32.
 #include "common.cuh"
+#include "expert_act.cuh"
 #include "operand.cuh"
 
 namespace lily {
@@ -294,19 +295,6 @@ __global__ void moe_align_kernel(const int* __restrict__ chosen, int pairs, int 
 // the output is the activation in T.  MODE 1: A rows are the rows of `a` in grouped order, the output float32.  MODE 2: as
 // mode 0 for ungated experts, W = the up rows alone.
 constexpr int EBM = 32, EBN = 64, EBK = 16;
-
-// act 0: the clamped gate; 1: silu(g) u
-__device__ __forceinline__ float expert_gate(int act, float g, float u, float limit, float alpha) {
-    if (act == 1) return (g / (1.f + expf(-g))) * u;
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return (g / (1.f + expf(-alpha * g))) * (u + 1.f);
-}
-
-__device__ __forceinline__ float squared_relu(float z) {
-    const float r = fmaxf(z, 0.f);
-    return r * r;
-}
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)

@@ -85,6 +85,8 @@ _SIGNATURES = {
     "lily_moe_choose": [_vp, _i, _i, _sz, _i, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp],
     "lily_moe_align": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp],
     "lily_moe_gemm": [_i, _vp, _i, _vp, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _f, _f, _vp, _i, _vp],
+    "lily_moe_up_few": [_vp, _i, _i, _i, _vp, _i, _vp, _i, _i, _vp, _i, _f, _f, _vp, _vp],
+    "lily_moe_down_few": [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _vp, _i, _vp, _i, _i, _sz, _vp, _vp, _vp],
     "lily_moe_combine": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _sz, _vp, _vp, _i, _vp],
     "lily_moe_gather": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp],
     "lily_moe_activation": [_vp, _i, _i, _vp, _i, _f, _f, _vp, _vp, _i, _vp, _vp],
@@ -143,6 +145,8 @@ def library():
         lib.lily_latent_attention_tc_col_blocks.argtypes = [_i]
         lib.lily_latent_attention_tc_col_blocks.restype = _i
         lib.lily_moe_tile_rows.restype = _i
+        lib.lily_moe_few_takes.argtypes = [_i, _i, _i, _i, _i]
+        lib.lily_moe_few_takes.restype = _i
         lib.lily_delta_rule_max_head_dim.restype = _i
         lib.lily_selective_scan_max_state.restype = _i
         lib.lily_mlstm_max_head_dim.restype = _i
@@ -1508,12 +1512,21 @@ def head_gate(ov: torch.Tensor, gate_rows: torch.Tensor, g0: int, out_dtype: tor
 
 @dataclass
 class ExpertRouting:
-    """A step's routing for one layer, all on the device: ``chosen`` / ``weights`` [tokens, top]; the pairs (token, choice)
-    of experts that have weights grouped by expert (``offsets``, ``order``, ``place``) and the tiles the grouped
-    products run over."""
+    """A step's routing for one layer, all on the device: ``chosen`` / ``weights`` [tokens, top]."""
 
     chosen: torch.Tensor
     weights: torch.Tensor
+    experts: int                             # router outputs that have weights
+    top: int
+    gate: Optional[torch.Tensor] = None      # float32 [tokens]: the shared expert's gate
+    grouped: Optional["ExpertGroups"] = None # made by the first product that asks for it (``expert_groups``)
+
+
+@dataclass
+class ExpertGroups:
+    """The pairs (token, choice) of experts that have weights grouped by expert (``offsets``, ``order``, ``place``) and the
+    tiles the grouped products run over."""
+
     offsets: torch.Tensor
     order: torch.Tensor
     place: torch.Tensor
@@ -1521,8 +1534,6 @@ class ExpertRouting:
     tile_row: torch.Tensor
     tile_count: torch.Tensor
     max_tiles: int
-    top: int
-    gate: Optional[torch.Tensor] = None      # float32 [tokens]: the shared expert's gate
 
 
 def moe_route(h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.Tensor], top: int, experts: int,
@@ -1548,12 +1559,7 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.
     if scores not in ("softmax", "sigmoid"):
         raise KernelError(f"moe_route: no scores {scores!r} (have softmax, sigmoid)")
     dev = h.device
-    pairs = tokens * top
-    tile_rows = int(library().lily_moe_tile_rows())
-    max_tiles = -(-pairs // tile_rows) + experts
-    ints = torch.empty(3 * pairs + experts + 1 + 2 * max_tiles + 1, dtype=torch.int32, device=dev)
-    chosen, order, place, offsets, tile_expert, tile_row, tile_count = torch.split(
-        ints, [pairs, pairs, pairs, experts + 1, max_tiles, max_tiles, 1])
+    chosen = torch.empty((tokens, top), dtype=torch.int32, device=dev)
     weights = torch.empty((tokens, top), dtype=torch.float32, device=dev)
     gate = torch.empty((tokens,), dtype=torch.float32, device=dev) if shared_gate else None
     how = (outputs, top, int(scores == "sigmoid"), int(renormalise), int(groups), int(keep_groups), _p(chosen), _p(weights), _p(gate))
@@ -1564,10 +1570,21 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.
         _call("lily_moe_choose", *_operand(z, tokens, router.shape[0], "moe_route"), router.shape[0], tokens, _p(correction), *how, _stream())
     else:
         _call("lily_moe_route", _p(h), tokens, width, _p(router), _p(correction), *how, _dt(h), _stream())
-    _call("lily_moe_align", _p(chosen), pairs, experts, _p(offsets), _p(order), _p(place), _p(tile_expert), _p(tile_row),
-          _p(tile_count), max_tiles, _stream())
-    return ExpertRouting(chosen.view(tokens, top), weights, offsets, order, place, tile_expert, tile_row, tile_count,
-                         max_tiles, top, gate)
+    return ExpertRouting(chosen, weights, experts, top, gate)
+
+
+def expert_groups(r: ExpertRouting) -> ExpertGroups:
+    """The routing's pairs grouped by expert, by a kernel of one block at the first call."""
+    if r.grouped is None:
+        pairs, experts = r.chosen.numel(), r.experts
+        max_tiles = -(-pairs // int(library().lily_moe_tile_rows())) + experts
+        ints = torch.empty(2 * pairs + experts + 1 + 2 * max_tiles + 1, dtype=torch.int32, device=r.chosen.device)
+        order, place, offsets, tile_expert, tile_row, tile_count = torch.split(
+            ints, [pairs, pairs, experts + 1, max_tiles, max_tiles, 1])
+        _call("lily_moe_align", _p(r.chosen), pairs, experts, _p(offsets), _p(order), _p(place), _p(tile_expert), _p(tile_row),
+              _p(tile_count), max_tiles, _stream())
+        r.grouped = ExpertGroups(offsets, order, place, tile_expert, tile_row, tile_count, max_tiles)
+    return r.grouped
 
 
 _OWN_GROUPED = os.environ.get("LILY_B200_GROUPED_GEMM", "") == "own"
@@ -1578,6 +1595,18 @@ def grouped_library_takes(dtype: torch.dtype, width: int, ff: int) -> bool:
     units); everything else, and float32 always, runs on this package's grouped kernel."""
     return (dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and hasattr(torch, "_grouped_mm")
             and not _OWN_GROUPED)
+
+
+_FEW_TOKENS = os.environ.get("LILY_B200_EXPERTS_FEW", "1") != "0"
+
+
+def few_tokens_take(r: "ExpertRouting", h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, gated: bool) -> bool:
+    """Whether the step's few tokens go through the two kernels that stream the chosen experts' weights."""
+    experts, width, ff = w_down.shape
+    return (_FEW_TOKENS and h.dtype == w_gate_up.dtype == w_down.dtype == torch.bfloat16 and experts == r.experts
+            and tuple(w_gate_up.shape) == (experts, 2 * ff if gated else ff, width) and w_down.shape[1] == h.shape[1]
+            and bool(library().lily_moe_few_takes(h.shape[0], r.top, experts, width, ff))
+            and (w_gate_up.data_ptr() | w_down.data_ptr() | h.data_ptr()) % 16 == 0)
 
 
 EXPERT_ACTIVATIONS = {"swish_clamped": 0, "silu": 1, "relu2": 2}      # "relu2": ungated
@@ -1605,18 +1634,28 @@ def moe_experts(h: torch.Tensor, routing: ExpertRouting, w_gate_up: torch.Tensor
     experts = w_down.shape[0] if w_down.dim() == 3 else 0
     ff = w_down.shape[2] if experts else 0
     act_code, in_weight = EXPERT_ACTIVATIONS[activation], _p(r.weights) if weight_on_input else None
+    sh = (None, _F32, 1, 0) if shared is None else _operand(shared, tokens, width, "moe_experts shared")
+    out = torch.empty((tokens, width), dtype=torch.float32, device=h.device)
+    if experts and few_tokens_take(r, h, w_gate_up, w_down, gated):
+        act = torch.empty((pairs, ff), dtype=h.dtype, device=h.device)
+        _call("lily_moe_up_few", _p(h), width, tokens, width, _p(w_gate_up), ff, _p(r.chosen), r.top, experts, in_weight, act_code,
+              float(limit), float(alpha), _p(act), _stream())
+        _call("lily_moe_down_few", _p(act), ff, _p(w_down), width, _p(r.chosen), None if weight_on_input else _p(r.weights), tokens,
+              r.top, experts, _p(h), width, *sh, _p(r.gate), _p(out), _stream())
+        return out
+    grouped = expert_groups(r)
     if experts and grouped_library_takes(h.dtype, width, ff):
         # bfloat16: the library's grouped product over the rows in grouped order (groups end at offsets[1:])
-        ends = r.offsets[1:]
+        ends = grouped.offsets[1:]
         rows = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
-        _call("lily_moe_gather", _p(h), width, _p(r.offsets), experts, _p(r.order), r.top, pairs, _p(rows), _stream())
+        _call("lily_moe_gather", _p(h), width, _p(grouped.offsets), experts, _p(grouped.order), r.top, pairs, _p(rows), _stream())
         gate_up = torch._grouped_mm(rows, w_gate_up.transpose(1, 2), offs=ends)
         act = torch.empty((pairs, ff), dtype=h.dtype, device=h.device)
         if not gated:
-            _call("lily_moe_relu2", _p(gate_up), ff, pairs, _p(act), in_weight, _p(r.offsets), experts, _p(r.order), _stream())
+            _call("lily_moe_relu2", _p(gate_up), ff, pairs, _p(act), in_weight, _p(grouped.offsets), experts, _p(grouped.order), _stream())
         else:
             _call("lily_moe_activation", _p(gate_up), ff, pairs, _p(act), act_code, float(limit), float(alpha), in_weight,
-                  _p(r.offsets), experts, _p(r.order), _stream())
+                  _p(grouped.offsets), experts, _p(grouped.order), _stream())
         y = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)
     else:
         y = torch.empty((max(pairs, 1), width), dtype=torch.float32, device=h.device)
@@ -1624,14 +1663,12 @@ def moe_experts(h: torch.Tensor, routing: ExpertRouting, w_gate_up: torch.Tensor
             if w_gate_up.dtype != h.dtype or w_down.dtype != h.dtype or tuple(w_gate_up.shape) != (experts, 2 * ff if gated else ff, width):
                 raise KernelError(f"moe_experts: weights {tuple(w_gate_up.shape)} / {tuple(w_down.shape)} {w_down.dtype} for inputs {tuple(h.shape)} {h.dtype}")
             act = torch.empty((max(pairs, 1), ff), dtype=h.dtype, device=h.device)
-            _call("lily_moe_gemm", 0 if gated else 2, _p(h), h.stride(0), _p(w_gate_up), ff, width, _p(r.offsets), _p(r.order), r.top,
-                  _p(r.tile_expert), _p(r.tile_row), _p(r.tile_count), r.max_tiles, _p(act), act_code, float(limit), float(alpha),
+            _call("lily_moe_gemm", 0 if gated else 2, _p(h), h.stride(0), _p(w_gate_up), ff, width, _p(grouped.offsets), _p(grouped.order), r.top,
+                  _p(grouped.tile_expert), _p(grouped.tile_row), _p(grouped.tile_count), grouped.max_tiles, _p(act), act_code, float(limit), float(alpha),
                   in_weight, _dt(h), _stream())
-            _call("lily_moe_gemm", 1, _p(act), ff, _p(w_down), width, ff, _p(r.offsets), _p(r.order), r.top, _p(r.tile_expert),
-                  _p(r.tile_row), _p(r.tile_count), r.max_tiles, _p(y), 0, 0.0, 0.0, None, _dt(h), _stream())
-    sh = (None, _F32, 1, 0) if shared is None else _operand(shared, tokens, width, "moe_experts shared")
-    out = torch.empty((tokens, width), dtype=torch.float32, device=h.device)
-    _call("lily_moe_combine", _p(y), _dt(y), _p(h), _p(r.place), None if weight_on_input else _p(r.weights), tokens, r.top, width,
+            _call("lily_moe_gemm", 1, _p(act), ff, _p(w_down), width, ff, _p(grouped.offsets), _p(grouped.order), r.top, _p(grouped.tile_expert),
+                  _p(grouped.tile_row), _p(grouped.tile_count), grouped.max_tiles, _p(y), 0, 0.0, 0.0, None, _dt(h), _stream())
+    _call("lily_moe_combine", _p(y), _dt(y), _p(h), _p(grouped.place), None if weight_on_input else _p(r.weights), tokens, r.top, width,
           *sh, _p(r.gate), _p(out), _dt(h), _stream())
     return out
 

@@ -777,3 +777,36 @@ def test_attention_fp32_wide_and_element_by_element(nq, nkv, d, dv, page, window
             ref.attention_prefill(q, cache, table, cu, pre, *tiles, want, nq, nkv, d, page, d ** -0.5, window, **opts)
             ops().attention_prefill(q, cache, table, cu, pre, *tiles, got, nq, nkv, d, page, d ** -0.5, window, **opts)
             torch.testing.assert_close(got, want, **tol(torch.float32))
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("width,ff,experts,identity,top,activation,on_input,shared", [
+    (64, 64, 3, 0, 2, "silu", False, False), (192, 320, 16, 2, 4, "swish_clamped", False, False),
+    (2048, 2048, 16, 0, 3, "relu2", False, True), (128, 192, 40, 0, 8, "silu", True, True), (256, 64, 2, 6, 7, "swish_clamped", False, True),
+    (64, 128, 256, 0, 8, "relu2", True, False)])
+def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, activation, on_input, shared):
+    """The kernels that stream the chosen experts' weights (up to 16 tokens and 128 pairs; beyond, the grouped products): odd
+    numbers of tokens, experts nobody chose, steps of identity choices alone, fewer tiles of k than warps."""
+    g = torch.Generator(device=DEV).manual_seed(tokens * 7 + width)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    bf = torch.bfloat16
+    h = rand(tokens, width).to(bf)
+    router = rand(experts + identity + (1 if shared else 0), width) * 0.5
+    gu = (rand(experts, (1 if activation == "relu2" else 2) * ff, width) / width ** 0.5).to(bf)
+    dn = (rand(experts, width, ff) / ff ** 0.5).to(bf)
+    sh = rand(2, tokens, width) if shared else None
+    r = ops().moe_route(h, router, None, top, experts, shared_gate=shared, outputs=experts + identity)
+    got = ops().moe_experts(h, r, gu, dn, 7.0, 1.702, activation=activation, weight_on_input=on_input, shared=sh)
+    plain = ref.ExpertRouting(r.chosen, r.weights, top, r.gate)
+    want = ref.moe_experts(h, plain, gu, dn, 7.0, 1.702, activation=activation, weight_on_input=on_input, shared=sh)
+    # the activations are rounded to 8 bits once here, 2^-9 of each of ff terms; the grouped products round their outputs too
+    scale = float(want.abs().max())
+    assert float((got - want).abs().max()) < 1.6e-2 * scale
+    # a token's sum does not depend on its neighbours, bit for bit, while both take the same kernels
+    if tokens * top <= 128 and tokens <= 16:
+        keep = slice(tokens - 1, tokens)
+        alone = ops().moe_route(h[keep], router, None, top, experts, shared_gate=shared, outputs=experts + identity)
+        assert torch.equal(alone.chosen, r.chosen[keep])
+        one = ops().moe_experts(h[keep].contiguous(), alone, gu, dn, 7.0, 1.702, activation=activation, weight_on_input=on_input,
+                                shared=sh[:, keep].contiguous() if shared else None)
+        assert torch.equal(one, got[keep])
