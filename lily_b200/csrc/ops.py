@@ -64,6 +64,8 @@ _SIGNATURES = {
     "lily_diff_combine": [_vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _f, _f, _i, _vp],
     "lily_ssd_scan": [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp,
                       _i, _vp, _vp, _i, _vp],
+    "lily_ssd_step": [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "lily_wkv_step": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "lily_ssd_combine": [_vp, _sz, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "lily_gated_group_rmsnorm": [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _f, _i, _vp],
     "lily_latent_attention_prefill_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
@@ -145,6 +147,10 @@ def library():
         lib.lily_latent_attention_tc_col_blocks.argtypes = [_i]
         lib.lily_latent_attention_tc_col_blocks.restype = _i
         lib.lily_moe_tile_rows.restype = _i
+        lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
+        lib.lily_ssd_step_takes.restype = _i
+        lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
+        lib.lily_wkv_step_takes.restype = _i
         lib.lily_moe_few_takes.argtypes = [_i, _i, _i, _i, _i]
         lib.lily_moe_few_takes.restype = _i
         lib.lily_delta_rule_max_head_dim.restype = _i
@@ -1236,6 +1242,10 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
     common = (_p(xbc), channels, _p(proj), proj.shape[1], int(dt_col), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
               state.shape[1], _p(y), _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
     sizes = (heads, head_dim, n_state, groups, _dt(xbc))
+    if n == requests and library().lily_ssd_step_takes(_p(state), state.shape[1], n_state):
+        # one token a request (a decode step): a kernel that moves the state and stages nothing
+        _call("lily_ssd_step", *common, int(requests), *sizes, _stream())
+        return y
     if plan is None or plan.direct is None:
         _call("lily_ssd_scan", *common, int(requests), *sizes, None, None, None, 0, None, None, 0, _stream())
         return y
@@ -1421,6 +1431,10 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
     y = torch.empty((tokens, heads * d), dtype=torch.float32, device=r.device)
     common = (_p(r), _p(k), _p(v), stride, _p(log_decay), _p(u), _p(state), state.stride(0), _p(y),
               _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
+    if tokens == requests and library().lily_wkv_step_takes(_p(state), state.stride(0), _p(v), stride, d, _dt(r)):
+        # one token a request (a decode step): a kernel that moves the matrices and stages nothing
+        _call("lily_wkv_step", *common, requests, heads, d, _dt(r), _stream())
+        return y
     if plan is None:
         _call("lily_wkv_scan", *common, requests, heads, d, _dt(r), 0, None, None, None, None, None, _stream())
         return y

@@ -810,3 +810,51 @@ def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, acti
         one = ops().moe_experts(h[keep].contiguous(), alone, gu, dn, 7.0, 1.702, activation=activation, weight_on_input=on_input,
                                 shared=sh[:, keep].contiguous() if shared else None)
         assert torch.equal(one, got[keep])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("requests,heads,groups,pd,n_state", [
+    (1, 2, 1, 64, 128), (9, 64, 8, 64, 128), (3, 6, 3, 24, 64), (2, 4, 2, 7, 20), (5, 8, 1, 33, 256), (2, 2, 2, 16, 300), (300, 2, 1, 80, 512),
+    (4, 3, 1, 5, 17)])
+def test_ssd_scan_of_one_token_a_request(dtype, requests, heads, groups, pd, n_state):
+    """A decode step's scan: rows of a head that no warp fills, states of one to four pieces a lane, many and few requests; a state
+    that is no multiple of four takes the general kernel."""
+    g = torch.Generator(device=DEV).manual_seed(requests + pd)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    inner = heads * pd
+    xbc, proj = rand(requests, inner + 2 * groups * n_state).to(dtype), rand(requests, 5 + heads).to(dtype)
+    vec = [rand(heads) for _ in range(3)]
+    state = rand(requests + 2, inner * n_state + 4 * (requests % 2))
+    cu = torch.arange(requests + 1, device=DEV, dtype=torch.int32)
+    slots = (torch.randperm(requests + 1, device=DEV, generator=g) + 1)[:requests].to(torch.int32)
+    mine, theirs = state.clone(), state.clone()
+    got = ops().ssd_scan(xbc, proj, 5, *vec, mine, cu, slots, requests, heads, pd, n_state, groups)
+    want = ref.ssd_scan(xbc, proj, 5, *vec, theirs, cu, slots, requests, heads, pd, n_state, groups)
+    # float32 throughout: n_state products a sum, 2^-24 each
+    torch.testing.assert_close(got, want, rtol=2e-5, atol=2e-5 * n_state ** 0.5)
+    torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("requests,heads,d", [(1, 32, 64), (7, 3, 32), (40, 2, 128), (2, 5, 256), (3, 4, 48)])
+def test_wkv_scan_of_one_token_a_request(dtype, requests, heads, d):
+    g = torch.Generator(device=DEV).manual_seed(requests + d)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    r, k, v = (rand(requests, heads * d).to(dtype) for _ in range(3))
+    lw, u = -torch.exp(rand(requests, heads * d)), rand(heads, d)
+    state = rand(requests + 2, heads * d * d + 8)
+    cu = torch.arange(requests + 1, device=DEV, dtype=torch.int32)
+    slots = (torch.randperm(requests + 1, device=DEV, generator=g) + 1)[:requests].to(torch.int32)
+    mine, theirs = state.clone(), state.clone()
+    got = ops().wkv_scan(r, k, v, lw, u, mine, cu, slots, requests, heads, d)
+    want = ref.wkv_scan(r, k, v, lw, u, theirs, cu, slots, requests, heads, d)
+    torch.testing.assert_close(got, want, rtol=2e-5, atol=2e-5 * d ** 0.5)
+    torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("tokens,rank,cols", [(1, 1, 5), (2, 64, 2048), (8, 31, 130), (9, 33, 257), (21, 200, 128)])
+def test_wkv_decay_by_rows_asked_for_ahead(tokens, rank, cols):
+    g = torch.Generator(device=DEV).manual_seed(rank)
+    a, w2t, w0 = (torch.randn(*s, device=DEV, generator=g) for s in ((tokens, rank), (rank, cols), (cols,)))
+    w2t = w2t / rank ** 0.5
+    torch.testing.assert_close(ops().wkv_decay(a, w2t, w0), ref.wkv_decay(a, w2t, w0), rtol=1e-5, atol=1e-6)
