@@ -1,0 +1,158 @@
+// Matrix product for up to 16 tokens whose result is wanted whole: out[m][n] = sum_k x[m][k] w[n][k] (+ bias[n]), bfloat16 in,
+// float32 sums, bfloat16 or float32 out.  (gemm_skinny.cu leaves float32 partial sums to a consumer that adds them up; this
+// kernel serves the ones that want finished rows: projections with a convolution, a recurrence or a table behind them.)
+//
+// Bound by reading w once.  A block of eight warps takes tiles of 16 weight rows, each warp an eighth of k: tiles of [16 rows][64 k]
+// by cp.async in a ring of the warp's own, the tokens' [8 or 16][64 k] beside them, ldmatrix and mma.sync m16n8k16 (weight rows on
+// the 16-row side, tokens on the 8-column side); the eighths meet in shared memory.  Two blocks a SM walk the tiles as one pipeline
+// each, up to 96 KB in flight a SM, and the first stages of w, which depends on no one, are asked for before the kernel ahead has
+// finished: a 2,048 x 2,048 product has all of its weights on the way by then.
+// A token's sums run in the same order whatever else is in the step.
+//
+// Against the library's product in a chain of norms and products, us (w at the copy rate): N x K 64 x 2,048 5.1 -> 2.0; 2,048 x
+// 2,048 7.9 -> 3.2 (1.3) with 5 tokens, 6.4 -> 3.8 with 16; 2,048 x 4,096 12 -> 4.5 (2.6); 10,304 x 2,048 9.8 -> 7.9 (6.5) with 8, 11.3 ->
+// 9.1 with 16; 24,576 x 4,096 35.3 -> 31.5 (31.2), 35.8 -> 34.2 with 16; 32,000 x 4,096 46 -> 39 (41), 47 -> 41.
+#include "common.cuh"
+#include "mma.cuh"
+
+namespace lily {
+namespace fewrows {
+
+using mma16::cp_async_commit;
+using mma16::cp_async_wait;
+using mma16::ldmatrix_x4;
+using mma16::mma_bf16;
+using mma16::smem_u32;
+
+constexpr int KT = 64, PITCH = KT * 2, WARPS = 8, ROWS = 16;
+__host__ __device__ constexpr int stages(int nt) { return nt == 1 ? 4 : 3; }
+__host__ __device__ constexpr int stage_bytes(int nt) { return (ROWS + nt * 8) * PITCH; }
+__host__ __device__ constexpr int part_floats(int nt) { return WARPS * nt * 8 * ROWS; }
+__host__ __device__ constexpr int smem_bytes(int nt) { return WARPS * stages(nt) * stage_bytes(nt) + part_floats(nt) * (int)sizeof(float); }
+static_assert(smem_bytes(1) <= 113 * 1024 && smem_bytes(2) <= 113 * 1024, "two blocks a SM");
+
+template <int NT>
+__global__ void __launch_bounds__(WARPS * 32)
+gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const void* __restrict__ bias, int bias_f32,
+                void* __restrict__ out, int out_f32, int M, int N, int K) {
+    constexpr int STAGES = stages(NT), STAGE = stage_bytes(NT);
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
+    const uint32_t ring = smem_u32(smem + warp * STAGES * STAGE);
+    float* part = reinterpret_cast<float*>(smem + WARPS * STAGES * STAGE);      // [warp][NT * 8][16 rows]
+    const int kblocks = K / KT, per = (kblocks + WARPS - 1) / WARPS, kb0 = warp * per, nkb = max(0, min(per, kblocks - kb0));
+    const int tiles = (N + ROWS - 1) / ROWS, mine = (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1, steps = mine * nkb;
+
+    // a copy of the warp covers four rows of 128 bytes; rows beyond N repeat the last one
+    const int r4 = lane >> 3, piece = lane & 7;
+    int w_tile = blockIdx.x, w_kb = 0, x_kb = 0;
+    auto issue_w = [&](int step) {
+        const uint32_t base = ring + (step % STAGES) * STAGE;
+        const __nv_bfloat16* src = w + (size_t)(kb0 + w_kb) * KT + piece * 8;
+#pragma unroll
+        for (int i = 0; i < ROWS / 4; ++i) {
+            const int r = i * 4 + r4;
+            asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;\n" ::"r"(base + r * PITCH + (((piece ^ r) & 7) << 4)),
+                         "l"(src + (size_t)min(w_tile * ROWS + r, N - 1) * K) : "memory");
+        }
+        if (++w_kb == nkb) w_kb = 0, w_tile += gridDim.x;
+    };
+    auto issue_x = [&](int step) {
+        const uint32_t base = ring + (step % STAGES) * STAGE + ROWS * PITCH;
+#pragma unroll
+        for (int i = 0; i < NT * 2; ++i) {
+            const int r = i * 4 + r4;
+            mma16::cp_async16(base + r * PITCH + (((piece ^ r) & 7) << 4), x + (size_t)min(r, M - 1) * K + (size_t)(kb0 + x_kb) * KT + piece * 8, r < M);
+        }
+        if (++x_kb == nkb) x_kb = 0;
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < steps) issue_w(s);
+    pdl_wait();
+    pdl_launch_dependents();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < steps) issue_x(s);
+        cp_async_commit();
+    }
+
+    int step = 0;
+    for (int it = 0; it < mine; ++it) {
+        float acc[NT][4] = {};
+        for (int kb = 0; kb < nkb; ++kb, ++step) {
+            cp_async_wait<STAGES - 2>();
+            __syncwarp();
+            if (step + STAGES - 1 < steps) {
+                issue_w(step + STAGES - 1);
+                issue_x(step + STAGES - 1);
+            }
+            cp_async_commit();
+            const uint32_t stage = ring + (step % STAGES) * STAGE;
+            uint32_t xf[NT][8];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {                // a read brings the tokens' numbers of two steps of 16 k
+                    const int r = lane & 7, ch = q * 4 + (lane >> 3);
+                    ldmatrix_x4(stage + (ROWS + nt * 8 + r) * PITCH + (((ch ^ r) & 7) << 4), xf[nt][4 * q], xf[nt][4 * q + 1], xf[nt][4 * q + 2],
+                                xf[nt][4 * q + 3]);
+                }
+#pragma unroll
+            for (int kk = 0; kk < KT / 16; ++kk) {
+                uint32_t a[4];
+                const int r = lane & 15, ch = kk * 2 + (lane >> 4);
+                ldmatrix_x4(stage + r * PITCH + (((ch ^ r) & 7) << 4), a[0], a[1], a[2], a[3]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[nt], a, xf[nt][2 * kk], xf[nt][2 * kk + 1]);
+            }
+        }
+        if (it > 0) __syncthreads();                         // the tile before has been added up
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[(warp * NT * 8 + nt * 8 + 2 * c + (j & 1)) * ROWS + g + (j >> 1) * 8] = acc[nt][j];
+        __syncthreads();
+        const int n0 = (blockIdx.x + it * gridDim.x) * ROWS;
+        for (int i = tid; i < M * ROWS; i += WARPS * 32) {
+            const int m = i / ROWS, n = n0 + i % ROWS;
+            if (n >= N) continue;
+            float v = 0.f;
+#pragma unroll
+            for (int q = 0; q < WARPS; ++q) v += part[q * NT * 8 * ROWS + i];
+            if (bias) v += bias_f32 ? ((const float*)bias)[n] : __bfloat162float(((const __nv_bfloat16*)bias)[n]);
+            if (out_f32) ((float*)out)[(size_t)m * N + n] = v;
+            else ((__nv_bfloat16*)out)[(size_t)m * N + n] = __float2bfloat16_rn(v);
+        }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+}  // namespace fewrows
+}  // namespace lily
+
+using namespace lily;
+
+// Whether the kernel takes the product; up to 16 tokens it is ahead of the library's at every size measured (above).
+LILY_API int lily_gemm_few_takes(int M, int N, int K) {
+    return M >= 1 && M <= 16 && N >= 1 && K >= fewrows::KT && K % fewrows::KT == 0;
+}
+
+LILY_API int lily_gemm_few(const void* x, const void* w, const void* bias, int bias_f32, void* out, int out_f32, int M, int N, int K,
+                           cudaStream_t stream) {
+    LILY_REQUIRE(lily_gemm_few_takes(M, N, K), "gemm_few: M=%d N=%d K=%d", M, N, K);
+    LILY_REQUIRE((((uintptr_t)x | (uintptr_t)w) & 15) == 0, "gemm_few: operands do not start on 16 bytes");
+    const int tiles = (N + fewrows::ROWS - 1) / fewrows::ROWS, grid = min(tiles, 2 * sm_count());
+#define GO(NT)                                                                                                              \
+    do {                                                                                                                    \
+        auto kern = fewrows::gemm_few_kernel<NT>;                                                                           \
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fewrows::smem_bytes(NT));   \
+        LILY_REQUIRE(e == cudaSuccess, "gemm_few: %s", cudaGetErrorString(e));                                              \
+        launch_pdl(kern, dim3(grid), dim3(fewrows::WARPS * 32), fewrows::smem_bytes(NT), stream, (const __nv_bfloat16*)x,   \
+                   (const __nv_bfloat16*)w, bias, bias_f32, out, out_f32, M, N, K);                                         \
+    } while (0)
+    if (M <= 8) GO(1); else GO(2);
+#undef GO
+    LILY_CHECK_LAUNCH("gemm_few");
+    return 0;
+}

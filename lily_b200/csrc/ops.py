@@ -34,6 +34,7 @@ _SIGNATURES = {
     "lily_skinny_gemm": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "lily_skinny_swiglu": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lily_cast": [_vp, _i, _vp, _i, _sz, _vp],
+    "lily_gemm_few": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
     "lily_gemm_fp32": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_attention_prefill_simt": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp, _vp],
     "lily_attention_decode_simt": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp, _vp],
@@ -147,6 +148,8 @@ def library():
         lib.lily_latent_attention_tc_col_blocks.argtypes = [_i]
         lib.lily_latent_attention_tc_col_blocks.restype = _i
         lib.lily_moe_tile_rows.restype = _i
+        lib.lily_gemm_few_takes.argtypes = [_i, _i, _i]
+        lib.lily_gemm_few_takes.restype = _i
         lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
         lib.lily_ssd_step_takes.restype = _i
         lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
@@ -414,8 +417,8 @@ def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x [M, K] . weight [N, K]^T (+ bias)``.  float32: this package's FFMA kernel.
-    bfloat16: cuBLAS with float32 accumulation; ``out_dtype=float32`` keeps the accumulator's
-    precision (used for the logits)."""
+    bfloat16: up to 16 rows this package's kernel that streams the weights (``few_rows_take``), else cuBLAS, both with
+    float32 accumulation; ``out_dtype=float32`` keeps the accumulator's precision (used for the logits)."""
     _dev(x, weight, bias)
     m, k = x.shape
     n = weight.shape[0]
@@ -427,6 +430,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             raise KernelError("float32 linear takes a float32 bias")
         _call("lily_gemm_fp32", _p(x), _p(weight), _p(bias), _p(out), m, n, k, k, n, _stream())
         return out
+    if few_rows_take(x, weight) and out_dtype in (None, torch.bfloat16, torch.float32) and (bias is None or bias.numel() == n):
+        out = torch.empty((m, n), dtype=out_dtype or x.dtype, device=x.device)
+        _call("lily_gemm_few", _p(x), _p(weight), _p(bias), int(bias is not None and bias.dtype == torch.float32), _p(out),
+              int(out.dtype == torch.float32), m, n, k, _stream())
+        return out
     if _OWN_PLAIN_GEMM and out_dtype is None and m >= TC_MIN_ROWS and gemm_tc_takes(x, weight):
         return gemm_tc(x, weight, bias.to(x.dtype) if bias is not None else None)
     if out_dtype == torch.float32:
@@ -437,6 +445,16 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if bias is not None:
         return torch.addmm(bias.to(x.dtype), x, weight.t())
     return torch.mm(x, weight.t())
+
+
+_FEW_ROWS = os.environ.get("LILY_B200_GEMM_FEW", "1") != "0"
+
+
+def few_rows_take(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether a product of a few tokens goes to the kernel that streams the weights and finishes its rows."""
+    m, k = x.shape
+    return (_FEW_ROWS and m <= 16 and x.dtype == weight.dtype == torch.bfloat16 and bool(library().lily_gemm_few_takes(m, weight.shape[0], k))
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
 TC_MIN_ROWS = 65          # products of more rows than this go to the tcgen05 kernel when it takes the shape

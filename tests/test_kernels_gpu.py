@@ -858,3 +858,22 @@ def test_wkv_decay_by_rows_asked_for_ahead(tokens, rank, cols):
     a, w2t, w0 = (torch.randn(*s, device=DEV, generator=g) for s in ((tokens, rank), (rank, cols), (cols,)))
     w2t = w2t / rank ** 0.5
     torch.testing.assert_close(ops().wkv_decay(a, w2t, w0), ref.wkv_decay(a, w2t, w0), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("n,k", [(1, 64), (15, 128), (64, 448), (331, 512), (2048, 2048), (5000, 576), (10304, 192)])
+@pytest.mark.parametrize("m", [1, 3, 8, 9, 16])
+def test_linear_of_a_few_rows(m, n, k):
+    """bfloat16 products of up to 16 rows: tiles of rows and eighths of k that are not whole, fewer tiles of k than warps, several
+    tiles a block; with and without a bias, both result types."""
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    x, w = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((m, k), (n, k)))
+    b = torch.randn(n, device=DEV, generator=g)
+    want = x.double() @ w.double().t()
+    got = ops().linear(x, w, out_dtype=torch.float32)
+    # float32 sums of exact products: 2^-24 of sqrt(k) terms near one, and the largest of m * n
+    assert float((got - want).abs().max()) < 4e-6 * (k ** 0.5) * 4
+    assert float((ops().linear(x, w, b, out_dtype=torch.float32) - (want + b)).abs().max()) < 4e-6 * (k ** 0.5) * 4
+    assert torch.equal(ops().linear(x, w), got.bfloat16())
+    low = ops().linear(x, w, b.bfloat16())
+    assert float((low - (want + b.bfloat16())).abs().max()) < 2 ** -8 * float(want.abs().max() + 4)
+    assert torch.equal(ops().linear(x[-1:].contiguous(), w), ops().linear(x, w)[-1:])
