@@ -7,13 +7,18 @@
 // the 16-row side, tokens on the 8-column side); the eighths meet in shared memory.  Two blocks a SM walk the tiles as one pipeline
 // each, up to 96 KB in flight a SM, and the first stages of w, which depends on no one, are asked for before the kernel ahead has
 // finished: a 2,048 x 2,048 product has all of its weights on the way by then.
-// A token's sums run in the same order whatever else is in the step.
+// A token's sums run in the same order whatever else is in the step.  With the gate/up product's activation (GATED) the tile's two
+// halves are the gate and the up rows of 8 outputs.
 //
 // Against the library's product in a chain of norms and products, us (w at the copy rate): N x K 64 x 2,048 5.1 -> 2.0; 2,048 x
 // 2,048 7.9 -> 3.2 (1.3) with 5 tokens, 6.4 -> 3.8 with 16; 2,048 x 4,096 12 -> 4.5 (2.6); 10,304 x 2,048 9.8 -> 7.9 (6.5) with 8, 11.3 ->
-// 9.1 with 16; 24,576 x 4,096 35.3 -> 31.5 (31.2), 35.8 -> 34.2 with 16; 32,000 x 4,096 46 -> 39 (41), 47 -> 41.
+// 9.1 with 16; 24,576 x 4,096 35.3 -> 31.5 (31.2), 35.8 -> 34.2 with 16; 32,000 x 4,096 46 -> 39 (41), 47 -> 41.  Gate/up with SiLU, against
+// stretches of (128 outputs, 64 k) dealt out evenly and finished through scratch by the block that comes last: 8,192 x 2,048 14.6 ->
+// 11.5 (10.4), 12,288 x 4,096 36.9 -> 30.7 (31.2), 25,600 x 5,120 85 -> 75 (81), 28,672 x 8,192 155 -> 139 (146).
 #include "common.cuh"
 #include "mma.cuh"
+
+#include <cstdlib>
 
 namespace lily {
 namespace fewrows {
@@ -31,10 +36,17 @@ __host__ __device__ constexpr int part_floats(int nt) { return WARPS * nt * 8 * 
 __host__ __device__ constexpr int smem_bytes(int nt) { return WARPS * stages(nt) * stage_bytes(nt) + part_floats(nt) * (int)sizeof(float); }
 static_assert(smem_bytes(1) <= 113 * 1024 && smem_bytes(2) <= 113 * 1024, "two blocks a SM");
 
-template <int NT>
+// The gate/up product with its activation (GATED): w holds runs of `run` gate rows and the `run` up rows of the same outputs, a tile is
+// the 8 gate rows and the 8 up rows of 8 outputs, and the sums meet in the activation instead of in `out`'s row.
+struct Gate {
+    int run, act;                  // act 0: SiLU, 1: GELU in its tanh form, 2: clamped
+    float limit, alpha;
+};
+
+template <int NT, bool GATED>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const void* __restrict__ bias, int bias_f32,
-                void* __restrict__ out, int out_f32, int M, int N, int K) {
+                void* __restrict__ out, int out_f32, int M, int N, int K, const Gate gate) {
     constexpr int STAGES = stages(NT), STAGE = stage_bytes(NT);
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
@@ -45,6 +57,11 @@ gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 
     // a copy of the warp covers four rows of 128 bytes; rows beyond N repeat the last one
     const int r4 = lane >> 3, piece = lane & 7;
+    auto row_of = [&](int tile, int r) {
+        if (!GATED) return min(tile * ROWS + r, N - 1);
+        const int o = tile * 8 + (r & 7);                    // N / 2 outputs, a multiple of 8, as a run is
+        return o / gate.run * 2 * gate.run + o % gate.run + (r < 8 ? 0 : gate.run);
+    };
     int w_tile = blockIdx.x, w_kb = 0, x_kb = 0;
     auto issue_w = [&](int step) {
         const uint32_t base = ring + (step % STAGES) * STAGE;
@@ -53,7 +70,7 @@ gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         for (int i = 0; i < ROWS / 4; ++i) {
             const int r = i * 4 + r4;
             asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;\n" ::"r"(base + r * PITCH + (((piece ^ r) & 7) << 4)),
-                         "l"(src + (size_t)min(w_tile * ROWS + r, N - 1) * K) : "memory");
+                         "l"(src + (size_t)row_of(w_tile, r) * K) : "memory");
         }
         if (++w_kb == nkb) w_kb = 0, w_tile += gridDim.x;
     };
@@ -113,19 +130,49 @@ gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
             for (int j = 0; j < 4; ++j) part[(warp * NT * 8 + nt * 8 + 2 * c + (j & 1)) * ROWS + g + (j >> 1) * 8] = acc[nt][j];
         __syncthreads();
-        const int n0 = (blockIdx.x + it * gridDim.x) * ROWS;
-        for (int i = tid; i < M * ROWS; i += WARPS * 32) {
-            const int m = i / ROWS, n = n0 + i % ROWS;
-            if (n >= N) continue;
+        const int tile = blockIdx.x + it * gridDim.x;
+        auto sum = [&](int m, int r) {
             float v = 0.f;
 #pragma unroll
-            for (int q = 0; q < WARPS; ++q) v += part[q * NT * 8 * ROWS + i];
+            for (int q = 0; q < WARPS; ++q) v += part[q * NT * 8 * ROWS + m * ROWS + r];
+            return v;
+        };
+        if (GATED) {
+            for (int i = tid; i < M * 8; i += WARPS * 32) {
+                const int m = i / 8, o = tile * 8 + i % 8;
+                float g_ = sum(m, i % 8), u = sum(m, i % 8 + 8);
+                if (gate.act == 2) {                         // the clamped form: g' sigmoid(alpha g') (u' + 1)
+                    g_ = fminf(g_, gate.limit);
+                    u = fminf(fmaxf(u, -gate.limit), gate.limit) + 1.f;
+                }
+                // act(g) = g * sigmoid(t): t = g for SiLU; t = 2 sqrt(2/pi) (g + 0.044715 g^3) for the tanh form of GELU; alpha g for the clamped form
+                const float t = gate.act == 0 ? g_ : (gate.act == 2 ? gate.alpha * g_ : 1.5957691216057308f * (g_ + 0.044715f * g_ * g_ * g_));
+                ((__nv_bfloat16*)out)[(size_t)m * (N / 2) + o] = __float2bfloat16_rn(g_ / (1.f + __expf(-t)) * u);
+            }
+            continue;
+        }
+        for (int i = tid; i < M * ROWS; i += WARPS * 32) {
+            const int m = i / ROWS, n = tile * ROWS + i % ROWS;
+            if (n >= N) continue;
+            float v = sum(m, i % ROWS);
             if (bias) v += bias_f32 ? ((const float*)bias)[n] : __bfloat162float(((const __nv_bfloat16*)bias)[n]);
             if (out_f32) ((float*)out)[(size_t)m * N + n] = v;
             else ((__nv_bfloat16*)out)[(size_t)m * N + n] = __float2bfloat16_rn(v);
         }
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+template <int NT, bool GATED>
+static int launch(int grid, const void* x, const void* w, const void* bias, int bias_f32, void* out, int out_f32, int M, int N, int K,
+                  const Gate& gate, cudaStream_t stream) {
+    auto kern = gemm_few_kernel<NT, GATED>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(NT));
+    LILY_REQUIRE(e == cudaSuccess, "gemm_few: %s", cudaGetErrorString(e));
+    launch_pdl(kern, dim3(grid), dim3(WARPS * 32), smem_bytes(NT), stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, bias_f32,
+               out, out_f32, M, N, K, gate);
+    LILY_CHECK_LAUNCH("gemm_few");
+    return 0;
 }
 
 }  // namespace fewrows
@@ -143,16 +190,38 @@ LILY_API int lily_gemm_few(const void* x, const void* w, const void* bias, int b
     LILY_REQUIRE(lily_gemm_few_takes(M, N, K), "gemm_few: M=%d N=%d K=%d", M, N, K);
     LILY_REQUIRE((((uintptr_t)x | (uintptr_t)w) & 15) == 0, "gemm_few: operands do not start on 16 bytes");
     const int tiles = (N + fewrows::ROWS - 1) / fewrows::ROWS, grid = min(tiles, 2 * sm_count());
-#define GO(NT)                                                                                                              \
-    do {                                                                                                                    \
-        auto kern = fewrows::gemm_few_kernel<NT>;                                                                           \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fewrows::smem_bytes(NT));   \
-        LILY_REQUIRE(e == cudaSuccess, "gemm_few: %s", cudaGetErrorString(e));                                              \
-        launch_pdl(kern, dim3(grid), dim3(fewrows::WARPS * 32), fewrows::smem_bytes(NT), stream, (const __nv_bfloat16*)x,   \
-                   (const __nv_bfloat16*)w, bias, bias_f32, out, out_f32, M, N, K);                                         \
-    } while (0)
-    if (M <= 8) GO(1); else GO(2);
-#undef GO
-    LILY_CHECK_LAUNCH("gemm_few");
-    return 0;
+    if (M <= 8) return fewrows::launch<1, false>(grid, x, w, bias, bias_f32, out, out_f32, M, N, K, fewrows::Gate{}, stream);
+    return fewrows::launch<2, false>(grid, x, w, bias, bias_f32, out, out_f32, M, N, K, fewrows::Gate{}, stream);
+}
+
+// out [M, I] bfloat16 = act(x . gate^T) * (x . up^T), up to 16 tokens; w [2 I, K] holds runs of `run` gate rows and the `run` up
+// rows of the same outputs (run == I: all gate rows, then all up rows).
+LILY_API int lily_swiglu_few_takes(int M, int I, int K, int run) {
+    return lily_gemm_few_takes(M, I, K) && I >= 8 && run >= 8 && run % 8 == 0 && I % run == 0;
+}
+
+// How a caller is to form the gate/up product and its activation: 0: this kernel does not take it (more than 8 tokens among
+// them), 1: here, 2: it takes it, but the product and the activation as a pass of its own are the answer (several tokens of an input that
+// the kernel before this one could not stage, for which that pair was ahead; it is 2 us behind now).  LILY_B200_SWIGLU_X=global
+// answers as if no input could be staged.
+LILY_API int lily_swiglu_few_verdict(int M, int I, int K, int run) {
+    if (M > 8 || !lily_swiglu_few_takes(M, I, K, run)) return 0;
+    static const bool never_staged = [] {
+        const char* v = getenv("LILY_B200_SWIGLU_X");
+        return v && v[0] == 'g';
+    }();
+    const long long kblocks = K / fewrows::KT, units = (I + 127) / 128 * kblocks, a_block = (units + sm_count() - 1) / sm_count();
+    const bool staged = !never_staged && min(a_block, kblocks) <= 66;        // 66 KB beside 160 KB of rings
+    return !staged && (long long)M * K > 3 * 8192 ? 2 : 1;
+}
+
+LILY_API int lily_swiglu_few(const void* x, const void* w, void* out, int M, int I, int K, int run, int act, float limit, float alpha,
+                             cudaStream_t stream) {
+    LILY_REQUIRE(lily_swiglu_few_takes(M, I, K, run), "swiglu_few: M=%d I=%d K=%d run=%d", M, I, K, run);
+    LILY_REQUIRE(act >= 0 && act <= 2 && (act != 2 || limit > 0.f), "swiglu_few: activation %d (0: SiLU, 1: GELU, tanh form, 2: clamped with a positive limit)", act);
+    LILY_REQUIRE((((uintptr_t)x | (uintptr_t)w) & 15) == 0, "swiglu_few: operands do not start on 16 bytes");
+    const int grid = min(I / 8, 2 * sm_count());
+    const fewrows::Gate gate{run, act, limit, alpha};
+    if (M <= 8) return fewrows::launch<1, true>(grid, x, w, nullptr, 0, out, 0, M, 2 * I, K, gate, stream);
+    return fewrows::launch<2, true>(grid, x, w, nullptr, 0, out, 0, M, 2 * I, K, gate, stream);
 }

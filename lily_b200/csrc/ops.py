@@ -32,9 +32,9 @@ _SIGNATURES = {
     "lily_qk_norm_rope_write": [_vp, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i,
                                 _i, _i, _i, _i, _i, _sz, _i, _i, _f, _vp, _i, _i, _vp],
     "lily_skinny_gemm": [_vp, _vp, _vp, _i, _i, _i, _i, _vp],
-    "lily_skinny_swiglu": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lily_cast": [_vp, _i, _vp, _i, _sz, _vp],
     "lily_gemm_few": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
+    "lily_swiglu_few": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp],
     "lily_gemm_fp32": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_attention_prefill_simt": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp, _vp],
     "lily_attention_decode_simt": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp, _vp],
@@ -122,8 +122,6 @@ def library():
         lib.lily_skinny_gemm_max_rows.restype = _i
         lib.lily_skinny_gemm_splits.argtypes = [_i, _i, _i]
         lib.lily_skinny_gemm_splits.restype = _i
-        lib.lily_skinny_swiglu_need.argtypes = [_i, _i, _i, _i, ctypes.POINTER(_sz), ctypes.POINTER(_i)]
-        lib.lily_skinny_swiglu_need.restype = _i
         lib.lily_attention_prefill_mma_rows.restype = _i
         lib.lily_attention_prefill_tc_rows.restype = _i
         lib.lily_attention_prefill_tc_takes.argtypes = [_i, _i]
@@ -150,6 +148,8 @@ def library():
         lib.lily_moe_tile_rows.restype = _i
         lib.lily_gemm_few_takes.argtypes = [_i, _i, _i]
         lib.lily_gemm_few_takes.restype = _i
+        lib.lily_swiglu_few_verdict.argtypes = [_i, _i, _i, _i]
+        lib.lily_swiglu_few_verdict.restype = _i
         lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
         lib.lily_ssd_step_takes.restype = _i
         lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
@@ -457,6 +457,16 @@ def few_rows_take(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
+def few_rows_whole_pays(m: int, n: int, k: int) -> bool:
+    """Whether finished float32 rows are the faster way to a product that its consumer would also add up from slices of k:
+    while the 16-row tiles fit the device in one turn (two blocks a SM; a second, partly filled turn costs more than
+    the slices' sums) and a block's share of k is short or there are blocks for every SM.  Measured with the norm that adds
+    the slices up, us, slices / whole: 2,048 x 2,048 4.2 / 3.4 with 2 tokens, 5.4 / 3.5 with 8; 4,096 x 4,096 8.0 / 7.2; 4,096 x 12,288
+    19.0 / 17.7; 2,048 x 8,192 8.1 / 8.5 with 1, 8.6 / 10.3 with 12; 6,144 x 4,096 9.6 / 10.6."""
+    tiles = -(-n // 16)
+    return tiles <= 2 * sm_count() and (k <= 4096 or tiles > sm_count())
+
+
 TC_MIN_ROWS = 65          # products of more rows than this go to the tcgen05 kernel when it takes the shape
 
 
@@ -524,11 +534,14 @@ def linear_split(x: torch.Tensor, weight: torch.Tensor, splits: Optional[int] = 
     lib = library()
     if m > lib.lily_skinny_gemm_max_rows() or m < 1 or weight.shape[1] != k or k % 64:
         return None
-    if splits is None:
+    own_rule = splits is None
+    if own_rule:
         splits = int(lib.lily_skinny_gemm_splits(m, n, k))
     if splits < 1:
         return None
     _dev(x, weight)
+    if own_rule and few_rows_whole_pays(m, n, k) and few_rows_take(x, weight):
+        return linear(x, weight, out_dtype=torch.float32).unsqueeze(0)
     parts = torch.empty((splits, m, n), dtype=torch.float32, device=x.device)
     _call("lily_skinny_gemm", _p(x), _p(weight), _p(parts), m, n, k, splits, _stream())
     return parts
@@ -547,18 +560,16 @@ def linear_auto(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
 
 def swiglu_skinny_need(tokens: int, intermediate: int, hidden: int, dtype: torch.dtype,
                        block: Optional[int] = None, whenever_possible: bool = False) -> Optional[Tuple[int, int]]:
-    """(float32 of scratch, int32 counters) that ``swiglu_skinny`` wants for this shape, or None when it does not
-    take it (more than 8 tokens, not bfloat16, K not a multiple of 64) or, unless ``whenever_possible``, when the
-    library product followed by SiLU*mul is the faster pair for it (several tokens of a very wide input): the caller
-    then forms the product and SiLU*mul separately.  ``LILY_B200_SWIGLU=library`` always answers None."""
+    """(float32 of scratch, int32 counters) that ``swiglu_skinny`` is given for this shape (it uses neither), or None when it
+    does not take it (more than 8 tokens, not bfloat16, K not a multiple of 64) or, unless ``whenever_possible``, for
+    several tokens of a very wide input: the caller then forms the product and SiLU*mul separately.
+    ``LILY_B200_SWIGLU=library`` always answers None."""
     if dtype != torch.bfloat16 or _LIBRARY_SWIGLU:
         return None
-    floats, counters = _sz(0), _i(0)
-    verdict = library().lily_skinny_swiglu_need(int(tokens), int(intermediate), int(hidden), int(block or intermediate),
-                                                ctypes.byref(floats), ctypes.byref(counters))
+    verdict = library().lily_swiglu_few_verdict(int(tokens), int(intermediate), int(hidden), int(block or intermediate))
     if verdict == 0 or (verdict == 2 and not whenever_possible):
         return None
-    return int(floats.value), int(counters.value)
+    return 4, 1
 
 
 _LIBRARY_SWIGLU = os.environ.get("LILY_B200_SWIGLU", "") == "library"
@@ -569,8 +580,8 @@ def swiglu_skinny(x: torch.Tensor, gate_up: torch.Tensor, block: Optional[int], 
                   limit: float = 0.0, alpha: float = 1.0) -> torch.Tensor:
     """``act(x . gate^T) * (x . up^T)`` [tokens, I] for up to 8 tokens in one kernel that streams the fused
     gate/up matrix [2 I, K] once (rows in alternating runs of ``block`` gate and up rows; None: all gate, then all
-    up).  ``scratch`` (float32) and ``counters`` (int32, zero before the first call; the kernel leaves them zero)
-    are sized by ``swiglu_skinny_need``."""
+    up).  ``scratch`` and ``counters`` are sized by
+    ``swiglu_skinny_need`` and left as they are."""
     _dev(x, gate_up, scratch, counters, out)
     m, k = x.shape
     inter = gate_up.shape[0] // 2
@@ -581,8 +592,8 @@ def swiglu_skinny(x: torch.Tensor, gate_up: torch.Tensor, block: Optional[int], 
         raise KernelError(f"swiglu_skinny: {need[0]} float32 of scratch and {need[1]} int32 counters needed")
     if out is None:
         out = torch.empty((m, inter), dtype=torch.bfloat16, device=x.device)
-    _call("lily_skinny_swiglu", _p(x), _p(gate_up), _p(out), _p(scratch), _p(counters), m, inter, k, int(block or inter),
-          GATE_ACTIVATIONS[activation], float(limit), float(alpha), _stream())
+    _call("lily_swiglu_few", _p(x), _p(gate_up), _p(out), m, inter, k, int(block or inter), GATE_ACTIVATIONS[activation],
+          float(limit), float(alpha), _stream())
     return out
 
 

@@ -877,3 +877,28 @@ def test_linear_of_a_few_rows(m, n, k):
     low = ops().linear(x, w, b.bfloat16())
     assert float((low - (want + b.bfloat16())).abs().max()) < 2 ** -8 * float(want.abs().max() + 4)
     assert torch.equal(ops().linear(x[-1:].contiguous(), w), ops().linear(x, w)[-1:])
+
+
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh", "swish_clamped"])
+@pytest.mark.parametrize("m,inter,k,run", [(1, 8, 64, 8), (5, 72, 192, 24), (8, 3000, 576, 8), (3, 2432, 512, 128)])
+def test_gate_up_of_a_few_rows(activation, m, inter, k, run):
+    """Every activation in the product's epilogue, runs of all lengths, several tiles a block and fewer outputs than a tile's rows."""
+    g = torch.Generator(device=DEV).manual_seed(m + k)
+    x = torch.randn(m, k, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(2 * inter, k, device=DEV, generator=g) * 2 * k ** -0.5).bfloat16()
+    how = dict(limit=1.5, alpha=1.702) if activation == "swish_clamped" else {}
+    need = ops().swiglu_skinny_need(m, inter, k, torch.bfloat16, run, whenever_possible=True)
+    got = ops().swiglu_skinny(x, w, run, torch.zeros(need[0], device=DEV), torch.zeros(need[1], device=DEV, dtype=torch.int32),
+                              activation=activation, **how)
+    want = ref.silu_mul((x.double() @ w.double().t()).float(), torch.float32, block=run, activation=activation, **how)
+    assert float((got.float() - want).abs().max()) < 2 ** -8 * float(want.abs().max())      # rounded once, to 8 bits
+
+
+def test_linear_split_in_one_plane():
+    """Where finished rows are the faster way the product comes as one float32 plane, the same numbers as its slices added up."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    for m, n, k in ((2, 2048, 2048), (16, 4096, 12288), (8, 24, 64)):
+        x, w = torch.randn(m, k, device=DEV, generator=g).bfloat16(), torch.randn(n, k, device=DEV, generator=g).bfloat16()
+        one = ops().linear_split(x, w)
+        assert tuple(one.shape) == (1, m, n) and one.dtype == torch.float32
+        assert float((one[0] - x.double() @ w.double().t()).abs().max()) < 4e-6 * (k ** 0.5) * 4
