@@ -101,6 +101,8 @@ struct Params {
     int bt_stride, tiles, nq, nkv, page_size, window;
     int keep_first;                       // with a window: keys at positions below this stay visible whatever the distance
     float scale_log2;                     // softmax scale times log2(e) (log2(e) alone under a cap)
+    int sink;                             // the softmax's denominator holds one more unit: a key of score 0 without a value
+    size_t plane;                         // elements between the planes of `out` (grid z): plane z weighs the values of kv head (own + z) % nkv
     float cap, cap_in;                    // cap > 0: scores become cap * tanh(score * cap_in), cap_in = scale / cap
 };
 
@@ -197,7 +199,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
     if (warp == 0) {
         if (lane == 0) {
-            const int kvh = head / (p.nq / p.nkv);
+            const int kvh = head / (p.nq / p.nkv), vh = (kvh + (int)blockIdx.z) % p.nkv;
             const int* table = p.block_table + (size_t)req * p.bt_stride;
             mbar_expect_tx(q_full, TILE);
             for (int dh = 0; dh < DH; ++dh) tma_load_3d(q_smem + dh * SUB, &map_q, q_full, dh * 64, head, q_begin + start);
@@ -225,7 +227,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 mbar_expect_tx(v_full + 8 * s, TILE);
                 for (int h = 0; h < 2; ++h)
                     for (int dh = 0; dh < DH; ++dh)
-                        tma_load_4d(v_smem + s * TILE + dh * SUB + h * BOX, &map_kv, v_full + 8 * s, dh * 64, off[h], p.nkv + kvh, page[h]);
+                        tma_load_4d(v_smem + s * TILE + dh * SUB + h * BOX, &map_kv, v_full + 8 * s, dh * 64, off[h], p.nkv + vh, page[h]);
                 ++issued_v;
             }
             if (*abort_flag) {
@@ -298,7 +300,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         const int pos = pos0 + row;
-        float m_used = -INFINITY, l = 0.f;
+        float m_used = p.sink ? 0.f : -INFINITY, l = 0.f;
         bool ok = true;
         // The threads of a row hand each other one float per tile (the maximum of their keys; at the end
         // their sum) through words of shared memory whose two lowest mantissa bits carry a sequence
@@ -374,6 +376,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             const float m_new = fmaxf(m_used, row_max);
             if (j == 0) {
                 m_used = m_new;
+                if (p.sink && part == 0) l = ex2(-m_used * p.scale_log2);       // the unit, against the row's maximum
             } else {
                 const bool grow = (m_new - m_used) * p.scale_log2 > GROW_LOG2;      // also when m_used is -inf
                 if (__any_sync(0xffffffffu, grow)) {
@@ -453,7 +456,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (ok) {
             tc_fence_after();
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            __nv_bfloat16* dst = p.out + ((size_t)(q_begin + start + row) * p.nq + head) * D + part * OCOLS;
+            __nv_bfloat16* dst = p.out + blockIdx.z * p.plane + ((size_t)(q_begin + start + row) * p.nq + head) * D + part * OCOLS;
 #pragma unroll 1
             for (int c = 0; c < OCOLS / 32; ++c) {
                 float o[32];
@@ -565,7 +568,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
 
     if (warp == 0) {
         if (lane == 0) {
-            const int kvh = head0 / (p.nq / p.nkv);
+            const int kvh = head0 / (p.nq / p.nkv), vh = (kvh + (int)blockIdx.z) % p.nkv;
             const int* table = p.block_table + (size_t)req * p.bt_stride;
             mbar_expect_tx(q_full, NH2 * TILE);
             for (int h = 0; h < NH2; ++h)
@@ -595,7 +598,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 mbar_expect_tx(v_full + 8 * s, TILE);
                 for (int h = 0; h < 2; ++h)
                     for (int dh = 0; dh < DH; ++dh)
-                        tma_load_4d(v_smem + s * TILE + dh * SUB + h * BOX, &map_kv, v_full + 8 * s, dh * 64, off[h], p.nkv + kvh, page[h]);
+                        tma_load_4d(v_smem + s * TILE + dh * SUB + h * BOX, &map_kv, v_full + 8 * s, dh * 64, off[h], p.nkv + vh, page[h]);
                 ++issued_v;
             }
             if (*abort_flag) {
@@ -689,7 +692,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         const uint32_t my_s = tmem + lane_addr + (uint32_t)(h * BKV), my_o = tmem_o + lane_addr + (uint32_t)(h * D);
         const int pos = pos0 + row;
-        float m_used = -INFINITY, l = 0.f;
+        float m_used = p.sink ? 0.f : -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < n && ok; ++j) {
             { FA_TIC(); ok = mbar_wait(s_full + 8 * h, (uint32_t)(j & 1), abort_flag, 7); FA_TOC(8 + h, row == 0); }
@@ -724,6 +727,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
             FA_TOC(10 + h, row == 0);
             if (j == 0) {
                 m_used = m_new;
+                if (p.sink) l = ex2(-m_used * p.scale_log2);
             } else {
                 const bool grow = (m_new - m_used) * p.scale_log2 > GROW_LOG2;      // also when m_used is -inf
                 if (__any_sync(0xffffffffu, grow)) {
@@ -788,7 +792,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
         if (ok) {
             tc_fence_after();
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            __nv_bfloat16* dst = p.out + ((size_t)(q_begin + start + row) * p.nq + head0 + h) * D;
+            __nv_bfloat16* dst = p.out + blockIdx.z * p.plane + ((size_t)(q_begin + start + row) * p.nq + head0 + h) * D;
 #pragma unroll 1
             for (int c = 0; c < D / 32; ++c) {
                 float o[32];
@@ -816,7 +820,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
 
 // Launches the kernel of head size D with one head or two heads a block (the shared memory limits are raised once).
 template <int D>
-static int launch(bool two, int nq, int tiles, cudaStream_t stream, const CUtensorMap& map_q, const CUtensorMap& map_kv, const Params& p) {
+static int launch(bool two, int nq, int tiles, int planes, cudaStream_t stream, const CUtensorMap& map_q, const CUtensorMap& map_kv, const Params& p) {
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_one(D));
@@ -829,9 +833,9 @@ static int launch(bool two, int nq, int tiles, cudaStream_t stream, const CUtens
         configured = true;
     }
     if (two)
-        launch_pdl(attention_prefill_tc2_kernel<D>, dim3(nq / 2, tiles), dim3(THREADS2), (size_t)smem_two(D), stream, map_q, map_kv, p);
+        launch_pdl(attention_prefill_tc2_kernel<D>, dim3(nq / 2, tiles, planes), dim3(THREADS2), (size_t)smem_two(D), stream, map_q, map_kv, p);
     else
-        launch_pdl(attention_prefill_tc_kernel<D>, dim3(nq, tiles), dim3(THREADS), (size_t)smem_one(D), stream, map_q, map_kv, p);
+        launch_pdl(attention_prefill_tc_kernel<D>, dim3(nq, tiles, planes), dim3(THREADS), (size_t)smem_one(D), stream, map_q, map_kv, p);
     return 0;
 }
 
@@ -870,13 +874,16 @@ LILY_API int lily_attention_tc_status() {
 
 // The arguments of lily_attention_prefill_mma with tiles of 128 rows, plus the number of pages of
 // the layer (`kv` is [num_pages, 2, nkv, page_size, d]) and of new tokens (`q` is [tokens, nq, d]);
-// heads_per_block 1 or 2 names the kernel, 0 leaves the choice to the launcher.
+// heads_per_block 1 or 2 names the kernel, 0 leaves the choice to the launcher.  sink: the softmax's denominator holds one more
+// unit.  planes: plane z of `out` ([planes][tokens, nq, d]) holds every head's weights over the values of kv head (its own + z) % nkv,
+// all in one launch (2,000 tokens, 16 heads over 4 of 128: four launches of the mma.sync kernel 4 x 108 us, this one 112).
 LILY_API int lily_attention_prefill_tc(const void* q, const void* kv, void* out, const int* block_table, int bt_stride,
                                        const int* cu_seqlens, const int* prefix_lens, const int* tile_req,
                                        const int* tile_start, int tiles, int nq, int nkv, int d, int page_size, int window,
                                        float scale, int tokens, int num_pages, int heads_per_block, float softcap,
-                                       int keep_first, cudaStream_t stream) {
+                                       int keep_first, int sink, int planes, cudaStream_t stream) {
     if (tiles == 0) return 0;
+    LILY_REQUIRE(planes >= 1 && planes <= nkv, "attention_prefill_tc: %d planes of %d kv heads", planes, nkv);
     LILY_REQUIRE(lily_attention_prefill_tc_takes(d, page_size), "attention_prefill_tc: head size %d, page size %d (takes 64 or 128, and multiples of 64)",
                  d, page_size);
     LILY_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_prefill_tc: %d query heads over %d kv heads", nq, nkv);
@@ -908,7 +915,7 @@ LILY_API int lily_attention_prefill_tc(const void* q, const void* kv, void* out,
     fa::Params p{};
     p.block_table = block_table; p.cu_seqlens = cu_seqlens; p.prefix_lens = prefix_lens; p.tile_req = tile_req;
     p.tile_start = tile_start; p.out = (__nv_bfloat16*)out; p.bt_stride = bt_stride; p.tiles = tiles; p.nq = nq; p.nkv = nkv;
-    p.page_size = page_size; p.window = window;
+    p.page_size = page_size; p.window = window; p.sink = sink; p.plane = (size_t)tokens * nq * d;
     p.keep_first = window > 0 && keep_first > 0 ? keep_first : 0;
     p.cap = softcap > 0.f ? softcap : 0.f;
     p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
@@ -919,8 +926,8 @@ LILY_API int lily_attention_prefill_tc(const void* q, const void* kv, void* out,
     const bool even = (nq / nkv) % 2 == 0;
     LILY_REQUIRE(heads_per_block >= 0 && heads_per_block <= 2 && (heads_per_block != 2 || even),
                  "attention_prefill_tc: %d heads a block with %d query heads per kv head", heads_per_block, nq / nkv);
-    const bool two = heads_per_block == 2 || (heads_per_block == 0 && even && (long)tiles * (nq / 2) >= sms);
-    const int rc = d == 64 ? fa::launch<64>(two, nq, tiles, stream, map_q, map_kv, p) : fa::launch<128>(two, nq, tiles, stream, map_q, map_kv, p);
+    const bool two = heads_per_block == 2 || (heads_per_block == 0 && even && (long)tiles * planes * (nq / 2) >= sms);
+    const int rc = d == 64 ? fa::launch<64>(two, nq, tiles, planes, stream, map_q, map_kv, p) : fa::launch<128>(two, nq, tiles, planes, stream, map_q, map_kv, p);
     if (rc) return rc;
     LILY_CHECK_LAUNCH("attention_prefill_tc");
     return 0;

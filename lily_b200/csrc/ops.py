@@ -40,7 +40,7 @@ _SIGNATURES = {
     "lily_attention_decode_simt": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp, _vp],
     "lily_attention_combine": [_vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_attention_prefill_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp],
-    "lily_attention_prefill_tc": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _f, _i, _vp],
+    "lily_attention_prefill_tc": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _f, _i, _i, _i, _vp],
     "lily_attention_decode_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _vp],
     "lily_attention_decode_mma_fused": [_vp, _i, _sz, _i, _vp, _vp, _i, _f, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _vp,
                                         _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _vp],
@@ -674,6 +674,8 @@ def prefill_tile_rows(dtype: torch.dtype = torch.float32, d: int = 0, page_size:
         # a tile height names its kernel; where both kernels' tiles hold one token (65 heads and more) it is the tcgen05 one
         return many if latent_tcgen05(dtype, d, dv, page_size) and (many == few or new_tokens * heads >= LATENT_TC_MIN_ROWS) else few
     if (sink or all_values) and sink_on_tensor_cores(dtype, d, dv, values_in_keys, softcap):
+        if not _MMA_SINK and uses_tcgen05_attention(dtype, d, page_size, new_tokens):
+            return int(lib.lily_attention_prefill_tc_rows())
         return int(lib.lily_attention_prefill_mma_rows())
     if sink or all_values:
         return int(lib.lily_attention_prefill_simt_rows())
@@ -710,14 +712,25 @@ def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torc
     (tcgen05 only) 1 or 2 picks between its one-head and its two-head form; 0 lets the launcher choose."""
     _dev(q, kv_layer, block_table, cu_seqlens, prefix_lens, tile_req, tile_start, out, sinks)
     _check_sinks(sinks, nq, sink or all_values)
-    planes = all_values and out.dim() == 3            # one launch of the mma.sync kernel a kv head (``all_values_sums``)
+    planes = all_values and out.dim() == 3            # a plane a kv head (``all_values_sums``)
     if q.dtype != kv_layer.dtype or out.dtype != (torch.float32 if all_values and not planes else q.dtype):
         raise KernelError("attention: q, cache and out must share a dtype (sums over all kv heads' values on CUDA cores are float32)")
     if (sink or all_values) and sink_on_tensor_cores(q.dtype, d, dv, values_in_keys, softcap) and (planes or not all_values):
-        if (tile_rows or 0) not in (0, int(library().lily_attention_prefill_mma_rows())):
-            raise KernelError(f"attention_prefill: the sink runs in tiles of {library().lily_attention_prefill_mma_rows()} rows")
+        lib = library()
+        on_tc = (tile_rows == int(lib.lily_attention_prefill_tc_rows()) and not _MMA_SINK
+                 and bool(lib.lily_attention_prefill_tc_takes(int(d), int(page_size))))
+        if not on_tc and (tile_rows or 0) not in (0, int(lib.lily_attention_prefill_mma_rows())):
+            raise KernelError(f"attention_prefill: the sink runs in tiles of {lib.lily_attention_prefill_mma_rows()} rows"
+                              f" (or {lib.lily_attention_prefill_tc_rows()} where the tcgen05 kernel takes the shape)")
         if planes and tuple(out.shape) != (nkv, q.shape[0], nq * d):
             raise KernelError(f"attention_prefill: planes of sums are [{nkv}, tokens, nq * d]")
+        if on_tc:
+            _call("lily_attention_prefill_tc", _p(q), _p(kv_layer), _p(out), _i32(block_table, "block_table"), block_table.shape[-1],
+                  _i32(cu_seqlens, "cu_seqlens"), _i32(prefix_lens, "prefix_lens"), _i32(tile_req, "tile_req"),
+                  _i32(tile_start, "tile_start"), tile_req.numel(), nq, nkv, d, page_size, int(window or 0), float(scale), q.shape[0],
+                  kv_layer.shape[0], int(heads_per_block), float(softcap or 0.0), int(keep_first or 0) if window else 0,
+                  int(bool(sink)), nkv if planes else 1, _stream())
+            return
         for shift in range(nkv if planes else 1):
             _call("lily_attention_prefill_mma", _p(q), _p(kv_layer), out[shift].data_ptr() if planes else _p(out),
                   _i32(block_table, "block_table"), block_table.shape[-1], _i32(cu_seqlens, "cu_seqlens"),
@@ -768,7 +781,7 @@ def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torc
                               f"page size {page_size}")
         if not (q.is_contiguous() and out.is_contiguous() and kv_layer.is_contiguous()):
             raise KernelError("attention_prefill: the tcgen05 kernel takes contiguous q, out and cache")
-        _call("lily_attention_prefill_tc", *common, q.shape[0], kv_layer.shape[0], int(heads_per_block), cap, keep_first, _stream())
+        _call("lily_attention_prefill_tc", *common, q.shape[0], kv_layer.shape[0], int(heads_per_block), cap, keep_first, 0, 1, _stream())
     elif tensor_cores:
         _call("lily_attention_prefill_mma", *common, cap, keep_first, 0, 0, _stream())
     else:
@@ -778,12 +791,13 @@ def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torc
 _MERGED_SHIFTS = os.environ.get("LILY_B200_MERGED_SHIFTS", "1") != "0"
 ALL_VALUES_COLUMNS = 512       # value columns a query row of the CUDA-core kernels gathers in one launch
 _SIMT_SINK = os.environ.get("LILY_B200_SINK_ATTENTION", "") == "simt"
+_MMA_SINK = os.environ.get("LILY_B200_SINK_ATTENTION", "") == "mma"        # prompts stay on the mma.sync kernel
 
 
 def sink_on_tensor_cores(dtype: torch.dtype, d: int, dv: Optional[int] = None, values_in_keys: bool = False,
                          softcap: Optional[float] = None) -> bool:
-    """Whether attention with a sink (and, in one launch a kv head, with the values of all kv heads) runs on the mma.sync
-    kernels: bfloat16, keys and values of one head size that those kernels take; else the CUDA-core kernels."""
+    """Whether attention with a sink (and with the values of all kv heads) runs on the tensor-core kernels (prompts of
+    TC_ATTENTION_MIN_TOKENS on the tcgen05 kernel where it takes the shape, the rest on mma.sync): bfloat16, keys and values of one head size that those kernels take; else the CUDA-core kernels."""
     return (not _SIMT_SINK and not values_in_keys and int(dv or d) == d and uses_tensor_cores(dtype, d))
 
 

@@ -902,3 +902,32 @@ def test_linear_split_in_one_plane():
         one = ops().linear_split(x, w)
         assert tuple(one.shape) == (1, m, n) and one.dtype == torch.float32
         assert float((one[0] - x.double() @ w.double().t()).abs().max()) < 4e-6 * (k ** 0.5) * 4
+
+
+@pytest.mark.parametrize("heads_per_block", [1, 2])
+@pytest.mark.parametrize("nq,nkv,d,window,sink,planes", [(16, 4, 128, None, True, True), (4, 2, 64, None, False, True), (6, 3, 64, 100, True, True),
+                                                         (8, 4, 128, None, True, False)])
+def test_attention_prefill_tcgen05_sink_and_planes(nq, nkv, d, window, sink, planes, heads_per_block):
+    """The sink's unit and the planes of values of every kv head on the tcgen05 kernel: one-row tiles, cached prefixes, rows whose
+    scores all lie far below the sink's and rows with a key far above it."""
+    o, page = ops(), 64
+    prefixes, news = [0, 17, 130, 300], [1, 200, 129, 64]
+    cache, table, q, cu, pre = _attention_case(torch.bfloat16, nq, nkv, d, page, prefixes, news, window, spike=True)
+    q[5:40] = (q[5:40].float() * 6).bfloat16()
+    rows = int(o.library().lily_attention_prefill_tc_rows())
+    tiles = _tiles_of(news, rows)
+    shape = (nkv, len(q), nq * d) if planes else (len(q), nq * d)
+    got = torch.zeros(shape, device=DEV, dtype=torch.bfloat16)
+    o.attention_prefill(q, cache, table, cu, pre, *tiles, got, nq, nkv, d, page, d ** -0.5, window, tile_rows=rows, sink=sink,
+                        all_values=planes, heads_per_block=heads_per_block)
+    assert o.attention_tc_status() == 0
+    if planes:
+        wide = torch.zeros(len(q), nq * nkv * d, device=DEV)
+        ref.attention_prefill(q, cache, table, cu, pre, *tiles, wide, nq, nkv, d, page, d ** -0.5, window, sink=sink, all_values=True)
+        wide = wide.view(len(q), nq, nkv, d)
+        own = torch.arange(nq, device=DEV) // (nq // nkv)
+        want = torch.stack([wide[:, torch.arange(nq, device=DEV), (own + z) % nkv] for z in range(nkv)]).reshape(shape)
+    else:
+        want = torch.zeros(shape, device=DEV)
+        ref.attention_prefill(q, cache, table, cu, pre, *tiles, want, nq, nkv, d, page, d ** -0.5, window, sink=sink)
+    torch.testing.assert_close(got.float(), want.float(), **tol(torch.bfloat16))
