@@ -67,6 +67,7 @@ _SIGNATURES = {
                       _i, _vp, _vp, _i, _vp],
     "lily_ssd_step": [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
     "lily_wkv_step": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "lily_ssd_chunk": [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
     "lily_ssd_combine": [_vp, _sz, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "lily_gated_group_rmsnorm": [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _f, _i, _vp],
     "lily_latent_attention_prefill_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
@@ -146,6 +147,8 @@ def library():
         lib.lily_latent_attention_tc_col_blocks.argtypes = [_i]
         lib.lily_latent_attention_tc_col_blocks.restype = _i
         lib.lily_moe_tile_rows.restype = _i
+        lib.lily_ssd_chunk_takes.argtypes = [_vp, _i, _i, _i, _i, _i]
+        lib.lily_ssd_chunk_takes.restype = _i
         lib.lily_gemm_few_takes.argtypes = [_i, _i, _i]
         lib.lily_gemm_few_takes.restype = _i
         lib.lily_swiglu_few_verdict.argtypes = [_i, _i, _i, _i]
@@ -1214,6 +1217,8 @@ def causal_conv(proj: torch.Tensor, col0: int, channels: int, weight: torch.Tens
 SCAN_CHUNK = 128        # tokens a chunk of a long portion (doubled while the chunk states would pass SCAN_WORKSPACE)
 SCAN_DIRECT = 192       # portions up to this many tokens run in one piece, from and to the state in the slot
 SCAN_WORKSPACE = 1 << 29
+SCAN_FINE = 17          # tokens from which a portion is worth the tensor-core kernels' chunks (a token by itself takes about a
+                        # microsecond of a block, three launches and a padded tile 30)
 
 
 @dataclass
@@ -1232,33 +1237,51 @@ class ScanPlan:
     long_count: Optional[torch.Tensor] = None
     num_long: int = 0
     chunk: int = 0                           # the longest chunk, in tokens
+    fine: Optional["ScanPlan"] = None        # the cut for the tensor-core kernels, where they could take chunks
+
+
+_SSD_CHUNKS = os.environ.get("LILY_B200_SSD_CHUNKS", "") != "scan"       # "scan": chunks run token by token
 
 
 def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0) -> ScanPlan:
     """Cuts the step's portions for the scan.  A portion of up to SCAN_DIRECT tokens (every decoded token) runs in one
     piece; a longer one in chunks of SCAN_CHUNK tokens that run side by side and are joined by ``ssd_combine``
-    (``state_floats``: the size of one scan state, which bounds how many chunks the workspace may hold)."""
-    longs = [r for r, n in enumerate(new_lens) if n > SCAN_DIRECT]
-    if not longs:
-        return ScanPlan(None, len(new_lens))
+    (``state_floats``: the size of one scan state, which bounds how many chunks the workspace may hold).  Where the
+    tensor-core kernels could take chunks, ``fine`` is the cut for them: chunks from SCAN_FINE tokens on."""
+    def cut(direct_most, chunk):
+        longs = [r for r, n in enumerate(new_lens) if n > direct_most]
+        direct = [r for r, n in enumerate(new_lens) if n <= direct_most]
+        creq, cstart, clen, lfirst, lcount = [], [], [], [], []
+        for r in longs:
+            lfirst.append(len(creq))
+            for s in range(0, new_lens[r], chunk):
+                creq.append(r)
+                cstart.append(s)
+                clen.append(min(chunk, new_lens[r] - s))
+            lcount.append(len(creq) - lfirst[-1])
+        return [direct, creq, cstart, clen, longs, lfirst, lcount], chunk
+
     chunk = SCAN_CHUNK
-    while chunk < 1024 and state_floats and sum(-(-new_lens[r] // chunk) for r in longs) * state_floats * 4 > SCAN_WORKSPACE:
+    while chunk < 1024 and state_floats and sum(-(-n // chunk) for n in new_lens if n > SCAN_DIRECT) * state_floats * 4 > SCAN_WORKSPACE:
         chunk *= 2
-    direct = [r for r, n in enumerate(new_lens) if n <= SCAN_DIRECT]
-    creq, cstart, clen, lfirst, lcount = [], [], [], [], []
-    for r in longs:
-        lfirst.append(len(creq))
-        for s in range(0, new_lens[r], chunk):
-            creq.append(r)
-            cstart.append(s)
-            clen.append(min(chunk, new_lens[r] - s))
-        lcount.append(len(creq) - lfirst[-1])
-    flat = direct + creq + cstart + clen + longs + lfirst + lcount
-    dev = torch.tensor(flat, dtype=torch.int32).to(device, non_blocking=True)
-    sizes = [len(direct)] + [len(creq)] * 3 + [len(longs)] * 3
-    parts = torch.split(dev, sizes)
-    return ScanPlan(parts[0], len(direct), parts[1], parts[2], parts[3], len(creq), parts[4], parts[5], parts[6], len(longs),
-                    chunk)
+    cuts = [cut(SCAN_DIRECT, chunk)] if max(new_lens, default=0) > SCAN_DIRECT else []
+    if (max(new_lens, default=0) >= SCAN_FINE and chunk == SCAN_CHUNK
+            and sum(-(-n // chunk) for n in new_lens if n >= SCAN_FINE) * max(state_floats, 1) * 4 <= SCAN_WORKSPACE):
+        cuts.append(cut(SCAN_FINE - 1, chunk))
+    if not cuts:
+        return ScanPlan(None, len(new_lens))
+    # one copy to the device for all lists
+    lists = [part for parts, _ in cuts for part in parts]
+    dev = torch.tensor([x for part in lists for x in part], dtype=torch.int32).to(device, non_blocking=True)
+    split = torch.split(dev, [len(part) for part in lists])
+    plans = []
+    for i, (parts, size) in enumerate(cuts):
+        p = split[7 * i:7 * i + 7]
+        plans.append(ScanPlan(p[0], len(parts[0]), p[1], p[2], p[3], len(parts[1]), p[4], p[5], p[6], len(parts[4]), size))
+    if max(new_lens) <= SCAN_DIRECT:
+        return ScanPlan(None, len(new_lens), fine=plans[0])
+    plans[0].fine = plans[1] if len(plans) > 1 else None
+    return plans[0]
 
 
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
@@ -1289,6 +1312,11 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
         # one token a request (a decode step): a kernel that moves the state and stages nothing
         _call("lily_ssd_step", *common, int(requests), *sizes, _stream())
         return y
+    fine = plan.fine if plan is not None else None
+    tensor_cores = (fine is not None and xbc.dtype == torch.bfloat16 and _SSD_CHUNKS
+                    and bool(library().lily_ssd_chunk_takes(_p(xbc), channels, heads, head_dim, n_state, fine.chunk)))
+    if tensor_cores:
+        plan = fine
     if plan is None or plan.direct is None:
         _call("lily_ssd_scan", *common, int(requests), *sizes, None, None, None, 0, None, None, 0, _stream())
         return y
@@ -1301,18 +1329,27 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
         raise KernelError(f"ssd_scan: a float32 workspace of {need} entries needed")
     chunk_state, chunk_decay = workspace, workspace[plan.num_chunks * inner * n_state:]
     items = (_p(plan.chunk_req), _p(plan.chunk_start), _p(plan.chunk_len))
-    _call("lily_ssd_scan", *common, plan.num_chunks, *sizes, *items, 1, _p(chunk_state), _p(chunk_decay), plan.chunk, _stream())
+
+    def run(outputs):
+        if tensor_cores:
+            _call("lily_ssd_chunk", _p(xbc), channels, _p(proj), proj.shape[1], int(dt_col), _p(dt_bias), _p(a_log), _p(d_skip), _p(y),
+                  _i32(cu_seqlens, "cu_seqlens"), plan.num_chunks, heads, head_dim, n_state, groups, *items, _p(chunk_state),
+                  _p(chunk_decay), plan.chunk, int(outputs), _stream())
+        else:
+            _call("lily_ssd_scan", *common, plan.num_chunks, *sizes, *items, 2 if outputs else 1, _p(chunk_state), _p(chunk_decay),
+                  plan.chunk, _stream())
+
+    run(outputs=False)
     _call("lily_ssd_combine", _p(state), state.shape[1], _i32(slots, "slots"), _p(chunk_state), _p(chunk_decay),
           _p(plan.long_req), _p(plan.long_first), _p(plan.long_count), plan.num_long, heads, head_dim * n_state, _stream())
-    _call("lily_ssd_scan", *common, plan.num_chunks, *sizes, *items, 2, _p(chunk_state), _p(chunk_decay), plan.chunk, _stream())
+    run(outputs=True)
     return y
 
 
 def scan_workspace_floats(plan: Optional[ScanPlan], heads: int, head_dim: int, n_state: int) -> int:
     """float32 entries ``ssd_scan`` needs for this plan: a state and one decay a head for every chunk."""
-    if plan is None or not plan.num_chunks:
-        return 0
-    return plan.num_chunks * (heads * head_dim * n_state + heads)
+    chunks = 0 if plan is None else max(plan.num_chunks, plan.fine.num_chunks if plan.fine is not None else 0)
+    return chunks * (heads * head_dim * n_state + heads)
 
 
 def gated_group_rmsnorm(y: torch.Tensor, proj: torch.Tensor, gain: torch.Tensor, groups: int, eps: float) -> torch.Tensor:

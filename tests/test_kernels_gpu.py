@@ -931,3 +931,45 @@ def test_attention_prefill_tcgen05_sink_and_planes(nq, nkv, d, window, sink, pla
         want = torch.zeros(shape, device=DEV)
         ref.attention_prefill(q, cache, table, cu, pre, *tiles, want, nq, nkv, d, page, d ** -0.5, window, sink=sink)
     torch.testing.assert_close(got.float(), want.float(), **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("lens", [[17], [64, 5, 130], [128, 1, 257, 40], [16, 300]])
+@pytest.mark.parametrize("heads,groups,pd,n_state", [(4, 2, 64, 128), (3, 1, 16, 16), (2, 1, 80, 48), (8, 4, 128, 64)])
+def test_ssd_scan_in_chunks_on_the_tensor_cores(lens, heads, groups, pd, n_state):
+    """bfloat16 portions as chunks of matrix products: chunks and tiles that are not whole, short portions beside long ones, heads of
+    less and more than 64 columns, slow and fast decays (e^-30 a token) in one chunk; no further from 64 bits than token by token."""
+    from lily_b200.csrc import ops as o
+    g = torch.Generator(device=DEV).manual_seed(sum(lens) + pd)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    n, inner = sum(lens), heads * pd
+    xbc, proj = rand(n, inner + 2 * groups * n_state).bfloat16(), rand(n, 8 + heads).bfloat16()
+    dt_bias, a_log, d_skip = rand(heads), torch.linspace(-5.0, 3.0, heads, device=DEV), rand(heads)
+    state = rand(len(lens) + 1, inner * n_state)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device=DEV, dtype=torch.int32)
+    slots = torch.arange(len(lens), 0, -1, device=DEV, dtype=torch.int32)
+    plan = o.scan_plan(lens, DEV, inner * n_state)
+    assert plan.fine is not None and plan.fine.num_chunks
+    errs = []
+    x64, p64, s64 = xbc.double(), proj.double(), state.double()
+    want = torch.empty(n, inner, device=DEV, dtype=torch.float64)
+    per = heads // groups
+    for r in range(len(lens)):
+        s = s64[int(slots[r])].view(heads, pd, n_state)
+        for t in range(int(cu[r]), int(cu[r + 1])):
+            x = x64[t, :inner].view(heads, pd)
+            b, c = (x64[t, inner + k * groups * n_state:inner + (k + 1) * groups * n_state].view(groups, n_state).repeat_interleave(per, 0) for k in (0, 1))
+            dt = torch.nn.functional.softplus(p64[t, 4:4 + heads] + dt_bias.double())
+            s.copy_(torch.exp(-torch.exp(a_log.double()) * dt)[:, None, None] * s + (dt[:, None] * x)[:, :, None] * b[:, None, :])
+            want[t] = (torch.einsum("hpn,hn->hp", s, c) + d_skip.double()[:, None] * x).reshape(inner)
+    for chunks in (False, True):
+        o._SSD_CHUNKS = chunks
+        try:
+            mine = state.clone()
+            got = o.ssd_scan(xbc, proj, 4, dt_bias, a_log, d_skip, mine, cu, slots, len(lens), heads, pd, n_state, groups, plan=plan)
+        finally:
+            o._SSD_CHUNKS = True
+        errs.append((float((got.double() - want).norm() / want.norm()), float((mine.double() - s64)[1:].norm() / s64[1:].norm())))
+        assert torch.equal(mine[0], state[0])
+    # float32 sums either way: 2^-24 a product and term
+    assert errs[1][0] < 2e-6 and errs[1][1] < 2e-6, errs
+    assert errs[1][0] < errs[0][0] + 2e-8 and errs[1][1] < errs[0][1] + 2e-8, errs
