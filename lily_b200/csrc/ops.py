@@ -433,7 +433,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             raise KernelError("float32 linear takes a float32 bias")
         _call("lily_gemm_fp32", _p(x), _p(weight), _p(bias), _p(out), m, n, k, k, n, _stream())
         return out
-    if few_rows_take(x, weight) and out_dtype in (None, torch.bfloat16, torch.float32) and (bias is None or bias.numel() == n):
+    if (few_rows_take(x, weight) and out_dtype in (None, torch.bfloat16, torch.float32)
+            and (bias is None or bias.shape[-1] == bias.numel() == n)):
+        if bias is not None and bias.dtype not in (torch.float32, torch.bfloat16):
+            bias = bias.float()                                   # the kernel reads these two
         out = torch.empty((m, n), dtype=out_dtype or x.dtype, device=x.device)
         _call("lily_gemm_few", _p(x), _p(weight), _p(bias), int(bias is not None and bias.dtype == torch.float32), _p(out),
               int(out.dtype == torch.float32), m, n, k, _stream())

@@ -879,6 +879,19 @@ def test_linear_of_a_few_rows(m, n, k):
     assert torch.equal(ops().linear(x[-1:].contiguous(), w), ops().linear(x, w)[-1:])
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float64])
+@pytest.mark.parametrize("m", [1, 9, 16, 17])
+def test_linear_takes_a_bias_of_any_float_type(m, dtype):
+    """Few rows and many: a bias that no kernel reads as it is gets converted first."""
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x, w = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((m, 192), (40, 192)))
+    b = torch.randn(40, device=DEV, generator=g).to(dtype)
+    want = x.double() @ w.double().t() + b.double()
+    assert float((ops().linear(x, w, b, out_dtype=torch.float32) - want).abs().max()) < 4e-6 * (192 ** 0.5) * 4
+    low = ops().linear(x, w, b)                       # sum and bias are rounded to 8 bits, 2^-9 each
+    assert low.dtype == torch.bfloat16 and float((low - want).abs().max()) < 2 ** -8 * float(want.abs().max() + 4)
+
+
 @pytest.mark.parametrize("activation", ["silu", "gelu_tanh", "swish_clamped"])
 @pytest.mark.parametrize("m,inter,k,run", [(1, 8, 64, 8), (5, 72, 192, 24), (8, 3000, 576, 8), (3, 2432, 512, 128)])
 def test_gate_up_of_a_few_rows(activation, m, inter, k, run):
