@@ -13,6 +13,8 @@
 // B, C and x are the convolution's own bfloat16 numbers.  What meets the tensor cores as float32 (a weighted value, a decayed
 // score, an entry of the starting state) is cut into the sum of three bfloat16 numbers, all 24 bits of it, and multiplied three
 // times; the L are summed in float64 and kept as two float32, so that the difference of two large ones loses nothing.
+// (The chunked form of the scan is Dao and Gu's, "Transformers are SSMs", 2024.)  A number that is not finite reaches what it would token
+// by token: its own column and head, from its token on.
 // Bound by the tensor cores and the reads of shared memory that feed them.  The scan one token after another took a chunk's
 // 128 steps twice, each step a round of shared memory, FMAs and shuffles: 2,048 tokens, 64 heads of 64 x 128: 139 (own states) and
 // 270 us (outputs), now 33 and 92; against 64 bits the outputs are 1.0e-7 off in the 2-norm, where they were 2 to 4e-7.
@@ -51,15 +53,23 @@ struct Args {
 
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
-// Pairs of float32 numbers as three pairs of bfloat16 whose sum they are.
+// Pairs of float32 numbers as three pairs of bfloat16 whose sum they are; infinities are their own first part.
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     const float2 hf = __bfloat1622float2(h);
     hi = *reinterpret_cast<const uint32_t*>(&h);
-    split2(x - hf.x, y - hf.y, mid, lo);
+    split2(isinf(hf.x) ? 0.f : x - hf.x, isinf(hf.y) ? 0.f : y - hf.y, mid, lo);
 }
 
+// Which of a pair of bfloat16 numbers are infinities or NaN, as a mask over the pair's bits.
+__device__ __forceinline__ uint32_t not_finite(uint32_t pair) {
+    return ((pair & 0x7f80u) == 0x7f80u ? 0xffffu : 0u) | ((pair & 0x7f800000u) == 0x7f800000u ? 0xffff0000u : 0u);
+}
+
+__device__ __forceinline__ float half_of(uint32_t pair, int upper) { return __uint_as_float(upper ? pair & 0xffff0000u : pair << 16); }
+
 // A token's step size and L (as two numbers) for the chunk's tokens, a thread each; the chunk's L for everyone.  All threads call it.
+// e^-110 is zero in float32, so a decay beyond e^-200 counts as that: the sums stay finite and keep the bits of the slow decays behind it.
 struct Gates {
     float dt[CHUNK], hi[CHUNK], lo[CHUNK];
     double warp_sum[THREADS / 32];
@@ -68,7 +78,8 @@ __device__ __forceinline__ double chunk_gates(const Args& a, Gates& s, size_t to
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float A = -expf(a.a_log[head]);
     const float dt = tid < len ? softplus_f(__bfloat162float(a.proj[(tok0 + tid) * a.proj_stride + a.dt_col + head]) + a.dt_bias[head]) : 0.f;
-    double L = (double)(A * dt);
+    const float step = tid < len ? A * dt : 0.f;
+    double L = (double)(step < -200.f ? -200.f : step);          // (a NaN stays one)
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double left = __shfl_up_sync(0xffffffffu, L, o);
@@ -309,6 +320,20 @@ __global__ void __launch_bounds__(THREADS, 3) read_kernel(const Args a) {
             for (int u = 0; u < PV / 16; ++u)
                 ldmatrix_x4_trans(smem_u32(x_s + (k16 * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * XLD + u * 16 + ((lane >> 4) << 3)),
                                   xb[u][0], xb[u][1], xb[u][2], xb[u][3]);
+            // A weight of zero takes finite values away, but not infinities and NaN: in the run that a warp's tokens see only part of, those
+            // are left out of the product and meet the tokens that see them one by one.
+            uint32_t odd = 0;
+            if (s0 == start && k16 == warp) {
+#pragma unroll
+                for (int u = 0; u < PV / 16; ++u)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t m = not_finite(xb[u][q]);
+                        xb[u][q] &= ~m;
+                        odd |= m;
+                    }
+                odd = __any_sync(0xffffffffu, odd != 0);
+            }
             float sum[PV / 8][4] = {};
 #pragma unroll
             for (int part = 2; part >= 0; --part)
@@ -318,6 +343,30 @@ __global__ void __launch_bounds__(THREADS, 3) read_kernel(const Args a) {
                     mma_bf16(sum[2 * u + 1], w[part], xb[u][2], xb[u][3]);
                 }
             add<PV / 8>(o, sum);
+            if (odd) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+#pragma unroll 1
+                    for (int k = 0; k < 8; ++k) {
+                        const int row = warp * 16 + half * 8 + k, from = (lane & 28) | (k >> 1);
+                        float p_lo = 0.f, p_hi = 0.f;            // the key's weights of this lane's two tokens
+#pragma unroll
+                        for (int part = 0; part < 3; ++part) {
+                            p_lo += half_of(__shfl_sync(0xffffffffu, w[part][2 * half], from), k & 1);
+                            p_hi += half_of(__shfl_sync(0xffffffffu, w[part][2 * half + 1], from), k & 1);
+                        }
+#pragma unroll
+                        for (int j = 0; j < PV / 8; ++j) {
+                            const uint32_t pair = *reinterpret_cast<const uint32_t*>(x_s + row * XLD + j * 8 + 2 * c), m = not_finite(pair);
+#pragma unroll
+                            for (int q = 0; q < 2; ++q)
+                                if (m >> (16 * q) & 1) {
+                                    if (start + row <= t_lo) o[j][q] = fmaf(p_lo, half_of(pair, q), o[j][q]);
+                                    if (start + row <= t_hi) o[j][2 + q] = fmaf(p_hi, half_of(pair, q), o[j][2 + q]);
+                                }
+                        }
+                    }
+            }
         }
     }
     // the last turn's values are the tile's own tokens

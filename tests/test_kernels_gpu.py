@@ -986,3 +986,69 @@ def test_ssd_scan_in_chunks_on_the_tensor_cores(lens, heads, groups, pd, n_state
     # float32 sums either way: 2^-24 a product and term
     assert errs[1][0] < 2e-6 and errs[1][1] < 2e-6, errs
     assert errs[1][0] < errs[0][0] + 2e-8 and errs[1][1] < errs[0][1] + 2e-8, errs
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where,at", [("x", 3), ("x", 78), ("x", 150), ("B", 20), ("C", 21), ("dt", 37), ("state", 0)])
+def test_ssd_chunks_keep_non_finite_numbers_where_they_are(bad, where, at):
+    """A number that is not finite spoils its own column (value, state) and its own head from its token on, as it does token by
+    token: bit for bit nothing in earlier tokens, other columns, other heads or the other request."""
+    from lily_b200.csrc import ops as o
+    lens, heads, pd, n_state = [170, 40], 3, 80, 32
+    g = torch.Generator(device=DEV).manual_seed(at)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    n, inner = sum(lens), heads * pd
+    xbc, proj, state = rand(n, inner + 2 * n_state).bfloat16(), rand(n, heads).bfloat16(), rand(3, inner * n_state)
+    vec = [rand(heads), torch.tensor([-5.0, -2.0, -3.0], device=DEV), rand(heads)]
+    cu, slots = torch.tensor([0, 170, 210], device=DEV, dtype=torch.int32), torch.tensor([2, 1], device=DEV, dtype=torch.int32)
+    plan = o.scan_plan(lens, DEV, inner * n_state)
+
+    def run(xbc, proj, state):
+        state = state.clone()
+        return o.ssd_scan(xbc, proj, 0, *vec, state, cu, slots, 2, heads, pd, n_state, 1, plan=plan).view(n, heads, pd), state[1:].view(2, heads, pd, n_state)
+
+    y0, s0 = run(xbc, proj, state)
+    assert bool(y0.isfinite().all()) and bool(s0.isfinite().all())
+    xbc, proj, state = xbc.clone(), proj.clone(), state.clone()
+    same, held = torch.ones(n, heads, pd, dtype=torch.bool, device=DEV), torch.ones_like(s0, dtype=torch.bool)
+    if where == "x":
+        xbc[at, pd + 70] = bad                            # head 1, value column 70
+        same[at:170, 1, 70] = held[1, 1, 70] = False
+    elif where == "B":
+        xbc[at, inner + 5] = bad                          # state column 5 of every head
+        same[at:170], held[1, :, :, 5] = False, False
+    elif where == "C":
+        xbc[at, inner + n_state + 5] = bad
+        same[at] = False
+    elif where == "dt":
+        proj[at, 2] = bad
+        if bad == float("-inf"):                          # a step of size zero
+            assert bool(run(xbc, proj, state)[0].isfinite().all())
+            return
+        same[at:170, 2], held[1, 2] = False, False
+    else:
+        state[2].view(heads, pd, n_state)[0, 33, 7] = bad
+        same[:170, 0, 33] = held[1, 0, 33, 7] = False
+    y1, s1 = run(xbc, proj, state)
+    assert torch.equal(y1[same], y0[same]) and torch.equal(s1[held], s0[held])
+    if where != "dt":                                     # (behind an infinite step nothing of the state is left to be spoiled by)
+        assert not bool(y1[~same].isfinite().any()) and not bool(s1[~held].isfinite().any())
+    else:
+        assert not bool(y1[at, 2].isfinite().any())
+
+
+def test_ssd_chunks_where_a_decay_is_beyond_float32():
+    """exp(a_log) dt past the largest float32: the state is forgotten at every token, and what the token brings is all there is."""
+    from lily_b200.csrc import ops as o
+    n, heads, pd, n_state = 140, 2, 64, 64
+    g = torch.Generator(device=DEV).manual_seed(1)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    xbc, proj, state = rand(n, heads * pd + 2 * n_state).bfloat16(), rand(n, heads).abs().bfloat16() + 8, rand(2, heads * pd * n_state)
+    vec = [torch.zeros(heads, device=DEV), torch.tensor([88.0, 90.0], device=DEV), rand(heads)]
+    cu, slots = torch.tensor([0, n], device=DEV, dtype=torch.int32), torch.ones(1, device=DEV, dtype=torch.int32)
+    plan = o.scan_plan([n], DEV, heads * pd * n_state)
+    got = o.ssd_scan(xbc, proj, 0, *vec, state, cu, slots, 1, heads, pd, n_state, 1, plan=plan).double()
+    x, b, c = xbc.double().split([heads * pd, n_state, n_state], 1)
+    dt = torch.nn.functional.softplus(proj.double())
+    want = ((b * c).sum(1)[:, None] * dt + vec[2].double())[:, :, None] * x.view(n, heads, pd)
+    assert float((got.view_as(want) - want).norm() / want.norm()) < 2e-6
