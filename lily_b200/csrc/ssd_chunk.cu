@@ -53,12 +53,12 @@ struct Args {
 
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
-// Pairs of float32 numbers as three pairs of bfloat16 whose sum they are; infinities are their own first part.
+// Pairs of float32 numbers as three pairs of bfloat16 whose sum they are (an infinity becomes a NaN).
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     const float2 hf = __bfloat1622float2(h);
     hi = *reinterpret_cast<const uint32_t*>(&h);
-    split2(isinf(hf.x) ? 0.f : x - hf.x, isinf(hf.y) ? 0.f : y - hf.y, mid, lo);
+    split2(x - hf.x, y - hf.y, mid, lo);
 }
 
 // Which of a pair of bfloat16 numbers are infinities or NaN, as a mask over the pair's bits.
@@ -322,17 +322,19 @@ __global__ void __launch_bounds__(THREADS, 3) read_kernel(const Args a) {
                                   xb[u][0], xb[u][1], xb[u][2], xb[u][3]);
             // A weight of zero takes finite values away, but not infinities and NaN: in the run that a warp's tokens see only part of, those
             // are left out of the product and meet the tokens that see them one by one.
-            uint32_t odd = 0;
+            bool odd = false;
             if (s0 == start && k16 == warp) {
+                uint32_t any = 0;                                // an exponent of all ones leaves a half of zeros, which borrows
 #pragma unroll
                 for (int u = 0; u < PV / 16; ++u)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t m = not_finite(xb[u][q]);
-                        xb[u][q] &= ~m;
-                        odd |= m;
-                    }
-                odd = __any_sync(0xffffffffu, odd != 0);
+                    for (int q = 0; q < 4; ++q) any |= ((xb[u][q] & 0x7f807f80u) ^ 0x7f807f80u) - 0x00010001u;
+                odd = __any_sync(0xffffffffu, (any & 0x80008000u) != 0);
+                if (odd)
+#pragma unroll
+                    for (int u = 0; u < PV / 16; ++u)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) xb[u][q] &= ~not_finite(xb[u][q]);
             }
             float sum[PV / 8][4] = {};
 #pragma unroll

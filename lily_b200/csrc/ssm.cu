@@ -422,7 +422,10 @@ ssd_step_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__ p
 }
 
 // grid (ceil(elements / 256), long portions), block 256: one entry of the scan state through the chunks of a portion.  (A trip to
-// memory a chunk: 16 chunks of 64 heads of 64 x 128 took 53 us, now 12.)
+// memory a chunk took 53 us for 16 chunks of 64 heads of 64 x 128, four a trip take 13.  Eight a trip are no faster there, and the
+// registers they hold while this kernel waits are the next one's: own states, this and the outputs of 4 chunks of 16 heads of 64 x 64
+// in float32 99 us with one a trip, 113 with eight, 98 with four.)
+constexpr int AHEAD = 4;
 __global__ void ssd_combine_kernel(float* __restrict__ state, size_t state_stride, const int* __restrict__ slots,
                                    float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
                                    const int* __restrict__ long_req, const int* __restrict__ long_first,
@@ -435,16 +438,16 @@ __global__ void ssd_combine_kernel(float* __restrict__ state, size_t state_strid
     float* st = state + (size_t)slots[long_req[k]] * state_stride + e;
     float S = *st;
     const int first = long_first[k], count = long_count[k];
-    for (int c0 = 0; c0 < count; c0 += 8) {                // eight chunks' numbers asked for before the first is used
-        float own[8], decay[8];
+    for (int c0 = 0; c0 < count; c0 += AHEAD) {                // so many chunks' numbers asked for before the first is used
+        float own[AHEAD], decay[AHEAD];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < AHEAD; ++j) {
             const bool in = c0 + j < count;
             own[j] = in ? chunk_state[(size_t)(first + c0 + j) * elements + e] : 0.f;
             decay[j] = in ? chunk_decay[(size_t)(first + c0 + j) * heads + h] : 1.f;
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < AHEAD; ++j) {
             if (c0 + j < count) {
                 chunk_state[(size_t)(first + c0 + j) * elements + e] = S;
                 S = fmaf(decay[j], S, own[j]);
