@@ -32,13 +32,11 @@
 
 namespace lily {
 
-constexpr int ROWS = 32;      // query rows per block
+constexpr int MOST_ROWS = 32; // query rows per block
 constexpr int KEYS = 32;      // keys per tile (one per lane)
 constexpr int WARPS = 4;
-constexpr int RPW = ROWS / WARPS;
 
 template <int N> struct Count { static constexpr int value = N; };
-
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool in) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(dst);
@@ -50,10 +48,14 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool in) {
 // while this one is worked on, the pages of a tile's keys are looked up by the lanes at once, and scores and sums read four
 // numbers at a time; the sums keep their order.  Otherwise (bfloat16 is converted on the way) a tile is fetched element by
 // element when the one before is done.  Where few query heads share a kv head (decode) a warp has one row and does the work of
-// one.  Three rows of up to 250 keys, 16 heads of 128 over 4: 133 -> 44 us; 451 new tokens of three prompts: 127 -> 94 us.
-template <typename T, int DCH, bool DECODE, bool WIDE>
+// one: in a kernel of its own (LIVE 1) where elements come one by one, since a body for eight rows beside it takes the registers of
+// eight (8 requests of 250 keys, 16 heads of 80 over 4, bfloat16: 130 us with eight row slots, 93 with both bodies, 72 alone; eight heads a
+// kv head of 40: 87, 92 and 77), as a second body where the tiles come wide.
+// Three rows of up to 250 keys, 16 heads of 128 over 4, float32: 133 -> 44 us; 451 new tokens of three prompts: 127 -> 94 us.
+template <typename T, int DCH, bool DECODE, bool WIDE, int LIVE>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const AttnArgs a, const int bufs) {
+    constexpr int RPW = LIVE, ROWS = WARPS * LIVE;
     extern __shared__ __align__(16) float smem[];
     const int d = a.d, dv = a.v_all ? a.nkv * a.dv : a.dv;      // dv: the value columns a query row gathers
     const int krow = WIDE ? d + 4 : d + 1;     // lanes read a column of keys without bank conflicts (four columns where WIDE)
@@ -147,47 +149,59 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
     auto load_tile = [&](int ub, int buf) {
         float* Ks = Kt + buf * tile_floats;
         float* Vs = Ks + KEYS * krow;
-        // lane j looks key ub + j up
-        const int mine = ub + lane, mpos = mine < nkeep ? mine : klo + (mine - nkeep);
-        const int mpage = mine < uend ? table[mpos / a.page_size] : 0, mrow = mine < uend ? mpos % a.page_size : 0;
+        if constexpr (WIDE) {
+            // lane j looks key ub + j up
+            const int mine = ub + lane, mpos = mine < nkeep ? mine : klo + (mine - nkeep);
+            const int mpage = mine < uend ? table[mpos / a.page_size] : 0, mrow = mine < uend ? mpos % a.page_size : 0;
 #pragma unroll 4
-        for (int j = warp; j < KEYS; j += WARPS) {
-            const bool in = ub + j < uend;
-            const int row = __shfl_sync(0xffffffffu, mrow, j);
-            const T* base = kv + (size_t)__shfl_sync(0xffffffffu, mpage, j) * page_stride;
-            const T* ksrc = base + (size_t)kvh * khead + (size_t)row * d;
-            const T* vsrc = base + (size_t)a.nkv * khead + (size_t)(a.v_all ? 0 : (kvh + a.v_shift) % a.nkv) * vhead + (size_t)row * dv1;
-            if constexpr (WIDE) {
+            for (int j = warp; j < KEYS; j += WARPS) {
+                const bool in = ub + j < uend;
+                const int row = __shfl_sync(0xffffffffu, mrow, j);
+                const T* base = kv + (size_t)__shfl_sync(0xffffffffu, mpage, j) * page_stride;
+                const T* ksrc = base + (size_t)kvh * khead + (size_t)row * d;
+                const T* vsrc = base + (size_t)a.nkv * khead + (size_t)(a.v_all ? 0 : (kvh + a.v_shift) % a.nkv) * vhead + (size_t)row * dv1;
                 for (int c = lane * 4; c < d; c += 128) copy16(Ks + j * krow + c, ksrc + c, in);
                 if (a.v_all)
                     for (int c = lane * 4; c < dv; c += 128) copy16(Vs + j * dv + c, vsrc + (size_t)(c / dv1) * vhead + c % dv1, in);
                 else if (!a.v_in_k)
                     for (int c = lane * 4; c < dv; c += 128) copy16(Vs + j * dv + c, vsrc + c, in);
-            } else {
-                for (int c = lane; c < d; c += 32) Ks[j * krow + c] = in ? to_float(ksrc[c]) : 0.f;
-                if (a.v_all)
-                    for (int c = lane; c < dv; c += 32) Vs[j * dv + c] = in ? to_float(vsrc[(size_t)(c / dv1) * vhead + c % dv1]) : 0.f;
-                else if (!a.v_in_k)
-                    for (int c = lane; c < dv; c += 32) Vs[j * dv + c] = in ? to_float(vsrc[c]) : 0.f;
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        } else {
+            for (int j = warp; j < KEYS; j += WARPS) {
+                const int u = ub + j, kpos = u < nkeep ? u : klo + (u - nkeep);
+                if (u < uend) {
+                    const T* base = kv + (size_t)table[kpos / a.page_size] * page_stride;
+                    const T* ksrc = base + (size_t)kvh * khead + (size_t)(kpos % a.page_size) * d;
+                    const T* vsrc = base + (size_t)a.nkv * khead + (size_t)(a.v_all ? 0 : (kvh + a.v_shift) % a.nkv) * vhead + (size_t)(kpos % a.page_size) * dv1;
+                    for (int c = lane; c < d; c += 32) Ks[j * krow + c] = to_float(ksrc[c]);
+                    if (a.v_all)
+                        for (int c = lane; c < dv; c += 32) Vs[j * dv + c] = to_float(vsrc[(size_t)(c / dv1) * vhead + c % dv1]);
+                    else if (!a.v_in_k)
+                        for (int c = lane; c < dv; c += 32) Vs[j * dv + c] = to_float(vsrc[c]);
+                } else {
+                    for (int c = lane; c < d; c += 32) Ks[j * krow + c] = 0.f;
+                    if (!a.v_in_k)
+                        for (int c = lane; c < dv; c += 32) Vs[j * dv + c] = 0.f;
+                }
             }
         }
-        if constexpr (WIDE) asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    // one tile for the first LIVE row slots of every warp
-    auto work = [&](int ub, const float* Ks, const float* Vp, auto live) {
-        constexpr int LIVE = decltype(live)::value;
+    // one tile for the first SLOTS row slots of every warp
+    auto work = [&](int ub, const float* Ks, const float* Vp, auto slots) {
+        constexpr int SLOTS = decltype(slots)::value;
         // scores: lane j holds key ub + j for each of the warp's rows
-        float s[LIVE];
+        float s[SLOTS];
 #pragma unroll
-        for (int i = 0; i < LIVE; ++i) s[i] = 0.f;
+        for (int i = 0; i < SLOTS; ++i) s[i] = 0.f;
         const float* kmine = Ks + lane * krow;
         if constexpr (WIDE) {
 #pragma unroll 4
             for (int c = 0; c < d; c += 4) {
                 const float4 k4 = *reinterpret_cast<const float4*>(kmine + c);
 #pragma unroll
-                for (int i = 0; i < LIVE; ++i) {
+                for (int i = 0; i < SLOTS; ++i) {
                     const int r = DECODE ? i * WARPS + warp : warp * RPW + i;
                     const float4 q4 = *reinterpret_cast<const float4*>(Qs + r * d + c);
                     s[i] = fmaf(q4.w, k4.w, fmaf(q4.z, k4.z, fmaf(q4.y, k4.y, fmaf(q4.x, k4.x, s[i]))));
@@ -197,7 +211,7 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
             for (int c = 0; c < d; ++c) {
                 const float kval = kmine[c];
 #pragma unroll
-                for (int i = 0; i < LIVE; ++i) {
+                for (int i = 0; i < SLOTS; ++i) {
                     const int r = DECODE ? i * WARPS + warp : warp * RPW + i;
                     s[i] = fmaf(Qs[r * d + c], kval, s[i]);
                 }
@@ -206,7 +220,7 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
         const int u = ub + lane;
         const int kpos = u < nkeep ? u : klo + (u - nkeep);
 #pragma unroll
-        for (int i = 0; i < LIVE; ++i) {
+        for (int i = 0; i < SLOTS; ++i) {
             const bool seen = row_ok[i] && u < uend && kpos <= row_pos[i] &&
                               (a.window <= 0 || kpos > row_pos[i] - a.window || kpos < a.keep_first);
             const float sv = seen ? (cap > 0.f ? cap * tanhf(s[i] * cap_in) : s[i] * a.scale) : -INFINITY;
@@ -224,7 +238,7 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
         }
         __syncwarp();
         // p.v: lane owns output columns lane, lane + 32, ...
-        constexpr int JV = DCH <= 8 ? 4 : 1;            // keys at a time: more would not fit the registers of wide rows
+        constexpr int JV = (WIDE || LIVE == 1) && DCH <= 8 ? 4 : 1;     // keys at a time: more would not fit the registers
         for (int j = 0; j < KEYS; j += JV) {
             float v[JV][DCH];
 #pragma unroll
@@ -235,7 +249,7 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
                     v[k][c] = col < dv ? Vp[(j + k) * vrow + col] : 0.f;
                 }
 #pragma unroll
-            for (int i = 0; i < LIVE; ++i) {
+            for (int i = 0; i < SLOTS; ++i) {
                 const float* pi = Ps + (warp * RPW + i) * KEYS + j;
                 float p[JV];
                 if constexpr (JV == 4) {
@@ -266,8 +280,8 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
         }
         const float* Ks = Kt + buf * tile_floats;
         const float* Vp = a.v_in_k ? Ks : Ks + KEYS * krow;
-        if (DECODE && nrows <= WARPS) work(ub, Ks, Vp, Count<1>{});        // few query heads share a kv head: a row a warp
-        else work(ub, Ks, Vp, Count<RPW>{});
+        if (WIDE && DECODE && nrows <= WARPS) work(ub, Ks, Vp, Count<1>{});
+        else work(ub, Ks, Vp, Count<LIVE>{});
         if (WIDE && bufs == 1 && ub + KEYS < uend) {
             __syncthreads();
             load_tile(ub + KEYS, 0);
@@ -388,21 +402,21 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     }
 }
 
-static size_t smem_bytes(int d, int dv, int v_in_k, bool wide, int bufs) {
-    return sizeof(float) * ((size_t)ROWS * d + ROWS * KEYS + (size_t)bufs * (KEYS * (d + (wide ? 4 : 1)) + (v_in_k ? 0 : KEYS * dv)));
+static size_t smem_bytes(int rows, int d, int dv, int v_in_k, bool wide, int bufs) {
+    return sizeof(float) * ((size_t)rows * d + rows * KEYS + (size_t)bufs * (KEYS * (d + (wide ? 4 : 1)) + (v_in_k ? 0 : KEYS * dv)));
 }
 
 constexpr size_t SMEM_MOST = 227 * 1024;
 
-template <typename T, bool DECODE, bool WIDE>
+template <typename T, bool DECODE, bool WIDE, int LIVE>
 static int launch(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
     const int dvo = a.v_all ? a.nkv * a.dv : a.dv;
     const int dch = (dvo + 31) / 32;               // output columns a lane owns
-    const int bufs = WIDE && smem_bytes(a.d, dvo, a.v_in_k, WIDE, 2) <= SMEM_MOST ? 2 : 1;
-    const size_t smem = smem_bytes(a.d, dvo, a.v_in_k, WIDE, bufs);
+    const int bufs = WIDE && smem_bytes(WARPS * LIVE, a.d, dvo, a.v_in_k, WIDE, 2) <= SMEM_MOST ? 2 : 1;
+    const size_t smem = smem_bytes(WARPS * LIVE, a.d, dvo, a.v_in_k, WIDE, bufs);
 #define CASE(N)                                                                                          \
     case N: {                                                                                            \
-        auto kern = attention_simt_kernel<T, N, DECODE, WIDE>;                                               \
+        auto kern = attention_simt_kernel<T, N, DECODE, WIDE, LIVE>;                                         \
         static size_t granted = 48 * 1024;      /* set once per size, never while a graph is captured */  \
         if (smem > granted) {                                                                            \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -426,9 +440,14 @@ static int launch(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
 // 16 bytes, given that the cache does).
 template <bool DECODE>
 static int launch_typed(const AttnArgs& a, int dtype, dim3 grid, cudaStream_t stream) {
-    if (dtype == kBF16) return launch<__nv_bfloat16, DECODE, false>(a, grid, stream);
-    if (((a.d | a.dv) & 3) == 0 && ((uintptr_t)a.kv & 15) == 0) return launch<float, DECODE, true>(a, grid, stream);
-    return launch<float, DECODE, false>(a, grid, stream);
+    constexpr int ALL = MOST_ROWS / WARPS;
+    if (dtype == kF32 && ((a.d | a.dv) & 3) == 0 && ((uintptr_t)a.kv & 15) == 0) return launch<float, DECODE, true, ALL>(a, grid, stream);
+    if (DECODE && a.nq / a.nkv <= WARPS) {
+        if (dtype == kBF16) return launch<__nv_bfloat16, DECODE, false, DECODE ? 1 : ALL>(a, grid, stream);
+        return launch<float, DECODE, false, DECODE ? 1 : ALL>(a, grid, stream);
+    }
+    if (dtype == kBF16) return launch<__nv_bfloat16, DECODE, false, ALL>(a, grid, stream);
+    return launch<float, DECODE, false, ALL>(a, grid, stream);
 }
 
 static int check_common(const char* name, int nq, int nkv, int d, int page_size, int dv) {
@@ -499,7 +518,7 @@ LILY_API int lily_attention_combine(const float* scratch, void* out, int request
 }
 
 // Rows of a prefill tile: the host cuts each request's new tokens into tiles of this many.
-LILY_API int lily_attention_prefill_simt_rows() { return ROWS; }
+LILY_API int lily_attention_prefill_simt_rows() { return MOST_ROWS; }
 
 LILY_API size_t lily_attention_decode_scratch_floats(int requests, int nq, int d, int splits) {
     return splits > 1 ? (size_t)requests * nq * splits * (d + 2) : 0;
@@ -517,7 +536,7 @@ LILY_API int lily_attention_decode_simt(const void* q, const void* kv, void* out
     const int d_out = (flags & kAllValues) ? nkv * d_one : d_one;
     LILY_REQUIRE(splits >= 1 && splits <= 65535, "attention_decode: %d splits", splits);
     LILY_REQUIRE(splits == 1 || scratch != nullptr, "attention_decode: splits need scratch");
-    const int group = nq / nkv, chunks = (group + ROWS - 1) / ROWS;
+    const int group = nq / nkv, chunks = (group + MOST_ROWS - 1) / MOST_ROWS;
     AttnArgs a{};
     a.q = q; a.kv = kv; a.out = out; a.block_table = block_table; a.bt_stride = bt_stride;
     a.seq_lens = seq_lens; a.splits = splits; a.nq = nq; a.nkv = nkv; a.d = d; a.page_size = page_size;
