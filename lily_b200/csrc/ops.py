@@ -1220,8 +1220,7 @@ def causal_conv(proj: torch.Tensor, col0: int, channels: int, weight: torch.Tens
 SCAN_CHUNK = 128        # tokens a chunk of a long portion (doubled while the chunk states would pass SCAN_WORKSPACE)
 SCAN_DIRECT = 192       # portions up to this many tokens run in one piece, from and to the state in the slot
 SCAN_WORKSPACE = 1 << 29
-SCAN_FINE = 17          # tokens from which a portion is worth the tensor-core kernels' chunks (a token by itself takes about a
-                        # microsecond of a block, three launches and a padded tile 30)
+SCAN_FINE = 17          # tokens from which a portion can go to the tensor-core kernels' chunks
 
 
 @dataclass
@@ -1246,11 +1245,31 @@ class ScanPlan:
 _SSD_CHUNKS = os.environ.get("LILY_B200_SSD_CHUNKS", "") != "scan"       # "scan": chunks run token by token
 
 
-def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0) -> ScanPlan:
+def scan_chunks_pay(new_lens: Sequence[int], heads: int) -> bool:
+    """Whether the portions of SCAN_FINE tokens and more are faster as chunks of the tensor-core kernels than one token after
+    another in one piece each.  A token takes about 1.05 us of its block, and 0.0033 us a head once all blocks are busy; the chunks'
+    three launches take 20 us, 5 more where other rows need a fourth, and a chunk of up to 64 tokens 0.094 us a head.  Where a portion is
+    long enough to be cut anyway the others go with it.  Measured, us, in pieces / in chunks, 64 heads of 64 x 128: one portion of 17 tokens
+    21 / 26, of 24 28 / 26, of 64 67 / 27; eight of 17 32 / 65, of 32 50 / 65, of 48 71 / 66; 33 and 391 tokens 82 with the 33 in
+    one piece, 47 without."""
+    portions = [n for n in new_lens if n >= SCAN_FINE]
+    if not portions or max(portions) > SCAN_DIRECT:
+        return bool(portions)
+    pieces = max(1.05 * max(portions) + 4.0, 0.0033 * heads * sum(portions))
+    return pieces > 20.0 + 0.094 * heads * len(portions) + (5.0 if len(portions) < len(new_lens) else 0.0)
+
+
+def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0, chunks=True) -> ScanPlan:
     """Cuts the step's portions for the scan.  A portion of up to SCAN_DIRECT tokens (every decoded token) runs in one
     piece; a longer one in chunks of SCAN_CHUNK tokens that run side by side and are joined by ``ssd_combine``
-    (``state_floats``: the size of one scan state, which bounds how many chunks the workspace may hold).  Where the
-    tensor-core kernels could take chunks, ``fine`` is the cut for them: chunks from SCAN_FINE tokens on."""
+    (``state_floats``: the size of one scan state, which bounds how many chunks the workspace may hold).  ``fine`` is the cut for
+    the tensor-core kernels, chunks from SCAN_FINE tokens on, or None: ``chunks`` False leaves it out, and (dtype, heads, head
+    size, state, channels) makes it for a scan of those sizes, where its kernels take them and ``scan_chunks_pay``."""
+    if isinstance(chunks, tuple):
+        dtype, heads, head_dim, n_state, channels = chunks
+        chunks = (_SSD_CHUNKS and dtype == torch.bfloat16 and scan_chunks_pay(new_lens, heads)
+                  and bool(library().lily_ssd_chunk_takes(None, channels, heads, head_dim, n_state, SCAN_CHUNK)))
+
     def cut(direct_most, chunk):
         longs = [r for r, n in enumerate(new_lens) if n > direct_most]
         direct = [r for r, n in enumerate(new_lens) if n <= direct_most]
@@ -1268,7 +1287,7 @@ def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0) -> ScanPla
     while chunk < 1024 and state_floats and sum(-(-n // chunk) for n in new_lens if n > SCAN_DIRECT) * state_floats * 4 > SCAN_WORKSPACE:
         chunk *= 2
     cuts = [cut(SCAN_DIRECT, chunk)] if max(new_lens, default=0) > SCAN_DIRECT else []
-    if (max(new_lens, default=0) >= SCAN_FINE and chunk == SCAN_CHUNK
+    if (chunks and max(new_lens, default=0) >= SCAN_FINE and chunk == SCAN_CHUNK
             and sum(-(-n // chunk) for n in new_lens if n >= SCAN_FINE) * max(state_floats, 1) * 4 <= SCAN_WORKSPACE):
         cuts.append(cut(SCAN_FINE - 1, chunk))
     if not cuts:

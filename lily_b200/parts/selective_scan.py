@@ -113,7 +113,7 @@ class SelectiveScan(Mixer):
         step = ops.linear(low, self.w_dt, self.dt_bias, out_dtype=torch.float32)
         # long portions run as chunks side by side; the cut is planned once a step for layers of one state size
         plan = batch.plan(("scan_plan", self.scan_floats),
-                          lambda b: ops.scan_plan(b.h_new_lens, b.token_ids.device, self.scan_floats))
+                          lambda b: ops.scan_plan(b.h_new_lens, b.token_ids.device, self.scan_floats, chunks=False))
         need = ops.selective_workspace_floats(plan, s.inner, s.state)
         room = batch.workspace.floats("selective_chunks", need) if need and batch.workspace is not None else None
         if need and room is None:

@@ -1052,3 +1052,19 @@ def test_ssd_chunks_where_a_decay_is_beyond_float32():
     dt = torch.nn.functional.softplus(proj.double())
     want = ((b * c).sum(1)[:, None] * dt + vec[2].double())[:, :, None] * x.view(n, heads, pd)
     assert float((got.view_as(want) - want).norm() / want.norm()) < 2e-6
+
+
+def test_scan_plan_cuts_only_for_who_runs_it():
+    """No tensor-core cut, lists on the device or workspace for a scan that will not use them: float32, sizes the kernels refuse, the selective
+    scan, portions that are faster in one piece."""
+    o = ops()
+    floats, bf = 64 * 64 * 128, (torch.bfloat16, 64, 64, 128, 64 * 64 + 16 * 128)
+    for chunks in (False, (torch.float32,) + bf[1:], (torch.bfloat16, 64, 64, 136, 64 * 64 + 16 * 136)):
+        plan = o.scan_plan([190] * 64, DEV, floats, chunks=chunks)
+        assert plan.fine is None and plan.direct is None and o.scan_workspace_floats(plan, 64, 64, 128) == 0
+        plan = o.scan_plan([300] + [100] * 40, DEV, floats, chunks=chunks)
+        assert plan.fine is None and plan.num_chunks == 3 and o.scan_workspace_floats(plan, 64, 64, 128) == 3 * (floats + 64)
+    for lens, want in (([17], 0), ([24], 1), ([17] * 8, 0), ([32] * 8, 0), ([64] * 8, 8), ([1] * 16 + [17], 0), ([1] * 16 + [40], 1), ([33, 391], 5)):
+        plan = o.scan_plan(lens, DEV, floats, chunks=bf)
+        assert (plan.fine.num_chunks if plan.fine else 0) == want, lens
+        assert o.scan_workspace_floats(plan, 64, 64, 128) == want * (floats + 64)
