@@ -85,18 +85,20 @@ __global__ void token_shift_mix_kernel(const T* __restrict__ h, int tokens, int 
 // grid (ceil(tokens / 8), ceil(cols / 128)), block 128; a [tokens, rank] float32, w2t [rank, cols] float32 (the second
 // matrix of the low-rank pair, transposed so that neighbouring threads read neighbouring numbers), w0 [cols].  A block
 // takes eight tokens, so a number of w2t read once serves eight sums.
-// The loop over the rank waits for memory once for every DECAY_AHEAD rows of w2t; the first ones are asked for before the kernel
-// ahead has finished (they are weights).  Rank 64, 2,048 columns, 36 steps of 2 tokens and 3 of 1,920: 24.4 us on average with the
-// compiler's own four at a time, 11.7 now.
-constexpr int DECAY_TOKENS = 8, DECAY_AHEAD = 32;
+// With few blocks the loop over the rank waits for memory: AHEAD rows of w2t are asked for at once, the first before the kernel ahead has
+// finished (they are weights): rank 64, 2,048 columns, a row at a time / 32: 8.6 / 6.7 us with 1 token, 9.7 / 7.7 with 64.  With more
+// blocks than two a SM others run meanwhile, and the registers of 32 rows are in the way, so AHEAD is 0, a row at a time: 2,048 tokens
+// 52 us with 32, 35 so; 64 tokens, rank 256, 8,192 columns, 512 blocks, 49 and 32.
+constexpr int DECAY_TOKENS = 8;
+template <int AHEAD>
 __global__ void wkv_decay_kernel(const float* __restrict__ a, int tokens, int rank, const float* __restrict__ w2t,
                                  const float* __restrict__ w0, int cols, float* __restrict__ lw) {
     extern __shared__ float th[];          // [8][rank]: tanh(a[t, :])
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    float w[DECAY_AHEAD];
+    float w[AHEAD > 0 ? AHEAD : 1];
     auto ask = [&](int j0) {
 #pragma unroll
-        for (int j = 0; j < DECAY_AHEAD; ++j) w[j] = c < cols && j0 + j < rank ? w2t[(size_t)(j0 + j) * cols + c] : 0.f;
+        for (int j = 0; j < AHEAD; ++j) w[j] = c < cols && j0 + j < rank ? w2t[(size_t)(j0 + j) * cols + c] : 0.f;
     };
     ask(0);
     const float b = c < cols ? w0[c] : 0.f;
@@ -109,15 +111,23 @@ __global__ void wkv_decay_kernel(const float* __restrict__ a, int tokens, int ra
     float z[DECAY_TOKENS];
 #pragma unroll
     for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = 0.f;
-    for (int j0 = 0; j0 < rank; j0 += DECAY_AHEAD) {
-        const int now = min(DECAY_AHEAD, rank - j0);
+    if constexpr (AHEAD == 0) {
+        for (int j = 0; j < rank; ++j) {
+            const float one = w2t[(size_t)j * cols + c];
 #pragma unroll
-        for (int j = 0; j < DECAY_AHEAD; ++j)
-            if (j < now) {
+            for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = fmaf(th[t * rank + j], one, z[t]);
+        }
+    } else {
+        for (int j0 = 0; j0 < rank; j0 += AHEAD) {
+            const int now = min(AHEAD, rank - j0);
 #pragma unroll
-                for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = fmaf(th[t * rank + j0 + j], w[j], z[t]);
-            }
-        if (j0 + DECAY_AHEAD < rank) ask(j0 + DECAY_AHEAD);
+            for (int j = 0; j < AHEAD; ++j)
+                if (j < now) {
+#pragma unroll
+                    for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = fmaf(th[t * rank + j0 + j], w[j], z[t]);
+                }
+            if (j0 + AHEAD < rank) ask(j0 + AHEAD);
+        }
     }
 #pragma unroll
     for (int t = 0; t < DECAY_TOKENS; ++t)
@@ -461,7 +471,8 @@ LILY_API int lily_wkv_decay(const float* a, int tokens, int rank, const float* w
     LILY_REQUIRE(rank > 0 && cols > 0, "wkv_decay: rank=%d cols=%d", rank, cols);
     dim3 grid((tokens + DECAY_TOKENS - 1) / DECAY_TOKENS, (cols + 127) / 128), block(128);
     LILY_REQUIRE(grid.y <= 65535 && rank <= 1024, "wkv_decay: %d columns, rank %d", cols, rank);
-    launch_pdl(wkv_decay_kernel, grid, block, (size_t)DECAY_TOKENS * rank * sizeof(float), stream, a, tokens, rank, w2t, w0, cols, lw);
+    auto kern = (long long)grid.x * grid.y <= 2 * sm_count() ? wkv_decay_kernel<32> : wkv_decay_kernel<0>;
+    launch_pdl(kern, grid, block, (size_t)DECAY_TOKENS * rank * sizeof(float), stream, a, tokens, rank, w2t, w0, cols, lw);
     LILY_CHECK_LAUNCH("wkv_decay");
     return 0;
 }
