@@ -815,7 +815,7 @@ def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, acti
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("requests,heads,groups,pd,n_state", [
     (1, 2, 1, 64, 128), (9, 64, 8, 64, 128), (3, 6, 3, 24, 64), (2, 4, 2, 7, 20), (5, 8, 1, 33, 256), (2, 2, 2, 16, 300), (300, 2, 1, 80, 512),
-    (4, 3, 1, 5, 17)])
+    (4, 3, 1, 5, 17), (3, 2, 1, 9, 64), (3, 2, 1, 9, 68), (300, 4, 2, 70, 132), (2, 3, 1, 40, 260)])
 def test_ssd_scan_of_one_token_a_request(dtype, requests, heads, groups, pd, n_state):
     """A decode step's scan: rows of a head that no warp fills, states of one to four pieces a lane, many and few requests; a state
     that is no multiple of four takes the general kernel."""
