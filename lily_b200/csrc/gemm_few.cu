@@ -180,9 +180,24 @@ static int launch(int grid, const void* x, const void* w, const void* bias, int 
 
 using namespace lily;
 
-// Whether the kernel takes the product; up to 16 tokens it is ahead of the library's at every size measured (above).
+// Whether the kernel takes the product.
 LILY_API int lily_gemm_few_takes(int M, int N, int K) {
     return M >= 1 && M <= 16 && N >= 1 && K >= fewrows::KT && K % fewrows::KT == 0;
+}
+
+// Whether it is the faster way to the product than the library's.  A block has a tile's whole k to itself, so it falls behind where a
+// very long k meets too few tiles for the SMs, where a second turn of tiles leaves most blocks idle, and, beyond 8 tokens, whose
+// stages are three, where it is not ahead of the memory any more.  Library / here, timed over N from 16 to 128,256 and K from 512 to
+// 28,672:
+//   up to 8 tokens   1.05 to 3.5 but for K 28,672 with N up to 256 (0.85 to 0.94) and N 5,120 (320 tiles for 296 blocks) from K
+//                    9,728 on (0.89 to 0.97)
+//   9 to 16, tiles for one turn   1.0 to 2.7 up to K 18,944; beyond that 0.56 to 0.99 up to N 2,560, 0.97 to 1.2 from 3,072 on
+//   9 to 16, more tiles           0.99 to 1.7 up to K 4,096 (0.76 at K 512, 0.95 at 1,024 with N 128,256); beyond it 0.76 to 1.1
+LILY_API int lily_gemm_few_pays(int M, int N, int K) {
+    const int tiles = (N + fewrows::ROWS - 1) / fewrows::ROWS, slots = 2 * sm_count(), turns = (tiles + slots - 1) / slots;
+    if (M <= 8) return turns == 1 ? K <= 25600 || tiles >= 32 : K <= 8192 || 10ll * tiles >= 6ll * turns * slots;
+    if (turns == 1) return K <= 18944 || tiles >= 192;
+    return K <= 4096 && (turns <= 4 || K >= 2048);
 }
 
 LILY_API int lily_gemm_few(const void* x, const void* w, const void* bias, int bias_f32, void* out, int out_f32, int M, int N, int K,

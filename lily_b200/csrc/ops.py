@@ -151,6 +151,8 @@ def library():
         lib.lily_ssd_chunk_takes.restype = _i
         lib.lily_gemm_few_takes.argtypes = [_i, _i, _i]
         lib.lily_gemm_few_takes.restype = _i
+        lib.lily_gemm_few_pays.argtypes = [_i, _i, _i]
+        lib.lily_gemm_few_pays.restype = _i
         lib.lily_swiglu_few_verdict.argtypes = [_i, _i, _i, _i]
         lib.lily_swiglu_few_verdict.restype = _i
         lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
@@ -458,19 +460,20 @@ _FEW_ROWS = os.environ.get("LILY_B200_GEMM_FEW", "1") != "0"
 
 def few_rows_take(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether a product of a few tokens goes to the kernel that streams the weights and finishes its rows."""
-    m, k = x.shape
-    return (_FEW_ROWS and m <= 16 and x.dtype == weight.dtype == torch.bfloat16 and bool(library().lily_gemm_few_takes(m, weight.shape[0], k))
-            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
+    (m, k), n = x.shape, weight.shape[0]
+    return (_FEW_ROWS and m <= 16 and x.dtype == weight.dtype == torch.bfloat16 and bool(library().lily_gemm_few_takes(m, n, k))
+            and bool(library().lily_gemm_few_pays(m, n, k)) and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
 def few_rows_whole_pays(m: int, n: int, k: int) -> bool:
     """Whether finished float32 rows are the faster way to a product that its consumer would also add up from slices of k:
     while the 16-row tiles fit the device in one turn (two blocks a SM; a second, partly filled turn costs more than
-    the slices' sums) and a block's share of k is short or there are blocks for every SM.  Measured with the norm that adds
+    the slices' sums) and a block's share of k is short or there are blocks enough for every SM.  Measured with the norm that adds
     the slices up, us, slices / whole: 2,048 x 2,048 4.2 / 3.4 with 2 tokens, 5.4 / 3.5 with 8; 4,096 x 4,096 8.0 / 7.2; 4,096 x 12,288
-    19.0 / 17.7; 2,048 x 8,192 8.1 / 8.5 with 1, 8.6 / 10.3 with 12; 6,144 x 4,096 9.6 / 10.6."""
+    19.0 / 17.7; 2,048 x 8,192 8.1 / 8.5 with 1, 8.6 / 10.3 with 12; 6,144 x 4,096 9.6 / 10.6.  Slices over whole beyond K 4,096: N 2,560
+    (1.08 tiles a SM) 0.93 to 1.06, 3,072 (1.3) 0.98 to 1.1."""
     tiles = -(-n // 16)
-    return tiles <= 2 * sm_count() and (k <= 4096 or tiles > sm_count())
+    return tiles <= 2 * sm_count() and (k <= 4096 or 4 * tiles >= 5 * sm_count())
 
 
 TC_MIN_ROWS = 65          # products of more rows than this go to the tcgen05 kernel when it takes the shape

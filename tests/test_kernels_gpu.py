@@ -879,6 +879,20 @@ def test_linear_of_a_few_rows(m, n, k):
     assert torch.equal(ops().linear(x[-1:].contiguous(), w), ops().linear(x, w)[-1:])
 
 
+@pytest.mark.parametrize("m,n,k,here", [
+    (8, 32, 25600, True), (8, 32, 25664, False), (8, 512, 25664, True), (8, 5120, 8192, True), (8, 5120, 8256, False), (9, 1024, 18944, True),
+    (9, 1024, 19008, False), (9, 3072, 19008, True), (16, 5120, 4096, True), (16, 5120, 4160, False), (16, 40000, 2048, True), (16, 40000, 1984, False)])
+def test_linear_of_a_few_rows_on_both_sides_of_its_line(m, n, k, here):
+    """Where the kernel for few rows hands over to the library (with 148 SMs): the same numbers either way."""
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    x, w = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((m, k), (n, k)))
+    assert ops().few_rows_take(x, w) == here or ops().sm_count() != 148
+    want = x.double() @ w.double().t()
+    # the tensor cores cut off what they add to an accumulator: k / 16 additions of 2^-23 of at most the largest sum
+    assert float((ops().linear(x, w, out_dtype=torch.float32) - want).abs().max()) < k / 16 * 2 ** -23 * float(want.abs().max())
+    assert float((ops().linear(x, w) - want).abs().max()) < 2 ** -8 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float64])
 @pytest.mark.parametrize("m", [1, 9, 16, 17])
 def test_linear_takes_a_bias_of_any_float_type(m, dtype):
@@ -908,8 +922,17 @@ def test_gate_up_of_a_few_rows(activation, m, inter, k, run):
 
 
 def test_linear_split_in_one_plane():
-    """Where finished rows are the faster way the product comes as one float32 plane, the same numbers as its slices added up."""
+    """Where finished rows are the faster way the product comes as one float32 plane, the same numbers as its slices added up; at the
+    edges of that rule (1.25 tiles a SM and two, K 4,096) it comes in slices on the other side."""
     g = torch.Generator(device=DEV).manual_seed(0)
+    o, sms = ops(), ops().sm_count()
+    for n, k, whole in ((20 * sms, 4160, True), (20 * sms - 16, 4160, False), (20 * sms - 16, 4096, True), (32 * sms, 512, True), (32 * sms + 1, 512, False)):
+        assert o.few_rows_whole_pays(2, n, k) == whole
+        x, w = torch.randn(2, k, device=DEV, generator=g).bfloat16(), torch.randn(n, k, device=DEV, generator=g).bfloat16()
+        parts = o.linear_split(x, w)
+        assert (parts is not None and parts.shape[0] == 1) == whole or o.library().lily_skinny_gemm_splits(2, n, k) <= 1
+        if parts is not None:
+            assert float((parts.sum(0) - x.double() @ w.double().t()).abs().max()) < 4e-6 * (k ** 0.5) * 4
     for m, n, k in ((2, 2048, 2048), (16, 4096, 12288), (8, 24, 64)):
         x, w = torch.randn(m, k, device=DEV, generator=g).bfloat16(), torch.randn(n, k, device=DEV, generator=g).bfloat16()
         one = ops().linear_split(x, w)
