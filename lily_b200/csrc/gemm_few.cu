@@ -6,19 +6,19 @@
 // by cp.async in a ring of the warp's own, the tokens' [8 or 16][64 k] beside them, ldmatrix and mma.sync m16n8k16 (weight rows on
 // the 16-row side, tokens on the 8-column side); the eighths meet in shared memory.  Two blocks a SM walk the tiles as one pipeline
 // each, up to 96 KB in flight a SM, and the first stages of w, which depends on no one, are asked for before the kernel ahead has
-// finished: a 2,048 x 2,048 product has all of its weights on the way by then.
+// finished (three of the four tiles of k that a warp has at K 2,048).
 // A token's sums run in the same order whatever else is in the step.  With the gate/up product's activation (GATED) the tile's two
 // halves are the gate and the up rows of 8 outputs.
 //
-// Against the library's product in a chain of norms and products, us (w at the copy rate): N x K 64 x 2,048 5.1 -> 2.0; 2,048 x
+// What the product adds to a chain of norms and products, the library's and this one, us (in brackets w over the copy's rate, which is no
+// floor: w's first tiles come under the kernel ahead, and a copy writes as much as it reads; alone 24,576 x 4,096 takes 35): N x K 64 x 2,048
+// 5.1 -> 2.0; 2,048 x
 // 2,048 7.9 -> 3.2 (1.3) with 5 tokens, 6.4 -> 3.8 with 16; 2,048 x 4,096 12 -> 4.5 (2.6); 10,304 x 2,048 9.8 -> 7.9 (6.5) with 8, 11.3 ->
 // 9.1 with 16; 24,576 x 4,096 35.3 -> 31.5 (31.2), 35.8 -> 34.2 with 16; 32,000 x 4,096 46 -> 39 (41), 47 -> 41.  Gate/up with SiLU, against
 // stretches of (128 outputs, 64 k) dealt out evenly and finished through scratch by the block that comes last: 8,192 x 2,048 14.6 ->
 // 11.5 (10.4), 12,288 x 4,096 36.9 -> 30.7 (31.2), 25,600 x 5,120 85 -> 75 (81), 28,672 x 8,192 155 -> 139 (146).
 #include "common.cuh"
 #include "mma.cuh"
-
-#include <cstdlib>
 
 namespace lily {
 namespace fewrows {
@@ -209,25 +209,11 @@ LILY_API int lily_gemm_few(const void* x, const void* w, const void* bias, int b
     return fewrows::launch<2, false>(grid, x, w, bias, bias_f32, out, out_f32, M, N, K, fewrows::Gate{}, stream);
 }
 
-// out [M, I] bfloat16 = act(x . gate^T) * (x . up^T), up to 16 tokens; w [2 I, K] holds runs of `run` gate rows and the `run` up
-// rows of the same outputs (run == I: all gate rows, then all up rows).
+// out [M, I] bfloat16 = act(x . gate^T) * (x . up^T), up to 8 tokens; w [2 I, K] holds runs of `run` gate rows and the `run` up
+// rows of the same outputs (run == I: all gate rows, then all up rows).  Against the product followed by the activation, us: 12,288 x 4,096
+// 32.1 -> 31.0 with 1 token, 32.2 -> 31.3 with 8; 25,600 x 5,120 75.1 -> 73.8, 76.7 -> 75.6; 28,672 x 8,192 135.7 -> 136.6, 141.5 -> 139.5.
 LILY_API int lily_swiglu_few_takes(int M, int I, int K, int run) {
-    return lily_gemm_few_takes(M, I, K) && I >= 8 && run >= 8 && run % 8 == 0 && I % run == 0;
-}
-
-// How a caller is to form the gate/up product and its activation: 0: this kernel does not take it (more than 8 tokens among
-// them), 1: here, 2: it takes it, but the product and the activation as a pass of its own are the answer (several tokens of an input that
-// the kernel before this one could not stage, for which that pair was ahead; it is 2 us behind now).  LILY_B200_SWIGLU_X=global
-// answers as if no input could be staged.
-LILY_API int lily_swiglu_few_verdict(int M, int I, int K, int run) {
-    if (M > 8 || !lily_swiglu_few_takes(M, I, K, run)) return 0;
-    static const bool never_staged = [] {
-        const char* v = getenv("LILY_B200_SWIGLU_X");
-        return v && v[0] == 'g';
-    }();
-    const long long kblocks = K / fewrows::KT, units = (I + 127) / 128 * kblocks, a_block = (units + sm_count() - 1) / sm_count();
-    const bool staged = !never_staged && min(a_block, kblocks) <= 66;        // 66 KB beside 160 KB of rings
-    return !staged && (long long)M * K > 3 * 8192 ? 2 : 1;
+    return M <= 8 && lily_gemm_few_takes(M, I, K) && I >= 8 && run >= 8 && run % 8 == 0 && I % run == 0;
 }
 
 LILY_API int lily_swiglu_few(const void* x, const void* w, void* out, int M, int I, int K, int run, int act, float limit, float alpha,
@@ -237,6 +223,5 @@ LILY_API int lily_swiglu_few(const void* x, const void* w, void* out, int M, int
     LILY_REQUIRE((((uintptr_t)x | (uintptr_t)w) & 15) == 0, "swiglu_few: operands do not start on 16 bytes");
     const int grid = min(I / 8, 2 * sm_count());
     const fewrows::Gate gate{run, act, limit, alpha};
-    if (M <= 8) return fewrows::launch<1, true>(grid, x, w, nullptr, 0, out, 0, M, 2 * I, K, gate, stream);
-    return fewrows::launch<2, true>(grid, x, w, nullptr, 0, out, 0, M, 2 * I, K, gate, stream);
+    return fewrows::launch<1, true>(grid, x, w, nullptr, 0, out, 0, M, 2 * I, K, gate, stream);
 }

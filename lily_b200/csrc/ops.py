@@ -153,8 +153,8 @@ def library():
         lib.lily_gemm_few_takes.restype = _i
         lib.lily_gemm_few_pays.argtypes = [_i, _i, _i]
         lib.lily_gemm_few_pays.restype = _i
-        lib.lily_swiglu_few_verdict.argtypes = [_i, _i, _i, _i]
-        lib.lily_swiglu_few_verdict.restype = _i
+        lib.lily_swiglu_few_takes.argtypes = [_i, _i, _i, _i]
+        lib.lily_swiglu_few_takes.restype = _i
         lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
         lib.lily_ssd_step_takes.restype = _i
         lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
@@ -569,36 +569,30 @@ def linear_auto(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
 
 def swiglu_skinny_need(tokens: int, intermediate: int, hidden: int, dtype: torch.dtype,
                        block: Optional[int] = None, whenever_possible: bool = False) -> Optional[Tuple[int, int]]:
-    """(float32 of scratch, int32 counters) that ``swiglu_skinny`` is given for this shape (it uses neither), or None when it
-    does not take it (more than 8 tokens, not bfloat16, K not a multiple of 64) or, unless ``whenever_possible``, for
-    several tokens of a very wide input: the caller then forms the product and SiLU*mul separately.
-    ``LILY_B200_SWIGLU=library`` always answers None."""
-    if dtype != torch.bfloat16 or _LIBRARY_SWIGLU:
+    """None where ``swiglu_skinny`` does not take the shape (more than 8 tokens, not bfloat16, K not a multiple of 64): the caller
+    then forms the product and SiLU*mul separately.  Else (0, 0): the float32 of scratch and int32 counters it wants.
+    ``LILY_B200_SWIGLU=library`` always answers None.  (``whenever_possible`` asks for the shapes it takes although the pair is the
+    faster way; there are none.)"""
+    if dtype != torch.bfloat16 or _LIBRARY_SWIGLU or not library().lily_swiglu_few_takes(int(tokens), int(intermediate), int(hidden), int(block or intermediate)):
         return None
-    verdict = library().lily_swiglu_few_verdict(int(tokens), int(intermediate), int(hidden), int(block or intermediate))
-    if verdict == 0 or (verdict == 2 and not whenever_possible):
-        return None
-    return 4, 1
+    return 0, 0
 
 
 _LIBRARY_SWIGLU = os.environ.get("LILY_B200_SWIGLU", "") == "library"
 
 
-def swiglu_skinny(x: torch.Tensor, gate_up: torch.Tensor, block: Optional[int], scratch: torch.Tensor,
-                  counters: torch.Tensor, out: Optional[torch.Tensor] = None, activation: str = "silu",
+def swiglu_skinny(x: torch.Tensor, gate_up: torch.Tensor, block: Optional[int], scratch: Optional[torch.Tensor] = None,
+                  counters: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, activation: str = "silu",
                   limit: float = 0.0, alpha: float = 1.0) -> torch.Tensor:
     """``act(x . gate^T) * (x . up^T)`` [tokens, I] for up to 8 tokens in one kernel that streams the fused
     gate/up matrix [2 I, K] once (rows in alternating runs of ``block`` gate and up rows; None: all gate, then all
-    up).  ``scratch`` and ``counters`` are sized by
-    ``swiglu_skinny_need`` and left as they are."""
+    up).  ``scratch`` and ``counters`` are left as they are."""
     _dev(x, gate_up, scratch, counters, out)
     m, k = x.shape
     inter = gate_up.shape[0] // 2
-    need = swiglu_skinny_need(m, inter, k, x.dtype, block, whenever_possible=True)
-    if need is None or gate_up.dtype != torch.bfloat16 or gate_up.shape[1] != k:
+    if (swiglu_skinny_need(m, inter, k, x.dtype, block, whenever_possible=True) is None or gate_up.dtype != torch.bfloat16
+            or gate_up.shape[1] != k):
         raise KernelError(f"swiglu_skinny: x {tuple(x.shape)} {x.dtype} against {tuple(gate_up.shape)} {gate_up.dtype}")
-    if scratch.dtype != torch.float32 or scratch.numel() < need[0] or counters.dtype != torch.int32 or counters.numel() < need[1]:
-        raise KernelError(f"swiglu_skinny: {need[0]} float32 of scratch and {need[1]} int32 counters needed")
     if out is None:
         out = torch.empty((m, inter), dtype=torch.bfloat16, device=x.device)
     _call("lily_swiglu_few", _p(x), _p(gate_up), _p(out), m, inter, k, int(block or inter), GATE_ACTIVATIONS[activation],

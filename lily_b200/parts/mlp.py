@@ -75,11 +75,9 @@ class SwiGLU(FeedForward):
         how = {} if self.spec.activation == "silu" else {"activation": self.spec.activation}
         if self.spec.activation == "swish_clamped":
             how.update(limit=self.spec.limit, alpha=self.spec.alpha)
-        few = ops.swiglu_skinny_need(x.shape[0], self.spec.intermediate_size, self.spec.hidden_size, x.dtype, self.block)
-        if few is not None and batch.workspace is not None:
+        if ops.swiglu_skinny_need(x.shape[0], self.spec.intermediate_size, self.spec.hidden_size, x.dtype, self.block) is not None:
             # a few tokens: one kernel streams the fused matrix and applies the activation and the product to its own sums
-            act = ops.swiglu_skinny(x, self.w_gate_up, self.block, batch.workspace.floats("swiglu", few[0]),
-                                    batch.workspace.counters("swiglu", few[1]), **how)
+            act = ops.swiglu_skinny(x, self.w_gate_up, self.block, **how)
         elif self.block and ops.gate_up_fused_pays(x.shape[0], self.w_gate_up.shape[0]) and ops.gemm_tc_takes(x, self.w_gate_up):
             act = ops.gemm_tc(x, self.w_gate_up, silu_mul_block=True, **how)
         else:

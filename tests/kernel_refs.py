@@ -192,11 +192,10 @@ def linear_auto(x, weight, bias=None):
 
 
 def swiglu_skinny_need(tokens, intermediate, hidden, dtype, block=None, whenever_possible=False):
-    return (16, 4) if dtype == torch.bfloat16 and tokens <= 8 and hidden % 64 == 0 else None
+    return (0, 0) if dtype == torch.bfloat16 and tokens <= 8 and hidden % 64 == 0 else None
 
 
-def swiglu_skinny(x, gate_up, block, scratch, counters, out=None, activation="silu", limit=0.0, alpha=1.0):
-    assert int(counters.abs().sum()) == 0           # the kernel finds them zero and leaves them zero
+def swiglu_skinny(x, gate_up, block, scratch=None, counters=None, out=None, activation="silu", limit=0.0, alpha=1.0):
     return silu_mul(linear(x, gate_up, out_dtype=torch.float32), x.dtype, block=block, activation=activation, limit=limit, alpha=alpha)
 
 

@@ -1,7 +1,6 @@
 """Each CUDA kernel alone against its plain PyTorch statement (tests/kernel_refs.py), at sizes
 other than the engine's: odd widths, head sizes in steps of 16, any grouping, windows, page edges."""
 
-import os
 
 import pytest
 import torch
@@ -143,22 +142,10 @@ SWIGLU_SHAPES = [(8, 12288, 4096, 128), (1, 12288, 4096, 128), (5, 1408, 512, 12
                  (3, 264, 1088, 8), (7, 25600, 5120, 128), (8, 352, 128, None), (2, 128, 12288, 64)]
 
 
-def test_skinny_swiglu_with_x_from_global_memory():
-    """The kernel's other form (the lanes read x from global memory; taken when x of a block's stretch does not fit
-    beside the rings) on every shape: the form is chosen by an environment variable read once, so a fresh process."""
-    import subprocess, sys
-    code = (f"import sys; sys.path.insert(0, {os.path.dirname(os.path.abspath(__file__))!r}); import test_kernels_gpu as t\n"
-            "for shape in t.SWIGLU_SHAPES: t.test_skinny_swiglu(*shape)")
-    done = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LILY_B200_SWIGLU_X="global"),
-                          capture_output=True, text=True, timeout=600)
-    assert done.returncode == 0, done.stderr[-2000:]
-
-
 @pytest.mark.parametrize("m,inter,k,run", SWIGLU_SHAPES)
 def test_skinny_swiglu(m, inter, k, run):
     """The gate/up product with SiLU*mul in one weight-streaming kernel against the plain statement: tall and low
-    matrices (row blocks finished by one block or by several, whose stretches end anywhere), deep k (more units a
-    block than a row block has), both layouts of the fused matrix, 1 to 8 tokens; twice over the same scratch, and a
+    matrices, deep k, both layouts of the fused matrix, 1 to 8 tokens; scratch and counters left as they are, and a
     token's result does not depend on its neighbours."""
     o = ops()
     g = torch.Generator(device=DEV).manual_seed(12)
@@ -179,9 +166,8 @@ def test_skinny_swiglu(m, inter, k, run):
     alone = o.swiglu_skinny(x[:1].contiguous(), w, run, scratch, counters)
     assert torch.equal(alone[0], got[0])
     assert o.swiglu_skinny_need(9, inter, k, torch.bfloat16, run) is None
-    # several tokens of an input too wide to stage beside the rings: the kernel takes it, the library pair is preferred
-    from_global = os.environ.get("LILY_B200_SWIGLU_X") == "global" or (m, inter, k) == (7, 25600, 5120)
-    assert (o.swiglu_skinny_need(m, inter, k, torch.bfloat16, run) is None) == (from_global and m * k > 3 * 8192)
+    assert o.swiglu_skinny_need(m, inter, k, torch.bfloat16, run) is not None
+    assert torch.equal(o.swiglu_skinny(x, w, run), got)
     assert o.swiglu_skinny_need(m, inter, k, torch.float32, run) is None
     assert o.swiglu_skinny_need(m, inter, k + 8, torch.bfloat16, run) is None
 
