@@ -14,8 +14,8 @@
 //          outputs are never written and nothing is left to combine.  The ring starts on the first experts while the up
 //          kernel still runs (the choices are older than that kernel).
 //
-// The line lies at 16 tokens and 128 pairs, as far as the columns' fragments go; up to there both kernels are ahead of the
-// grouping, the library's two grouped products and the sum, us with router and choice (weights read at the copy rate):
+// The kernels take up to 16 tokens and 128 pairs, as far as the columns' fragments go (lily_moe_few_pays says where they are the faster
+// way); against the grouping, the library's two grouped products and the sum, us with router and choice (weights read at the copy rate):
 // 16 experts of 2,048 x 2,048, gated, top 4: 62 -> 31 (16) with 1 token, 84 -> 42 (25) with 2, 120 -> 76 (57) with 8, 125 -> 96
 // (62) with 16; 64 of 4,096 x 1,536, top 8: 116 -> 70 (47), 172 -> 115 (89), 364 -> 276 (237), 498 -> 459 (328).  The columns
 // ride in the ring beside the weights: read by the lanes in pieces of 4 bytes, 8 tokens took 113 us and 16 took 162.
@@ -313,6 +313,16 @@ using namespace lily;
 LILY_API int lily_moe_few_takes(int tokens, int top, int experts, int width, int ff) {
     return tokens >= 1 && tokens <= 16 && tokens * top <= few::MAX_PAIRS && experts >= 1 && experts <= few::MAX_EXPERTS &&
            width > 0 && ff > 0 && width % few::KT == 0 && ff % few::KT == 0;
+}
+
+// Whether they are the faster way.  A block of the down kernel takes every chosen expert's 16 rows, 1.25 us for 1,000 numbers of them up to 8
+// tokens and 1.85 beyond (an expert counts 512 at least, a tile of k a warp), where the grouped products take 1 us a 1,000 for a width of
+// 1,000 and 33 us of launches and grouping: a wide layer is always ahead, a narrow one while it meets few experts or short ones.
+// Grouped / here, 64 experts, top 8: width 512, ff 2,048: 1.60 with 1 token, 1.13 with 2, 0.89 with 4, 0.60 with 16; width 1,024: 1.45,
+// 1.28, 1.15, 0.86; width 1,024, ff 512: 2.00, 1.68, 1.37, 1.02; from width 2,048 on 1.05 to 3.
+LILY_API int lily_moe_few_pays(int tokens, int top, int experts, int width, int ff) {
+    const long long chosen = min(experts, tokens * top), a_number = tokens <= 8 ? 1250 : 1850;
+    return width >= a_number || chosen * max(ff, 512) * (a_number - width) <= 33000000;
 }
 
 // act [tokens * top, ff] from h [tokens, ldh]: W [experts, 2 ff, width] (an expert's gate rows, then its up rows) with

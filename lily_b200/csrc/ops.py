@@ -161,6 +161,8 @@ def library():
         lib.lily_wkv_step_takes.restype = _i
         lib.lily_moe_few_takes.argtypes = [_i, _i, _i, _i, _i]
         lib.lily_moe_few_takes.restype = _i
+        lib.lily_moe_few_pays.argtypes = [_i, _i, _i, _i, _i]
+        lib.lily_moe_few_pays.restype = _i
         lib.lily_delta_rule_max_head_dim.restype = _i
         lib.lily_selective_scan_max_state.restype = _i
         lib.lily_mlstm_max_head_dim.restype = _i
@@ -1714,11 +1716,13 @@ _FEW_TOKENS = os.environ.get("LILY_B200_EXPERTS_FEW", "1") != "0"
 
 
 def few_tokens_take(r: "ExpertRouting", h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, gated: bool) -> bool:
-    """Whether the step's few tokens go through the two kernels that stream the chosen experts' weights."""
+    """Whether the step's few tokens go through the two kernels that stream the chosen experts' weights: where those take
+    the step and are the faster way."""
     experts, width, ff = w_down.shape
     return (_FEW_TOKENS and h.dtype == w_gate_up.dtype == w_down.dtype == torch.bfloat16 and experts == r.experts
             and tuple(w_gate_up.shape) == (experts, 2 * ff if gated else ff, width) and w_down.shape[1] == h.shape[1]
             and bool(library().lily_moe_few_takes(h.shape[0], r.top, experts, width, ff))
+            and bool(library().lily_moe_few_pays(h.shape[0], r.top, experts, width, ff))
             and (w_gate_up.data_ptr() | w_down.data_ptr() | h.data_ptr()) % 16 == 0)
 
 

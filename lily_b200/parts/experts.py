@@ -18,9 +18,10 @@ be added, times ``sigmoid(W_sg h)``, one number a token: ``W_sg`` is one more ro
 returned in float32 as one plane of partial sums for the next residual add.
 
 Routing, grouping by expert and the grouped products all stay on the device (``ops.moe_route``, ``ops.moe_experts``):
-nothing is read back by the host, so a step replays from a CUDA graph, and each (token, choice) pair is a row of a
-grouped product whose sum runs over k in a fixed order, so a token's result does not depend on its neighbours in the
-batch.
+nothing is read back by the host, so a step replays from a CUDA graph.  A (token, choice) pair's sums run over k in an order that is
+fixed for the kernels that take the step: a row of the grouped products, or, in a step of up to 16 tokens, a column of the kernels
+that stream the chosen experts' weights.  So a token's result does not depend on its neighbours among steps that take the same
+kernels; between the two it differs by the order of float32 sums and, in bfloat16, by the grouped gate and up sums being rounded.
 """
 
 from __future__ import annotations

@@ -769,7 +769,7 @@ def test_attention_fp32_wide_and_element_by_element(nq, nkv, d, dv, page, window
 @pytest.mark.parametrize("width,ff,experts,identity,top,activation,on_input,shared", [
     (64, 64, 3, 0, 2, "silu", False, False), (192, 320, 16, 2, 4, "swish_clamped", False, False),
     (2048, 2048, 16, 0, 3, "relu2", False, True), (128, 192, 40, 0, 8, "silu", True, True), (256, 64, 2, 6, 7, "swish_clamped", False, True),
-    (64, 128, 256, 0, 8, "relu2", True, False)])
+    (64, 128, 256, 0, 8, "relu2", True, False), (1216, 512, 64, 0, 8, "silu", False, False), (1856, 2048, 12, 0, 8, "silu", False, False)])
 def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, activation, on_input, shared):
     """The kernels that stream the chosen experts' weights (up to 16 tokens and 128 pairs; beyond, the grouped products): odd
     numbers of tokens, experts nobody chose, steps of identity choices alone, fewer tiles of k than warps."""
@@ -789,7 +789,8 @@ def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, acti
     scale = float(want.abs().max())
     assert float((got - want).abs().max()) < 1.6e-2 * scale
     # a token's sum does not depend on its neighbours, bit for bit, while both take the same kernels
-    if tokens * top <= 128 and tokens <= 16:
+    few = lambda n: bool(ops().library().lily_moe_few_takes(n, top, experts, width, ff) and ops().library().lily_moe_few_pays(n, top, experts, width, ff))
+    if few(tokens) and few(1):
         keep = slice(tokens - 1, tokens)
         alone = ops().moe_route(h[keep], router, None, top, experts, shared_gate=shared, outputs=experts + identity)
         assert torch.equal(alone.chosen, r.chosen[keep])
