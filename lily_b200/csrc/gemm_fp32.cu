@@ -300,21 +300,23 @@ gemm_fp32_kernel(const float* __restrict__ A, const float* __restrict__ W, const
     }
 }
 
-// Whether a product goes to the kernel for few rows.  That one takes about 1.05 us for every million products of 8 rows
-// (W comes from L2 again for each 8, and a product's row is read from shared memory); the tile takes about 130 us for
-// 2,048 products of one wave of blocks and 0.8 of that for each further one, however many of its 64 rows are there.
-// Measured, rows / tile, us: N 2,048, K 2,048: 47 / 130 with 64 rows, 116 / 129 with 192, 154 / 129 with 256; N 16,384,
-// K 2,048: 46 / 140 with 3 rows, 116 / 140 with 24, 214 / 140 with 48.
-static bool few_rows(long long M, long long N, long long heads) {
-    const long long chunks = (M + 7) / 8, blocks = (M + BM - 1) / BM * ((N + BN - 1) / BN) * heads;
-    const long long waves = (blocks + sm_count() - 1) / sm_count();
-    return chunks <= 65535 && 10 * chunks * N * heads < 60000 * max(10ll, 8 * waves);
+// Whether a product goes to the kernel for few rows.  In units of 0.175 ns: that one takes, for every 2,048 numbers of k or part of them, 10
+// for every output column of 8 rows (W comes from L2 again for each 8, and a product's row is read from shared memory; 5.5 for a single
+// row), 25,000 for one row to 49,000 for 8 at least; the tile takes 13,000 and 290 for every k in one wave of blocks and 0.8 of that for each
+// further one, however many of its 64 rows are there.  Tile / rows, us: N 2,048, K 2,048: 121 / 40 with 64 rows, 122 / 119 with 200, 122 /
+// 187 with 300; N 8,192, K 2,048: 126 / 21 with 8, 127 / 139 with 64; N 512, K 512: 32 / 26 with 200, 32 / 42 with 300; 16 heads of N
+// 512, K 128: 9.4 / 17 with 8; N 64, K 32: 3.2 / 4.5 with 1.
+static bool few_rows(long long M, long long N, long long K, long long heads) {
+    const long long chunks = (M + 7) / 8, blocks = (M + BM - 1) / BM * ((N + BN - 1) / BN) * heads, m = min(M, 8ll);
+    const long long waves = (blocks + sm_count() - 1) / sm_count(), passes = (K + RUN * RUNS - 1) / (RUN * RUNS);
+    const long long rows = passes * max(22000 + 3400 * m, (96 + 13 * m) * chunks * N * heads / 20);
+    return chunks <= 65535 && rows < (13000 + 290 * K) * max(10ll, 8 * waves) / 10;
 }
 
 static int gemm_fp32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldc, int heads,
                      size_t a_head, size_t w_head, size_t c_head, cudaStream_t stream) {
     const bool vec = (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && ((K | lda) & 3) == 0 && ((a_head | w_head) & 3) == 0;
-    if (vec && few_rows(M, N, heads)) {
+    if (vec && few_rows(M, N, K, heads)) {
 #define LILY_ROWS(MB) return launch_rows<MB>(A, W, bias, C, M, N, K, lda, ldc, heads, a_head, w_head, c_head, stream)
         if (M == 1) LILY_ROWS(1);
         if (M == 2) LILY_ROWS(2);

@@ -714,7 +714,7 @@ def test_sample_frequencies():
     assert chi2 < 31.26                                         # df = 11, p = 0.001
 
 
-@pytest.mark.parametrize("n,k", [(16, 2048), (17, 2052), (2400, 4100), (5, 260), (4750, 516)])
+@pytest.mark.parametrize("n,k", [(16, 2048), (17, 2052), (2400, 4100), (5, 260), (4750, 516), (130, 32), (70, 64), (513, 132), (2048, 2304)])
 @pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6, 8, 9, 200, 257])
 def test_gemm_fp32_rows_and_tiles_give_the_same_bits(m, n, k):
     """Both kernels of the float32 product sum in the same order: a row is the same bits alone, in a few rows and in
