@@ -62,6 +62,14 @@ class _PinnedRing:
             self.events[i] = ev
 
 
+def _load_library_products(device) -> None:
+    """The library that prompts take their products from sets itself up in its first calls (0.15 s and, for float32 results, 0.05 s a
+    process): here, so that the first prompt does not wait for it.  Decode steps of up to 16 requests do not call it."""
+    x = torch.zeros((16, 64), dtype=torch.bfloat16, device=device)
+    torch.mm(x, x.t())
+    torch.mm(x, x.t(), out_dtype=torch.float32)
+
+
 class _DecodeGraph:
     """One captured decode step for up to ``bucket`` requests of up to ``max_len`` positions, about equally long
     (``even``) or not; ``even_matters`` says whether some part planned by that.  Its metadata lives
@@ -357,6 +365,8 @@ class ModelRunner:
         lily/model_executor/cuda_graph_runner.py:93,147-149)."""
         if not self.use_graphs:
             return []
+        if self.dtype == torch.bfloat16:
+            _load_library_products(self.device)
         want = self.graph_buckets if batch_sizes is None else sorted(
             {next(b for b in self.graph_buckets if b >= n) for n in batch_sizes if 1 <= n <= self.graph_buckets[-1]})
         classes = self.length_classes if max_len is None else [self._length_class(max_len)]

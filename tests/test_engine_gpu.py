@@ -333,3 +333,18 @@ def test_many_live_requests(which, dtype, live, graphs, monkeypatch):
                 assert not any(p.fused for p in decode)                            # too many blocks: the rotation kernel runs first
             elif dtype == "bfloat16":
                 assert any(p.fused for p in decode)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_capturing_readies_the_library_that_prompts_use(dtype, monkeypatch):
+    """Decode steps call no library product, so a captured runner has called it for the first prompt's sake: in bfloat16, which is
+    where prompts use it."""
+    from lily_b200.engine import runner as module
+    asked, mm = [], torch.mm
+    monkeypatch.setattr(module.torch, "mm", lambda *a, **k: asked.append(k.get("out_dtype")) or mm(*a, **k))
+    with tempfile.TemporaryDirectory() as tmp:
+        path, _ = model_dir(tiny_models.CONFIGS["tiny_qwen3"], 31, tmp)
+        runner = make_runner(path, dtype=dtype, device="cuda:0")
+        assert not asked
+        runner.capture_decode_graphs([1])
+    assert (None in asked and torch.float32 in asked) == (dtype == "bfloat16")
