@@ -1286,8 +1286,8 @@ def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0, chunks=Tru
     while chunk < 1024 and state_floats and sum(-(-n // chunk) for n in new_lens if n > SCAN_DIRECT) * state_floats * 4 > SCAN_WORKSPACE:
         chunk *= 2
     cuts = [cut(SCAN_DIRECT, chunk)] if max(new_lens, default=0) > SCAN_DIRECT else []
-    if (chunks and max(new_lens, default=0) >= SCAN_FINE and chunk == SCAN_CHUNK
-            and sum(-(-n // chunk) for n in new_lens if n >= SCAN_FINE) * max(state_floats, 1) * 4 <= SCAN_WORKSPACE):
+    fine = sum(-(-n // SCAN_CHUNK) for n in new_lens if n >= SCAN_FINE) if chunks and chunk == SCAN_CHUNK else 0
+    if 0 < 2 * fine <= 65535 and fine * max(state_floats, 1) * 4 <= SCAN_WORKSPACE:       # two tiles of outputs a chunk along the grid
         cuts.append(cut(SCAN_FINE - 1, chunk))
     if not cuts:
         return ScanPlan(None, len(new_lens))

@@ -1078,3 +1078,5 @@ def test_scan_plan_cuts_only_for_who_runs_it():
         plan = o.scan_plan(lens, DEV, floats, chunks=bf)
         assert (plan.fine.num_chunks if plan.fine else 0) == want, lens
         assert o.scan_workspace_floats(plan, 64, 64, 128) == want * (floats + 64)
+    # more chunks than a grid of the tensor-core kernels has room for
+    assert o.scan_plan([150] * 16383, DEV, 256).fine.num_chunks == 32766 and o.scan_plan([150] * 16384, DEV, 256).fine is None
