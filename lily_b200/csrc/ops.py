@@ -669,9 +669,11 @@ def latent_attention_status() -> int:
 
 def prefill_tile_rows(dtype: torch.dtype = torch.float32, d: int = 0, page_size: int = 0, new_tokens: int = 0,
                       softcap: Optional[float] = None, dv: Optional[int] = None, values_in_keys: bool = False,
-                      heads: int = 0, keep_first: int = 0, sink: bool = False, all_values: bool = False) -> int:
+                      heads: int = 0, keep_first: int = 0, sink: bool = False, all_values: bool = False,
+                      new_lens: Optional[Sequence[int]] = None) -> int:
     """New tokens per tile of the prefill kernel that will take this precision, head size (``dv`` for the values
-    where it differs), page size, number of new tokens and kind of scores and mask."""
+    where it differs), page size, number of new tokens and kind of scores and mask.  ``new_lens``: the tokens of each portion (one
+    portion where not given), which the forms with a sink or all heads' values are chosen by, with ``heads`` query heads."""
     lib = library()
     if values_in_keys and heads and latent_tensor_cores(dtype, d, dv, softcap=softcap):
         few = int(lib.lily_latent_attention_mma_tile_tokens(int(heads)))
@@ -679,7 +681,8 @@ def prefill_tile_rows(dtype: torch.dtype = torch.float32, d: int = 0, page_size:
         # a tile height names its kernel; where both kernels' tiles hold one token (65 heads and more) it is the tcgen05 one
         return many if latent_tcgen05(dtype, d, dv, page_size) and (many == few or new_tokens * heads >= LATENT_TC_MIN_ROWS) else few
     if (sink or all_values) and sink_on_tensor_cores(dtype, d, dv, values_in_keys, softcap):
-        if not _MMA_SINK and uses_tcgen05_attention(dtype, d, page_size, new_tokens):
+        if (not _MMA_SINK and uses_tcgen05_attention(dtype, d, page_size, new_tokens)
+                and sink_prompts_on_tcgen05(d, [new_tokens] if new_lens is None else new_lens, heads, all_values)):
             return int(lib.lily_attention_prefill_tc_rows())
         return int(lib.lily_attention_prefill_mma_rows())
     if sink or all_values:
@@ -688,6 +691,20 @@ def prefill_tile_rows(dtype: torch.dtype = torch.float32, d: int = 0, page_size:
     if same and uses_tcgen05_attention(dtype, d, page_size, new_tokens):
         return int(lib.lily_attention_prefill_tc_rows())
     return int(lib.lily_attention_prefill_mma_rows() if same and uses_tensor_cores(dtype, d) else lib.lily_attention_prefill_simt_rows())
+
+
+def sink_prompts_on_tcgen05(d: int, new_lens: Sequence[int], heads: int, planes: bool) -> bool:
+    """Whether prompts with a sink are faster on the tcgen05 kernel, tiles of 128 tokens and (``planes``) the values of all kv heads in
+    one launch, than on the mma.sync kernel, tiles of 64 and a launch a kv head.  What its tiles hold of padding decides, unless there are
+    few of them and planes save launches; heads of 64, whose tiles the mma.sync kernel walks as fast, want full tiles.  Measured, mma.sync /
+    tcgen05: 16 heads over 4 of 128, planes: 128 tokens 4.4, 2 x 64 4.0, 8 x 64 2.2, 16 x 32 0.83, 2,000 3.9; own values: 128 1.2, 16 x 64 0.75,
+    2,000 3.4; heads of 64, 16 over 2, planes: 128 1.6, 16 x 32 0.53, 6 x 100 1.04; own values: 128 0.84, 400 0.99, 1,000 1.9."""
+    tokens, wide, narrow = sum(new_lens), sum(-(-n // 128) for n in new_lens) * 128, sum(-(-n // 64) for n in new_lens) * 64
+    if d < 128 and not planes:
+        return tokens >= 400 * len(new_lens)
+    if planes and wide * heads <= (16384 if d >= 128 else 8192):
+        return True
+    return wide <= (1.75 if d >= 128 else 1.1) * narrow
 
 
 def attention_tc_status() -> int:
@@ -705,8 +722,8 @@ def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torc
     ``sinks`` (float32, one number a query head): the softmax's denominator holds exp(sinks[h]) as well, a key without a
     value whose score is not scaled (the kernels over cached latents and the CUDA-core kernel).
     ``sink``: the softmax's denominator holds one more unit (a key of score 0 that has no value).  ``all_values``: every
-    query head's weights meet the values of all kv heads, ``out`` is float32 [tokens, nq * nkv * dv] (``head_mix``
-    follows).  Both run on the CUDA-core kernel.  ``softcap``: scores
+    query head's weights meet the values of all kv heads, ``out`` is what ``all_values_sums`` gives (``head_mix``
+    follows).  ``softcap``: scores
     become softcap * tanh(score * scale / softcap) before the softmax; ``keep_first``: beside a window, keys at
     positions below this stay visible; ``dv``: the
     value head size where it differs from d (CUDA-core kernels; ``out`` is then [tokens, nq * dv]).
@@ -802,7 +819,7 @@ _MMA_SINK = os.environ.get("LILY_B200_SINK_ATTENTION", "") == "mma"        # pro
 def sink_on_tensor_cores(dtype: torch.dtype, d: int, dv: Optional[int] = None, values_in_keys: bool = False,
                          softcap: Optional[float] = None) -> bool:
     """Whether attention with a sink (and with the values of all kv heads) runs on the tensor-core kernels (prompts of
-    TC_ATTENTION_MIN_TOKENS on the tcgen05 kernel where it takes the shape, the rest on mma.sync): bfloat16, keys and values of one head size that those kernels take; else the CUDA-core kernels."""
+    TC_ATTENTION_MIN_TOKENS on the tcgen05 kernel where it takes the shape and ``sink_prompts_on_tcgen05``, the rest on mma.sync): bfloat16, keys and values of one head size that those kernels take; else the CUDA-core kernels."""
     return (not _SIMT_SINK and not values_in_keys and int(dv or d) == d and uses_tensor_cores(dtype, d))
 
 
@@ -813,17 +830,17 @@ def all_values_decode_rows(dtype: torch.dtype, requests: int, nkv: int, d: int, 
 
 
 def all_values_in_planes(dtype: torch.dtype, nkv: int, d: int, dv: Optional[int] = None) -> bool:
-    """Whether attention over the values of all kv heads runs as one launch a kv head (``all_values_sums`` then gives
-    planes): on the mma.sync kernels, and on the CUDA-core kernels when a row of ``nkv * dv`` columns would pass 512."""
+    """Whether attention over the values of all kv heads gives a plane a kv head (``all_values_sums``): on the tensor-core
+    kernels, and on the CUDA-core kernels when a row of ``nkv * dv`` columns would pass 512."""
     return sink_on_tensor_cores(dtype, d, dv) or nkv * int(dv or d) > ALL_VALUES_COLUMNS
 
 
 def all_values_sums(dtype: torch.dtype, tokens: int, nq: int, nkv: int, d: int, dv: Optional[int], device) -> torch.Tensor:
     """The tensor that ``attention_prefill`` / ``attention_decode`` with ``all_values`` fill and ``head_mix`` reads.  On
     the CUDA-core kernels float32 [tokens, nq * nkv * dv]: a query head's row holds its weights' sums over every kv
-    head's values.  On the mma.sync kernels, and on the CUDA-core kernels when such a row would pass their 512 columns,
+    head's values.  On the tensor-core kernels, and on the CUDA-core kernels when such a row would pass their 512 columns,
     ``nkv`` planes [nkv, tokens, nq * dv] in ``dtype``: plane s holds, for a query head of kv head g, the sums over the
-    values of kv head (g + s) % nkv (one launch a plane)."""
+    values of kv head (g + s) % nkv (a launch a plane but on the tcgen05 kernel)."""
     dv = int(dv or d)
     if all_values_in_planes(dtype, nkv, d, dv):
         return torch.empty((nkv, tokens, nq * dv), dtype=dtype, device=device)

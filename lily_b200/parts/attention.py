@@ -253,7 +253,7 @@ class Attention(Mixer):
                 wide = s.talk and not ops.all_values_in_planes(dtype, s.num_kv_heads, s.head_dim, s.value_dim)
                 sized = dict(sized, cuda_cores=True, dv=s.num_kv_heads * s.value_dim if wide else s.value_dim)
             else:
-                sized = dict(sized, fusable=False)      # one launch a kv head of the mma.sync kernel, queries prepared ahead
+                sized = dict(sized, fusable=False)      # queries are prepared ahead
 
         def make(b):
             nd = b.num_decode
@@ -270,7 +270,8 @@ class Attention(Mixer):
                 decode = dataclasses.replace(decode, fused=False)
             rows = tiles = None
             if b.num_requests > nd:
-                rows = ops.prefill_tile_rows(dtype, s.head_dim, page, b.num_tokens - nd, **capped, **tiled)
+                portions = {"heads": s.num_heads, "new_lens": b.h_new_lens[nd:]} if s.sink or s.talk else {}
+                rows = ops.prefill_tile_rows(dtype, s.head_dim, page, b.num_tokens - nd, **capped, **tiled, **portions)
                 tiles = ops.prefill_tiles(b.h_prefix_lens, b.h_new_lens, nd, rows, b.token_ids.device)
             return AttentionPlan(decode, rows, tiles)
         return batch.plan(key, make)

@@ -223,7 +223,7 @@ def uses_tensor_cores(dtype, d):
 
 
 def prefill_tile_rows(dtype=None, d=0, page_size=0, new_tokens=0, softcap=None, dv=None, values_in_keys=False, heads=0,
-                      keep_first=0, sink=False, all_values=False):
+                      keep_first=0, sink=False, all_values=False, new_lens=None):
     return 32
 
 

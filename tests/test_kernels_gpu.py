@@ -956,6 +956,42 @@ def test_attention_prefill_tcgen05_sink_and_planes(nq, nkv, d, window, sink, pla
     torch.testing.assert_close(got.float(), want.float(), **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("nq,nkv,d,window,keep,cap,planes", [
+    (4, 4, 128, None, 0, None, True), (3, 3, 64, None, 0, 20.0, False), (8, 2, 128, 90, 70, None, False), (4, 2, 64, 64, 3, 15.0, True),
+    (6, 6, 128, 100, 130, 30.0, True)])
+def test_sink_prompts_with_caps_kept_positions_and_single_heads(nq, nkv, d, window, keep, cap, planes):
+    """A sink with a soft cap, with kept first positions beside a window, and one query head a kv head: the same from the tcgen05 and the
+    mma.sync kernels' tiles, and as the plain statement."""
+    o, page = ops(), 64
+    prefixes, news = [0, 30, 200], [40, 129, 200]
+    cache, table, q, cu, pre = _attention_case(torch.bfloat16, nq, nkv, d, page, prefixes, news, window, spike=True)
+    shape = (nkv, len(q), nq * d) if planes else (len(q), nq * d)
+    how = dict(sink=True, all_values=planes, softcap=cap, keep_first=keep)
+    if planes:
+        wide = torch.zeros(len(q), nq * nkv * d, device=DEV)
+        ref.attention_prefill(q, cache, table, cu, pre, *_tiles_of(news, 32), wide, nq, nkv, d, page, d ** -0.5, window, **how)
+        wide, heads = wide.view(len(q), nq, nkv, d), torch.arange(nq, device=DEV)
+        want = torch.stack([wide[:, heads, (heads // (nq // nkv) + z) % nkv] for z in range(nkv)]).reshape(shape)
+    else:
+        want = torch.zeros(shape, device=DEV)
+        ref.attention_prefill(q, cache, table, cu, pre, *_tiles_of(news, 32), want, nq, nkv, d, page, d ** -0.5, window, **how)
+    for rows in (int(o.library().lily_attention_prefill_tc_rows()), int(o.library().lily_attention_prefill_mma_rows())):
+        got = torch.zeros(shape, device=DEV, dtype=torch.bfloat16)
+        o.attention_prefill(q, cache, table, cu, pre, *_tiles_of(news, rows), got, nq, nkv, d, page, d ** -0.5, window, tile_rows=rows, **how)
+        assert o.attention_tc_status() == 0
+        torch.testing.assert_close(got.float(), want.float(), **tol(torch.bfloat16))
+
+
+def test_sink_prompts_take_the_tiles_they_fill():
+    o = ops()
+    rows = lambda d, news, heads, planes: o.prefill_tile_rows(torch.bfloat16, d, 64, sum(news), sink=True, all_values=planes, heads=heads, new_lens=news)
+    for d, news, heads, planes, want in ((128, [128], 16, False, 128), (128, [127], 16, False, 64), (128, [16] * 16, 32, False, 64), (128, [16] * 16, 32, True, 64),
+                                         (128, [64] * 2, 16, True, 128), (128, [300, 45, 211, 127, 512], 16, True, 128), (64, [300], 16, False, 64),
+                                         (64, [400], 16, False, 128), (64, [16] * 8, 16, True, 64), (64, [256] * 4, 16, True, 128)):
+        assert rows(d, news, heads, planes) == want, (d, news, heads, planes)
+    assert o.prefill_tile_rows(torch.bfloat16, 128, 64, 500, sink=True) == 128
+
+
 @pytest.mark.parametrize("lens", [[17], [64, 5, 130], [128, 1, 257, 40], [16, 300]])
 @pytest.mark.parametrize("heads,groups,pd,n_state", [(4, 2, 64, 128), (3, 1, 16, 16), (2, 1, 80, 48), (8, 4, 128, 64)])
 def test_ssd_scan_in_chunks_on_the_tensor_cores(lens, heads, groups, pd, n_state):
