@@ -157,8 +157,12 @@ def library():
         lib.lily_swiglu_few_takes.restype = _i
         lib.lily_ssd_step_takes.argtypes = [_vp, _sz, _i]
         lib.lily_ssd_step_takes.restype = _i
+        lib.lily_ssd_step_pays.argtypes = [_i, _i, _i, _i, _i]
+        lib.lily_ssd_step_pays.restype = _i
         lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
         lib.lily_wkv_step_takes.restype = _i
+        lib.lily_wkv_step_pays.argtypes = [_i, _i, _i]
+        lib.lily_wkv_step_pays.restype = _i
         lib.lily_moe_few_takes.argtypes = [_i, _i, _i, _i, _i]
         lib.lily_moe_few_takes.restype = _i
         lib.lily_moe_few_pays.argtypes = [_i, _i, _i, _i, _i]
@@ -1346,7 +1350,8 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.
     common = (_p(xbc), channels, _p(proj), proj.shape[1], int(dt_col), _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
               state.shape[1], _p(y), _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
     sizes = (heads, head_dim, n_state, groups, _dt(xbc))
-    if n == requests and library().lily_ssd_step_takes(_p(state), state.shape[1], n_state):
+    if (n == requests and library().lily_ssd_step_takes(_p(state), state.shape[1], n_state)
+            and library().lily_ssd_step_pays(n, heads, head_dim, n_state, _dt(xbc))):
         # one token a request (a decode step): a kernel that moves the state and stages nothing
         _call("lily_ssd_step", *common, int(requests), *sizes, _stream())
         return y
@@ -1549,7 +1554,8 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
     y = torch.empty((tokens, heads * d), dtype=torch.float32, device=r.device)
     common = (_p(r), _p(k), _p(v), stride, _p(log_decay), _p(u), _p(state), state.stride(0), _p(y),
               _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
-    if tokens == requests and library().lily_wkv_step_takes(_p(state), state.stride(0), _p(v), stride, d, _dt(r)):
+    if (tokens == requests and library().lily_wkv_step_takes(_p(state), state.stride(0), _p(v), stride, d, _dt(r))
+            and library().lily_wkv_step_pays(tokens, heads, d)):
         # one token a request (a decode step): a kernel that moves the matrices and stages nothing
         _call("lily_wkv_step", *common, requests, heads, d, _dt(r), _stream())
         return y

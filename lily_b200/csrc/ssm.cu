@@ -337,10 +337,6 @@ ssd_scan_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__ p
 // memory between three barriers and reads the state in runs of a lane, which a prompt pays once and a token every time.)
 // grid (heads, requests, ceil(head_dim / (8 RB))), block 256: a warp takes RB rows of the head's state; n_state up to 128 NI, a
 // multiple of four, its rows on 16 bytes.  64 heads of 64 x 128: 8 requests 12.2 -> 8.0 us (33 MB: 5.2 at the copy rate), one 6.1 -> 2.8.
-// The lines lie at rows of more than 64 numbers, where more than half of the lanes have some, and of 256, where a lane's registers end:
-// between them this kernel is ahead from 1 to 256 requests; us, the kernel above / this one, 64 heads of 64 rows: 16 numbers a row, 64
-// requests 13 / 30; 64 numbers, 256 requests 137 / 167; 96, 8 requests 9.3 / 6.3, 256 requests 212 / 191; 256, 64 requests 131 / 117;
-// 272, 256 requests 736 / 831.
 template <typename T, int NI, int RB>
 __global__ void __launch_bounds__(256)
 ssd_step_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__ proj, int proj_stride, int dt_col,
@@ -642,10 +638,19 @@ LILY_API int lily_ssd_scan(const void* xbc, int channels, const void* proj, int 
     return 0;
 }
 
-// The same scan, arranged for requests that bring one token each (others are taken): whether it is the faster one for this state and the
-// state's rows are on 16 bytes.
+// The same scan, arranged for requests that bring one token each (others are taken): whether the state's rows are on 16 bytes.
 LILY_API int lily_ssd_step_takes(const float* state, size_t state_stride, int n_state) {
-    return n_state % 4 == 0 && n_state > 64 && n_state <= 256 && state_stride % 4 == 0 && (uintptr_t)state % 16 == 0;
+    return n_state % 4 == 0 && n_state >= 4 && n_state <= 512 && state_stride % 4 == 0 && (uintptr_t)state % 16 == 0;
+}
+
+// Whether it is the faster one: always for rows of 68 to 256 numbers; shorter rows leave more than half of a warp's lanes idle, which
+// tells once the device is full, and in bfloat16 so do the registers of longer ones.  The scan / this one, us, 64 heads of 64 rows: 16
+// numbers a row, 2 requests 3.6 / 3.6, 64 requests 13 / 30; 64 numbers, 1 request 4.1 / 2.7, 256 requests 137 / 167; 96, 256 requests
+// 212 / 191; 256, 64 requests 131 / 117; 272, 1 request 7.4 / 4.0, 256 requests 736 / 831 (24 heads, 300 numbers, float32: 307 / 230).
+LILY_API int lily_ssd_step_pays(int requests, int heads, int pd, int n_state, int dtype) {
+    const long long blocks = (long long)requests * heads * ((pd + 63) / 64);
+    if (n_state <= 64) return blocks <= (n_state < 48 ? 128 : 4096);
+    return n_state <= 256 || dtype == kF32 || blocks <= 1024;
 }
 
 LILY_API int lily_ssd_step(const void* xbc, int channels, const void* proj, int proj_stride, int dt_col, const float* dt_bias,
@@ -655,9 +660,9 @@ LILY_API int lily_ssd_step(const void* xbc, int channels, const void* proj, int 
     LILY_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0 && pd >= 1, "ssd_step: %d heads over %d groups, head size %d", heads, groups, pd);
     LILY_REQUIRE(lily_ssd_step_takes(state, state_stride, n_state), "ssd_step: state %d, rows of %zu", n_state, state_stride);
     LILY_REQUIRE(requests <= 65535, "ssd_step: %d requests", requests);
-    const int ni = n_state <= 128 ? 1 : 2;
+    const int ni = n_state <= 128 ? 1 : (n_state <= 256 ? 2 : 4);
     // eight rows a warp where that still gives every SM two blocks, fewer for a few requests
-    int rb = ni == 1 ? 8 : 4;
+    int rb = ni == 1 ? 8 : (ni == 2 ? 4 : 2);
     while (rb > 2 && (long long)heads * requests * ((pd + 8 * rb - 1) / (8 * rb)) < 2 * sm_count()) rb >>= 1;
     dim3 grid(heads, requests, (pd + 8 * rb - 1) / (8 * rb));
 #define GO(T, N, R)                                                                                                          \
@@ -666,7 +671,8 @@ LILY_API int lily_ssd_step(const void* xbc, int channels, const void* proj, int 
 #define GO_T(T)                                                                                                     \
     do {                                                                                                            \
         if (ni == 1) { if (rb == 8) GO(T, 1, 8); else if (rb == 4) GO(T, 1, 4); else GO(T, 1, 2); }                 \
-        else { if (rb == 4) GO(T, 2, 4); else GO(T, 2, 2); }                                                        \
+        else if (ni == 2) { if (rb == 4) GO(T, 2, 4); else GO(T, 2, 2); }                                           \
+        else GO(T, 4, 2);                                                                                           \
     } while (0)
     if (dtype == kBF16) GO_T(__nv_bfloat16); else GO_T(float);
 #undef GO_T

@@ -280,9 +280,8 @@ __global__ void __launch_bounds__(256, 3) wkv_scan_kernel(const T* __restrict__ 
 
 // A step that brings each request one token (any number is taken, one after another).  Bound by reading and writing the
 // matrices once: a thread has four neighbouring value columns (16 bytes) of every 1,024 / d-th key row, asks for eight of them at once and
-// goes on in turns of eight, so nothing but a token's vectors is staged.  grid (heads, requests), block 256; d is 64, 128 or 256,
-// its rows on 16 bytes.  2 requests, 32 heads of 64 x 64: 5.0 -> 2.9 us.  (Matrices of 32 x 32 are four KB a block, which the scan's smaller
-// blocks read faster: 64 heads, 64 requests 14 us there, 27 here.)
+// goes on in turns of eight, so nothing but a token's vectors is staged.  grid (heads, requests), block 256; d is 32, 64, 128 or 256,
+// its rows on 16 bytes.  2 requests, 32 heads of 64 x 64: 5.0 -> 2.9 us.
 template <typename T>
 __global__ void __launch_bounds__(256)
 wkv_step_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, int in_stride, const float* __restrict__ lw,
@@ -520,9 +519,13 @@ LILY_API int lily_wkv_scan(const void* r, const void* k, const void* v, int in_s
 // The same recurrence, arranged for requests that bring one token each (others are taken).
 LILY_API int lily_wkv_step_takes(const float* state, size_t state_stride, const void* v, int in_stride, int d, int dtype) {
     const size_t four = dtype == kBF16 ? 8 : 16;
-    return (d == 64 || d == 128 || d == 256) && state_stride % 4 == 0 && (uintptr_t)state % 16 == 0 && in_stride % 4 == 0 &&
+    return (d == 32 || d == 64 || d == 128 || d == 256) && state_stride % 4 == 0 && (uintptr_t)state % 16 == 0 && in_stride % 4 == 0 &&
            (uintptr_t)v % four == 0;
 }
+
+// Whether it is the faster one: matrices of 32 x 32 are four KB a block of 256 threads, which the scan's smaller blocks read faster
+// once the device is full (64 heads: 4.3 / 2.9 us with 1 request, 5.6 / 5.1 with 8, 14 / 27 with 64; larger matrices are ahead throughout).
+LILY_API int lily_wkv_step_pays(int requests, int heads, int d) { return d > 32 || (long long)requests * heads <= 512; }
 
 LILY_API int lily_wkv_step(const void* r, const void* k, const void* v, int in_stride, const float* lw, const float* u, float* state,
                            size_t state_stride, float* y, const int* cu_seqlens, const int* slots, int requests, int heads, int d, int dtype,

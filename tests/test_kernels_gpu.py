@@ -802,7 +802,8 @@ def test_experts_of_a_few_tokens(tokens, width, ff, experts, identity, top, acti
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("requests,heads,groups,pd,n_state", [
     (1, 2, 1, 64, 128), (9, 64, 8, 64, 128), (3, 6, 3, 24, 64), (2, 4, 2, 7, 20), (5, 8, 1, 33, 256), (2, 2, 2, 16, 300), (300, 2, 1, 80, 512),
-    (4, 3, 1, 5, 17), (3, 2, 1, 9, 64), (3, 2, 1, 9, 68), (300, 4, 2, 70, 132), (2, 3, 1, 40, 260)])
+    (4, 3, 1, 5, 17), (3, 2, 1, 9, 64), (3, 2, 1, 9, 68), (300, 4, 2, 70, 132), (2, 3, 1, 40, 260),
+    (64, 2, 1, 64, 44), (65, 2, 1, 64, 44), (256, 4, 1, 64, 260), (257, 4, 1, 64, 260)])
 def test_ssd_scan_of_one_token_a_request(dtype, requests, heads, groups, pd, n_state):
     """A decode step's scan: rows of a head that no warp fills, states of one to four pieces a lane, many and few requests; a state
     that is no multiple of four takes the general kernel."""
@@ -823,7 +824,7 @@ def test_ssd_scan_of_one_token_a_request(dtype, requests, heads, groups, pd, n_s
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("requests,heads,d", [(1, 32, 64), (7, 3, 32), (40, 2, 128), (2, 5, 256), (3, 4, 48)])
+@pytest.mark.parametrize("requests,heads,d", [(1, 32, 64), (7, 3, 32), (40, 2, 128), (2, 5, 256), (3, 4, 48), (64, 8, 32), (65, 8, 32)])
 def test_wkv_scan_of_one_token_a_request(dtype, requests, heads, d):
     g = torch.Generator(device=DEV).manual_seed(requests + d)
     rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
