@@ -192,12 +192,15 @@ LILY_API int lily_gemm_few_takes(int M, int N, int K) {
 //   up to 8 tokens   1.05 to 3.5 but for K 28,672 with N up to 256 (0.85 to 0.94) and N 5,120 (320 tiles for 296 blocks) from K
 //                    9,728 on (0.89 to 0.97)
 //   9 to 16, tiles for one turn   1.0 to 2.7 up to K 18,944; beyond that 0.56 to 0.99 up to N 2,560, 0.97 to 1.2 from 3,072 on
-//   9 to 16, more tiles           0.99 to 1.7 up to K 4,096 (0.76 at K 512, 0.95 at 1,024 with N 128,256); beyond it 0.76 to 1.1
+//   9 to 16, more tiles           0.99 to 1.7 up to K 4,096 (0.76 at K 512, 0.95 at 1,024 with N 128,256; 1.09 at 1,024 with 50,000);
+//                                 beyond it 0.76 to 0.99 in up to four turns, but 1.02 to 1.06 up to K 12,288 where two or three turns
+//                                 are full (N 8,192 and 12,288), and 0.97 to 1.15 in five turns and more
 LILY_API int lily_gemm_few_pays(int M, int N, int K) {
     const int tiles = (N + fewrows::ROWS - 1) / fewrows::ROWS, slots = 2 * sm_count(), turns = (tiles + slots - 1) / slots;
     if (M <= 8) return turns == 1 ? K <= 25600 || tiles >= 32 : K <= 8192 || 10ll * tiles >= 6ll * turns * slots;
     if (turns == 1) return K <= 18944 || tiles >= 192;
-    return K <= 4096 && (turns <= 4 || K >= 2048);
+    if (turns <= 4) return K <= 4096 || (turns <= 3 && K <= 12288 && 10ll * tiles >= 8ll * turns * slots);
+    return K >= (turns <= 16 ? 1024 : 2048);
 }
 
 LILY_API int lily_gemm_few(const void* x, const void* w, const void* bias, int bias_f32, void* out, int out_f32, int M, int N, int K,

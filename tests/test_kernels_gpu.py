@@ -869,7 +869,8 @@ def test_linear_of_a_few_rows(m, n, k):
 
 @pytest.mark.parametrize("m,n,k,here", [
     (8, 32, 25600, True), (8, 32, 25664, False), (8, 512, 25664, True), (8, 5120, 8192, True), (8, 5120, 8256, False), (9, 1024, 18944, True),
-    (9, 1024, 19008, False), (9, 3072, 19008, True), (16, 5120, 4096, True), (16, 5120, 4160, False), (16, 40000, 2048, True), (16, 40000, 1984, False)])
+    (9, 1024, 19008, False), (9, 3072, 19008, True), (16, 5120, 4096, True), (16, 5120, 4160, False), (16, 40000, 1024, True), (16, 40000, 960, False),
+    (16, 18944, 4160, False), (16, 18960, 4160, True), (16, 8192, 12288, True), (16, 8192, 12352, False), (16, 80000, 1984, False)])
 def test_linear_of_a_few_rows_on_both_sides_of_its_line(m, n, k, here):
     """Where the kernel for few rows hands over to the library (with 148 SMs): the same numbers either way."""
     g = torch.Generator(device=DEV).manual_seed(n + k)
