@@ -429,7 +429,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x [M, K] . weight [N, K]^T (+ bias)``.  float32: this package's FFMA kernel.
     bfloat16: up to 16 rows this package's kernel that streams the weights (``few_rows_take``), else cuBLAS, both with
-    float32 accumulation; ``out_dtype=float32`` keeps the accumulator's precision (used for the logits)."""
+    float32 accumulation; ``out_dtype=float32`` keeps the accumulator's precision (used for the logits).
+    ``weight`` is at rest: the kernels for few rows (as ``linear_split`` and ``swiglu_skinny``) read its first tiles while the kernel
+    launched before may still run, so it must not be what that kernel of this package writes."""
     _dev(x, weight, bias)
     m, k = x.shape
     n = weight.shape[0]
