@@ -63,11 +63,13 @@ class _PinnedRing:
 
 
 def _load_library_products(device) -> None:
-    """The library that prompts take their products from sets itself up in its first calls (0.15 s and, for float32 results, 0.05 s a
-    process): here, so that the first prompt does not wait for it.  Decode steps of up to 16 requests do not call it."""
+    """The library that prompts take their products from sets itself up in its first calls (0.15 s and, for the forms with a
+    float32 result or a bias, 0.05 s and more a process): here, so that the first prompt does not wait for it.  Decode steps of up to 16
+    requests do not call it."""
     x = torch.zeros((16, 64), dtype=torch.bfloat16, device=device)
     torch.mm(x, x.t())
     torch.mm(x, x.t(), out_dtype=torch.float32)
+    torch.addmm(x[0, :16], x, x.t())
 
 
 class _DecodeGraph:
