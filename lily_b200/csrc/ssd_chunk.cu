@@ -17,7 +17,7 @@
 // by token: its own column and head, from its token on.
 // Bound by the tensor cores and the reads of shared memory that feed them.  The scan one token after another took a chunk's
 // 128 steps twice, each step a round of shared memory, FMAs and shuffles: 2,048 tokens, 64 heads of 64 x 128: 139 (own states) and
-// 270 us (outputs), now 33 and 92; against 64 bits the outputs are 1.0e-7 off in the 2-norm, where they were 2 to 4e-7.
+// 270 us (outputs), now 33 and 94; against 64 bits the outputs are 1.0e-7 off in the 2-norm, where they were 2 to 4e-7.
 #include "common.cuh"
 #include "mma.cuh"
 
