@@ -702,13 +702,13 @@ def prefill_tile_rows(dtype: torch.dtype = torch.float32, d: int = 0, page_size:
 def sink_prompts_on_tcgen05(d: int, new_lens: Sequence[int], heads: int, planes: bool) -> bool:
     """Whether prompts with a sink are faster on the tcgen05 kernel, tiles of 128 tokens and (``planes``) the values of all kv heads in
     one launch, than on the mma.sync kernel, tiles of 64 and a launch a kv head.  What its tiles hold of padding decides, unless there are
-    few of them and planes save launches; heads of 64, whose tiles the mma.sync kernel walks as fast, want full tiles.  Measured, mma.sync /
+    few of them, or one portion, and planes save launches; heads of 64, whose tiles the mma.sync kernel walks as fast, want full tiles.  Measured, mma.sync /
     tcgen05: 16 heads over 4 of 128, planes: 128 tokens 4.4, 2 x 64 4.0, 8 x 64 2.2, 16 x 32 0.83, 2,000 3.9; own values: 128 1.2, 16 x 64 0.75,
-    2,000 3.4; heads of 64, 16 over 2, planes: 128 1.6, 16 x 32 0.53, 6 x 100 1.04; own values: 128 0.84, 400 0.99, 1,000 1.9."""
+    2,000 3.4; heads of 64, 16 over 2, planes: 128 1.6, 300 1.75, 16 x 32 0.53, 6 x 100 1.04; own values: 128 0.84, 400 0.99, 1,000 1.9."""
     tokens, wide, narrow = sum(new_lens), sum(-(-n // 128) for n in new_lens) * 128, sum(-(-n // 64) for n in new_lens) * 64
     if d < 128 and not planes:
         return tokens >= 400 * len(new_lens)
-    if planes and wide * heads <= (16384 if d >= 128 else 8192):
+    if planes and (len(new_lens) == 1 or wide * heads <= (16384 if d >= 128 else 8192)):
         return True
     return wide <= (1.75 if d >= 128 else 1.1) * narrow
 

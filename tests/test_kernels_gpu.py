@@ -989,7 +989,8 @@ def test_sink_prompts_take_the_tiles_they_fill():
     rows = lambda d, news, heads, planes: o.prefill_tile_rows(torch.bfloat16, d, 64, sum(news), sink=True, all_values=planes, heads=heads, new_lens=news)
     for d, news, heads, planes, want in ((128, [128], 16, False, 128), (128, [127], 16, False, 64), (128, [16] * 16, 32, False, 64), (128, [16] * 16, 32, True, 64),
                                          (128, [64] * 2, 16, True, 128), (128, [300, 45, 211, 127, 512], 16, True, 128), (64, [300], 16, False, 64),
-                                         (64, [400], 16, False, 128), (64, [16] * 8, 16, True, 64), (64, [256] * 4, 16, True, 128)):
+                                         (64, [400], 16, False, 128), (64, [16] * 8, 16, True, 64), (64, [256] * 4, 16, True, 128),
+                                         (64, [300], 32, True, 128), (64, [300, 20], 32, True, 64)):
         assert rows(d, news, heads, planes) == want, (d, news, heads, planes)
     assert o.prefill_tile_rows(torch.bfloat16, 128, 64, 500, sink=True) == 128
 
