@@ -450,6 +450,10 @@ static int launch_typed(const AttnArgs& a, int dtype, dim3 grid, cudaStream_t st
     return launch<float, DECODE, false, ALL>(a, grid, stream);
 }
 
+// attention_decode_f32.cu: float32 decode rows whose keys are cut over warps
+bool attention_decode_f32_takes(const AttnArgs& a);
+int attention_decode_f32(const AttnArgs& a, int requests, cudaStream_t stream);
+
 static int check_common(const char* name, int nq, int nkv, int d, int page_size, int dv) {
     LILY_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "%s: %d query heads do not group over %d kv heads", name, nq, nkv);
     // dv < 0: the values are the first -dv columns of the key rows
@@ -550,7 +554,8 @@ LILY_API int lily_attention_decode_simt(const void* q, const void* kv, void* out
     a.part_ml = scratch ? scratch + (size_t)requests * nq * splits * d_out : nullptr;
     dim3 grid(requests, nkv * chunks, splits);
     LILY_REQUIRE(grid.y <= 65535, "attention_decode: %d kv heads", nkv);
-    int rc = launch_typed<true>(a, dtype, grid, stream);
+    int rc = dtype == kF32 && attention_decode_f32_takes(a) ? attention_decode_f32(a, requests, stream)
+                                                            : launch_typed<true>(a, dtype, grid, stream);
     if (rc) return rc;
     LILY_CHECK_LAUNCH("attention_decode");
     if (splits > 1) {

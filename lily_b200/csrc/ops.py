@@ -1031,6 +1031,13 @@ def whole_rows_pay(pairs: int, sm_count: int = 148) -> bool:
     return last == 0 or last >= 0.45 * places
 
 
+def f32_rows_take(dtype: torch.dtype, group: int, d: int, dv: int) -> bool:
+    """Whether float32 decode rows go to the kernel that cuts a row's keys over warps (attention_decode_f32.cu).  One block of 16 warps a SM:
+    its ranges are cut for one wave of blocks and at least 64 keys, one round of a block.  Whole / in such ranges, us: 3 rows of 250
+    keys, 4 kv heads of 128: 10.6 / 6.8 (with the combine kernel), of 150 8.2 / 7.5; 1 row of 64 keys 4.9 / 6.6, which stays whole."""
+    return dtype == torch.float32 and group <= 8 and d % 4 == 0 and dv % 4 == 0 and max(d, dv) <= 256
+
+
 def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, d: int, max_seq_len: int,
                           even: bool = False, dv: Optional[int] = None, values_in_keys: bool = False,
                           keep_first: int = 0, fusable: bool = True, cuda_cores: bool = False, page_size: int = 0) -> DecodePlan:
@@ -1063,7 +1070,10 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
     if even and tensor_cores and d <= 128 and _WHOLE_ROWS and whole_rows_pay(pairs, sm_count()):
         return DecodePlan(1, fusable and pairs <= 2 * sm_count(), 0, "whole rows", 3)
     room = (lambda s: decode_clusters(d, s, group)) if tensor_cores else None
-    splits = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), clusters=room)
+    if f32_rows_take(dtype, group, d, dv) and not values_in_keys and not cuda_cores:
+        splits = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), blocks_per_sm=1, min_keys=64, max_splits=12)
+    else:
+        splits = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), clusters=room)
     in_clusters = tensor_cores and splits > 1 and pairs <= decode_clusters(d, splits, group)
     fused = fusable and tensor_cores and pairs * splits <= 3 * sm_count()
     arm = "single" if splits == 1 else ("cluster" if in_clusters else "wave")

@@ -765,6 +765,33 @@ def test_attention_fp32_wide_and_element_by_element(nq, nkv, d, dv, page, window
             torch.testing.assert_close(got, want, **tol(torch.float32))
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("window,keep,cap,sinks", [(None, 0, None, False), (70, 0, 30.0, False), (70, 9, None, False), (None, 0, None, True)])
+@pytest.mark.parametrize("nq,nkv,d,dv,page", [(2, 2, 4, 8, 16), (4, 2, 132, 128, 16), (9, 3, 128, 64, 64), (14, 2, 128, 128, 8), (16, 2, 256, 252, 16),
+                                              (7, 1, 100, 100, 1)])
+def test_attention_decode_fp32_keys_over_warps(nq, nkv, d, dv, page, window, keep, cap, sinks, splits):
+    """float32 decode rows whose keys are cut over warps: fewer query heads than the kernel's one, two, four or eight, one piece of
+    128 columns and two, rows that end inside a warp's four keys and inside a round of all warps, ranges without keys, the
+    window's and the kept positions, a sink a head, a row so far ahead that its weight is all there is."""
+    seqs = [1, 2, 5, 31, 33, 64, 65, 257]
+    g = torch.Generator(device=DEV).manual_seed(d + dv + splits)
+    width = max(-(-s // page) for s in seqs)
+    cache = torch.randn(len(seqs) * width + 1, page * nkv * (d + dv), device=DEV, generator=g)
+    cache[0] = float("nan")                                    # a page that no row owns
+    table = (torch.randperm(len(seqs) * width, device=DEV, generator=g) + 1).view(len(seqs), width).to(torch.int32)
+    q = torch.randn(len(seqs), nq * d, device=DEV, generator=g)
+    q[3] *= 40.0
+    opts = dict(dv=dv, keep_first=keep, softcap=cap)
+    if sinks:
+        opts["sinks"] = torch.randn(nq, device=DEV, generator=g) * 3.0
+    seq_t = torch.tensor(seqs, device=DEV, dtype=torch.int32)
+    got, want = (torch.zeros(len(seqs), nq * dv, device=DEV) for _ in range(2))
+    scratch = torch.full((max(ops().decode_scratch_floats(len(seqs), nq, dv, splits), 1),), float("nan"), device=DEV)
+    ref.attention_decode(q, cache, table, seq_t, want, None, 1, nq, nkv, d, page, d ** -0.5, window, **opts)
+    ops().attention_decode(q, cache, table, seq_t, got, scratch, splits, nq, nkv, d, page, d ** -0.5, window, **opts)
+    torch.testing.assert_close(got, want, **tol(torch.float32))
+
+
 @pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16, 17])
 @pytest.mark.parametrize("width,ff,experts,identity,top,activation,on_input,shared", [
     (64, 64, 3, 0, 2, "silu", False, False), (192, 320, 16, 2, 4, "swish_clamped", False, False),
