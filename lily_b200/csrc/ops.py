@@ -1074,6 +1074,13 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
         splits = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), blocks_per_sm=1, min_keys=64, max_splits=12)
     else:
         splits = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), clusters=room)
+    if tensor_cores and max_seq_len >= 384:
+        # Short rows: ranges of 128 keys (two tiles a block) as long as the clusters merge them.  Ranges of 256 / 128, us: 1 row of 900 keys, 4 kv
+        # heads 8.1 / 6.7, of 2,000 9.2 / 7.7; 8 rows of 400 keys 8.3 / 7.3, of 900 over 8 kv heads 12.9 / 12.3; 20 of 500 11.3 / 10.6; but 16 of
+        # 200 keys over 8 kv heads 9.1 whole, 10.2 in two.
+        finer = choose_decode_splits(requests, nkv, max_seq_len, sm_count=sm_count(), min_keys=128, clusters=room)
+        if finer > splits and pairs <= decode_clusters(d, finer, group):
+            splits = finer
     in_clusters = tensor_cores and splits > 1 and pairs <= decode_clusters(d, splits, group)
     fused = fusable and tensor_cores and pairs * splits <= 3 * sm_count()
     arm = "single" if splits == 1 else ("cluster" if in_clusters else "wave")
