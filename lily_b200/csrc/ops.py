@@ -58,6 +58,7 @@ _SIGNATURES = {
     "lily_add_normed_rmsnorm": [_vp, _vp, _i, _i, _sz, _vp, _f, _f, _vp, _i, _vp, _i, _vp, _i, _i, _f, _i, _i, _vp],
     "lily_head_mix": [_vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_delta_rule": [_vp, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _vp],
+    "lily_delta_chunks": [_vp, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _f, _f, _vp],
     "lily_selective_scan": [_vp, _vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _vp, _vp, _vp],
     "lily_selective_combine": [_vp, _sz, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp],
     "lily_activation": [_vp, _i, _i, _sz, _vp, _i, _sz, _i, _f, _f, _vp],
@@ -168,6 +169,10 @@ def library():
         lib.lily_moe_few_pays.argtypes = [_i, _i, _i, _i, _i]
         lib.lily_moe_few_pays.restype = _i
         lib.lily_delta_rule_max_head_dim.restype = _i
+        lib.lily_delta_chunks_take.argtypes = [_vp, _i, _i, _i, _i, _i, _i, _i, _i]
+        lib.lily_delta_chunks_take.restype = _i
+        lib.lily_delta_chunk_tokens.restype = _i
+        lib.lily_delta_chunk_floats.restype = _i
         lib.lily_selective_scan_max_state.restype = _i
         lib.lily_mlstm_max_head_dim.restype = _i
         lib.lily_mlstm_chunk_takes.argtypes = [_i, _i]
@@ -2063,16 +2068,69 @@ def delta_rule_max_head_dim() -> int:
     return int(library().lily_delta_rule_max_head_dim())
 
 
+@dataclass
+class DeltaPlan:
+    """How a step's delta rule is cut: the first ``singles`` requests bring one token each and run token by token, the portions of
+    the others go in chunks.  The lists are int32 on the device, requests counted from ``singles`` on."""
+
+    singles: int
+    item_req: torch.Tensor
+    item_start: torch.Tensor
+    first_item: torch.Tensor
+    items: int
+
+
+def delta_chunks_pay(new_lens: Sequence[int], heads: int, d: int, dv: int) -> bool:
+    """Whether portions are faster as chunks of 64 tokens on the tensor cores than one token after another.  Token by token the longest
+    portion's chain counts, 0.42 us a token with heads of 128, or the blocks of 8 value columns once they fill the device; in chunks 25 us
+    and the longest portion's chain, 3.6 us a chunk, or the blocks of 16 columns, one a SM.  Measured, us, one after another / in chunks, 16 heads
+    of 128 x 128 over 4: one portion of 33 tokens 19 / 28, of 64 31 / 29, of 100 47 / 32, of 1,999 843 / 141; 32 of 8 83 / 158; 12 of
+    24 77 / 75, of 40 118 / 76, of 170 460 / 156; 32 heads over 8: one of 2,048 1,045 / 279, three of 700 974 / 286; 8 heads of 64 x 64:
+    one of 2,048 531 / 116."""
+    longest, tokens = max(new_lens), sum(new_lens)
+    tiles = [-(-n // 64) for n in new_lens]
+    alone = 4.0 + (0.24 + 0.76 * min(d, 128) / 128) * max(0.42 * longest, 0.00012 * tokens * heads * dv)
+    return alone > 25.0 + max(3.6 * max(tiles), 0.0019 * sum(tiles) * heads * dv)
+
+
+def delta_plan(new_lens: Sequence[int], dtype: torch.dtype, heads: int, kv_heads: int, d: int, dv: int, device) -> Optional[DeltaPlan]:
+    """None when every token runs by itself: decode steps, short portions, float32, and sizes the chunk kernels do not take.
+    (The requests that bring one token come first in a step.)"""
+    singles = next((i for i, n in enumerate(new_lens) if n != 1), len(new_lens))
+    lens = new_lens[singles:]
+    lib = library()
+    chunk = int(lib.lily_delta_chunk_tokens())
+    if dtype != torch.bfloat16 or not lens or not lib.lily_delta_chunks_take(None, 8, 0, kv_heads * d, 2 * kv_heads * d, heads, kv_heads, d, dv):
+        return None
+    items = sum(-(-n // chunk) for n in lens)
+    if not delta_chunks_pay(lens, heads, d, dv) or items * heads * int(lib.lily_delta_chunk_floats()) * 4 > SCAN_WORKSPACE:
+        return None
+    req, start, first = [], [], []
+    for r, n in enumerate(lens):
+        first.append(len(req))
+        req += [r] * -(-n // chunk)
+        start += range(0, n, chunk)
+    flat = torch.tensor(req + start + first, dtype=torch.int32).to(device, non_blocking=True)
+    parts = torch.split(flat, [items, items, len(lens)])
+    return DeltaPlan(singles, parts[0], parts[1], parts[2], items)
+
+
+def delta_workspace_floats(plan: Optional[DeltaPlan], heads: int) -> int:
+    return 0 if plan is None else plan.items * heads * int(library().lily_delta_chunk_floats())
+
+
 def delta_rule(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, a_log: torch.Tensor, dt_bias: torch.Tensor,
                state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, requests: int, heads: int, kv_heads: int,
-               d: int, dv: int, unit_eps: float, q_scale: float) -> torch.Tensor:
+               d: int, dv: int, unit_eps: float, q_scale: float, plan: Optional[DeltaPlan] = None,
+               workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The gated delta rule over each request's new tokens, from and to ``state[slot, :heads * dv * d]`` (float32,
     a head's matrix as [dv, d]).  ``qkv`` [tokens, (2 kv_heads) d + heads dv]: q, k, v behind their convolution and
     activation; ``proj`` [tokens, width]: ``heads`` columns from ``b_col`` (the write strength before its sigmoid) and
     from ``a_col`` (the decay's input).  q and k are made unit vectors per head here (``unit_eps`` inside the root; q
     times ``q_scale``); the decay is ``exp(-exp(a_log) softplus(a + dt_bias))``.  Returns float32 [tokens, heads * dv],
-    each token read out after its own write."""
-    _dev(qkv, proj, a_log, dt_bias, state, cu_seqlens, slots)
+    each token read out after its own write.  With a ``plan`` (``delta_plan``) portions run in chunks on the tensor cores through
+    ``workspace`` (float32, ``delta_workspace_floats``; made here when absent)."""
+    _dev(qkv, proj, a_log, dt_bias, state, cu_seqlens, slots, workspace)
     n = qkv.shape[0]
     if qkv.shape[1] != 2 * kv_heads * d + heads * dv or proj.shape[0] != n or qkv.dtype != proj.dtype:
         raise KernelError("delta_rule: qkv is [tokens, 2 kv_heads d + heads dv] in the projection's dtype")
@@ -2080,9 +2138,24 @@ def delta_rule(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, a_
             or a_log.numel() != heads or dt_bias.numel() != heads or state.dtype != torch.float32 or state.dim() != 2:
         raise KernelError("delta_rule: columns out of range, or decay constants / state not float32")
     y = torch.empty((n, heads * dv), dtype=torch.float32, device=qkv.device)
-    _call("lily_delta_rule", _p(qkv), qkv.shape[1], 0, kv_heads * d, 2 * kv_heads * d, _p(proj), proj.shape[1], int(b_col),
-          int(a_col), _p(a_log), _p(dt_bias), _p(state), state.shape[1], _p(y), _i32(cu_seqlens, "cu_seqlens"),
-          _i32(slots, "slots"), int(requests), n, heads, kv_heads, d, dv, float(unit_eps), float(q_scale), _dt(qkv), _stream())
+    columns = (_p(qkv), qkv.shape[1], 0, kv_heads * d, 2 * kv_heads * d, _p(proj), proj.shape[1], int(b_col), int(a_col), _p(a_log),
+               _p(dt_bias), _p(state), state.shape[1], _p(y))
+    cu, slot = _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots")
+    if plan is not None and not (qkv.dtype == torch.bfloat16 and library().lily_delta_chunks_take(*columns[:5], heads, kv_heads, d, dv)):
+        plan = None                       # (rows that do not start on 16 bytes)
+    if plan is None or plan.singles:
+        _call("lily_delta_rule", *columns, cu, slot, int(requests) if plan is None else plan.singles, n if plan is None else plan.singles,
+              heads, kv_heads, d, dv, float(unit_eps), float(q_scale), _dt(qkv), _stream())
+    if plan is not None:
+        need = delta_workspace_floats(plan, heads)
+        if workspace is None:
+            workspace = torch.empty(need, dtype=torch.float32, device=qkv.device)
+        if workspace.dtype != torch.float32 or workspace.numel() < need:
+            raise KernelError(f"delta_rule: a float32 workspace of {need} entries needed")
+        _call("lily_delta_chunks", *columns, cu + 4 * plan.singles, slot + 4 * plan.singles, int(requests) - plan.singles, _p(plan.item_req),
+              _p(plan.item_start), _p(plan.first_item), plan.items, _p(workspace), heads, kv_heads, d, dv, float(unit_eps), float(q_scale),
+              _stream())
+        launches["count"] += 1            # two kernels
     return y
 
 

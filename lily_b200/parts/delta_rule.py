@@ -127,9 +127,16 @@ class DeltaRule(Mixer):
         proj = ops.linear(x, self.w_in)                                       # [tokens, q | k | v | gate | beta | alpha]
         qkv = ops.causal_conv_silu(proj, 0, s.channels, self.conv_w, None, state, self.matrix_floats, chunk_req,
                                    chunk_start, batch.cu_seqlens, batch.slots, chunk)
+        chunks = {}
+        if batch.num_tokens > batch.num_requests and hasattr(ops, "delta_plan"):       # (a stand-in may run token by token only)
+            plan = batch.plan(("delta_plan", s.heads, s.kv_heads, s.head_dim, s.v_head_dim), lambda b: ops.delta_plan(
+                b.h_new_lens, x.dtype, s.heads, s.kv_heads, s.head_dim, s.v_head_dim, x.device))
+            if plan is not None:
+                floats = ops.delta_workspace_floats(plan, s.heads)
+                chunks = {"plan": plan, "workspace": batch.workspace.floats("delta_chunks", floats) if batch.workspace is not None else None}
         y = ops.delta_rule(qkv, proj, s.channels + s.inner, s.channels + s.inner + s.heads, self.a_log, self.dt_bias, state,
                            batch.cu_seqlens, batch.slots, batch.num_requests, s.heads, s.kv_heads, s.head_dim, s.v_head_dim,
-                           s.unit_eps, s.head_dim ** -0.5)
+                           s.unit_eps, s.head_dim ** -0.5, **chunks)
         gate = proj[:, s.channels:s.channels + s.inner]
         normed = ops.group_rmsnorm_gate(y, gate, self.gain, s.heads, s.norm_eps)
         return ops.linear_auto(normed, self.w_o)

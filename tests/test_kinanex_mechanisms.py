@@ -328,6 +328,77 @@ def test_delta_rule_reads_after_hundreds_of_steps_what_the_first_token_wrote(dev
           torch.float32)
 
 
+# ------------------------------------------------------------------ the delta rule in chunks
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[64], [1, 1, 33, 2, 130], [65, 63, 16, 15, 257]])
+@pytest.mark.parametrize("heads,kvh,d,dv", [(2, 2, 16, 16), (6, 1, 48, 32), (4, 4, 64, 16), (10, 2, 80, 48), (4, 1, 128, 128)])
+def test_delta_rule_in_chunks(monkeypatch, lens, heads, kvh, d, dv):
+    """Portions in chunks of 64 tokens on the tensor cores, beside single tokens: chunks and tiles of 16 tokens that end early, head sizes that fill
+    no run of 64 or 128, more value heads a key head than are prepared at a time, states carried in and out of their slots."""
+    ops = ops_for("cuda")
+    monkeypatch.setattr(ops, "delta_chunks_pay", lambda *a: True)
+    data = [delta_inputs(n, heads, kvh, d, dv, 40 + i, torch.bfloat16) for i, n in enumerate(lens)]
+    a_log, dt_bias = data[0][2], data[0][3]
+    before = [delta_inputs(3, heads, kvh, d, dv, 60 + i, torch.bfloat16) for i in range(len(lens))]
+    state = torch.zeros((len(lens) + 1, heads * d * dv + 3), device="cuda")
+    state[:, -3:] = 7.0
+    slots = i32(list(range(len(lens), 0, -1)), "cuda")
+    run = lambda rows, ns, plan: ops.delta_rule(torch.cat([x[0] for x in rows]).cuda(), torch.cat([x[1] for x in rows]).cuda(), 3, 3 + heads, a_log.cuda(),
+                                                dt_bias.cuda(), state, i32([0] + torch.tensor(ns).cumsum(0).tolist(), "cuda"), slots, len(ns), heads, kvh,
+                                                d, dv, 1e-6, d ** -0.5, plan=plan)
+    run(before, [3] * len(lens), None)
+    plan = ops.delta_plan(lens, torch.bfloat16, heads, kvh, d, dv, torch.device("cuda"))
+    assert plan is not None and plan.singles == lens.count(1)
+    y = run(data, lens, plan).view(-1, heads, dv)
+    after = run(before, [3] * len(lens), None).view(len(lens), 3, heads, dv)
+    at = 0
+    for i, n in enumerate(lens):
+        rows = [torch.cat([b, x, b]) for b, x in zip(before[i][:2], data[i][:2])]
+        want = plain_delta(rows[0], rows[1], a_log, dt_bias, heads, kvh, d, dv)
+        got = torch.cat([y[at:at + n], after[i]]).cpu()
+        at += n
+        # sums of d + 64 products, each rounded to 2^-24, in four such products one behind the other
+        bound = 4 * (d + 64) ** 0.5 * 2.0 ** -24
+        assert float((got - want[3:]).norm() / want[3:].norm()) < bound
+    assert float((state[:, -3:] - 7.0).abs().max()) == 0.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("token", [5, 15, 64, 100])
+@pytest.mark.parametrize("what", ["v", "k", "q", "alpha", "infinite v"])
+def test_delta_rule_in_chunks_keeps_what_is_not_finite_behind_its_token(monkeypatch, token, what):
+    ops = ops_for("cuda")
+    monkeypatch.setattr(ops, "delta_chunks_pay", lambda *a: True)
+    heads, kvh, d, dv, n = 4, 2, 64, 32, 140
+    qkv, proj, a_log, dt_bias = (x.cuda() for x in delta_inputs(n, heads, kvh, d, dv, 3, torch.bfloat16))
+    plan = ops.delta_plan([n], torch.bfloat16, heads, kvh, d, dv, torch.device("cuda"))
+
+    def run():
+        state = torch.zeros((2, heads * d * dv), device="cuda")
+        return ops.delta_rule(qkv, proj, 3, 3 + heads, a_log, dt_bias, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, heads, kvh, d, dv, 1e-6,
+                              d ** -0.5, plan=plan).view(n, heads, dv), state
+    clean, _ = run()
+    if what in ("v", "infinite v"):
+        qkv[token, 2 * kvh * d + dv + 9] = float("nan") if what == "v" else float("inf")      # value head 1, column 9
+    elif what == "alpha":
+        proj[token, 3 + heads + 1] = float("nan")
+    else:
+        qkv[token, (kvh * d if what == "k" else 0) + 7] = float("nan")                         # query/key head 0: value heads 0 and 1
+    y, state = run()
+    hit = torch.zeros(n, heads, dv, dtype=torch.bool, device="cuda")
+    if what == "q":
+        hit[token, :2] = True
+    elif what == "k":
+        hit[token:, :2] = True
+    elif what == "alpha":
+        hit[token:, 1] = True
+    else:
+        hit[token:, 1, 9] = True
+    assert not torch.isfinite(y[hit]).any() and torch.isfinite(y[~hit]).all()
+    torch.testing.assert_close(y[~hit], clean[~hit], atol=1e-5, rtol=1e-5)
+    assert bool(torch.isfinite(state).all()) == (what == "q")
+
 # ------------------------------------------------------------------ the selective scan
 
 def plain_scan(x, low, rank, step, z, a_log, d_skip):
