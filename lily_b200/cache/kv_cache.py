@@ -79,11 +79,19 @@ class KVCacheManager:
                     (need.kv_heads * page_size * (need.head_dim + value_columns(need)),)
                 data = torch.zeros((layers, num_pages + 1, *shape), dtype=dtype, device=device)
             self.groups.append(CacheGroup(need, layers, GroupTables(num_pages, page_size, need.window, need.keep_first), data))
-        self.states: List[Optional[torch.Tensor]] = []
         self.state_needs = list(states)
-        for need in states:
-            self.states.append(None if device is None else
-                               torch.zeros((max_requests + 1, *need.shape), dtype=need.dtype, device=device))
+        # states of one kind lie in one tensor [of that kind, slots, ...], so that a request's rows of all of them are zeroed at once
+        kinds: Dict[StateNeed, List[int]] = {}
+        for i, need in enumerate(self.state_needs):
+            kinds.setdefault(need, []).append(i)
+        self._state_kinds: List[torch.Tensor] = []
+        self.states: List[Optional[torch.Tensor]] = [None] * len(self.state_needs)
+        if device is not None:
+            for need, members in kinds.items():
+                rows = torch.zeros((len(members), max_requests + 1, *need.shape), dtype=need.dtype, device=device)
+                self._state_kinds.append(rows)
+                for k, i in enumerate(members):
+                    self.states[i] = rows[k]
         self.lengths: Dict[int, int] = {}            # slot -> positions whose pages are held
 
     # ---- requests ------------------------------------------------------------
@@ -92,9 +100,8 @@ class KVCacheManager:
         slot = self.slots.alloc()
         for g in self.groups:
             g.tables.open(slot)
-        for s in self.states:
-            if s is not None:
-                s[slot].zero_()
+        for rows in self._state_kinds:
+            rows[:, slot].zero_()
         self.lengths[slot] = 0
         return slot
 

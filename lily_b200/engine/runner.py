@@ -25,7 +25,7 @@ from lily_b200.config.model_config import read_model_dir
 from lily_b200.config.registry import architecture_names, resolve_architecture
 from lily_b200.config.server_args import ServerArgs
 from lily_b200.engine import check
-from lily_b200.engine.batch import FUTURE, StepBatch, StepEntry, Workspace, build_step_batch, order_entries, rows_are_even
+from lily_b200.engine.batch import FUTURE, StepBatch, StepEntry, Workspace, build_step_batch, order_entries, rows_are_even, wire_array
 from lily_b200.engine.profiler import DecodeProfiler
 from lily_b200.models.assembled import AssembledModel
 from lily_b200.parts.base import BuildContext, ModelSpec
@@ -289,6 +289,7 @@ class ModelRunner:
             raise ValueError("a step needs at least one entry")
         vocab = self.spec.vocab_size
         seen = set()
+        arrays = []
         for e in entries:
             if e.slot not in self.seq_lens:
                 raise KeyError(f"request slot {e.slot} is not open")
@@ -297,8 +298,13 @@ class ModelRunner:
             seen.add(e.slot)
             if len(e.tokens) == 0:
                 raise ValueError("an entry brings at least one token")
-            if not (len(e.tokens) == 1 and int(e.tokens[0]) == FUTURE) and any(not (0 <= int(t) < vocab) for t in e.tokens):
+            try:
+                ids = wire_array(e)
+            except OverflowError:
+                raise ValueError(f"token id outside [0, {vocab})") from None
+            if not (len(e.tokens) == 1 and int(e.tokens[0]) == FUTURE) and not (0 <= ids.min() and ids.max() < vocab):
                 raise ValueError(f"token id outside [0, {vocab})")
+            arrays.append(ids)
             if self.seq_lens[e.slot] + len(e.tokens) > self.context_len:
                 raise ValueError(f"request would reach {self.seq_lens[e.slot] + len(e.tokens)} positions; "
                                  f"the context length is {self.context_len}")
@@ -328,7 +334,7 @@ class ModelRunner:
             len(entries) * max((len(t) for t in g), default=1) for g in tables) + 8
         pinned, ring_index = self._ring.take(need) if self._ring is not None else (None, -1)
         batch = build_step_batch(ordered, prefix, tables, self.device, workspace=self.workspace, pinned=pinned,
-                                 logit_rows=rows)
+                                 logit_rows=rows, token_arrays=[arrays[i] for i in order])
         if self._ring is not None:
             self._ring.mark(ring_index)
         batch.future_tokens = self.future_tokens

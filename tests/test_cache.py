@@ -135,3 +135,19 @@ def test_table_stamps_change_with_the_table_and_are_never_shared():
     assert b == a
     cache.grow(b, 40)
     assert not {cache.table_stamp(0, b), cache.table_stamp(1, b)} & seen
+
+
+def test_a_new_request_zeroes_its_row_of_every_state_and_no_other():
+    """States of one kind share a tensor: rows of other slots and of other kinds stay, and each state keeps its own shape and type."""
+    import torch
+    from lily_b200.cache.kv_cache import KVCacheManager
+    from lily_b200.parts.base import CacheNeed, StateNeed
+    needs = [StateNeed((2, 3)), StateNeed((5,)), StateNeed((2, 3)), StateNeed((5,), torch.bfloat16)]
+    cache = KVCacheManager([(CacheNeed(1, 16, None), 1)], needs, page_size=8, num_pages=4, max_requests=3, max_context=32,
+                           dtype=torch.float32, device=torch.device("cpu"))
+    for state, need in zip(cache.states, needs):
+        assert state.shape == (4, *need.shape) and state.dtype == need.dtype and state.is_contiguous()
+        state.fill_(1.0)
+    slot = cache.open_request()
+    for state in cache.states:
+        assert not state[slot].any() and bool((state[[s for s in range(4) if s != slot]] == 1).all())

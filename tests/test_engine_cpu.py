@@ -68,6 +68,28 @@ def test_wanted_rows_come_in_the_given_order(setup):
     assert float((out - want).abs().max()) < TOL
 
 
+def test_a_step_takes_ids_of_any_kind_and_refuses_others(setup):
+    """Ids come as a list, a tuple, an array or a tensor, and as numbers that are whole; one outside the vocabulary anywhere in a portion is
+    refused before a page is taken."""
+    import numpy as np
+    from lily_b200.engine.batch import StepEntry
+    cfg, _, path = setup
+    v = cfg["vocab_size"]
+    ids = tiny_models.random_tokens(7, v, 4)
+    runner = make_runner(path)
+    outs = []
+    for tokens in (ids, tuple(ids), np.array(ids), np.array(ids, dtype=np.int16), torch.tensor(ids), [float(t) for t in ids], [np.int64(t) for t in ids]):
+        slot = runner.open_request()
+        outs.append(runner.step([StepEntry(slot, tokens, [6])]))
+        runner.close_request(slot)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    slot = runner.open_request()
+    for bad in (ids[:3] + [v] + ids[3:], [-1] + ids, ids + [1 << 40], [v], [-(1 << 40)], np.array(ids + [v])):
+        with pytest.raises(ValueError, match="token id"):
+            runner.step([StepEntry(slot, bad, [0])])
+    assert runner.cache.held_pages() == [0] * len(runner.cache.groups)
+
+
 def test_decode_splits_follow_the_clusters_that_fit():
     """With the kernel's answer on how many clusters of s blocks fit (a B200's, head size 128), the most ranges
     whose clusters are all resident; without it, or with more rows than clusters of two, the wave rule."""
