@@ -82,13 +82,15 @@ __global__ void token_shift_mix_kernel(const T* __restrict__ h, int tokens, int 
 
 // ---------------------------------------------------------------------------- the decay's logarithm
 
-// grid (ceil(tokens / 8), ceil(cols / 128)), block 128; a [tokens, rank] float32, w2t [rank, cols] float32 (the second
-// matrix of the low-rank pair, transposed so that neighbouring threads read neighbouring numbers), w0 [cols].  A block
-// takes eight tokens, so a number of w2t read once serves eight sums.
-// With few blocks the loop over the rank waits for memory: AHEAD rows of w2t are asked for at once, the first before the kernel ahead has
-// finished (they are weights): rank 64, 2,048 columns, a row at a time / 32: 8.6 / 6.7 us with 1 token, 9.7 / 7.7 with 64.  With more
-// blocks than two a SM others run meanwhile, and the registers of 32 rows are in the way, so AHEAD is 0, a row at a time: 2,048 tokens
-// 52 us with 32, 35 so; 64 tokens, rank 256, 8,192 columns, 512 blocks, 49 and 32.
+template <int N> struct Number { static constexpr int value = N; };
+
+// a [tokens, rank] float32, w2t [rank, cols] float32 (the second matrix of the low-rank pair, transposed so that neighbouring threads
+// read neighbouring numbers), w0 [cols].  Every kernel sums over the rank in order.
+//
+// Few blocks (at most two a SM): grid (ceil(tokens / 8), ceil(cols / 128)), block 128, a column a thread.  The loop over the rank would wait
+// for memory, so AHEAD rows of w2t are asked for at once, the first before the kernel ahead has finished (they are weights), and only the
+// tokens that are there are summed.  Rank 64, 2,048 columns, us (a row at a time / 32 rows and eight sums whatever the tokens / now): 1 token
+// 8.6 / 6.5 / 2.0, 2 tokens - / 6.5 / 4.1, 64 tokens 9.7 / 7.6 / 6.8; rank 256, 8,192 columns, 1 token - / 23 / 6.3.
 constexpr int DECAY_TOKENS = 8;
 template <int AHEAD>
 __global__ void wkv_decay_kernel(const float* __restrict__ a, int tokens, int rank, const float* __restrict__ w2t,
@@ -118,20 +120,70 @@ __global__ void wkv_decay_kernel(const float* __restrict__ a, int tokens, int ra
             for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = fmaf(th[t * rank + j], one, z[t]);
         }
     } else {
-        for (int j0 = 0; j0 < rank; j0 += AHEAD) {
-            const int now = min(AHEAD, rank - j0);
+        auto sum = [&](auto most, int j0, int now) {
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j)
                 if (j < now) {
 #pragma unroll
-                    for (int t = 0; t < DECAY_TOKENS; ++t) z[t] = fmaf(th[t * rank + j0 + j], w[j], z[t]);
+                    for (int t = 0; t < decltype(most)::value; ++t) z[t] = fmaf(th[t * rank + j0 + j], w[j], z[t]);
                 }
+        };
+        for (int j0 = 0; j0 < rank; j0 += AHEAD) {
+            const int now = min(AHEAD, rank - j0);
+            if (nt == 1) sum(Number<1>{}, j0, now);
+            else if (nt == 2) sum(Number<2>{}, j0, now);
+            else if (nt <= 4) sum(Number<4>{}, j0, now);
+            else sum(Number<DECAY_TOKENS>{}, j0, now);
             if (j0 + AHEAD < rank) ask(j0 + AHEAD);
         }
     }
 #pragma unroll
     for (int t = 0; t < DECAY_TOKENS; ++t)
         if (t < nt) lw[(size_t)(t0 + t) * cols + c] = -expf(z[t] + b);
+}
+
+// Many blocks: bound by FFMA and the reads that feed it, so a thread has four columns of 16 tokens, 64 multiply-adds for one 16-byte read of
+// w2t and four of the tokens' tanh.  grid (ceil(tokens / 16), ceil(cols / 512)), block 128; cols a multiple of four, rows on 16 bytes (other
+// shapes stay with AHEAD 0 above).  Rank 64, 2,048 columns, 1,920 tokens: 33 -> 17 us (7 at the FFMA rate); 64 tokens,
+// rank 256, 8,192 columns: 49 -> 34.
+constexpr int WIDE_TOKENS = 16;
+__global__ void __launch_bounds__(128) wkv_decay_wide_kernel(const float* __restrict__ a, int tokens, int rank, const float* __restrict__ w2t,
+                                                             const float* __restrict__ w0, int cols, float* __restrict__ lw) {
+    extern __shared__ __align__(16) float th[];          // [rank][16]: tanh(a[t, :])
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    pdl_enter_small();
+    const int t0 = blockIdx.x * WIDE_TOKENS, nt = min(WIDE_TOKENS, tokens - t0);
+    for (int i = threadIdx.x; i < WIDE_TOKENS * rank; i += 128) {
+        const int t = i / rank, j = i - t * rank;
+        th[j * WIDE_TOKENS + t] = t < nt ? tanhf(a[(size_t)t0 * rank + i]) : 0.f;
+    }
+    __syncthreads();
+    if (c >= cols) return;
+    float z[WIDE_TOKENS][4] = {};
+    const float4* src = reinterpret_cast<const float4*>(w2t + c);
+    const size_t step = cols / 4;
+#pragma unroll 4
+    for (int j = 0; j < rank; ++j) {
+        const float4 w = src[j * step];
+#pragma unroll
+        for (int t = 0; t < WIDE_TOKENS; t += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(th + j * WIDE_TOKENS + t);
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                z[t + e][0] = fmaf(xs[e], w.x, z[t + e][0]);
+                z[t + e][1] = fmaf(xs[e], w.y, z[t + e][1]);
+                z[t + e][2] = fmaf(xs[e], w.z, z[t + e][2]);
+                z[t + e][3] = fmaf(xs[e], w.w, z[t + e][3]);
+            }
+        }
+    }
+    const float4 b = *reinterpret_cast<const float4*>(w0 + c);
+#pragma unroll
+    for (int t = 0; t < WIDE_TOKENS; ++t)
+        if (t < nt)
+            *reinterpret_cast<float4*>(lw + (size_t)(t0 + t) * cols + c) =
+                make_float4(-expf(z[t][0] + b.x), -expf(z[t][1] + b.y), -expf(z[t][2] + b.z), -expf(z[t][3] + b.w));
 }
 
 // ---------------------------------------------------------------------------- the recurrence
@@ -471,8 +523,14 @@ LILY_API int lily_wkv_decay(const float* a, int tokens, int rank, const float* w
     LILY_REQUIRE(rank > 0 && cols > 0, "wkv_decay: rank=%d cols=%d", rank, cols);
     dim3 grid((tokens + DECAY_TOKENS - 1) / DECAY_TOKENS, (cols + 127) / 128), block(128);
     LILY_REQUIRE(grid.y <= 65535 && rank <= 1024, "wkv_decay: %d columns, rank %d", cols, rank);
-    auto kern = (long long)grid.x * grid.y <= 2 * sm_count() ? wkv_decay_kernel<32> : wkv_decay_kernel<0>;
-    launch_pdl(kern, grid, block, (size_t)DECAY_TOKENS * rank * sizeof(float), stream, a, tokens, rank, w2t, w0, cols, lw);
+    const bool few = (long long)grid.x * grid.y <= 2 * sm_count();
+    if (!few && cols % 4 == 0 && (((uintptr_t)w2t | (uintptr_t)w0 | (uintptr_t)lw) & 15) == 0 && rank <= 512) {
+        launch_pdl(wkv_decay_wide_kernel, dim3((tokens + WIDE_TOKENS - 1) / WIDE_TOKENS, (cols + 511) / 512), block,
+                   (size_t)WIDE_TOKENS * rank * sizeof(float), stream, a, tokens, rank, w2t, w0, cols, lw);
+    } else {
+        auto kern = few ? (rank <= 32 ? wkv_decay_kernel<32> : wkv_decay_kernel<64>) : wkv_decay_kernel<0>;
+        launch_pdl(kern, grid, block, (size_t)DECAY_TOKENS * rank * sizeof(float), stream, a, tokens, rank, w2t, w0, cols, lw);
+    }
     LILY_CHECK_LAUNCH("wkv_decay");
     return 0;
 }

@@ -867,7 +867,8 @@ def test_wkv_scan_of_one_token_a_request(dtype, requests, heads, d):
     torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
 
 
-@pytest.mark.parametrize("tokens,rank,cols", [(1, 1, 5), (2, 64, 2048), (8, 31, 130), (9, 33, 257), (21, 200, 128), (2364, 33, 128), (2371, 33, 130)])
+@pytest.mark.parametrize("tokens,rank,cols", [(1, 1, 5), (2, 64, 2048), (8, 31, 130), (9, 33, 257), (21, 200, 128), (2364, 33, 128), (2371, 33, 130), (3, 130, 384),
+                                              (4, 64, 64), (5, 65, 100), (1193, 64, 516), (2380, 5, 132)])
 def test_wkv_decay_by_rows_asked_for_ahead(tokens, rank, cols):
     g = torch.Generator(device=DEV).manual_seed(rank)
     a, w2t, w0 = (torch.randn(*s, device=DEV, generator=g) for s in ((tokens, rank), (rank, cols), (cols,)))
