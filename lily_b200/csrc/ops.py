@@ -58,6 +58,7 @@ _SIGNATURES = {
     "lily_add_normed_rmsnorm": [_vp, _vp, _i, _i, _sz, _vp, _f, _f, _vp, _i, _vp, _i, _vp, _i, _i, _f, _i, _i, _vp],
     "lily_head_mix": [_vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_delta_rule": [_vp, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _vp],
+    "lily_wkv_chunk": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
     "lily_delta_chunks": [_vp, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _f, _f, _vp],
     "lily_selective_scan": [_vp, _vp, _i, _i, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _vp, _vp, _vp],
     "lily_selective_combine": [_vp, _sz, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp],
@@ -160,6 +161,8 @@ def library():
         lib.lily_ssd_step_takes.restype = _i
         lib.lily_ssd_step_pays.argtypes = [_i, _i, _i, _i, _i]
         lib.lily_ssd_step_pays.restype = _i
+        lib.lily_wkv_chunk_takes.argtypes = [_vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i]
+        lib.lily_wkv_chunk_takes.restype = _i
         lib.lily_wkv_step_takes.argtypes = [_vp, _sz, _vp, _i, _i, _i]
         lib.lily_wkv_step_takes.restype = _i
         lib.lily_wkv_step_pays.argtypes = [_i, _i, _i]
@@ -1508,14 +1511,16 @@ def wkv_max_head_dim() -> int:
 
 WKV_CHUNK = 64          # tokens a chunk of a long portion
 WKV_DIRECT = 128        # portions up to this many tokens run in one piece, from and to the matrices in the slot
+WKV_FINE = 33           # tokens from which a portion can go to the tensor-core kernels' chunks
 
 
 @dataclass
 class WkvPlan:
     """How a step's recurrence is cut: portions up to ``WKV_DIRECT`` tokens run whole; longer ones as chunks of
     ``WKV_CHUNK`` tokens side by side (each first from zero, then, once ``wkv_combine`` has walked the chunks, from the
-    matrices it starts from).  The lists are device int32; ``short_cu`` / ``short_slots`` describe the short portions
-    as requests of their own."""
+    matrices it starts from).  The lists are device int32; ``short_reqs`` names the requests of the short portions.  ``fine`` is the cut
+    for the tensor-core kernels, whose chunks begin at ``WKV_FINE`` tokens: one portion of 17 tokens, 32 heads of 64, 19.7 us whole / 16.3 in
+    chunks, of 33 33 / 17, of 128 115 / 19; 12 of 24 33 / 37, of 40 50 / 41; 20 single tokens and 100 100 / 34."""
 
     items: int
     item_req: Optional[torch.Tensor]
@@ -1527,33 +1532,43 @@ class WkvPlan:
     long_count: Optional[torch.Tensor]
     short_reqs: Optional[torch.Tensor]      # requests that run whole (None: all of them)
     shorts: int
+    fine: Optional["WkvPlan"] = None
 
 
 def wkv_plan(new_lens: Sequence[int], device) -> Optional[WkvPlan]:
-    """None when every portion runs whole."""
-    if not new_lens or max(new_lens) <= WKV_DIRECT:
+    """None when every portion runs whole whatever kernels take it.  A plan without items has a cut for the tensor-core kernels only."""
+    if not new_lens or max(new_lens) < WKV_FINE:
         return None
-    item_req, item_start, item_len, long_req, long_first, long_count, short = [], [], [], [], [], [], []
-    for r, n in enumerate(new_lens):
-        if n <= WKV_DIRECT:
-            short.append(r)
-            continue
-        long_req.append(r)
-        long_first.append(len(item_req))
-        long_count.append(-(-n // WKV_CHUNK))
-        for s0 in range(0, n, WKV_CHUNK):
-            item_req.append(r)
-            item_start.append(s0)
-            item_len.append(min(WKV_CHUNK, n - s0))
-    flat = torch.tensor(item_req + item_start + item_len + long_req + long_first + long_count + short, dtype=torch.int32)
-    flat = flat.to(device, non_blocking=True)
-    a, b = len(item_req), len(long_req)
-    parts = torch.split(flat, [a, a, a, b, b, b, len(short)])
-    return WkvPlan(a, parts[0], parts[1], parts[2], b, parts[3], parts[4], parts[5], parts[6] if short else None, len(short))
+
+    def cut(direct):
+        item_req, item_start, item_len, long_req, long_first, long_count, short = [], [], [], [], [], [], []
+        for r, n in enumerate(new_lens):
+            if n <= direct:
+                short.append(r)
+                continue
+            long_req.append(r)
+            long_first.append(len(item_req))
+            long_count.append(-(-n // WKV_CHUNK))
+            for s0 in range(0, n, WKV_CHUNK):
+                item_req.append(r)
+                item_start.append(s0)
+                item_len.append(min(WKV_CHUNK, n - s0))
+        return [item_req, item_start, item_len, long_req, long_first, long_count, short]
+
+    cuts = [cut(WKV_FINE - 1)] + ([cut(WKV_DIRECT)] if max(new_lens) > WKV_DIRECT else [])
+    lists = [part for parts in cuts for part in parts]
+    flat = torch.tensor([x for part in lists for x in part], dtype=torch.int32).to(device, non_blocking=True)      # one copy for all lists
+    split = torch.split(flat, [len(part) for part in lists])
+    plan = None
+    for i, parts in enumerate(cuts):
+        p = split[7 * i:7 * i + 7]
+        plan = WkvPlan(len(parts[0]), p[0], p[1], p[2], len(parts[3]), p[3], p[4], p[5], p[6] if parts[6] else None, len(parts[6]), plan)
+    return plan if len(cuts) > 1 else WkvPlan(0, None, None, None, 0, None, None, None, None, 0, plan)
 
 
 def wkv_workspace_floats(plan: Optional[WkvPlan], heads: int, d: int) -> int:
-    return 0 if plan is None else plan.items * heads * (d * d + d)
+    items = 0 if plan is None else max(plan.items, plan.fine.items if plan.fine is not None else 0)
+    return items * heads * (d * d + d)
 
 
 def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch.Tensor, u: torch.Tensor,
@@ -1583,7 +1598,11 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
         # one token a request (a decode step): a kernel that moves the matrices and stages nothing
         _call("lily_wkv_step", *common, requests, heads, d, _dt(r), _stream())
         return y
-    if plan is None:
+    tensor_cores = (plan is not None and plan.fine is not None and r.dtype == torch.bfloat16 and plan.fine.items <= 65535 and bool(
+        library().lily_wkv_chunk_takes(_p(r), _p(k), _p(v), stride, _p(log_decay), _p(u), heads, d, WKV_CHUNK)))
+    if tensor_cores:
+        plan = plan.fine
+    if plan is None or not plan.items:
         _call("lily_wkv_scan", *common, requests, heads, d, _dt(r), 0, None, None, None, None, None, _stream())
         return y
     need = wkv_workspace_floats(plan, heads, d)
@@ -1591,11 +1610,19 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
         raise KernelError(f"wkv_scan: chunks need a float32 workspace of {need}")
     ws_state = workspace
     ws_decay = workspace[plan.items * heads * d * d:]
-    chunks = (_p(plan.item_req), _p(plan.item_start), _p(plan.item_len), _p(ws_state), _p(ws_decay))
-    _call("lily_wkv_scan", *common, plan.items, heads, d, _dt(r), 1, *chunks, _stream())
+    items = (_p(plan.item_req), _p(plan.item_start), _p(plan.item_len), _p(ws_state), _p(ws_decay))
+
+    def run(outputs):
+        if tensor_cores:
+            _call("lily_wkv_chunk", _p(r), _p(k), _p(v), stride, _p(log_decay), _p(u), _p(y), _i32(cu_seqlens, "cu_seqlens"), plan.items, heads, d,
+                  *items, WKV_CHUNK, int(outputs), _stream())
+        else:
+            _call("lily_wkv_scan", *common, plan.items, heads, d, _dt(r), 2 if outputs else 1, *items, _stream())
+
+    run(outputs=False)
     _call("lily_wkv_combine", _p(state), state.stride(0), _i32(slots, "slots"), _p(ws_state), _p(ws_decay), _p(plan.long_req),
           _p(plan.long_first), _p(plan.long_count), plan.longs, heads, d, _stream())
-    _call("lily_wkv_scan", *common, plan.items, heads, d, _dt(r), 2, *chunks, _stream())
+    run(outputs=True)
     if plan.shorts:
         # the short portions of the same step run whole, from and to their slots
         _call("lily_wkv_scan", *common, plan.shorts, heads, d, _dt(r), 3, _p(plan.short_reqs), None, None, None, None, _stream())

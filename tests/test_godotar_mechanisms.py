@@ -161,6 +161,76 @@ def test_recurrence_in_chunks_side_by_side(heads, d):
         assert float((kept - want_state.float()).abs().max()) < 3e-5 * max(1.0, float(want_state.abs().max()))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[64], [1, 1, 33, 2, 130], [65, 63, 49, 34, 257]])
+@pytest.mark.parametrize("heads,d,strided", [(3, 16, False), (2, 48, True), (5, 64, False)])
+def test_recurrence_in_chunks_on_the_tensor_cores(lens, heads, d, strided):
+    """bfloat16 portions from 33 tokens on, beside shorter ones and single tokens: segments and chunks that end early, heads of fewer than 64
+    channels, decays from none to faster than float32 holds, rows that lie apart, matrices carried in and out of the slots."""
+    from lily_b200.csrc import ops
+    g = torch.Generator().manual_seed(d + len(lens))
+    n, hd = sum(lens), heads * d
+    wide = torch.randn(n, 3 * hd, generator=g).bfloat16().cuda()
+    r, k, v = (wide[:, i * hd:(i + 1) * hd] if strided else wide[:, i * hd:(i + 1) * hd].contiguous() for i in range(3))
+    lw = -torch.exp(torch.rand(n, hd, generator=g) * 8 - 6)
+    lw[:, 1], lw[:, 2], lw[5:, 3] = 0.0, -300.0, -40.0
+    u = torch.randn(heads, d, generator=g)
+    state = torch.randn(len(lens) + 1, hd * d + 3, generator=g)
+    slots = list(range(len(lens), 0, -1))
+    plan = ops.wkv_plan(lens, torch.device("cuda"))
+    assert plan.fine.longs == sum(m > 32 for m in lens) and plan.fine.shorts == sum(m <= 32 for m in lens)
+    mine = state.cuda()
+    y = ops.wkv_scan(r, k, v, lw.cuda(), u.cuda(), mine, i32([0] + torch.tensor(lens).cumsum(0).tolist(), "cuda"), i32(slots, "cuda"), len(lens), heads, d,
+                     plan=plan, workspace=torch.empty(ops.wkv_workspace_floats(plan, heads, d), device="cuda")).cpu().view(n, heads, d)
+    rd, kd, vd, w = (x.double().cpu().view(n, heads, d) for x in (r, k, v, torch.exp(lw.double())))
+    at = 0
+    for q, m in enumerate(lens):
+        S = state[slots[q], :hd * d].double().view(heads, d, d)
+        for t in range(at, at + m):
+            kv = kd[t][:, :, None] * vd[t][:, None]
+            want = torch.einsum("hi,hij->hj", rd[t], S + u.double()[:, :, None] * kv)
+            # sums of up to d + 64 products of 16 bits each in a few roundings of 2^-24, where the largest are some sixteen times one
+            assert float((y[t] - want).abs().max()) < 16 * 4 * (d + 64) ** 0.5 * 2.0 ** -24 * max(1.0, float(want.abs().max())), (q, t - at)
+            S = w[t][:, :, None] * S + kv
+        at += m
+        kept = mine[slots[q], :hd * d].cpu().view(heads, d, d)
+        assert float((kept - S).norm() / S.norm()) < 4 * 8 * 2.0 ** -24 * 4
+    assert torch.equal(mine[:, hd * d:].cpu(), state[:, hd * d:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("token", [5, 15, 64, 100])
+@pytest.mark.parametrize("what", ["r", "k", "v", "infinite v", "decay"])
+def test_recurrence_in_chunks_keeps_what_is_not_finite_behind_its_token(token, what):
+    from lily_b200.csrc import ops
+    g = torch.Generator().manual_seed(7)
+    heads, d, n = 2, 64, 140
+    r, k, v = (torch.randn(n, heads * d, generator=g).bfloat16().cuda() for _ in range(3))
+    lw, u = -torch.exp(torch.rand(n, heads * d, generator=g) * 4 - 4).cuda(), torch.randn(heads, d, generator=g).cuda()
+    plan = ops.wkv_plan([n], torch.device("cuda"))
+
+    def run():
+        state = torch.zeros(2, heads * d * d, device="cuda")
+        y = ops.wkv_scan(r, k, v, lw, u, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, heads, d, plan=plan,
+                         workspace=torch.empty(ops.wkv_workspace_floats(plan, heads, d), device="cuda"))
+        return y.view(n, heads, d), state
+    clean, _ = run()
+    {"r": r, "k": k, "v": v, "infinite v": v, "decay": lw}[what][token, d + 9] = float("inf") if what == "infinite v" else float("nan")      # head 1, channel 9
+    y, state = run()
+    hit = torch.zeros(n, heads, d, dtype=torch.bool, device="cuda")
+    if what == "r":
+        hit[token, 1] = True
+    elif what == "decay":
+        hit[token + 1:, 1] = True                              # the state a token reads is from before its own decay
+    elif what == "k":
+        hit[token:, 1] = True
+    else:
+        hit[token:, 1, 9] = True
+    assert not torch.isfinite(y[hit]).any() and torch.isfinite(y[~hit]).all()
+    torch.testing.assert_close(y[~hit], clean[~hit], atol=1e-4, rtol=1e-5)
+    assert bool(torch.isfinite(state).all()) == (what == "r")
+
+
 @pytest.mark.parametrize("device", DEVICES)
 def test_recurrence_remembers_the_first_token(device):
     """With decays next to one, a value written by the first token is read 400 tokens later, through 399 decoded
