@@ -86,6 +86,15 @@ class Workspace:
 
 
 @dataclass
+class Lane:
+    """Where one of a block's sublayers that read the same input may run beside the others: a stream (None: the current one) and scratch
+    of its own."""
+
+    stream: Any
+    workspace: Workspace
+
+
+@dataclass
 class StepBatch:
     num_tokens: int
     num_requests: int
@@ -111,6 +120,7 @@ class StepBatch:
     workspace: Optional[Workspace] = None
     future_tokens: Optional[torch.Tensor] = None     # int32 [request slots]: what negative token ids stand for
     plans: Dict[Any, Any] = field(default_factory=dict)
+    lanes: Sequence[Lane] = ()                       # a block may run sublayers side by side on these (captured decode steps)
 
     @property
     def num_prefill_requests(self) -> int:
@@ -124,6 +134,24 @@ class StepBatch:
     def fresh(self) -> List[bool]:
         """Requests whose first token comes in this step."""
         return [p == 0 for p in self.h_prefix_lens]
+
+    def branch(self, lane: Lane, behind: Any, work: Callable[[], Any]):
+        """Runs ``work`` on a lane, behind the event ``behind`` and with the lane's scratch; gives its result and the event at its end, for
+        the stream that goes on with the result to wait for (None: a lane without a stream is the current one).  Buffers are ordered
+        by that fork and join: what the current stream allocated is to be let go of behind the join, and what the lane allocated
+        goes back to the lane, whose next work starts behind the next fork."""
+        held, self.workspace = self.workspace, lane.workspace
+        try:
+            if lane.stream is None:
+                return work(), None
+            lane.stream.wait_event(behind)
+            with torch.cuda.stream(lane.stream):
+                result = work()
+                end = torch.cuda.Event()
+                end.record(lane.stream)
+            return result, end
+        finally:
+            self.workspace = held
 
     def plan(self, key: Any, make: Callable[["StepBatch"], Any]) -> Any:
         """What a part worked out for this step, made once and shared by every layer that asks with the same

@@ -25,7 +25,7 @@ from lily_b200.config.model_config import read_model_dir
 from lily_b200.config.registry import architecture_names, resolve_architecture
 from lily_b200.config.server_args import ServerArgs
 from lily_b200.engine import check
-from lily_b200.engine.batch import FUTURE, StepBatch, StepEntry, Workspace, build_step_batch, order_entries, rows_are_even, wire_array
+from lily_b200.engine.batch import FUTURE, Lane, StepBatch, StepEntry, Workspace, build_step_batch, order_entries, rows_are_even, wire_array
 from lily_b200.engine.profiler import DecodeProfiler
 from lily_b200.models.assembled import AssembledModel
 from lily_b200.parts.base import BuildContext, ModelSpec
@@ -113,13 +113,19 @@ class _DecodeGraph:
         self._rows: List[List[int]] = [[0] * b for _ in self.widths]       # the stamp of the table each row holds
         self.fill([], [], [[] for _ in self.widths], [], [[] for _ in self.widths])
         self.static.copy_(self.host)
+        # Sublayers that read the same input are captured as branches of the graph (``StepBatch.branch``), on streams of the runner's.  The
+        # first run goes one after another and makes what the step keeps (plans, scratch, kernel attributes) in one order; the
+        # second takes the branches' streams, whose library workspaces must be there before the capture.
+        self.batch.lanes = lanes = [Lane(None, Workspace(runner.device)) for _ in range(runner.model.lanes)]
         stream = torch.cuda.Stream(device=runner.device)
         stream.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(stream), torch.no_grad():
-            for _ in range(2):                      # sizes the workspace and sets kernel attributes
+        for streams in ([None] * len(lanes), runner.lane_streams()):
+            for lane, own in zip(lanes, streams):
+                lane.stream = own
+            with torch.cuda.stream(stream), torch.no_grad():
                 runner.model.forward(self.batch, runner.cache)
-        torch.cuda.current_stream().wait_stream(stream)
-        torch.cuda.synchronize()
+            torch.cuda.current_stream().wait_stream(stream)
+            torch.cuda.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         counter = runner.model.ctx.ops.launches
         before = counter["count"]
@@ -224,6 +230,7 @@ class ModelRunner:
         self.steps_run = 0
         self.tokens_run = 0
         self.graph_steps = 0
+        self._lane_streams: List["torch.cuda.Stream"] = []
         self._graphs: Dict[Tuple[int, int, bool], _DecodeGraph] = {}      # by (batch bucket, length class, rows even)
         self.use_graphs = self.device.type == "cuda" and not args.disable_cuda_graph and self.model.graph_safe
         max_bs = args.cuda_graph_max_bs or min(self.max_requests, 256)
@@ -240,6 +247,13 @@ class ModelRunner:
             self.length_classes.append(bound)
             bound *= 2
         self.length_classes.append(self.context_len)
+
+    def lane_streams(self) -> List["torch.cuda.Stream"]:
+        """The streams that captured steps put branches on, above the default priority: what runs there is a chain of short kernels
+        beside products that stream weights."""
+        while len(self._lane_streams) < self.model.lanes:
+            self._lane_streams.append(torch.cuda.Stream(device=self.device, priority=-1))
+        return self._lane_streams
 
     # ---- construction ---------------------------------------------------------------
 

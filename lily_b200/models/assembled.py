@@ -106,6 +106,12 @@ class AssembledModel:
         return kept
 
     @property
+    def lanes(self) -> int:
+        """Streams beside the step's own that a captured step's blocks can use: those a block takes, and a last one for their feed-forwards."""
+        return (max((getattr(b, "lanes", 0) for b in self.blocks), default=0)
+                + max((getattr(getattr(b, "feed_forward", None), "lanes", 0) for b in self.blocks), default=0))
+
+    @property
     def graph_safe(self) -> bool:
         return all(m.graph_safe for b in self.blocks for m in b.mixers)
 

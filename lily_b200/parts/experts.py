@@ -94,6 +94,10 @@ class RoutedExperts(FeedForward):
             self.shared = build_part("feed_forward", form, f"{prefix}.{spec.name('shared')}", ctx)
         self.parts = () if self.shared is None else (self.shared,)
 
+    @property
+    def lanes(self) -> int:
+        return 0 if self.shared is None else 1
+
     def _expert(self, e: int, role: str) -> str:
         return f"{self.prefix}.{self.spec.name('expert').format(e)}.{self.spec.name(role)}"
 
@@ -139,9 +143,19 @@ class RoutedExperts(FeedForward):
     def forward(self, x, batch):
         s, ops = self.spec, self.ctx.ops
         grouped = {"groups": s.groups, "keep_groups": s.keep_groups} if s.groups > 1 else {}
-        routing = ops.moe_route(x, self.router, self.correction, s.top, s.experts, scores=s.scores, renormalise=s.renormalise,
-                                shared_gate=self.shared is not None, outputs=s.outputs, **grouped)
-        shared = None if self.shared is None else self.shared.forward(x, batch)
+        route = lambda: ops.moe_route(x, self.router, self.correction, s.top, s.experts, scores=s.scores, renormalise=s.renormalise,
+                                      shared_gate=self.shared is not None, outputs=s.outputs, **grouped)
+        if self.shared is not None and getattr(batch, "lanes", ()):
+            # a captured decode step: the shared expert's three short kernels beside the routing's two (6 us a layer of 2,048 columns)
+            ready = torch.cuda.Event()
+            ready.record()
+            shared, end = batch.branch(batch.lanes[-1], ready, lambda: self.shared.forward(x, batch))
+            routing = route()
+            if end is not None:
+                torch.cuda.current_stream().wait_event(end)
+        else:
+            routing = route()
+            shared = None if self.shared is None else self.shared.forward(x, batch)
         out = ops.moe_experts(x, routing, self.w_gate_up, self.w_down, s.limit, s.alpha, activation=s.activation,
                               weight_on_input=s.weight_on == "input", shared=shared)
         return out.unsqueeze(0)                   # float32 [1, tokens, hidden]: one plane of partial sums
