@@ -1267,6 +1267,7 @@ def causal_conv(proj: torch.Tensor, col0: int, channels: int, weight: torch.Tens
 SCAN_CHUNK = 128        # tokens a chunk of a long portion (doubled while the chunk states would pass SCAN_WORKSPACE)
 SCAN_DIRECT = 192       # portions up to this many tokens run in one piece, from and to the state in the slot
 SCAN_WORKSPACE = 1 << 29
+SCAN_ROWS = 64          # tokens a chunk of the scan with a state vector a channel (at most 16 entries); half of that for few tokens and channels
 SCAN_FINE = 17          # tokens from which a portion can go to the tensor-core kernels' chunks
 
 
@@ -1287,6 +1288,7 @@ class ScanPlan:
     num_long: int = 0
     chunk: int = 0                           # the longest chunk, in tokens
     fine: Optional["ScanPlan"] = None        # the cut for the tensor-core kernels, where they could take chunks
+    rows: Optional["ScanPlan"] = None        # the cut for the scan with a state vector a channel of few entries
 
 
 _SSD_CHUNKS = os.environ.get("LILY_B200_SSD_CHUNKS", "") != "scan"       # "scan": chunks run token by token
@@ -1310,8 +1312,9 @@ def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0, chunks=Tru
     """Cuts the step's portions for the scan.  A portion of up to SCAN_DIRECT tokens (every decoded token) runs in one
     piece; a longer one in chunks of SCAN_CHUNK tokens that run side by side and are joined by ``ssd_combine``
     (``state_floats``: the size of one scan state, which bounds how many chunks the workspace may hold).  ``fine`` is the cut for
-    the tensor-core kernels, chunks from SCAN_FINE tokens on, or None: ``chunks`` False leaves it out, and (dtype, heads, head
+    the tensor-core kernels, chunks from SCAN_FINE tokens on, or None: ``chunks`` False makes ``rows`` in its place (for the scan with a state vector a channel), and (dtype, heads, head
     size, state, channels) makes it for a scan of those sizes, where its kernels take them and ``scan_chunks_pay``."""
+    by_channel = chunks is False
     if isinstance(chunks, tuple):
         dtype, heads, head_dim, n_state, channels = chunks
         chunks = (_SSD_CHUNKS and dtype == torch.bfloat16 and scan_chunks_pay(new_lens, heads)
@@ -1337,6 +1340,17 @@ def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0, chunks=Tru
     fine = sum(-(-n // SCAN_CHUNK) for n in new_lens if n >= SCAN_FINE) if chunks and chunk == SCAN_CHUNK else 0
     if 0 < 2 * fine <= 65535 and fine * max(state_floats, 1) * 4 <= SCAN_WORKSPACE:       # two tiles of outputs a chunk along the grid
         cuts.append(cut(SCAN_FINE - 1, chunk))
+    rows = None
+    if by_channel and cuts:
+        # The scan with a state vector a channel: shorter chunks, within the same workspace.  Chunks of 32 / 64 / 128, us, 4,096 channels of 16
+        # entries: 260 tokens 46 / 63 / 100, 400 63 / 77 / 100, 300 + 211 + 512 168 / 170 / 231, 1,999 186 / 174 / 191; 8,192 channels,
+        # 2,048 tokens 392 / 307 / 308.
+        longs = [n for n in new_lens if n > SCAN_DIRECT]
+        size = SCAN_ROWS if sum(longs) * state_floats > 1 << 26 else SCAN_ROWS // 2
+        while size < 1024 and sum(-(-n // size) for n in longs) * state_floats * 4 > SCAN_WORKSPACE:
+            size *= 2
+        rows = len(cuts)
+        cuts.append(cut(SCAN_DIRECT, size))
     if not cuts:
         return ScanPlan(None, len(new_lens))
     # one copy to the device for all lists
@@ -1347,6 +1361,9 @@ def scan_plan(new_lens: Sequence[int], device, state_floats: int = 0, chunks=Tru
     for i, (parts, size) in enumerate(cuts):
         p = split[7 * i:7 * i + 7]
         plans.append(ScanPlan(p[0], len(parts[0]), p[1], p[2], p[3], len(parts[1]), p[4], p[5], p[6], len(parts[4]), size))
+    if rows is not None:
+        plans[0].rows = plans[rows]
+        return plans[0]
     if max(new_lens) <= SCAN_DIRECT:
         return ScanPlan(None, len(new_lens), fine=plans[0])
     plans[0].fine = plans[1] if len(plans) > 1 else None
@@ -2190,16 +2207,25 @@ def selective_scan_max_state() -> int:
     return int(library().lily_selective_scan_max_state())
 
 
-def selective_workspace_floats(plan: Optional[ScanPlan], inner: int, n_state: int) -> int:
-    """Float32 scratch the chunks of ``plan`` need: a state and a sum of steps a chunk.  0 when the long portions are
-    better run in one piece each: the chunked form does the recurrence's work twice, which pays while the blocks of the
-    whole portions (16 channels a block) leave most of the device's warp slots empty (measured, 2,048 tokens of one
-    request, 16 state entries: 4,096 channels 564 -> 419 us in chunks, 8,192 channels 666 -> 816 us)."""
+def _selective_cut(plan: Optional[ScanPlan], inner: int, n_state: int) -> Optional[ScanPlan]:
+    """The cut a scan with a state vector a channel takes, None for one piece a portion.  The chunked form does the recurrence's work twice,
+    but with up to 16 entries its kernels take less than half of the time a channel and token (one request of 2,048 tokens, 8,192 channels
+    694 us in pieces, 307 in chunks; four of 512, 4,096 channels 251 and 172).  With more entries it pays while the blocks of the
+    whole portions (16 channels a block) leave most of the device's warp slots empty (measured, 2,048 tokens of one request, 16 state
+    entries on the kernel of both: 4,096 channels 564 -> 419 us in chunks, 8,192 channels 666 -> 816 us)."""
+    if plan is not None and n_state <= 16 and plan.rows is not None:
+        plan = plan.rows
     if plan is None or not plan.num_chunks:
-        return 0
-    if plan.num_long * -(-inner // 16) > 2.5 * sm_count():
-        return 0
-    return plan.num_chunks * inner * (n_state + 1)
+        return None
+    if n_state > 16 and plan.num_long * -(-inner // 16) > 2.5 * sm_count():
+        return None
+    return plan
+
+
+def selective_workspace_floats(plan: Optional[ScanPlan], inner: int, n_state: int) -> int:
+    """Float32 scratch the chunks of ``plan`` need: a state and a sum of steps a chunk.  0 when the portions run in one piece each."""
+    plan = _selective_cut(plan, inner, n_state)
+    return 0 if plan is None else plan.num_chunks * inner * (n_state + 1)
 
 
 def selective_scan(x: torch.Tensor, low: torch.Tensor, b_col: int, step: torch.Tensor, proj: torch.Tensor, z_col: int,
@@ -2224,6 +2250,7 @@ def selective_scan(x: torch.Tensor, low: torch.Tensor, b_col: int, step: torch.T
     common = (_p(x), _p(low), low.shape[1], int(b_col), int(b_col) + n, _p(step), _p(proj), proj.shape[1], int(z_col), _p(a),
               _p(d_skip), _p(state), state.shape[1], _p(out), _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
     need = selective_workspace_floats(plan, inner, n)
+    plan = _selective_cut(plan, inner, n)
     if not need:
         _call("lily_selective_scan", *common, int(requests), tokens, inner, n, _dt(x), None, None, None, 0, None, None, _stream())
         return out

@@ -486,6 +486,38 @@ def test_selective_scan_long_portions_in_chunks_side_by_side(device, dtype, inne
                 at += ns[r]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner,state_n", [(130, 1), (64, 4), (257, 7), (128, 16), (40, 13)])
+@pytest.mark.parametrize("lens", [[193], [1, 1, 192, 224, 7], [225, 321, 1024]])
+def test_selective_scan_a_channel_a_thread(lens, inner, state_n, dtype):
+    """The cut the mixer makes: portions beyond 192 tokens in chunks, entries that fill the kernels' 4, 8 or 16 and that do not, channels
+    that end inside a block, last chunks, tiles and steps of four that are not whole, beside portions in one piece."""
+    ops = ops_for("cuda")
+    g = torch.Generator().manual_seed(inner + len(lens))
+    rank, n = 6, sum(lens)
+    x, low = torch.randn(n, inner, generator=g).to(dtype), torch.randn(n, rank + 2 * state_n, generator=g).to(dtype)
+    step, proj = torch.randn(n, inner, generator=g) - 1.0, torch.randn(n, 2 * inner, generator=g).to(dtype)
+    step[3] = 25.0                                                 # past where softplus is the identity; the decays go below float32
+    a_log, d_skip = torch.randn(inner, state_n, generator=g), torch.randn(inner, generator=g)
+    plan = ops.scan_plan(lens, torch.device("cuda"), inner * state_n, chunks=False)
+    assert plan.rows.num_long == sum(m > 192 for m in lens) and plan.rows.num_direct == sum(m <= 192 for m in lens)
+    need = ops.selective_workspace_floats(plan, inner, state_n)
+    state = torch.zeros((len(lens) + 1, inner * state_n + 3), device="cuda")
+    state[:, -3:] = 7.0
+    y = ops.selective_scan(x.cuda(), low.cuda(), rank, step.cuda(), proj.cuda(), inner, (-torch.exp(a_log)).cuda(), d_skip.cuda(), state,
+                           i32([0] + torch.tensor(lens).cumsum(0).tolist(), "cuda"), i32(list(range(len(lens), 0, -1)), "cuda"), len(lens), plan=plan,
+                           workspace=torch.empty(need, device="cuda"))
+    at = 0
+    for i, m in enumerate(lens):
+        want = plain_scan(x[at:at + m], low[at:at + m], rank, step[at:at + m], proj[at:at + m, inner:], a_log, d_skip)
+        close(y[at:at + m], want, dtype, scale=float(want.abs().max()))
+        if dtype == torch.float32:                                 # a sum of state_n products behind a chain of rounded decays
+            assert float((y[at:at + m].cpu() - want).norm() / want.norm()) < 16 * 2.0 ** -24 * 4
+        at += m
+    assert float((state[:, -3:] - 7.0).abs().max()) == 0.0
+
+
 # ------------------------------------------------------------------ feed-forward, layer scale, frequencies
 
 @pytest.mark.parametrize("device", DEVICES)
