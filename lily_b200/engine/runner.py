@@ -15,6 +15,7 @@ sizing follows model_runner.py:160-242.
 from __future__ import annotations
 
 import logging
+import threading
 import time
 from typing import Any, Dict, List, Optional, Sequence, Tuple
 
@@ -72,6 +73,23 @@ def _load_library_products(device) -> None:
     torch.addmm(x[0, :16], x, x.t())
 
 
+_CAPTURING = threading.local()
+
+
+def _lane_streams(device, count: int, library: bool) -> List["torch.cuda.Stream"]:
+    """The streams that a capture puts branches on, above the default priority: what runs there is a chain of short kernels beside
+    products that stream weights.  A thread captures one step at a time and a replay does not use them, so a thread has one set a
+    device for all its captures (with a set a runner the allocator's segments for them took up to 0.4 s a capture).  ``library``: the
+    library's products have their workspaces there, which must not be made while a graph is captured."""
+    held = vars(_CAPTURING).setdefault((torch.device(device), library), [])
+    while len(held) < count:
+        held.append(torch.cuda.Stream(device=device, priority=-1))
+        if library:
+            with torch.cuda.stream(held[-1]):
+                _load_library_products(device)
+    return held[:count]
+
+
 class _DecodeGraph:
     """One captured decode step for up to ``bucket`` requests of up to ``max_len`` positions, about equally long
     (``even``) or not; ``even_matters`` says whether some part planned by that.  Its metadata lives
@@ -113,19 +131,18 @@ class _DecodeGraph:
         self._rows: List[List[int]] = [[0] * b for _ in self.widths]       # the stamp of the table each row holds
         self.fill([], [], [[] for _ in self.widths], [], [[] for _ in self.widths])
         self.static.copy_(self.host)
-        # Sublayers that read the same input are captured as branches of the graph (``StepBatch.branch``), on streams of the runner's.  The
-        # first run goes one after another and makes what the step keeps (plans, scratch, kernel attributes) in one order; the
-        # second takes the branches' streams, whose library workspaces must be there before the capture.
+        # Sublayers that read the same input are captured as branches of the graph (``StepBatch.branch``).  The runs ahead of the capture go
+        # one after another, so that what the step keeps (plans, scratch, kernel attributes) is made in one order.
         self.batch.lanes = lanes = [Lane(None, Workspace(runner.device)) for _ in range(runner.model.lanes)]
         stream = torch.cuda.Stream(device=runner.device)
         stream.wait_stream(torch.cuda.current_stream())
-        for streams in ([None] * len(lanes), runner.lane_streams()):
-            for lane, own in zip(lanes, streams):
-                lane.stream = own
-            with torch.cuda.stream(stream), torch.no_grad():
+        with torch.cuda.stream(stream), torch.no_grad():
+            for _ in range(2):                      # sizes the workspace and sets kernel attributes
                 runner.model.forward(self.batch, runner.cache)
-            torch.cuda.current_stream().wait_stream(stream)
-            torch.cuda.synchronize()
+        torch.cuda.current_stream().wait_stream(stream)
+        for lane, own in zip(lanes, _lane_streams(runner.device, len(lanes), runner.dtype == torch.bfloat16)):
+            lane.stream = own
+        torch.cuda.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         counter = runner.model.ctx.ops.launches
         before = counter["count"]
@@ -230,7 +247,6 @@ class ModelRunner:
         self.steps_run = 0
         self.tokens_run = 0
         self.graph_steps = 0
-        self._lane_streams: List["torch.cuda.Stream"] = []
         self._graphs: Dict[Tuple[int, int, bool], _DecodeGraph] = {}      # by (batch bucket, length class, rows even)
         self.use_graphs = self.device.type == "cuda" and not args.disable_cuda_graph and self.model.graph_safe
         max_bs = args.cuda_graph_max_bs or min(self.max_requests, 256)
@@ -247,13 +263,6 @@ class ModelRunner:
             self.length_classes.append(bound)
             bound *= 2
         self.length_classes.append(self.context_len)
-
-    def lane_streams(self) -> List["torch.cuda.Stream"]:
-        """The streams that captured steps put branches on, above the default priority: what runs there is a chain of short kernels
-        beside products that stream weights."""
-        while len(self._lane_streams) < self.model.lanes:
-            self._lane_streams.append(torch.cuda.Stream(device=self.device, priority=-1))
-        return self._lane_streams
 
     # ---- construction ---------------------------------------------------------------
 

@@ -44,7 +44,7 @@ def test_branches_give_the_bits_of_one_stream(monkeypatch, design, config, dtype
                     out.append(runner.step([StepEntry(slots[r], [ids[r][at[r]]], [0]) for r in live]).clone())
                     for r in live:
                         at[r] += 1
-                assert runner.graph_steps == 40 and len(runner._lane_streams) == (lanes if branches else 0)
+                assert runner.graph_steps == 40 and all(len(g.batch.lanes) == (lanes if branches else 0) for g in runner._graphs.values())
                 return out, [s[1:].clone() for s in runner.cache.states]          # row 0 is the padded rows'
         (one, states), (many, states_many) = run(False), run(True)
         assert all(torch.equal(a, b) for a, b in zip(one, many)) and all(torch.equal(a, b) for a, b in zip(states, states_many))
