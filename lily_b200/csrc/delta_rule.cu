@@ -173,6 +173,133 @@ __global__ void __launch_bounds__(DELTA_THREADS) delta_rule_kernel(const DeltaAr
     }
 }
 
+// A step that brings each request one token (any number is taken, one after another).  Bound by reading and writing the state once: a warp
+// has RB value columns of a head, a lane four neighbouring entries of each (and the four 128 further), all asked for at once, and nothing
+// is staged.  A token needs three sums over the key entries beside the (S^T k)_j and (S^T q)_j; the latter are summed by halving what a lane
+// holds at each exchange, so that the lanes of a column end with its two sums, and go out again as u_j.  grid (heads, requests,
+// ceil(dv / (8 RB))), block 256; d a multiple of four up to 128 NI, the state's rows on 16 bytes.  16
+// heads of 128 x 128: 5 requests 9.0 -> 4.5 us, one 5.0 -> 2.7; 32 heads: 64 requests 154 -> 68 (268 MB: 4.0 TB/s); 8 heads of 256 x
+// 256, 64 requests: 281 -> 51.
+template <typename T, int NI, int RB>
+__global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
+    pdl_enter_small();
+    const int head = blockIdx.x, req = blockIdx.y, lane = threadIdx.x & 31, j0 = (blockIdx.z * 8 + (threadIdx.x >> 5)) * RB;
+    const int d = a.d, dv = a.dv, kvh = head / (a.heads / a.kv_heads);
+    const int tok0 = a.cu_seqlens[req], len = a.cu_seqlens[req + 1] - tok0;
+    if (len <= 0 || j0 >= dv) return;
+    float* st = a.state + (size_t)a.slots[req] * a.state_stride + ((size_t)head * dv + j0) * d;
+    float4 S[RB][NI];
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int e = lane * 4 + 128 * i;
+            S[r][i] = j0 + r < dv && e < d ? *reinterpret_cast<const float4*>(st + (size_t)r * d + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    const float rate = expf(a.a_log[head]), dt_bias = a.dt_bias[head];
+    constexpr int GROUP = 32 / RB;                               // lanes that end with a column's sums
+    const int mine = lane / GROUP;
+    for (int t = 0; t < len; ++t) {
+        const T* src = (const T*)a.qkv + (size_t)(tok0 + t) * a.qkv_stride;
+        const T* gates = (const T*)a.proj + (size_t)(tok0 + t) * a.proj_stride + head;
+        float4 k[NI], q[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int e = lane * 4 + 128 * i;
+            k[i] = q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (e < d) {
+                const T *kp = src + a.k_col + (size_t)kvh * d + e, *qp = src + a.q_col + (size_t)kvh * d + e;
+                k[i] = make_float4(to_float(kp[0]), to_float(kp[1]), to_float(kp[2]), to_float(kp[3]));
+                q[i] = make_float4(to_float(qp[0]), to_float(qp[1]), to_float(qp[2]), to_float(qp[3]));
+            }
+        }
+        const float value = j0 + mine < dv ? to_float(src[a.v_col + (size_t)head * dv + j0 + mine]) : 0.f;
+        const float alpha = to_float(gates[a.a_col]) + dt_bias, beta = 1.f / (1.f + expf(-to_float(gates[a.b_col])));
+        const float decay = expf(-rate * (alpha > 20.f ? alpha : log1pf(expf(alpha))));
+        float kk = 0.f, qq = 0.f, kq = 0.f, sum[2 * RB];
+        auto dot = [](const float4& x, const float4& y, float s) { return fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s)))); };
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            kk = dot(k[i], k[i], kk);
+            qq = dot(q[i], q[i], qq);
+            kq = dot(k[i], q[i], kq);
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            sum[2 * r] = sum[2 * r + 1] = 0.f;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                sum[2 * r] = dot(S[r][i], k[i], sum[2 * r]);
+                sum[2 * r + 1] = dot(S[r][i], q[i], sum[2 * r + 1]);
+            }
+        }
+        kk = warp_sum(kk);
+        qq = warp_sum(qq);
+        kq = warp_sum(kq);
+#pragma unroll
+        for (int off = 16, n = 2 * RB; off > 0; off >>= 1) {
+            if (n > 1) {
+                n >>= 1;
+                const bool upper = lane & off;
+#pragma unroll
+                for (int i = 0; i < RB; ++i)
+                    if (i < n) {
+                        const float give = upper ? sum[i] : sum[i + n], keep = upper ? sum[i + n] : sum[i];
+                        sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+                    }
+            } else sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], off);
+        }
+        // the first half of a column's lanes has (S^T k), the second (S^T q)
+        const float other = __shfl_xor_sync(0xffffffffu, sum[0], GROUP / 2);
+        const bool second = lane & (GROUP / 2);
+        const float fk = 1.f / sqrtf(kk + a.unit_eps), fq = a.q_scale / sqrtf(qq + a.unit_eps);
+        const float sk = (second ? other : sum[0]) * fk, sq = (second ? sum[0] : other) * fq;
+        const float u = beta * (value - decay * sk);
+        if (lane % GROUP == 0 && j0 + mine < dv)
+            a.y[(size_t)(tok0 + t) * a.heads * dv + (size_t)head * dv + j0 + mine] = fmaf(decay, sq, kq * fk * fq * u);
+        const float ku = u * fk;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            const float w = __shfl_sync(0xffffffffu, ku, r * GROUP);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                float4& x = S[r][i];
+                x.x = fmaf(k[i].x, w, decay * x.x), x.y = fmaf(k[i].y, w, decay * x.y);
+                x.z = fmaf(k[i].z, w, decay * x.z), x.w = fmaf(k[i].w, w, decay * x.w);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int e = lane * 4 + 128 * i;
+            if (j0 + r < dv && e < d) *reinterpret_cast<float4*>(st + (size_t)r * d + e) = S[r][i];
+        }
+}
+
+// Whether a step of one token a request goes to the kernel above: keys of 16 leave most of its lanes idle (64 requests, 32 heads of 16 x 16: 9.7
+// us in the kernel of the prompts, 15.1 here; heads of 20 x 20, 16: 9.6 and 8.9).
+static bool delta_step_takes(const DeltaArgs& a, int requests) {
+    return a.d > 16 && a.d % 4 == 0 && a.d <= 256 && ((uintptr_t)a.state & 15) == 0 && a.state_stride % 4 == 0 && requests <= 65535;
+}
+
+template <typename T>
+static void launch_step(const DeltaArgs& a, int requests, cudaStream_t stream) {
+    // eight columns a warp where that still gives every SM two blocks, fewer for a few requests
+    int rb = a.d <= 128 ? 8 : 4;
+    while (rb > 2 && (long long)a.heads * requests * ((a.dv + 8 * rb - 1) / (8 * rb)) < 2 * sm_count()) rb >>= 1;
+    const dim3 grid(a.heads, requests, (a.dv + 8 * rb - 1) / (8 * rb)), block(256);
+    if (a.d <= 128) {
+        if (rb == 8) launch_pdl(delta_step_kernel<T, 1, 8>, grid, block, 0, stream, a);
+        else if (rb == 4) launch_pdl(delta_step_kernel<T, 1, 4>, grid, block, 0, stream, a);
+        else launch_pdl(delta_step_kernel<T, 1, 2>, grid, block, 0, stream, a);
+    } else {
+        if (rb == 4) launch_pdl(delta_step_kernel<T, 2, 4>, grid, block, 0, stream, a);
+        else launch_pdl(delta_step_kernel<T, 2, 2>, grid, block, 0, stream, a);
+    }
+}
+
 }  // namespace lily
 
 using namespace lily;
@@ -193,6 +320,12 @@ LILY_API int lily_delta_rule(const void* qkv, int qkv_stride, int q_col, int k_c
     a.proj = proj; a.proj_stride = proj_stride; a.b_col = b_col; a.a_col = a_col; a.a_log = a_log; a.dt_bias = dt_bias;
     a.state = state; a.state_stride = state_stride; a.y = y; a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.heads = heads; a.kv_heads = kv_heads; a.d = d; a.dv = dv; a.unit_eps = unit_eps; a.q_scale = q_scale;
+    if (tokens == requests && delta_step_takes(a, requests)) {
+        if (dtype == kBF16) launch_step<__nv_bfloat16>(a, requests, stream);
+        else launch_step<float>(a, requests, stream);
+        LILY_CHECK_LAUNCH("delta_rule");
+        return 0;
+    }
     dim3 grid(requests, heads, (dv + DELTA_COLS - 1) / DELTA_COLS), block(DELTA_THREADS);
     const int rows = (d + DL - 1) / DL;
     const bool ahead = tokens > requests;               // some request brings more than one token

@@ -328,6 +328,26 @@ def test_delta_rule_reads_after_hundreds_of_steps_what_the_first_token_wrote(dev
           torch.float32)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("requests,heads,kvh,d,dv", [(1, 2, 1, 20, 3), (3, 4, 2, 64, 17), (40, 16, 4, 128, 70), (2, 3, 3, 132, 9), (80, 4, 2, 256, 64), (5, 2, 2, 16, 16)])
+def test_delta_rule_of_one_token_a_request(dtype, requests, heads, kvh, d, dv):
+    """A decode step: key entries that end inside a lane's reach and beyond the first 128, value columns that end inside a warp's eight, four or
+    two, slots in another order than the rows."""
+    ops = ops_for("cuda")
+    qkv, proj, a_log, dt_bias = delta_inputs(3 * requests, heads, kvh, d, dv, d, dtype)
+    state = torch.zeros((requests + 1, -(-(heads * d * dv + 1) // 4) * 4), device="cuda")
+    state[:, -1] = 7.0
+    slots = i32(list(range(requests, 0, -1)), "cuda")
+    cu = i32(list(range(requests + 1)), "cuda")
+    got = [ops.delta_rule(qkv[s::3].contiguous().cuda(), proj[s::3].contiguous().cuda(), 3, 3 + heads, a_log.cuda(), dt_bias.cuda(), state, cu, slots, requests,
+                          heads, kvh, d, dv, 1e-6, d ** -0.5).cpu() for s in range(3)]
+    for r in range(requests):
+        want = plain_delta(qkv[3 * r:3 * r + 3], proj[3 * r:3 * r + 3], a_log, dt_bias, heads, kvh, d, dv)
+        close(torch.stack([g[r] for g in got]).view(3, heads, dv), want, torch.float32)
+    assert float((state[:, -1] - 7.0).abs().max()) == 0.0
+
+
 # ------------------------------------------------------------------ the delta rule in chunks
 
 @pytest.mark.gpu
