@@ -103,7 +103,8 @@ class ParallelBlock(Block):
         """The sublayers as branches that start behind the norm and end ahead of the sum: a decode step's mixers are chains of short
         kernels, which leave the memory idle while the feed-forward's weights could stream.  With the layer sizes of 2,048 columns,
         a request of two prompts and 12 steps of four Godotar layers 6,025 -> 5,199 us, of eight prompts and 24 steps of four
-        Zirurax layers 9,313 -> 7,981."""
+        Zirurax layers 9,313 -> 7,981 (5,700 and 8,940 with the first mixer on the step's own stream and the feed-forward on a lane: its
+        products fill the SMs whenever they start, and are best out of the way first)."""
         ready = torch.cuda.Event()
         ready.record()
         outs, ends = [], []
