@@ -204,10 +204,14 @@ __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
     __shared__ float red[MEAN_MAX][33];
     __shared__ float share[MEAN_MAX][CL];
     cg::cluster_group cluster = cg::this_cluster();
-    pdl_enter_small();
     const size_t base = (size_t)blockIdx.y * a.width;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;       // this thread's four columns
-    float4 v[MEAN_MAX];
+    float4 v[MEAN_MAX], gain[MEAN_MAX], f = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < MEAN_MAX; ++k)                               // the gains depend on no one
+        if (k < a.count) gain[k] = *reinterpret_cast<const float4*>(a.gain[k] + i);
+    pdl_enter_small();
+    if (a.add.p) f = a.add.four(base + i);                           // with the inputs, not behind the cluster's barrier
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int k = 0; k < MEAN_MAX; ++k) {
@@ -243,16 +247,13 @@ __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
 #pragma unroll
             for (int r = 0; r < CL; ++r) total += share[k][r];       // same order in every block
             const float inv = rsqrtf(total / (float)a.width + a.eps);
-            const float4 g = *reinterpret_cast<const float4*>(a.gain[k] + i);
+            const float4 g = gain[k];
             o.x += (v[k].x * inv) * g.x; o.y += (v[k].y * inv) * g.y;
             o.z += (v[k].z * inv) * g.z; o.w += (v[k].w * inv) * g.w;
         }
     }
     o.x *= a.scale; o.y *= a.scale; o.z *= a.scale; o.w *= a.scale;
-    if (a.add.p) {
-        const float4 f = a.add.four(base + i);
-        o.x += f.x; o.y += f.y; o.z += f.z; o.w += f.w;
-    }
+    if (a.add.p) o.x += f.x, o.y += f.y, o.z += f.z, o.w += f.w;
     *reinterpret_cast<float4*>(a.out + base + i) = o;
 }
 
