@@ -867,6 +867,27 @@ def test_wkv_scan_of_one_token_a_request(dtype, requests, heads, d):
     torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("rows,hidden", [(1, 1024), (3, 1056), (64, 2048), (65, 2048), (70, 516), (5, 1028), (66, 4100), (3, 8192), (9, 9000), (2, 1027)])
+@pytest.mark.parametrize("planes,gains,bias,write", [((1, 17), 2, True, True), ((9, 0), 1, False, True), ((0, 0), 2, True, False), ((8, None), 0, False, True)])
+def test_add_rmsnorm_multi_in_pieces(rows, hidden, planes, gains, bias, write):
+    """Rows over a cluster, in a block's registers (whole and with a last piece that few threads have) and a number at a time; sums of one to
+    seventeen planes (0: bfloat16, None: no such sum), outputs and stream as the plain statement."""
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    deltas = [None if n is None else (rand(n, rows, hidden) if n else rand(rows, hidden).bfloat16()) for n in planes]
+    vectors, b = [rand(hidden) for _ in range(gains)], rand(hidden) if bias else None
+    mine, theirs = rand(rows, hidden), None
+    theirs, kept = mine.clone(), mine.clone()
+    got = ops().add_rmsnorm_multi(mine, deltas, vectors, 1e-6, torch.bfloat16, b, write)
+    want = ref.add_rmsnorm_multi(theirs, deltas, vectors, 1e-6, torch.bfloat16, b, write)
+    assert len(got) == gains
+    for x, y in zip(got, want):
+        torch.testing.assert_close(x.float(), y.float(), rtol=1e-2, atol=1e-2)             # one rounding to bfloat16 apart
+    torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
+    if not write:
+        assert torch.equal(mine, kept)
+
+
 @pytest.mark.parametrize("tokens,rank,cols", [(1, 1, 5), (2, 64, 2048), (8, 31, 130), (9, 33, 257), (21, 200, 128), (2364, 33, 128), (2371, 33, 130), (3, 130, 384),
                                               (4, 64, 64), (5, 65, 100), (1193, 64, 516), (2380, 5, 132)])
 def test_wkv_decay_by_rows_asked_for_ahead(tokens, rank, cols):
