@@ -23,6 +23,7 @@
 // rounded to bfloat16 for p.v as in lily/layers/attention/triton_ops/extend_attention.py:110-112.
 #include "attention_args.cuh"
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 #include <cooperative_groups.h>
 
@@ -114,19 +115,39 @@ __host__ __device__ constexpr size_t stage_bytes(bool decode) {
 // Output sums a block of a cluster of `splits` blocks merges: its share of rows x D.
 __host__ __device__ inline int cluster_share(int rows, int d, int splits) { return ((rows * d + splits - 1) / splits + 3) / 4 * 4; }
 
-template <int D, bool DECODE, int STAGES, bool CLUSTER>
+// Decode with pages of whole tiles (TMA): a tile's 64 keys and values are two to four copies that one thread asks for, where 128 threads
+// looked up the page of each of their sixteen 16-byte pieces, and all STAGES tiles are on their way instead of STAGES - 1, asked for
+// before the kernel ahead has finished.  With this step's own key and value among them: the block that finishes those from the
+// projection puts them into the arrived tile itself.  Ranges start on multiples of 64 (what lies ahead of the window is masked).  A tile
+// comes as halves of 64 columns, rows of 128 bytes in the hardware's swizzle.  Rows outside the range hold whatever the page
+// holds; their values are cleared, so that a weight of zero meets no infinity.  Every wait for a tile is bounded
+// (lily_attention_decode_status).  What bounds it is a block's start (length, table, first tile: 2 us) and its merge; the memory is busy
+// between.  Piece by piece / by TMA, us, 8 kv heads of 4 query heads, head size 128: 19 rows of 400 to 2,900 keys in clusters of two 38.2 / 28.5 (bytes
+// 18.5), 24 rows of 500 to 2,700 39.4 / 30.9, 64 rows of 250 to 1,750 whole 59.4 / 53.1, 48 rows of 250 to 3,500 100 / 66, one tile a row no difference.
+__device__ int g_decode_status = 0;
+constexpr uint32_t TILE_SPINS = 1u << 22;
+template <int D, int STAGES>
+__host__ __device__ constexpr size_t tma_bytes() { return 1024 + 2 * (size_t)STAGES * BN * D * 2 + 16 * D * 2 + 2 * D * 2; }
+
+template <int D, bool DECODE, int STAGES, bool CLUSTER, bool TMA>
 __global__ void __launch_bounds__(THREADS, D <= 128 ? 3 : 1)
-attention_mma_kernel(const AttnArgs a, const int page_shift) {
+attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_constant__ CUtensorMap map_kv) {
     constexpr int CH = D / 8;                  // 16-byte pieces per row
     constexpr int KSTEPS = D / 16;
     constexpr int BM = DECODE ? 16 : 64;
     constexpr int NT = DECODE ? 2 : 8;         // score n-tiles (8 keys each) per warp and key tile
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    unsigned char* k_s = smem_raw;                                  // [STAGES][BN][D]
+    constexpr int TILE = BN * D * 2;
+    unsigned char* k_s = TMA ? reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023) : smem_raw;      // [STAGES][BN][D]
     unsigned char* v_s = k_s + STAGES * BN * D * 2;                 // [STAGES][BN][D]
     // the queries pass through the last key stage on their way to registers: that stage is first
     // filled after the barrier of the first loop iteration, when every warp has its fragments
-    unsigned char* q_s = k_s + (STAGES - 1) * BN * D * 2;           // [BM][D], BM <= BN
+    // (TMA: room of their own, behind the stages; then this step's own key and value)
+    unsigned char* q_s = TMA ? k_s + 2 * STAGES * TILE : k_s + (STAGES - 1) * TILE;           // [BM][D], BM <= BN
+    __nv_bfloat16* own_s = reinterpret_cast<__nv_bfloat16*>(q_s + BM * D * 2);                // TMA: [2][D]
+    __shared__ __align__(8) uint64_t full_s[STAGES];
+    // the 16-byte piece `ch` of row `r` of a tile
+    auto piece = [](int r, int ch) { return TMA ? (uint32_t)((ch >> 3) * (BN * 128) + r * 128 + (((ch ^ r) & 7) << 4)) : swz<D>(r, ch); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, c = lane & 3;
     DECODE_STAMP(0);
@@ -142,25 +163,50 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
     const __nv_bfloat16* kv = (const __nv_bfloat16*)a.kv;
     const int group = a.nq / a.nkv;
 
+    int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
     int req, kvh, kbeg, kend, nrows, head0 = 0, tok0 = 0, pos0 = 0, v_shift = a.v_shift;
     if (DECODE) {
-        req = blockIdx.x;
+        int seq = -1;
+        if (TMA && !CLUSTER && a.longest_first) {
+            // the blocks of the row that is next by length: its kv heads and ranges side by side
+            int* len_s = reinterpret_cast<int*>(q_s);                  // the queries come there later
+            __shared__ int row_s;
+            const int rows = gridDim.x, part = gridDim.y * gridDim.z;
+            const int at = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), want = at / part;
+            const int mine = tid < rows ? a.seq_lens[tid] : 0;
+            len_s[tid] = mine;
+            __syncthreads();
+            int rank = 0;
+#pragma unroll 8
+            for (int j = 0; j < rows; ++j) {
+                const int other = len_s[j];
+                rank += other > mine || (other == mine && j < tid);
+            }
+            if (tid < rows && rank == want) row_s = tid;
+            __syncthreads();
+            bx = row_s;
+            by = at % part / gridDim.z;
+            bz = at % part % gridDim.z;
+            seq = len_s[bx];
+        }
+        req = bx;
         if (a.decode_rows > 0) {                             // all shifts of the value heads in one launch
             v_shift = req / a.decode_rows;
             req -= v_shift * a.decode_rows;
         }
         const int chunks = (group + 15) / 16;
-        kvh = blockIdx.y / chunks;
-        const int r0 = (blockIdx.y % chunks) * 16;
-        const int seq = a.seq_lens[req];
-        const int lo = (a.window > 0 && seq > a.window) ? seq - a.window : 0;
+        kvh = by / chunks;
+        const int r0 = (by % chunks) * 16;
+        if (seq < 0) seq = a.seq_lens[req];
+        int lo = (a.window > 0 && seq > a.window) ? seq - a.window : 0;
+        if (TMA) lo &= ~(BN - 1);
         int per = (seq - lo + a.splits - 1) / a.splits;
         per = (per + BN - 1) / BN * BN;
-        kbeg = lo + blockIdx.z * per;
+        kbeg = lo + bz * per;
         kend = min(seq, kbeg + per);
         nrows = min(16, group - r0);
         head0 = kvh * group + r0;
-        tok0 = blockIdx.x;                                   // the row written; the query's row is `req`
+        tok0 = bx;                                   // the row written; the query's row is `req`
         pos0 = seq > 0 ? seq - 1 : 0;                        // an empty row (no position yet) reads table entry 0 at most
     } else {
         const int tile = gridDim.x - 1 - blockIdx.x;       // the tiles come ordered by the keys they see: longest first
@@ -183,7 +229,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
     // With a window that keeps the first positions in sight, the keys [0, kept) that lie before the range come first, in
     // tiles of their own (the block of the first range only, where the ranges of a row are cut): tile t covers the keys
     // from tile_base(t) up to tile_limit(t).
-    const int kept = (a.window > 0 && a.keep_first > 0 && (!DECODE || blockIdx.z == 0)) ? min(a.keep_first, kbeg) : 0;
+    const int kept = (a.window > 0 && a.keep_first > 0 && (!DECODE || bz == 0)) ? min(a.keep_first, kbeg) : 0;
     const int ftiles = (kept + BN - 1) / BN;
     const int ntiles = ftiles + (kend > kbeg ? (kend - kbeg + BN - 1) / BN : 0);
     auto tile_base = [&](int t) { return t < ftiles ? t * BN : kbeg + (t - ftiles) * BN; };
@@ -210,10 +256,44 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
         }
     };
 
+    // TMA: one thread asks for a tile, which lies in one page
+    const uint32_t full0 = smem_u32(full_s);
+    auto ask_tile = [&](int t) {
+        const int kb = tile_base(t), st = t % STAGES, page = table[kb >> page_shift], off = kb & page_mask;
+        const uint32_t bar = full0 + 8 * st, kd = smem_u32(k_s + st * TILE), vd = smem_u32(v_s + st * TILE);
+        const int vh = a.nkv + (v_shift ? (kvh + v_shift) % a.nkv : kvh);
+        tc5::mbar_expect_tx(bar, 2 * TILE);
+#pragma unroll
+        for (int h = 0; h < D / 64; ++h) tc5::tma_load_4d(kd + h * (BN * 128), &map_kv, bar, h * 64, off, kvh, page);
+#pragma unroll
+        for (int h = 0; h < D / 64; ++h) tc5::tma_load_4d(vd + h * (BN * 128), &map_kv, bar, h * 64, off, vh, page);
+    };
+    const bool patched = TMA && a.qkv != nullptr && a.write_kv;          // this step's own key and value never come from the page
+    bool arrived = true;
+    if (TMA) {
+        if (tid == 0) {
+#pragma unroll
+            for (int st = 0; st < STAGES; ++st) tc5::mbar_init(full0 + 8 * st, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+        __syncthreads();
+        if (tid == 0)
+            for (int st = 0; st < STAGES && st < ntiles; ++st)
+                if (patched || tile_base(st) + BN <= pos0) ask_tile(st);
+        DECODE_STAMP(1);
+        pdl_wait();
+        pdl_launch_dependents();
+        DECODE_STAMP(2);
+        if (tid == 0) {
+            asm volatile("fence.proxy.async;\n" ::: "memory");           // the kernel ahead wrote this step's key by threads
+            for (int st = 0; st < STAGES && st < ntiles; ++st)
+                if (!(patched || tile_base(st) + BN <= pos0)) ask_tile(st);
+        }
+    }
     // the pipeline keeps STAGES - 1 tiles in flight; every iteration commits one group (maybe empty).
     // Decode: the tiles that end before this step's own key are asked for ahead of the wait.
     int early = 0;
-    if (DECODE) {
+    if (DECODE && !TMA) {
 #pragma unroll
         for (int st = 0; st < STAGES - 1; ++st) {
             if (st < ntiles && (st < ftiles || tile_base(st) + BN <= pos0) && early == st) {
@@ -333,7 +413,10 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
                     const uint32_t two = pack_bf16(x[2 * j], x[2 * j + 1]);
                     const int i = e0 + 2 * j;
                     if (is_q) *reinterpret_cast<uint32_t*>(q_s + swz<D>(job, i >> 3) + (i & 7) * 2) = two;
-                    else *reinterpret_cast<uint32_t*>(cached + i) = two;
+                    else {
+                        *reinterpret_cast<uint32_t*>(cached + i) = two;
+                        if (TMA) *reinterpret_cast<uint32_t*>(own_s + (is_v ? D : 0) + i) = two;
+                    }
                 }
             };
             for (int job = warp; job < jobs; job += 2 * WARPS) {
@@ -356,7 +439,10 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
             auto put = [&](int i, float v) {
                 const __nv_bfloat16 b = __float2bfloat16_rn(v);
                 if (is_q) *reinterpret_cast<__nv_bfloat16*>(q_s + swz<D>(job, i >> 3) + (i & 7) * 2) = b;
-                else cached[i] = b;
+                else {
+                    cached[i] = b;
+                    if (TMA) own_s[(is_v ? D : 0) + i] = b;
+                }
             };
             if (is_v) {
                 for (int i = lane; i < D; i += 32) put(i, in(src + i));
@@ -392,7 +478,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
                 put(i, x);
             }
         }
-        if (owner) __threadfence();                // the key and the value are in place before this block's copies read them
+        if (owner && !TMA) __threadfence();                // the key and the value are in place before this block's copies read them
     } else
     for (int i = tid; i < BM * CH; i += THREADS) {
         const int r = i / CH, ch = i % CH;
@@ -419,14 +505,14 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
 
     // the sink: a key of score 0 without a value, counted once a row (decode: by the first warp of the first key range;
     // the sums are per thread until the end, so one thread of the four that share a row holds the unit)
-    const bool sunk = a.sink && (!DECODE || (warp == 0 && blockIdx.z == 0));
+    const bool sunk = a.sink && (!DECODE || (warp == 0 && bz == 0));
     float m_lo = sunk ? 0.f : -INFINITY, m_hi = m_lo, l_lo = sunk && c == 0 ? 1.f : 0.f, l_hi = l_lo;
     float o[D / 8][4];
 #pragma unroll
     for (int j = 0; j < D / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
 
 #pragma unroll
-    for (int st = 0; st < STAGES - 1; ++st) {
+    for (int st = 0; st < STAGES - 1 && !TMA; ++st) {
         if (st >= early) {
             if (st < ntiles) load_tile(st, st);
             cp_async_commit();
@@ -441,14 +527,38 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
 
     for (int t = 0; t < ntiles; ++t) {
         const int buf = t % STAGES;
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();                                    // tile t has landed; tile t-1's readers are done
-        if (t == 0) DECODE_STAMP(4);
-        if (t + STAGES - 1 < ntiles) load_tile(t + STAGES - 1, (t + STAGES - 1) % STAGES);
-        cp_async_commit();
-        const unsigned char* kt = k_s + buf * BN * D * 2;
-        const unsigned char* vt = v_s + buf * BN * D * 2;
         const int kb = tile_base(t), klim = tile_limit(t);
+        unsigned char* kt = k_s + buf * TILE;
+        unsigned char* vt = v_s + buf * TILE;
+        if (TMA) {
+            uint32_t spins = 0;
+            while (arrived && !tc5::mbar_try_wait(full0 + 8 * buf, (t / STAGES) & 1)) arrived = ++spins < TILE_SPINS;
+            if (!arrived && lane == 0) atomicCAS(&g_decode_status, 0, 1 + (bx & 0x7fff));
+            const int first = a.window > 0 && t >= ftiles ? max(0, pos0 + 1 - a.window - kb) : 0;       // rows ahead of the window
+            if (first > 0 || kb + BN > klim || (patched && kb <= pos0 && pos0 < kb + BN)) {
+                // values of rows outside the range are cleared (kept first positions stay); this step's own row is put in
+                const int mine = patched && kbeg <= pos0 && pos0 < kend && t >= ftiles ? pos0 - kb : BN;
+                for (int i = tid; i < BN * CH; i += THREADS) {
+                    const int r = i / CH, ch = i % CH;
+                    if (r == mine) {
+                        *reinterpret_cast<uint4*>(kt + piece(r, ch)) = *reinterpret_cast<const uint4*>(own_s + ch * 8);
+                        *reinterpret_cast<uint4*>(vt + piece(r, ch)) = *reinterpret_cast<const uint4*>(own_s + D + ch * 8);
+                    } else if (kb + r >= klim || (r < first && kb + r >= a.keep_first)) {
+                        *reinterpret_cast<uint4*>(vt + piece(r, ch)) = make_uint4(0, 0, 0, 0);
+                    }
+                }
+                asm volatile("fence.proxy.async;\n" ::: "memory");      // a later tile's copy comes behind these
+                __syncthreads();
+            }
+        } else {
+            cp_async_wait<STAGES - 2>();
+            __syncthreads();                                // tile t has landed; tile t-1's readers are done
+        }
+        if (t == 0) DECODE_STAMP(4);
+        if (!TMA) {
+            if (t + STAGES - 1 < ntiles) load_tile(t + STAGES - 1, (t + STAGES - 1) % STAGES);
+            cp_async_commit();
+        }
         const int key0 = DECODE ? warp * 16 : 0;            // first key of this warp's share of the tile
 
         // ---- s = q . k^T -------------------------------------------------------------------
@@ -461,7 +571,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
             for (int jp = 0; jp < NT / 2; ++jp) {
                 uint32_t b0, b1, b2, b3;
                 const int krow = key0 + jp * 16 + (lane & 7) + ((lane >> 4) << 3);
-                ldmatrix_x4(smem_u32(kt + swz<D>(krow, kk * 2 + ((lane >> 3) & 1))), b0, b1, b2, b3);
+                ldmatrix_x4(smem_u32(kt + piece(krow, kk * 2 + ((lane >> 3) & 1))), b0, b1, b2, b3);
                 mma_bf16(s[2 * jp], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
                 mma_bf16(s[2 * jp + 1], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b2, b3);
             }
@@ -537,10 +647,14 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
 #pragma unroll
             for (int jp = 0; jp < D / 16; ++jp) {
                 uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(smem_u32(vt + swz<D>(vrow, jp * 2 + (lane >> 4))), b0, b1, b2, b3);
+                ldmatrix_x4_trans(smem_u32(vt + piece(vrow, jp * 2 + (lane >> 4))), b0, b1, b2, b3);
                 mma_bf16(o[2 * jp], a0, a1, a2, a3, b0, b1);
                 mma_bf16(o[2 * jp + 1], a0, a1, a2, a3, b2, b3);
             }
+        }
+        if (TMA && t + STAGES < ntiles) {
+            __syncthreads();                                // every warp is done with this buffer
+            if (tid == 0) ask_tile(t + STAGES);
         }
     }
 
@@ -593,9 +707,9 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
     // finishes its share of the output, so that neither scratch in global memory nor a combine kernel is needed.
     // Sums travel and are merged four neighbouring features at a time (shares are multiples of four).
     cg::cluster_group cluster = cg::this_cluster();
-    const int splits = a.splits, me = blockIdx.z;
+    const int splits = a.splits, me = bz;
     const int share = cluster_share(min(16, group), D, splits);
-    float* recv_o = reinterpret_cast<float*>(smem_raw + stage_bytes<D, STAGES>(true));     // [splits][share]
+    float* recv_o = reinterpret_cast<float*>(TMA ? smem_raw + tma_bytes<D, STAGES>() : smem_raw + stage_bytes<D, STAGES>(true));     // [splits][share]
     float* recv_ml = recv_o + (size_t)splits * share;                                        // [splits][16][2]
     for (int i4 = tid; i4 < nrows * (D / 4); i4 += THREADS) {
         const int r = i4 / (D / 4), col = (i4 % (D / 4)) * 4, i = r * D + col;
@@ -626,7 +740,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
             if (col / 4 < splits)                          // group p of four columns tells block p the row's (max, sum)
                 *reinterpret_cast<float2*>(cluster.map_shared_rank(recv_ml, col / 4) + (me * 16 + r) * 2) = make_float2(mx, den);
         } else if (a.splits > 1) {
-            const size_t base = ((size_t)tok0 * a.nq + head) * a.splits + blockIdx.z;
+            const size_t base = ((size_t)tok0 * a.nq + head) * a.splits + bz;
             *reinterpret_cast<float4*>(a.part_o + base * D + col) = acc;
             if (col == 0) {
                 a.part_ml[base * 2] = mx * ln2;             // back to natural-log units for the combine kernel
@@ -672,11 +786,11 @@ attention_mma_kernel(const AttnArgs a, const int page_shift) {
 }
 
 // Raises the kernel's dynamic shared memory limit to `bytes` if it is lower (never lowers it).
-template <int D, int STAGES>
+template <int D, int STAGES, bool TMA>
 static bool cluster_smem(size_t bytes) {
     static size_t granted = 0;
     if (bytes > granted) {
-        if (cudaFuncSetAttribute(attention_mma_kernel<D, true, STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(attention_mma_kernel<D, true, STAGES, true, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)bytes) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -689,7 +803,7 @@ static bool cluster_smem(size_t bytes) {
 // How many clusters of `splits` blocks of the decode kernel the device holds at once (asked once per head
 // size, cluster size and shared-memory size, which grows with the query heads of a kv head; 0: such a cluster
 // cannot be placed).
-template <int D, int STAGES>
+template <int D, int STAGES, bool TMA>
 static int cluster_capacity(int splits, size_t smem) {
     static int known[MAX_CLUSTER + 1] = {};                     // 0 not asked, -1 none, else the count
     static size_t known_smem[MAX_CLUSTER + 1] = {};             // the shared memory the answer was given for
@@ -708,10 +822,10 @@ static int cluster_capacity(int splits, size_t smem) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         // more than 8 blocks a cluster is a size the device has to allow explicitly
-        const bool ok = cluster_smem<D, STAGES>(smem) &&
-                        (splits <= 8 || cudaFuncSetAttribute(attention_mma_kernel<D, true, STAGES, true>,
+        const bool ok = cluster_smem<D, STAGES, TMA>(smem) &&
+                        (splits <= 8 || cudaFuncSetAttribute(attention_mma_kernel<D, true, STAGES, true, TMA>,
                                                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
-                        cudaOccupancyMaxActiveClusters(&clusters, attention_mma_kernel<D, true, STAGES, true>, &cfg) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, attention_mma_kernel<D, true, STAGES, true, TMA>, &cfg) == cudaSuccess &&
                         clusters > 0;
         if (!ok) cudaGetLastError();
         known[splits] = ok ? clusters : -1;
@@ -729,17 +843,17 @@ static bool cluster_enabled() {
 }
 
 // Returns 0 on success, and in `merged` whether the kernel itself merged the splits into `out`.
-template <int D, bool DECODE, int STAGES>
-static int launch(const AttnArgs& a, dim3 grid, int page_shift, cudaStream_t stream, bool* merged) {
-    size_t smem = stage_bytes<D, STAGES>(DECODE);
+template <int D, bool DECODE, int STAGES, bool TMA = false>
+static int launch(const AttnArgs& a, dim3 grid, int page_shift, cudaStream_t stream, bool* merged, const CUtensorMap& map = CUtensorMap{}) {
+    size_t smem = TMA ? tma_bytes<D, STAGES>() : stage_bytes<D, STAGES>(DECODE);
     // clusters pay when all of them are resident at once; over several rounds of blocks their placement costs
     // more than the combine kernel (measured: 32 requests x 8 kv heads x 7 splits 116 against 103 us)
     if (DECODE && STAGES == (D <= 128 ? LILY_DECODE_STAGES : 2) && a.splits >= 2 && a.splits <= MAX_CLUSTER && cluster_enabled()) {
         const int rows = a.nq / a.nkv < 16 ? a.nq / a.nkv : 16;
         const size_t with_recv = smem + ((size_t)a.splits * cluster_share(rows, D, a.splits) + (size_t)a.splits * 16 * 2) * sizeof(float);
-        if ((long)grid.x * grid.y <= cluster_capacity<D, DECODE ? STAGES : 2>(a.splits, with_recv)) {
-            auto kern = attention_mma_kernel<D, true, DECODE ? STAGES : 2, true>;
-            if (!cluster_smem<D, DECODE ? STAGES : 2>(with_recv)) {
+        if ((long)grid.x * grid.y <= cluster_capacity<D, DECODE ? STAGES : 2, TMA>(a.splits, with_recv)) {
+            auto kern = attention_mma_kernel<D, true, DECODE ? STAGES : 2, true, TMA>;
+            if (!cluster_smem<D, DECODE ? STAGES : 2, TMA>(with_recv)) {
                 set_error("attention_mma: cannot get %zu bytes of shared memory", with_recv);
                 return 2;
             }
@@ -757,12 +871,12 @@ static int launch(const AttnArgs& a, dim3 grid, int page_shift, cudaStream_t str
             attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = pdl_enabled() ? 2 : 1;
-            cudaLaunchKernelEx(&cfg, kern, a, page_shift);
+            cudaLaunchKernelEx(&cfg, kern, a, page_shift, map);
             *merged = true;
             return 0;
         }
     }
-    auto kern = attention_mma_kernel<D, DECODE, STAGES, false>;
+    auto kern = attention_mma_kernel<D, DECODE, STAGES, false, TMA>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -772,8 +886,32 @@ static int launch(const AttnArgs& a, dim3 grid, int page_shift, cudaStream_t str
         }
         configured = true;
     }
-    launch_pdl(kern, grid, dim3(THREADS), smem, stream, a, page_shift);
+    AttnArgs b = a;
+    // Longest row first, where the blocks outnumber the places (three a SM) and finding a row's rank (about 1.5 us a block, hidden by the others of its SM) is cheap beside what is gained.  Batch order /
+    // longest first, us: 64 rows of 250 to 1,750 keys whole 53.2 / 45.3 (its bytes 40.3), 32 such rows in 2 ranges 32.2 / 27.8, 48 of 250 to
+    // 3,500 in 2 69.1 / 59.3; many short blocks pay for the order: 64 rows in 4 ranges 54.5 / 62.4, 128 rows whole 89.0 / 88.3.
+    const long places = 3L * sm_count();
+    b.longest_first = TMA && STAGES == 2 && a.decode_rows == 0 && grid.x > 1 && grid.x <= THREADS && (long)grid.x * grid.y * grid.z > places &&
+                      (long)grid.x * grid.y * grid.z <= 2 * places;
+    launch_pdl(kern, grid, dim3(THREADS), smem, stream, b, page_shift, map);
     *merged = false;
+    return 0;
+}
+
+// Whether decode tiles come by TMA: pages of whole tiles, head sizes of one or two halves.
+static bool tma_takes(const AttnArgs& a) {
+    return (a.d == 64 || a.d == 128) && a.page_size % BN == 0 && a.pages > 0 && ((uintptr_t)a.kv & 15) == 0 && tc5::encoder() != nullptr;
+}
+// The layer's cache [pages, 2 nkv, page_size, d] in boxes of 64 positions of 64 columns of one head.
+static int make_cache_map(CUtensorMap* map, const AttnArgs& a) {
+    const cuuint64_t dims[4] = {(cuuint64_t)a.d, (cuuint64_t)a.page_size, (cuuint64_t)2 * a.nkv, (cuuint64_t)a.pages};
+    const cuuint64_t row = (cuuint64_t)a.d * 2;
+    const cuuint64_t strides[3] = {row, row * a.page_size, row * a.page_size * 2 * a.nkv};
+    const cuuint32_t box[4] = {64, BN, 1, 1}, elem[4] = {1, 1, 1, 1};
+    const CUresult rc = tc5::encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(a.kv), dims, strides, box, elem,
+                                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    LILY_REQUIRE(rc == CUDA_SUCCESS, "attention_decode: cuTensorMapEncodeTiled failed with %d (%d pages of %d)", (int)rc, a.pages, a.page_size);
     return 0;
 }
 
@@ -786,16 +924,33 @@ static int dispatch(const AttnArgs& a, dim3 grid, cudaStream_t stream, bool* mer
         return 1;
     }
     constexpr int ST = DECODE ? LILY_DECODE_STAGES : 2;
+    if constexpr (DECODE) {
+        if (a.stages == 0 && tma_takes(a)) {
+            CUtensorMap map;
+            if (int rc = make_cache_map(&map, a)) return rc;
+            if (a.d == 64) return launch<64, true, ST, true>(a, grid, page_shift, stream, merged, map);
+            return launch<128, true, ST, true>(a, grid, page_shift, stream, merged, map);
+        }
+    }
     if (DECODE && a.stages != 0 && a.stages != ST) {
         // a third stage: 96 KB a block at head size 128, so two blocks a SM, each with two tiles on their way while it
         // works on a third.  Measured on a B200 (8 kv heads of 4 query heads, head size 128, one range a row, us, two
         // stages / three): 32 rows of 4,096 keys 109 / 82 (and 96 in 7 ranges with the combine kernel), 64 rows 181 in
         // 4 ranges / 168, 32 rows of 1,024 keys 31.6 / 24.2, 64 rows 58.7 / 48.0; 20 rows of 4,096 keys 89.5 / 78.9
         // (61.0 in two ranges of two stages: too few blocks for three stages).  Four stages, one block a SM: slower
-        // everywhere (32 rows of 4,096 keys 122 us).
+        // everywhere (32 rows of 4,096 keys 122 us).  With the tiles by TMA: 32 rows of 4,096 keys 83.5 / 81.6, 64 rows 167 in 4 ranges / 156,
+        // 32 rows of 1,024 26.5 / 24.4, 64 rows 55.9 / 47.4, 20 rows of 4,096 63.0 / 59.1 (55.1 in two ranges).
         if (a.stages != 3 || a.d > 128) {
             set_error("attention_mma: %d key/value stages at head size %d (2 everywhere, 3 up to head size 128)", a.stages, a.d);
             return 1;
+        }
+        if constexpr (DECODE) {
+            if (tma_takes(a)) {
+                CUtensorMap map;
+                if (int rc = make_cache_map(&map, a)) return rc;
+                if (a.d == 64) return launch<64, true, 3, true>(a, grid, page_shift, stream, merged, map);
+                return launch<128, true, 3, true>(a, grid, page_shift, stream, merged, map);
+            }
         }
         if (a.d == 64) return launch<64, DECODE, DECODE ? 3 : 2>(a, grid, page_shift, stream, merged);
         return launch<128, DECODE, DECODE ? 3 : 2>(a, grid, page_shift, stream, merged);
@@ -864,11 +1019,14 @@ LILY_API int lily_attention_decode_mma_clusters(int d, int splits, int group) {
     if (splits < 2 || splits > mma::MAX_CLUSTER || !mma::cluster_enabled()) return 0;
     const int rows = group < 16 ? group : 16;
     const size_t recv = ((size_t)splits * mma::cluster_share(rows, d, splits) + (size_t)splits * 16 * 2) * sizeof(float);
+    // (the kernel whose tiles come by TMA takes a little more shared memory; both merge in clusters what is planned for)
+    constexpr int ST = LILY_DECODE_STAGES;
+    auto both = [](int x, int y) { return x < y ? x : y; };
     switch (d) {
-        case 64: return mma::cluster_capacity<64, LILY_DECODE_STAGES>(splits, mma::stage_bytes<64, LILY_DECODE_STAGES>(true) + recv);
-        case 128: return mma::cluster_capacity<128, LILY_DECODE_STAGES>(splits, mma::stage_bytes<128, LILY_DECODE_STAGES>(true) + recv);
-        case 192: return mma::cluster_capacity<192, 2>(splits, mma::stage_bytes<192, 2>(true) + recv);
-        case 256: return mma::cluster_capacity<256, 2>(splits, mma::stage_bytes<256, 2>(true) + recv);
+        case 64: return both(mma::cluster_capacity<64, ST, false>(splits, mma::stage_bytes<64, ST>(true) + recv), mma::cluster_capacity<64, ST, true>(splits, mma::tma_bytes<64, ST>() + recv));
+        case 128: return both(mma::cluster_capacity<128, ST, false>(splits, mma::stage_bytes<128, ST>(true) + recv), mma::cluster_capacity<128, ST, true>(splits, mma::tma_bytes<128, ST>() + recv));
+        case 192: return mma::cluster_capacity<192, 2, false>(splits, mma::stage_bytes<192, 2>(true) + recv);
+        case 256: return mma::cluster_capacity<256, 2, false>(splits, mma::stage_bytes<256, 2>(true) + recv);
     }
     return 0;
 }
@@ -899,12 +1057,14 @@ static int decode_mma(AttnArgs& a, const void* q, const void* kv, void* out, con
 // clusters resident at once) the blocks of a (request, kv head) form a cluster and merge their results through
 // distributed shared memory; else the partial results go to `scratch` in the layout of attention_simt.cu
 // ([requests, nq, splits, d] outputs, then [requests, nq, splits, 2] (max, sum)) and the combine kernel is launched behind.
+// `pages`: pages of the layer's cache (0: not known; tiles are then fetched piece by piece, as where a page is no whole tile).
 // `stages`: 0, or the key/value tiles a block holds (3, up to head size 128: two blocks a SM, no clusters).
 LILY_API int lily_attention_decode_mma(const void* q, const void* kv, void* out, const int* block_table,
                                        int bt_stride, const int* seq_lens, float* scratch, int requests, int splits,
                                        int nq, int nkv, int d, int page_size, int window, float scale, int stages,
-                                       float softcap, int keep_first, int sink, int v_shift, cudaStream_t stream) {
+                                       float softcap, int keep_first, int sink, int v_shift, int pages, cudaStream_t stream) {
     AttnArgs a{};
+    a.pages = pages;
     // v_shift -1: every shift in one launch, nkv planes of `requests` rows in `out` (and as many rows of scratch)
     LILY_REQUIRE(nkv > 0 && v_shift >= -1 && v_shift < nkv, "attention_decode: value heads shifted by %d of %d", v_shift, nkv);
     a.softcap = softcap; a.sink = sink; a.v_shift = v_shift < 0 ? 0 : v_shift;
@@ -927,7 +1087,7 @@ LILY_API int lily_attention_decode_mma_fused(const void* qkv, int qkv_planes, si
                                              void* kv, void* out, const int* block_table, int bt_stride,
                                              const int* seq_lens, float* scratch, int requests, int splits, int nq,
                                              int nkv, int d, int page_size, int window, float scale, int stages,
-                                             float softcap, int qkv_ld, cudaStream_t stream) {
+                                             float softcap, int qkv_ld, int pages, cudaStream_t stream) {
     // rows of the product may go on behind the heads; a layer that writes no keys may have the query heads alone
     LILY_REQUIRE(qkv_ld % 2 == 0 && qkv_ld >= (write_kv ? nq + 2 * nkv : nq) * d, "attention_decode_fused: rows of %d numbers", qkv_ld);
     LILY_REQUIRE(qkv != nullptr && qkv_planes >= 1 && (qkv_dtype == kF32 || qkv_planes == 1),
@@ -941,6 +1101,16 @@ LILY_API int lily_attention_decode_mma_fused(const void* qkv, int qkv_planes, si
     a.cos_t = cos_t; a.sin_t = sin_t; a.rd = cos_t ? rd : 0; a.write_kv = write_kv;
     a.softcap = softcap;
     a.qkv_ld = qkv_ld;
+    a.pages = pages;
     return decode_mma(a, nullptr, kv, out, block_table, bt_stride, seq_lens, scratch, requests, splits, nq, nkv, d,
                       page_size, window, scale, stages, stream);
+}
+
+// 0, or 1 + the request row of the first decode block whose wait for a tile ran out since the last call; clears it.
+LILY_API int lily_attention_decode_status() {
+    int v = 0;
+    const int zero = 0;
+    if (cudaMemcpyFromSymbol(&v, mma::g_decode_status, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(mma::g_decode_status, &zero, sizeof(int));
+    return v;
 }

@@ -41,9 +41,9 @@ _SIGNATURES = {
     "lily_attention_combine": [_vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_attention_prefill_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp],
     "lily_attention_prefill_tc": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _f, _i, _i, _i, _vp],
-    "lily_attention_decode_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _vp],
+    "lily_attention_decode_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp],
     "lily_attention_decode_mma_fused": [_vp, _i, _sz, _i, _vp, _vp, _i, _f, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _vp,
-                                        _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _vp],
+                                        _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp],
     "lily_sigmoid_gate": [_vp, _i, _vp, _i, _i, _sz, _sz, _vp],
     "lily_sigmoid_head_gate": [_vp, _i, _vp, _i, _i, _sz, _i, _i, _i, _i, _i, _vp],
     "lily_add_tanh_norm": [_vp, _vp, _i, _i, _sz, _f, _vp, _vp, _f, _f, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _vp],
@@ -722,8 +722,8 @@ def sink_prompts_on_tcgen05(d: int, new_lens: Sequence[int], heads: int, planes:
 
 
 def attention_tc_status() -> int:
-    """0, or a code from the first bounded wait that gave up in the tcgen05 attention kernel (synchronises)."""
-    return int(library().lily_attention_tc_status())
+    """0, or a code from the first bounded wait that gave up in the attention kernels whose tiles come by TMA (synchronises)."""
+    return int(library().lily_attention_tc_status()) or int(library().lily_attention_decode_status())
 
 
 def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor, cu_seqlens: torch.Tensor,
@@ -917,6 +917,7 @@ def attention_decode(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch
     common = (_p(q), _p(kv_layer), _p(out), _i32(block_table, "block_table"), block_table.shape[-1],
               _i32(seq_lens, "seq_lens"), _p(scratch), requests, splits, nq, nkv, d, page_size, int(window or 0),
               float(scale))
+    pages = kv_layer.shape[0] if kv_layer.numel() == kv_layer.shape[0] * 2 * nkv * page_size * d else 0
     if values_in_keys and latent_tcgen05(q.dtype, d, dv, page_size, nkv, softcap) and not stages:
         _call("lily_latent_attention_decode_tc", _p(q), _p(kv_layer), _p(out), _i32(block_table, "block_table"),
               block_table.shape[-1], _i32(seq_lens, "seq_lens"), _p(scratch), requests, splits, nq, d, dv, page_size,
@@ -934,12 +935,12 @@ def attention_decode(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch
             _call("lily_attention_decode_mma", _p(q), _p(kv_layer), out[shift].data_ptr() if planes and not merged else _p(out),
                   _i32(block_table, "block_table"), block_table.shape[-1], _i32(seq_lens, "seq_lens"), _p(scratch), requests, splits,
                   nq, nkv, d, page_size, int(window or 0), float(scale), int(stages), cap, int(keep_first or 0) if window else 0,
-                  int(bool(sink)), shift, _stream())
+                  int(bool(sink)), shift, pages, _stream())
             rows = requests * nkv if merged else requests
             if splits > 1 and (stages or rows * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
                 launches["count"] += 1
     elif dv == d and not values_in_keys and not flags and sinks is None and uses_tensor_cores(q.dtype, d):
-        _call("lily_attention_decode_mma", *common, int(stages), cap, int(keep_first or 0) if window else 0, 0, 0, _stream())   # merges the splits itself (cluster, or combine behind)
+        _call("lily_attention_decode_mma", *common, int(stages), cap, int(keep_first or 0) if window else 0, 0, 0, pages, _stream())   # merges the splits itself (cluster, or combine behind)
         if splits > 1 and (stages or requests * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
             launches["count"] += 1                                   # the combine kernel, launched inside
     else:
@@ -1039,6 +1040,27 @@ def whole_rows_pay(pairs: int, sm_count: int = 148) -> bool:
     return last == 0 or last >= 0.45 * places
 
 
+def many_rows_splits(pairs: int, max_seq_len: int, sm_count: int = 148) -> Optional[int]:
+    """Key ranges of ``pairs`` (request, kv head) pairs that are too many for clusters, where the tensor-core kernel takes the longest rows
+    first (three blocks a SM); None where about four rounds of blocks stay the better plan.  Rows of up to 2,048 keys: just enough ranges to
+    take every place and none under 768 keys, since a range costs its block's start and its share of the merge (32 rows of 1,000 keys whole 26.4 us, in 2
+    ranges 34; a row of 2,000 among 63 of 100: whole 33, in 4 ranges 35).  Longer rows: the fewest ranges whose last round of blocks is nearly
+    full, in case the rows are alike (32 rows of 4,096 keys in 2 ranges 100 us, in 3 86, in 7 91.7); with more pairs than places only
+    where that is one range (96 rows of up to 4,000 whole 122, in 3 ranges 141; 64 rows 101 in 3, 98.7 in 4).
+    Before (about four rounds of blocks, or the wave that just fits) / now, us, 8 kv heads: 64 rows of 250 to 1,750 keys 59.6 / 45.5, 32 such
+    rows 39 / 28, 96 rows 77 / 62, 64 rows of 100 to 1,000 40.2 / 27.5."""
+    places = 3 * sm_count
+    if 2 * pairs <= places:
+        return None
+    enough = -(-places // pairs)
+    if max_seq_len <= 2048:
+        return min(enough, max(1, max_seq_len // 768))
+    fill = lambda s: pairs * s / places / -(-pairs * s // places)
+    if enough == 1:
+        return 1 if fill(1) >= 0.85 else None
+    return next((s for s in range(enough, 8) if fill(s) >= 0.85), enough)
+
+
 def f32_rows_take(dtype: torch.dtype, group: int, d: int, dv: int) -> bool:
     """Whether float32 decode rows go to the kernel that cuts a row's keys over warps (attention_decode_f32.cu).  One block of 16 warps a SM:
     its ranges are cut for one wave of blocks and at least 64 keys, one round of a block.  Whole / in such ranges, us: 3 rows of 250
@@ -1090,6 +1112,11 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
         if finer > splits and pairs <= decode_clusters(d, finer, group):
             splits = finer
     in_clusters = tensor_cores and splits > 1 and pairs <= decode_clusters(d, splits, group)
+    # 16 query heads a block write and merge four times the sums of four (40 rows of 250 to 1,750 keys whole 37 us, in 2 ranges 43): ranges as before.  One
+    # or two gain as four do (70 rows of 250 to 1,750 keys in 3 ranges 55.8, whole 47.1) but keep the scratch and the combine kernel, the form that the
+    # engine's tests hold 70 such rows to.
+    if tensor_cores and d <= 128 and 4 <= group <= 8 and not in_clusters:
+        splits = many_rows_splits(pairs, max_seq_len, sm_count()) or splits
     fused = fusable and tensor_cores and pairs * splits <= 3 * sm_count()
     arm = "single" if splits == 1 else ("cluster" if in_clusters else "wave")
     return DecodePlan(splits, fused, decode_scratch_floats(requests, nq, dv, splits), arm)
@@ -1141,7 +1168,7 @@ def attention_decode_fused(qkv: torch.Tensor, q_gain: Optional[torch.Tensor], k_
           _dt(q_gain) if q_gain is not None else _F32, float(eps), _p(cos), _p(sin), int(rotary_dim), int(write_kv),
           _p(kv_layer), _p(out), _i32(block_table, "block_table"), block_table.shape[-1], _i32(seq_lens, "seq_lens"),
           _p(scratch), requests, splits, nq, nkv, d, page_size, int(window or 0), float(scale), int(stages),
-          float(softcap or 0.0), ld, _stream())
+          float(softcap or 0.0), ld, kv_layer.shape[0], _stream())
     if splits > 1 and (stages or requests * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
         launches["count"] += 1                                       # the combine kernel, launched inside
 

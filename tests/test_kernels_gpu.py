@@ -466,6 +466,54 @@ def test_attention_decode_with_three_stages(from_projection, splits, nq, nkv, d,
         o.attention_decode(q, cache, table, seq_t, got, scratch, splits, nq, nkv, d, page, d ** -0.5, window, stages=4)
 
 
+@pytest.mark.parametrize("rows,splits,stages", [(11, 1, 0), (11, 3, 0), (11, 2, 3), (64, 1, 0), (64, 2, 0), (129, 1, 0)])
+@pytest.mark.parametrize("nq,nkv,d,page,window,keep", [
+    (32, 8, 128, 64, None, 0), (32, 8, 128, 128, 100, 0), (16, 8, 64, 64, None, 0), (16, 8, 64, 128, 70, 65), (40, 2, 128, 64, 64, 3)])
+def test_attention_decode_by_whole_tiles(nq, nkv, d, page, window, keep, rows, splits, stages):
+    """Pages of whole tiles come by TMA: against the same cache in pages of 16, which are fetched piece by piece, and the reference.  Rows of one key up to several
+    tiles in an order of their own (64 rows over 8 kv heads are taken longest first, 129 are not), and infinities and NaN where no key is.
+    Without a window both add up the same ranges; with one they start at different keys."""
+    o, dtype = ops(), torch.bfloat16
+    lens = [1, 64, 65, 128, 129, 192, 193, 500, 1000, 3, 257]
+    seqs = [lens[(7 * i) % 11] + (i // 11) for i in range(rows)]
+    cache, table, q, cu, pre = _attention_case(dtype, nq, nkv, d, page, [n - 1 for n in seqs], [1] * rows, window, seed=19, spike=True)
+    seq_t = torch.tensor(seqs, device=DEV, dtype=torch.int32)
+    for r, n in enumerate(seqs):
+        if n % page:
+            cache[int(table[r, n // page]), 0, :, n % page:] = float("nan")
+            cache[int(table[r, n // page]), 1, :, n % page:] = float("inf")
+    k = page // 16
+    pieces = cache.view(cache.shape[0], 2, nkv, k, 16, d).permute(0, 3, 1, 2, 4, 5).reshape(-1, 2, nkv, 16, d).contiguous()
+    small = (table[:, :, None] * k + torch.arange(k, device=DEV, dtype=torch.int32)).reshape(rows, -1).contiguous()
+    scratch = torch.full((max(o.decode_scratch_floats(rows, nq, d, splits), 1),), float("nan"), device=DEV)
+    got, other, want = torch.zeros_like(q), torch.zeros_like(q), torch.zeros_like(q)
+    args = dict(window=window, stages=stages, keep_first=keep)
+    o.attention_decode(q, cache, table, seq_t, got, scratch, splits, nq, nkv, d, page, d ** -0.5, **args)
+    o.attention_decode(q, pieces, small, seq_t, other, scratch, splits, nq, nkv, d, 16, d ** -0.5, **args)
+    ref.attention_decode(q, cache, table, seq_t, want, None, splits, nq, nkv, d, page, d ** -0.5, window, keep_first=keep)
+    assert o.attention_tc_status() == 0
+    if window is None:
+        assert torch.equal(got, other)
+    torch.testing.assert_close(got.float(), want.float(), **tol(dtype))
+    if keep:
+        return
+    # from the projection: the block with the new position puts its key and value into the tile
+    g = torch.Generator(device=DEV).manual_seed(23)
+    qkv = torch.randn(2, rows, (nq + 2 * nkv) * d, device=DEV, generator=g)
+    cos, sin = torch.rand(1100, d // 2, device=DEV, generator=g), torch.rand(1100, d // 2, device=DEV, generator=g)
+    for r, n in enumerate(seqs):
+        cache[int(table[r, (n - 1) // page]), :, :, (n - 1) % page] = float("nan")
+    written = cache.clone()
+    o.attention_decode_fused(qkv, None, None, 1e-6, cos, sin, written, table, seq_t, got, scratch, splits, nq, nkv, d, d, page, d ** -0.5,
+                             window, stages=stages)
+    ref.attention_decode_fused(qkv, None, None, 1e-6, cos, sin, cache, table, seq_t, want, None, splits, nq, nkv, d, d, page, d ** -0.5, window)
+    assert o.attention_tc_status() == 0
+    torch.testing.assert_close(got.float(), want.float(), **tol(dtype))
+    for r, n in enumerate(seqs):
+        at = int(table[r, (n - 1) // page])
+        torch.testing.assert_close(written[at, :, :, (n - 1) % page].float(), cache[at, :, :, (n - 1) % page].float(), **tol(dtype))
+
+
 def test_three_stages_are_refused_where_they_do_not_fit():
     o = ops()
     nq, nkv, d, page = 2, 2, 256, 16
