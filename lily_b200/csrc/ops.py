@@ -1074,8 +1074,9 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
     """The plan for ``requests`` rows that bring one token each, none longer than ``max_seq_len`` positions.
     A step in which every request brings one token may hand the qkv product straight to the attention kernel
     (``fused``): every block then finishes its own queries, which costs less than a kernel of its own while all
-    blocks are resident at once (three a SM) and more when they run in several rounds (measured at batch 64:
-    2 % of the step).
+    blocks are resident at once (three a SM), and where each takes a whole row up to two rounds of them with four query heads (apart / fused, us,
+    8 kv heads: 64 rows of 250 to 1,750 keys 49.6 / 47.8, and the step 1,220 / 1,157; 110 rows 75.5 / 74.2, of 20 to 300 keys 27.3 / 27.8; 128 such
+    rows 29.8 / 31.5; eight query heads, 64 rows of 20 to 300 keys 20.5 / 21.1).
     ``cuda_cores``: the attention has options only the CUDA-core kernel has (a sink, values of all kv heads; ``dv`` is
     then the width of a head's output row).
     ``page_size``: of a cache of latents (``values_in_keys``), which says whether the tcgen05 kernel takes it.
@@ -1117,7 +1118,8 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
     # engine's tests hold 70 such rows to.
     if tensor_cores and d <= 128 and 4 <= group <= 8 and not in_clusters:
         splits = many_rows_splits(pairs, max_seq_len, sm_count()) or splits
-    fused = fusable and tensor_cores and pairs * splits <= 3 * sm_count()
+    in_rounds = splits == 1 and d <= 128 and 4 <= group <= 8 and pairs * group <= 24 * sm_count()
+    fused = fusable and tensor_cores and (pairs * splits <= 3 * sm_count() or in_rounds)
     arm = "single" if splits == 1 else ("cluster" if in_clusters else "wave")
     return DecodePlan(splits, fused, decode_scratch_floats(requests, nq, dv, splits), arm)
 
