@@ -51,7 +51,8 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool in) {
 // one: in a kernel of its own (LIVE 1) where elements come one by one, since a body for eight rows beside it takes the registers of
 // eight (8 requests of 250 keys, 16 heads of 80 over 4, bfloat16: 130 us with eight row slots, 93 with both bodies, 72 alone; eight heads a
 // kv head of 40: 87, 92 and 77), as a second body where the tiles come wide.
-// Three rows of up to 250 keys, 16 heads of 128 over 4, float32: 133 -> 44 us; 451 new tokens of three prompts: 127 -> 94 us.
+// Three rows of up to 250 keys, 16 heads of 128 over 4, float32: 133 -> 44 us (such rows now go to attention_decode_f32.cu, 6.8); 451 new tokens
+// of three prompts: 127 -> 94 us.
 template <typename T, int DCH, bool DECODE, bool WIDE, int LIVE>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const AttnArgs a, const int bufs) {
