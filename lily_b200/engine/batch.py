@@ -48,10 +48,14 @@ class StepEntry:
 
 def wire_array(entry: StepEntry) -> np.ndarray:
     """The entry's token ids as the device reads them, as int32 (an id beyond int32 raises OverflowError).  A prompt's ids are converted
-    and checked as an array, not one by one: 2,048 of them took the host 0.4 ms a step, now 0.05."""
-    if len(entry.tokens) > 1:
+    and checked as an array, not one by one: 2,048 of them took the host 0.4 ms a step, now 0.05.  (Bytes are a sequence of ids like any
+    other; ``array`` would take them for the memory of machine words.)"""
+    if len(entry.tokens) > 1 and not isinstance(entry.tokens, (bytes, bytearray)):
         try:
-            return np.frombuffer(array("i", entry.tokens), dtype=np.int32)
+            ids = np.frombuffer(array("i", entry.tokens), dtype=np.int32)
+            if len(ids) != len(entry.tokens):
+                raise ValueError(f"an entry of {len(entry.tokens)} tokens gives {len(ids)} ids")
+            return ids
         except TypeError:
             pass                                   # numbers that are no integers by type: int() below says what they are
     return np.frombuffer(array("i", entry.wire_tokens), dtype=np.int32)
@@ -218,6 +222,8 @@ def build_step_batch(entries: Sequence[StepEntry], prefix_lens: Sequence[int],
         token_arrays = [wire_array(e) for e in entries]
     out = host.numpy()
     for i, (p, ln) in enumerate(zip(prefix_lens, new_lens)):
+        if len(token_arrays[i]) != ln:
+            raise ValueError(f"{len(token_arrays[i])} ids for the {ln} tokens of an entry")
         out[cu[i]:cu[i + 1]] = token_arrays[i]
         out[n + cu[i]:n + cu[i + 1]] = np.arange(p, p + ln, dtype=np.int32)
         out[2 * n + cu[i]:2 * n + cu[i + 1]] = i
