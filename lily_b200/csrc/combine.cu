@@ -198,25 +198,26 @@ __global__ void normed_mean_kernel(const NormedMeanArgs a) {
 // The same for a few tokens (decode): a thread-block cluster of CL blocks shares one token, each block takes
 // width / CL columns (four a thread) and the blocks exchange their sums of squares through distributed shared
 // memory, so that 8 tokens keep 64 SMs busy instead of 8.  grid (CL, tokens), cluster (CL, 1, 1);
-// width % (4 * CL) == 0; block = width / (4 * CL) threads.
+// width % (4 * CL) == 0; block: width / (4 * CL) threads in whole warps.
 template <int CL>
 __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
     __shared__ float red[MEAN_MAX][33];
     __shared__ float share[MEAN_MAX][CL];
     cg::cluster_group cluster = cg::this_cluster();
     const size_t base = (size_t)blockIdx.y * a.width;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;       // this thread's four columns
+    const int pieces = a.width / (4 * CL), i = (blockIdx.x * pieces + threadIdx.x) * 4;       // this thread's four columns
+    const bool in = threadIdx.x < pieces;
     float4 v[MEAN_MAX], gain[MEAN_MAX], f = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < MEAN_MAX; ++k)                               // the gains depend on no one
-        if (k < a.count) gain[k] = *reinterpret_cast<const float4*>(a.gain[k] + i);
+        if (k < a.count && in) gain[k] = *reinterpret_cast<const float4*>(a.gain[k] + i);
     pdl_enter_small();
-    if (a.add.p) f = a.add.four(base + i);                           // with the inputs, not behind the cluster's barrier
+    if (a.add.p && in) f = a.add.four(base + i);                           // with the inputs, not behind the cluster's barrier
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int k = 0; k < MEAN_MAX; ++k) {
         float ssq = 0.f;
-        if (k < a.count) {
+        if (k < a.count && in) {
             v[k] = a.in[k].four(base + i);
             ssq = v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
         }
@@ -239,6 +240,7 @@ __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
         for (int k = 0; k < MEAN_MAX; ++k) cluster.map_shared_rank(&share[k][0], threadIdx.x)[blockIdx.x] = red[k][32];
     }
     cluster.sync();
+    if (!in) return;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < MEAN_MAX; ++k) {
@@ -343,10 +345,10 @@ LILY_API int lily_normed_mean(const void* const* ins, const int* dtypes, const i
     bool vec = width % 4 == 0 && a.add.vector_ok() && ((uintptr_t)out & 15) == 0;
     for (int k = 0; k < count; ++k) vec = vec && a.in[k].vector_ok() && ((uintptr_t)gains[k] & 15) == 0;
     constexpr int CL = 8;
-    if (vec && tokens <= 64 && width % (4 * CL) == 0 && width / (4 * CL) >= 32 && width / (4 * CL) <= 1024) {
+    if (const int share = vec && tokens <= 64 ? row_cluster_threads(width, CL) : 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(CL, tokens);
-        cfg.blockDim = dim3(width / (4 * CL));
+        cfg.blockDim = dim3(share);
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -72,6 +72,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Threads of each of the `blocks` of a cluster that share a row of `width` columns, four a thread: whole warps, since sums go over all lanes
+// (threads beyond a block's width / (4 * blocks) pieces bring zeros).  0: the row is not cut so.
+inline int row_cluster_threads(int width, int blocks) {
+    const int pieces = width / (4 * blocks);
+    return width % (4 * blocks) == 0 && pieces >= 32 && pieces <= 1024 ? (pieces + 31) / 32 * 32 : 0;
+}
+
 // Streaming multiprocessors of the current device (148 on a B200), asked once.
 inline int sm_count() {
     static int sms = 0;

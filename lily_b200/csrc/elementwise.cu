@@ -210,7 +210,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ resid, const Summed<IN> d
 // The same for a few rows (decode): a thread-block cluster of CL blocks shares one row, each block
 // takes hidden / CL columns (four per thread) and the blocks exchange their sums of squares
 // through distributed shared memory, so that 8 rows keep 64 SMs busy instead of 8.
-// grid (CL, rows), cluster (CL, 1, 1); hidden % (4 * CL) == 0; block = hidden / (4 * CL) threads.
+// grid (CL, rows), cluster (CL, 1, 1); hidden % (4 * CL) == 0; block: hidden / (4 * CL) threads in whole warps.
 template <typename T, typename W, typename IN, int CL>
 __global__ void add_rmsnorm_cluster_kernel(float* __restrict__ resid, const Summed<IN> delta,
                                            const W* __restrict__ weight, T* __restrict__ out,
@@ -221,14 +221,18 @@ __global__ void add_rmsnorm_cluster_kernel(float* __restrict__ resid, const Summ
     pdl_enter_small();
     const int m = blockIdx.y;
     const size_t src = (size_t)(rows ? rows[m] : m) * hidden;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;       // this thread's four columns
-    float4 v = load4(resid, src + i);
-    if (delta) {
-        const float4 dl = delta.four(src + i);
-        v.x += dl.x; v.y += dl.y; v.z += dl.z; v.w += dl.w;
-        if (write_residual) store4(resid, src + i, v);
+    const int pieces = hidden / (4 * CL), i = (blockIdx.x * pieces + threadIdx.x) * 4;       // this thread's four columns
+    const bool in = threadIdx.x < pieces;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f), g = v;
+    if (in) {
+        v = load4(resid, src + i);
+        if (delta) {
+            const float4 dl = delta.four(src + i);
+            v.x += dl.x; v.y += dl.y; v.z += dl.z; v.w += dl.w;
+            if (write_residual) store4(resid, src + i, v);
+        }
+        g = load4(weight, i);
     }
-    const float4 g = load4(weight, i);
     const float mine = block_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w, red);
     // each block tells every block of the cluster its sum; after the one barrier nobody touches another block's
     // shared memory again, so a block may leave as soon as it is done
@@ -238,7 +242,7 @@ __global__ void add_rmsnorm_cluster_kernel(float* __restrict__ resid, const Summ
 #pragma unroll
     for (int r = 0; r < CL; ++r) total += share[r];                  // same order in every block
     const float inv = rsqrtf(total / (float)hidden + eps);
-    store4(out + (size_t)m * hidden, i, make_float4((v.x * inv) * g.x, (v.y * inv) * g.y, (v.z * inv) * g.z, (v.w * inv) * g.w));
+    if (in) store4(out + (size_t)m * hidden, i, make_float4((v.x * inv) * g.x, (v.y * inv) * g.y, (v.z * inv) * g.z, (v.w * inv) * g.w));
 }
 
 
@@ -308,8 +312,11 @@ __global__ void add_rmsnorm_multi4_kernel(float* __restrict__ resid, const Summe
     float4 ga[NCH], gb[NCH];
 #pragma unroll
     for (int k = 0; k < NCH; ++k) {
-        at[k] = ((blockIdx.x * NCH + k) * blockDim.x + threadIdx.x) * 4;
-        if (CL > 1) {                                                // the gains depend on no one
+        at[k] = (k * blockDim.x + threadIdx.x) * 4;
+        if (CL > 1) {                                                // a block's share, which may end inside its last warp
+            const int pieces = hidden / (4 * CL);
+            at[k] = threadIdx.x < pieces ? (blockIdx.x * pieces + threadIdx.x) * 4 : hidden;
+            // the gains depend on no one
             ga[k] = out_a && at[k] < hidden ? load4(gain_a, at[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
             gb[k] = out_b && at[k] < hidden ? load4(gain_b, at[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -727,6 +734,9 @@ LILY_API int lily_scatter_tokens(const int* tokens, const int* logit_rows, const
     return 0;
 }
 
+// What row_cluster_threads says of the clusters of eight that share a row in the norms of a few rows.
+LILY_API int lily_row_cluster_threads(int width) { return row_cluster_threads(width, 8); }
+
 // `in_dtype` is the dtype of the summed input (delta, gate_up, qkv): the activation dtype with one
 // split, or float32 partial sums with `splits` slices `stride` elements apart.
 template <typename T, typename W, typename IN>
@@ -740,10 +750,10 @@ static void launch_add_rmsnorm(float* resid, const void* delta, int splits, size
     const int threads = hidden >= 2048 * per ? 512 : (hidden >= 1024 * per ? 256 : 128);
     const Summed<IN> d{(const IN*)delta, splits, stride};
     constexpr int CL = 8;
-    if (vec && out_rows <= 64 && hidden % (4 * CL) == 0 && hidden / (4 * CL) >= 32 && hidden / (4 * CL) <= 1024) {
+    if (const int share = vec && out_rows <= 64 ? row_cluster_threads(hidden, CL) : 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(CL, out_rows);
-        cfg.blockDim = dim3(hidden / (4 * CL));
+        cfg.blockDim = dim3(share);
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -805,10 +815,10 @@ static void launch_add_rmsnorm_multi(float* resid, const void* da, int sa, size_
     const bool vec = hidden % 4 == 0 && whole(resid, 4, 0) && whole(da, sizeof(INA), stra) && whole(db, sizeof(INB), strb) && whole(bias, 4, 0) &&
                      whole(gain_a, 4, 0) && whole(gain_b, 4, 0) && whole(out_a, sizeof(T), 0) && whole(out_b, sizeof(T), 0);
     constexpr int CL = 8;
-    if (vec && rows <= 64 && hidden % (4 * CL) == 0 && hidden / (4 * CL) >= 32 && hidden / (4 * CL) <= 1024) {
+    if (const int share = vec && rows <= 64 ? row_cluster_threads(hidden, CL) : 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(CL, rows);
-        cfg.blockDim = dim3(hidden / (4 * CL));
+        cfg.blockDim = dim3(share);
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;

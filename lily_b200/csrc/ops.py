@@ -135,6 +135,8 @@ def library():
         lib.lily_attention_decode_scratch_floats.argtypes = [_i, _i, _i, _i]
         lib.lily_attention_decode_scratch_floats.restype = _sz
         lib.lily_normed_mean_max.restype = _i
+        lib.lily_row_cluster_threads.argtypes = [_i]
+        lib.lily_row_cluster_threads.restype = _i
         lib.lily_wkv_max_head_dim.restype = _i
         lib.lily_latent_attention_mma_takes.argtypes = [_i, _i]
         lib.lily_latent_attention_mma_takes.restype = _i

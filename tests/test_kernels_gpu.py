@@ -915,7 +915,7 @@ def test_wkv_scan_of_one_token_a_request(dtype, requests, heads, d):
     torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
 
 
-@pytest.mark.parametrize("rows,hidden", [(1, 1024), (3, 1056), (64, 2048), (65, 2048), (70, 516), (5, 1028), (66, 4100), (3, 8192), (9, 9000), (2, 1027)])
+@pytest.mark.parametrize("rows,hidden", [(1, 1024), (3, 1056), (5, 1536), (2, 2560), (64, 2048), (65, 2048), (70, 516), (5, 1028), (66, 4100), (3, 8192), (9, 9000), (2, 1027)])
 @pytest.mark.parametrize("planes,gains,bias,write", [((1, 17), 2, True, True), ((9, 0), 1, False, True), ((0, 0), 2, True, False), ((8, None), 0, False, True)])
 def test_add_rmsnorm_multi_in_pieces(rows, hidden, planes, gains, bias, write):
     """Rows over a cluster, in a block's registers (whole and with a last piece that few threads have) and a number at a time; sums of one to
@@ -934,6 +934,26 @@ def test_add_rmsnorm_multi_in_pieces(rows, hidden, planes, gains, bias, write):
     torch.testing.assert_close(mine, theirs, rtol=1e-5, atol=1e-5)
     if not write:
         assert torch.equal(mine, kept)
+
+
+@pytest.mark.parametrize("hidden", [1024, 1056, 1536, 2560, 3584, 3616])
+@pytest.mark.parametrize("rows", [1, 9, 64])
+def test_norms_of_a_few_rows_over_clusters(rows, hidden):
+    """Rows over the eight blocks of a cluster whose shares end inside a warp, or do not: each sum is over the row's columns and nothing else, so a
+    column too much or too few (1.4e-4 of every result at 3,616 columns) is beyond what is allowed for three roundings of 2^-24."""
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    unit = lambda x: x * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-6)
+    resid, delta, gain = rand(rows, hidden), rand(3, rows, hidden), rand(hidden)
+    mine = resid.clone()
+    got = ops().add_rmsnorm(mine, delta, gain, 1e-6, torch.float32)
+    total = resid.double() + delta.double().sum(0)
+    torch.testing.assert_close(got.double(), unit(total) * gain, rtol=5e-5, atol=1e-5)
+    torch.testing.assert_close(mine.double(), total, rtol=1e-5, atol=1e-5)
+    a, b, f = rand(2, rows, hidden), rand(1, rows, hidden), rand(1, rows, hidden)
+    got = ops().normed_mean([a, b], [gain, resid[0].contiguous()], 1e-6, add=f)
+    want = (unit(a.double().sum(0)) * gain + unit(b[0].double()) * resid[0]) / 2 + f[0]
+    torch.testing.assert_close(got.double().view(rows, hidden), want, rtol=5e-5, atol=1e-5)
 
 
 @pytest.mark.parametrize("tokens,rank,cols", [(1, 1, 5), (2, 64, 2048), (8, 31, 130), (9, 33, 257), (21, 200, 128), (2364, 33, 128), (2371, 33, 130), (3, 130, 384),
