@@ -150,6 +150,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
     auto piece = [](int r, int ch) { return TMA ? (uint32_t)((ch >> 3) * (BN * 128) + r * 128 + (((ch ^ r) & 7) << 4)) : swz<D>(r, ch); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, c = lane & 3;
+    if (CLUSTER) cluster_arrive_started();
     DECODE_STAMP(0);
     DECODE_SPAN(0);
     // Prefill waits here for the kernel before it (which wrote q and this step's keys).  Decode
@@ -711,6 +712,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
     const int share = cluster_share(min(16, group), D, splits);
     float* recv_o = reinterpret_cast<float*>(TMA ? smem_raw + tma_bytes<D, STAGES>() : smem_raw + stage_bytes<D, STAGES>(true));     // [splits][share]
     float* recv_ml = recv_o + (size_t)splits * share;                                        // [splits][16][2]
+    if (CLUSTER) cluster_wait_started();
     for (int i4 = tid; i4 < nrows * (D / 4); i4 += THREADS) {
         const int r = i4 / (D / 4), col = (i4 % (D / 4)) * 4, i = r * D + col;
         float mw[4], mx = -INFINITY;

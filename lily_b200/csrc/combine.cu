@@ -204,6 +204,7 @@ __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
     __shared__ float red[MEAN_MAX][33];
     __shared__ float share[MEAN_MAX][CL];
     cg::cluster_group cluster = cg::this_cluster();
+    cluster_arrive_started();
     const size_t base = (size_t)blockIdx.y * a.width;
     const int pieces = a.width / (4 * CL), i = (blockIdx.x * pieces + threadIdx.x) * 4;       // this thread's four columns
     const bool in = threadIdx.x < pieces;
@@ -235,6 +236,7 @@ __global__ void normed_mean_cluster_kernel(const NormedMeanArgs a) {
     __syncthreads();
     // each block tells every block of the cluster its sums; after the one barrier nobody touches another block's
     // shared memory again
+    cluster_wait_started();
     if (threadIdx.x < CL) {
 #pragma unroll
         for (int k = 0; k < MEAN_MAX; ++k) cluster.map_shared_rank(&share[k][0], threadIdx.x)[blockIdx.x] = red[k][32];

@@ -110,6 +110,11 @@ __device__ __forceinline__ float xielu_fast(float z, float a, float b) {
     return z > 0.f ? fmaf(a * z, z, 0.5f * z) : fmaf(b, e, 0.5f * z);
 }
 
+// A block may touch another's shared memory only once that block runs: every thread arrives when it starts and waits ahead of its block's first
+// access.  The two lie around the wait for the kernel ahead and the loads, where the barrier costs nothing that shows.
+__device__ __forceinline__ void cluster_arrive_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

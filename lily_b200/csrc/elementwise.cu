@@ -218,6 +218,7 @@ __global__ void add_rmsnorm_cluster_kernel(float* __restrict__ resid, const Summ
     __shared__ float red[40];
     __shared__ float share[CL];                                      // every block's sum of squares, sent by its owner
     cg::cluster_group cluster = cg::this_cluster();
+    cluster_arrive_started();
     pdl_enter_small();
     const int m = blockIdx.y;
     const size_t src = (size_t)(rows ? rows[m] : m) * hidden;
@@ -236,6 +237,7 @@ __global__ void add_rmsnorm_cluster_kernel(float* __restrict__ resid, const Summ
     const float mine = block_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w, red);
     // each block tells every block of the cluster its sum; after the one barrier nobody touches another block's
     // shared memory again, so a block may leave as soon as it is done
+    cluster_wait_started();
     if (threadIdx.x < CL) cluster.map_shared_rank(&share[0], threadIdx.x)[blockIdx.x] = mine;
     cluster.sync();
     float total = 0.f;
@@ -307,6 +309,7 @@ __global__ void add_rmsnorm_multi4_kernel(float* __restrict__ resid, const Summe
                                           T* __restrict__ out_b, int hidden, float eps, int write_residual) {
     __shared__ float red[40];
     __shared__ float share[CL];
+    if (CL > 1) cluster_arrive_started();
     const size_t src = (size_t)blockIdx.y * hidden;
     int at[NCH];
     float4 ga[NCH], gb[NCH];
@@ -349,6 +352,7 @@ __global__ void add_rmsnorm_multi4_kernel(float* __restrict__ resid, const Summe
     if (CL > 1) {
         // each block tells every block of the cluster its sum; after the one barrier nobody touches another block's shared memory
         cg::cluster_group cluster = cg::this_cluster();
+        cluster_wait_started();
         if (threadIdx.x < CL) cluster.map_shared_rank(&share[0], threadIdx.x)[blockIdx.x] = total;
         cluster.sync();
         total = 0.f;

@@ -176,6 +176,7 @@ __global__ void add_normed_rmsnorm_cluster_kernel(const NormedAddArgs a) {
     __shared__ float red[40];
     __shared__ float share[2][CL];
     cg::cluster_group cluster = cg::this_cluster();
+    cluster_arrive_started();
     pdl_enter_small();
     const int m = blockIdx.y, hidden = a.hidden;
     const size_t src = (size_t)(a.rows ? a.rows[m] : m) * hidden;
@@ -184,6 +185,7 @@ __global__ void add_normed_rmsnorm_cluster_kernel(const NormedAddArgs a) {
     const float4 g = *reinterpret_cast<const float4*>(a.post_gain + i);
     float4 v = *reinterpret_cast<const float4*>(a.resid + src + i);
     float mine = 0.f, total = 0.f, inv_d = 1.f;
+    cluster_wait_started();
     if (a.normalise) {                                                  // the same branch in every block of the launch
         mine = block_sum(d.x * d.x + d.y * d.y + d.z * d.z + d.w * d.w, red);
         if (threadIdx.x < CL) cluster.map_shared_rank(&share[0][0], threadIdx.x)[blockIdx.x] = mine;

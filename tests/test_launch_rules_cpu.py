@@ -1,5 +1,8 @@
 """Rules of launches that can be looked at without a GPU: the host side of the kernel library, and its sources."""
 
+import os
+import re
+
 import pytest
 
 
@@ -23,3 +26,25 @@ def test_rows_over_clusters_take_whole_warps(lib):
         taken += 1
         assert threads % 32 == 0 and pieces <= threads < pieces + 32 and threads <= 1024, width
     assert taken == 993
+
+
+def test_no_block_writes_to_a_peer_that_may_not_have_started():
+    """In every kernel that writes into the shared memory of other blocks of its cluster, a barrier that all of them have reached stands ahead of
+    the first such write."""
+    from lily_b200.csrc import build
+    found = []
+    for name in build.SOURCES:
+        with open(os.path.join(build.HERE, name)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        # from one kernel's head to the next
+        heads = [m.start() for m in re.finditer(r"__global__", text)] + [len(text)]
+        for a, b in zip(heads, heads[1:]):
+            body = text[a:b]
+            write = re.search(r"map_shared_rank\([^;=]*=[^=]", body)
+            if write is None:
+                continue
+            found.append(name)
+            arrive, wait = body.find("cluster_arrive_started();"), body.find("cluster_wait_started();")
+            assert 0 < arrive < wait < write.start(), (name, body[:200])
+            assert body.count("cluster_arrive_started();") == body.count("cluster_wait_started();") == 1, name
+    assert sorted(found) == ["attention_mma.cu", "combine.cu", "elementwise.cu", "elementwise.cu", "sublayer.cu"]
