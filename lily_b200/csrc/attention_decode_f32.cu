@@ -75,7 +75,7 @@ attention_decode_f32_kernel(const AttnArgs a) {
                                            : make_float4(0.f, 0.f, 0.f, 0.f);
             o[h][c] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-    // after the exchanges lane l holds the sum of head l / (32 / G), key (l / (32 / N)) % KB (the first of two where N is 64)
+    // after the exchanges lane l holds the sum of head l / (32 / G), key (l / (32 / N)) % KB
     constexpr int PER_HEAD = 32 / G;
     const int head = lane / PER_HEAD;
     const bool sunk = a.sink && blockIdx.z == 0 && warp == 0 && head < group;
@@ -114,7 +114,7 @@ attention_decode_f32_kernel(const AttnArgs a) {
 #pragma unroll
         for (int off = REST; off < PER_HEAD; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
         const float m_new = fmaxf(m, mx);
-        float p = 0.f, alpha = 1.f;
+        float p = sv == sv ? 0.f : sv, alpha = 1.f;              // a NaN is no maximum: as a weight it reaches the row
         if (m_new > -INFINITY) {
             alpha = expf(m - m_new);
             p = expf(sv - m_new);
@@ -172,16 +172,14 @@ attention_decode_f32_kernel(const AttnArgs a) {
         for (int w = 0; w < WARPS; ++w) mx = fmaxf(mx, ml[(w * G + h) * 2]);
         float den = 0.f;
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (mx > -INFINITY) {
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) {
-                const float mw = ml[(w * G + h) * 2];
-                if (mw == -INFINITY && ml[(w * G + h) * 2 + 1] == 0.f) continue;          // no keys
-                const float f = expf(mw - mx);
-                const float4 t = *reinterpret_cast<const float4*>(merge + (w * G + h) * dv + col);
-                sum.x = fmaf(t.x, f, sum.x), sum.y = fmaf(t.y, f, sum.y), sum.z = fmaf(t.z, f, sum.z), sum.w = fmaf(t.w, f, sum.w);
-                den = fmaf(ml[(w * G + h) * 2 + 1], f, den);
-            }
+        for (int w = 0; w < WARPS; ++w) {
+            const float mw = ml[(w * G + h) * 2], lw = ml[(w * G + h) * 2 + 1];
+            if (mw == -INFINITY && lw == 0.f) continue;          // no keys
+            const float f = expf(mw - mx);
+            const float4 t = *reinterpret_cast<const float4*>(merge + (w * G + h) * dv + col);
+            sum.x = fmaf(t.x, f, sum.x), sum.y = fmaf(t.y, f, sum.y), sum.z = fmaf(t.z, f, sum.z), sum.w = fmaf(t.w, f, sum.w);
+            den = fmaf(lw, f, den);
         }
         const size_t row = (size_t)req * a.nq + kvh * group + h;
         if (a.splits > 1) {
@@ -192,7 +190,7 @@ attention_decode_f32_kernel(const AttnArgs a) {
                 a.part_ml[at * 2 + 1] = den;
             }
         } else {
-            const float inv = den > 0.f ? 1.f / den : 0.f;
+            const float inv = den == 0.f ? 0.f : 1.f / den;
             *reinterpret_cast<float4*>((float*)a.out + row * dv + col) = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv);
         }
     }

@@ -322,7 +322,7 @@ attention_simt_kernel(const AttnArgs a, const int bufs) {
 // block has four rows of threads and first brings every split's (max, sum) into shared memory, one a thread, and
 // forms the weights exp(m - max) there; each row of threads then sums every fourth split, loads that do not wait for
 // one another, and the first row adds the four partial sums up, in a fixed order.  (With dozens of splits the plain
-// loops are a chain of trips to L2: 22 us for 55 splits.)  Fewer splits (where the staging costs more than it saves:
+// loops are a chain of trips to L2: 22 us for 55 splits.)  A range whose sum is a NaN makes the row one, also where its maximum weighs nothing.  Fewer splits (where the staging costs more than it saves:
 // a step of 64 requests with 4 splits each 10.44 -> 10.53 ms) and more take the plain loops, a column in the order of
 // the splits.
 constexpr int COMBINE_STAGED = 256, COMBINE_ROWS = 4, COMBINE_D = 256;
@@ -372,7 +372,7 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
         if (row == 0) {
             float denom = 0.f;
             for (int s = 0; s < splits; ++s) denom += l_s[s] * w_s[s];
-            const float inv = denom > 0.f ? 1.f / denom : 0.f;
+            const float inv = denom == 0.f ? 0.f : 1.f / denom;
 #pragma unroll
             for (int j = 0; j < COMBINE_D / 128; ++j) {
                 const int c = threadIdx.x + j * 128;
@@ -390,9 +390,9 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
     float denom = 0.f;
     for (int s = 0; s < splits; ++s) {
         const float ms = part_ml[(base + s) * 2];
-        if (ms > -INFINITY) denom += part_ml[(base + s) * 2 + 1] * expf(ms - mx);
+        denom += part_ml[(base + s) * 2 + 1] * (ms > -INFINITY ? expf(ms - mx) : 0.f);
     }
-    const float inv = denom > 0.f ? 1.f / denom : 0.f;
+    const float inv = denom == 0.f ? 0.f : 1.f / denom;
     for (int c = threadIdx.x; c < d; c += blockDim.x) {
         float o = 0.f;
         for (int s = 0; s < splits; ++s) {

@@ -840,6 +840,41 @@ def test_attention_decode_fp32_keys_over_warps(nq, nkv, d, dv, page, window, kee
     torch.testing.assert_close(got, want, **tol(torch.float32))
 
 
+def _nan_keys_case(dtype, nq, nkv, d, page, seqs_places):
+    """A row for each (length, place of a key that is NaN in one column for the first kv head; None: no such key)."""
+    g = torch.Generator(device=DEV).manual_seed(d + len(seqs_places))
+    rows = len(seqs_places)
+    width = max(-(-n // page) for n, _ in seqs_places)
+    cache = torch.randn(rows * width + 1, 2, nkv, page, d, device=DEV, generator=g).to(dtype)
+    table = (torch.randperm(rows * width, device=DEV, generator=g) + 1).view(rows, width).to(torch.int32)
+    for r, (_, place) in enumerate(seqs_places):
+        if place is not None:
+            cache[int(table[r, place // page]), 0, 0, place % page, 3] = float("nan")
+    q = torch.randn(rows, nq * d, device=DEV, generator=g).to(dtype)
+    return cache, table, q, torch.tensor([n for n, _ in seqs_places], device=DEV, dtype=torch.int32)
+
+
+def _nan_keys_reach_their_rows(dtype, nq, nkv, d, page, splits, seqs, **opts):
+    cases = [(n, p) for n in seqs for p in sorted({None, 0, 4, 64, n - 1}, key=str) if p is None or p < n]
+    cache, table, q, seq_t = _nan_keys_case(dtype, nq, nkv, d, page, cases)
+    got, want = torch.zeros_like(q), torch.zeros_like(q)
+    scratch = torch.full((max(ops().decode_scratch_floats(len(cases), nq, d, splits), 1),), float("nan"), device=DEV)
+    ref.attention_decode(q, cache, table, seq_t, want, None, 1, nq, nkv, d, page, d ** -0.5, **opts)
+    ops().attention_decode(q, cache, table, seq_t, got, scratch, splits, nq, nkv, d, page, d ** -0.5, **opts)
+    first = nq // nkv * d                                      # the columns of the first kv head's query heads
+    for r, (n, place) in enumerate(cases):
+        assert bool(torch.isnan(got[r, :first]).all()) == (place is not None) and torch.isfinite(got[r, first:]).all(), (n, place)
+    torch.testing.assert_close(got.float(), want.float(), equal_nan=True, **tol(dtype))
+
+
+@pytest.mark.parametrize("splits", [1, 3, 9, 40])
+@pytest.mark.parametrize("nq,nkv,d,cap", [(2, 2, 128, None), (6, 2, 64, None), (8, 2, 128, 30.0), (16, 2, 128, None), (4, 2, 256, None)])
+def test_attention_decode_fp32_a_nan_key_reaches_its_row(nq, nkv, d, cap, splits):
+    """A key that is seen and whose score is a NaN makes the row one, wherever it lies: alone among its warp's four keys, in the first round of a
+    warp and in later ones, alone in its range; ranges merged by the combine kernel's plain loops and its staged ones."""
+    _nan_keys_reach_their_rows(torch.float32, nq, nkv, d, 16, splits, [1, 2, 5, 13, 65, 129, 257], softcap=cap)
+
+
 @pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16, 17])
 @pytest.mark.parametrize("width,ff,experts,identity,top,activation,on_input,shared", [
     (64, 64, 3, 0, 2, "silu", False, False), (192, 320, 16, 2, 4, "swish_clamped", False, False),
