@@ -725,14 +725,15 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
         float den = 0.f;
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            if (mw[w] > -INFINITY) {
+            const float lw = mml[(w * 16 + r) * 2 + 1];
+            if (mw[w] > -INFINITY || lw != 0.f) {          // (a NaN is no maximum, but makes the sum one)
                 const float f = exp2f(mw[w] - mx);
                 const float4 v = *reinterpret_cast<const float4*>(mo + (w * 16 + r) * D + col);
                 acc.x += v.x * f;
                 acc.y += v.y * f;
                 acc.z += v.z * f;
                 acc.w += v.w * f;
-                den += mml[(w * 16 + r) * 2 + 1] * f;
+                den += lw * f;
             }
         }
         const int head = head0 + r;
@@ -749,7 +750,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
                 a.part_ml[base * 2 + 1] = den;
             }
         } else {
-            const float inv = den > 0.f ? 1.f / den : 0.f;
+            const float inv = den == 0.f ? 0.f : 1.f / den;
             *reinterpret_cast<uint2*>((__nv_bfloat16*)a.out + ((size_t)tok0 * a.nq + head) * D + col) =
                 make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
         }
@@ -768,7 +769,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
             float den = 0.f;
             for (int sp = 0; sp < splits; ++sp) {           // in the order of the splits, whichever block merges
                 const float2 ml = *reinterpret_cast<const float2*>(recv_ml + (sp * 16 + r) * 2);
-                if (ml.x > -INFINITY) {
+                if (ml.x > -INFINITY || ml.y != 0.f) {
                     const float f = exp2f(ml.x - mx);
                     const float4 v = *reinterpret_cast<const float4*>(recv_o + sp * share + slot);
                     acc.x += v.x * f;
@@ -778,7 +779,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
                     den += ml.y * f;
                 }
             }
-            const float inv = den > 0.f ? 1.f / den : 0.f;
+            const float inv = den == 0.f ? 0.f : 1.f / den;
             *reinterpret_cast<uint2*>((__nv_bfloat16*)a.out + ((size_t)tok0 * a.nq + head0 + r) * D + col) =
                 make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
         }

@@ -875,6 +875,14 @@ def test_attention_decode_fp32_a_nan_key_reaches_its_row(nq, nkv, d, cap, splits
     _nan_keys_reach_their_rows(torch.float32, nq, nkv, d, 16, splits, [1, 2, 5, 13, 65, 129, 257], softcap=cap)
 
 
+@pytest.mark.parametrize("splits,stages", [(1, 0), (3, 0), (9, 0), (40, 0), (1, 3), (2, 3)])
+@pytest.mark.parametrize("nq,nkv,d,page", [(16, 4, 128, 16), (16, 4, 128, 64), (16, 8, 64, 128), (40, 2, 128, 64)])
+def test_attention_decode_bf16_a_nan_key_reaches_its_row(nq, nkv, d, page, splits, stages):
+    """The same on tensor cores, where a warp has 16 keys of every tile: ranges that end with one key, merged in the block, in clusters and by the
+    combine kernel; tiles piece by piece and by TMA."""
+    _nan_keys_reach_their_rows(torch.bfloat16, nq, nkv, d, page, splits, [1, 2, 65, 129, 193, 385], stages=stages)
+
+
 @pytest.mark.parametrize("tokens", [1, 2, 7, 8, 9, 16, 17])
 @pytest.mark.parametrize("width,ff,experts,identity,top,activation,on_input,shared", [
     (64, 64, 3, 0, 2, "silu", False, False), (192, 320, 16, 2, 4, "swish_clamped", False, False),
