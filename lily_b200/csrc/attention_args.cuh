@@ -20,6 +20,8 @@ struct AttnArgs {
     int nq, nkv, d, page_size, window;
     int pages;                // decode, tensor-core kernel: pages of the layer's cache (0: not known, tiles are then fetched piece by piece)
     int longest_first;        // decode, tensor-core kernel: 1 when blocks go to the rows in the order of their lengths
+    int tile_polls;           // decode, tensor-core kernel: polls before a wait for a tile gives up
+    int* lost;                // decode, tensor-core kernel: a word of the host's where it says so
     float scale;
     // decode, tensor-core kernel only: the qkv product as it leaves the projection (this kernel then norms and
     // rotates its own query heads, and the block whose key range holds the new position does the same for the

@@ -120,12 +120,12 @@ __host__ __device__ inline int cluster_share(int rows, int d, int splits) { retu
 // before the kernel ahead has finished.  With this step's own key and value among them: the block that finishes those from the
 // projection puts them into the arrived tile itself.  Ranges start on multiples of 64 (what lies ahead of the window is masked).  A tile
 // comes as halves of 64 columns, rows of 128 bytes in the hardware's swizzle.  Rows outside the range hold whatever the page
-// holds; their values are cleared, so that a weight of zero meets no infinity.  Every wait for a tile is bounded
-// (lily_attention_decode_status).  What bounds it is a block's start (length, table, first tile: 2 us) and its merge; the memory is busy
+// holds; their values are cleared, so that a weight of zero meets no infinity.  Every wait for a tile is bounded: where one runs out, a word
+// that the host reads says so (lily_attention_decode_status), no more tiles are asked for, those on their way are waited for (bounded
+// again) before their memory is used for something else, and the block's sums become NaN.  What bounds the kernel is a block's start (length, table, first tile: 2 us) and its merge; the memory is busy
 // between.  Piece by piece / by TMA, us, 8 kv heads of 4 query heads, head size 128: 19 rows of 400 to 2,900 keys in clusters of two 38.2 / 28.5 (bytes
 // 18.5), 24 rows of 500 to 2,700 39.4 / 30.9, 64 rows of 250 to 1,750 whole 59.4 / 53.1, 48 rows of 250 to 3,500 100 / 66, one tile a row no difference.
-__device__ int g_decode_status = 0;
-constexpr uint32_t TILE_SPINS = 1u << 22;
+constexpr int TILE_POLLS = 1 << 22;
 template <int D, int STAGES>
 __host__ __device__ constexpr size_t tma_bytes() { return 1024 + 2 * (size_t)STAGES * BN * D * 2 + 16 * D * 2 + 2 * D * 2; }
 
@@ -146,6 +146,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
     unsigned char* q_s = TMA ? k_s + 2 * STAGES * TILE : k_s + (STAGES - 1) * TILE;           // [BM][D], BM <= BN
     __nv_bfloat16* own_s = reinterpret_cast<__nv_bfloat16*>(q_s + BM * D * 2);                // TMA: [2][D]
     __shared__ __align__(8) uint64_t full_s[STAGES];
+    __shared__ int lost_s;                                          // TMA: a wait for a tile ran out
     // the 16-byte piece `ch` of row `r` of a tile
     auto piece = [](int r, int ch) { return TMA ? (uint32_t)((ch >> 3) * (BN * 128) + r * 128 + (((ch ^ r) & 7) << 4)) : swz<D>(r, ch); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -270,9 +271,10 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
         for (int h = 0; h < D / 64; ++h) tc5::tma_load_4d(vd + h * (BN * 128), &map_kv, bar, h * 64, off, vh, page);
     };
     const bool patched = TMA && a.qkv != nullptr && a.write_kv;          // this step's own key and value never come from the page
-    bool arrived = true;
+    int asked = 0;                                                      // tiles that were asked for (by the first thread)
     if (TMA) {
         if (tid == 0) {
+            lost_s = 0;
 #pragma unroll
             for (int st = 0; st < STAGES; ++st) tc5::mbar_init(full0 + 8 * st, 1);
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -290,6 +292,7 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
             for (int st = 0; st < STAGES && st < ntiles; ++st)
                 if (!(patched || tile_base(st) + BN <= pos0)) ask_tile(st);
         }
+        asked = min(STAGES, ntiles);
     }
     // the pipeline keeps STAGES - 1 tiles in flight; every iteration commits one group (maybe empty).
     // Decode: the tiles that end before this step's own key are asked for ahead of the wait.
@@ -532,9 +535,16 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
         unsigned char* kt = k_s + buf * TILE;
         unsigned char* vt = v_s + buf * TILE;
         if (TMA) {
-            uint32_t spins = 0;
-            while (arrived && !tc5::mbar_try_wait(full0 + 8 * buf, (t / STAGES) & 1)) arrived = ++spins < TILE_SPINS;
-            if (!arrived && lane == 0) atomicCAS(&g_decode_status, 0, 1 + (bx & 0x7fff));
+            int left = a.tile_polls;
+            while (left > 0 && !tc5::mbar_try_wait(full0 + 8 * buf, (t / STAGES) & 1))
+                if ((--left & 1023) == 0 && *(volatile int*)&lost_s) left = 0;
+            if (left == 0) {
+                lost_s = 1;
+                if (lane == 0) {
+                    *(volatile int*)a.lost = 1 + (bx & 0x7fff);
+                    __threadfence_system();
+                }
+            }
             const int first = a.window > 0 && t >= ftiles ? max(0, pos0 + 1 - a.window - kb) : 0;       // rows ahead of the window
             if (first > 0 || kb + BN > klim || (patched && kb <= pos0 && pos0 < kb + BN)) {
                 // values of rows outside the range are cleared (kept first positions stay); this step's own row is put in
@@ -655,7 +665,10 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
         }
         if (TMA && t + STAGES < ntiles) {
             __syncthreads();                                // every warp is done with this buffer
-            if (tid == 0) ask_tile(t + STAGES);
+            if (tid == 0 && !*(volatile int*)&lost_s) {
+                ask_tile(t + STAGES);
+                asked = t + STAGES + 1;
+            }
         }
     }
 
@@ -684,6 +697,13 @@ attention_mma_kernel(const AttnArgs a, const int page_shift, const __grid_consta
 
     // ---- decode: merge the four warps' partial results through shared memory ---------------------
     __syncthreads();                                        // every warp is done with the key/value tiles
+    if (TMA && lost_s) {
+        if (tid == 0)                                       // the last copy into each buffer
+            for (int t = max(0, asked - STAGES); t < asked; ++t)
+                for (int left = TILE_POLLS; left > 0 && !tc5::mbar_try_wait(full0 + 8 * (t % STAGES), (t / STAGES) & 1); --left) {}
+        l_lo = l_hi = __int_as_float(0x7fffffff);
+        __syncthreads();
+    }
     float* mo = reinterpret_cast<float*>(k_s);              // [4 warps][16 rows][D]
     float* mml = mo + 4 * 16 * D;                           // [4 warps][16 rows][2]
 #pragma unroll
@@ -1034,11 +1054,30 @@ LILY_API int lily_attention_decode_mma_clusters(int d, int splits, int group) {
     return 0;
 }
 
+// The host's word in which the decode kernel says that a wait for a tile ran out; made once, also while a graph is captured.
+static int* lost_word() {
+    static int* word = [] {
+        int* p = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (p) *p = 0;
+        return p;
+    }();
+    return word;
+}
+
 static int decode_mma(AttnArgs& a, const void* q, const void* kv, void* out, const int* block_table, int bt_stride,
                       const int* seq_lens, float* scratch, int requests, int splits, int nq, int nkv, int d, int page_size,
                       int window, float scale, int stages, cudaStream_t stream) {
     if (requests == 0) return 0;
     a.stages = stages;
+    a.lost = a.pages > 0 ? lost_word() : nullptr;
+    LILY_REQUIRE(a.pages <= 0 || a.lost != nullptr, "attention_decode: no word of the host's memory");
     LILY_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention_decode: %d query heads over %d kv heads", nq, nkv);
     LILY_REQUIRE(splits >= 1 && splits <= 65535 && page_size > 0, "attention_decode: splits=%d page_size=%d", splits, page_size);
     LILY_REQUIRE(splits == 1 || scratch != nullptr, "attention_decode: splits need scratch");
@@ -1061,13 +1100,15 @@ static int decode_mma(AttnArgs& a, const void* q, const void* kv, void* out, con
 // distributed shared memory; else the partial results go to `scratch` in the layout of attention_simt.cu
 // ([requests, nq, splits, d] outputs, then [requests, nq, splits, 2] (max, sum)) and the combine kernel is launched behind.
 // `pages`: pages of the layer's cache (0: not known; tiles are then fetched piece by piece, as where a page is no whole tile).
+// `polls`: how often a block asks whether a tile has arrived before it gives up.
 // `stages`: 0, or the key/value tiles a block holds (3, up to head size 128: two blocks a SM, no clusters).
 LILY_API int lily_attention_decode_mma(const void* q, const void* kv, void* out, const int* block_table,
                                        int bt_stride, const int* seq_lens, float* scratch, int requests, int splits,
                                        int nq, int nkv, int d, int page_size, int window, float scale, int stages,
-                                       float softcap, int keep_first, int sink, int v_shift, int pages, cudaStream_t stream) {
+                                       float softcap, int keep_first, int sink, int v_shift, int pages, int polls, cudaStream_t stream) {
     AttnArgs a{};
     a.pages = pages;
+    a.tile_polls = polls;
     // v_shift -1: every shift in one launch, nkv planes of `requests` rows in `out` (and as many rows of scratch)
     LILY_REQUIRE(nkv > 0 && v_shift >= -1 && v_shift < nkv, "attention_decode: value heads shifted by %d of %d", v_shift, nkv);
     a.softcap = softcap; a.sink = sink; a.v_shift = v_shift < 0 ? 0 : v_shift;
@@ -1090,7 +1131,7 @@ LILY_API int lily_attention_decode_mma_fused(const void* qkv, int qkv_planes, si
                                              void* kv, void* out, const int* block_table, int bt_stride,
                                              const int* seq_lens, float* scratch, int requests, int splits, int nq,
                                              int nkv, int d, int page_size, int window, float scale, int stages,
-                                             float softcap, int qkv_ld, int pages, cudaStream_t stream) {
+                                             float softcap, int qkv_ld, int pages, int polls, cudaStream_t stream) {
     // rows of the product may go on behind the heads; a layer that writes no keys may have the query heads alone
     LILY_REQUIRE(qkv_ld % 2 == 0 && qkv_ld >= (write_kv ? nq + 2 * nkv : nq) * d, "attention_decode_fused: rows of %d numbers", qkv_ld);
     LILY_REQUIRE(qkv != nullptr && qkv_planes >= 1 && (qkv_dtype == kF32 || qkv_planes == 1),
@@ -1105,15 +1146,17 @@ LILY_API int lily_attention_decode_mma_fused(const void* qkv, int qkv_planes, si
     a.softcap = softcap;
     a.qkv_ld = qkv_ld;
     a.pages = pages;
+    a.tile_polls = polls;
     return decode_mma(a, nullptr, kv, out, block_table, bt_stride, seq_lens, scratch, requests, splits, nq, nkv, d,
                       page_size, window, scale, stages, stream);
 }
 
-// 0, or 1 + the request row of the first decode block whose wait for a tile ran out since the last call; clears it.
-LILY_API int lily_attention_decode_status() {
-    int v = 0;
-    const int zero = 0;
-    if (cudaMemcpyFromSymbol(&v, mma::g_decode_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v != 0) cudaMemcpyToSymbol(mma::g_decode_status, &zero, sizeof(int));
+// 0, or 1 + the request row of a decode block whose wait for a tile ran out since the last call; clears it.  `wait`: behind all work
+// of the device; else as far as the host knows (the kernels it has waited for).
+LILY_API int lily_attention_decode_status(int wait) {
+    if (wait && cudaDeviceSynchronize() != cudaSuccess) return -1;
+    volatile int* word = lost_word();
+    const int v = word ? *word : 0;
+    if (v != 0) *word = 0;
     return v;
 }

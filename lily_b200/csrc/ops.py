@@ -41,9 +41,9 @@ _SIGNATURES = {
     "lily_attention_combine": [_vp, _vp, _i, _i, _i, _i, _i, _vp],
     "lily_attention_prefill_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp],
     "lily_attention_prefill_tc": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _f, _i, _i, _i, _vp],
-    "lily_attention_decode_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _vp],
+    "lily_attention_decode_mma": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _i, _i, _vp],
     "lily_attention_decode_mma_fused": [_vp, _i, _sz, _i, _vp, _vp, _i, _f, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp, _vp,
-                                        _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp],
+                                        _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _i, _vp],
     "lily_sigmoid_gate": [_vp, _i, _vp, _i, _i, _sz, _sz, _vp],
     "lily_sigmoid_head_gate": [_vp, _i, _vp, _i, _i, _sz, _i, _i, _i, _i, _i, _vp],
     "lily_add_tanh_norm": [_vp, _vp, _i, _i, _sz, _f, _vp, _vp, _f, _f, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _vp],
@@ -725,7 +725,16 @@ def sink_prompts_on_tcgen05(d: int, new_lens: Sequence[int], heads: int, planes:
 
 def attention_tc_status() -> int:
     """0, or a code from the first bounded wait that gave up in the attention kernels whose tiles come by TMA (synchronises)."""
-    return int(library().lily_attention_tc_status()) or int(library().lily_attention_decode_status())
+    return int(library().lily_attention_tc_status()) or int(library().lily_attention_decode_status(1))
+
+
+DECODE_POLLS = 1 << 22         # how often a decode block asks whether a tile has arrived before it gives up
+
+
+def attention_decode_lost() -> int:
+    """0, or 1 + the row of a decode block whose wait for a tile ran out (its outputs are NaN) in a kernel that the host has waited
+    for; clears it and waits for nothing."""
+    return int(library().lily_attention_decode_status(0))
 
 
 def attention_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor, cu_seqlens: torch.Tensor,
@@ -937,12 +946,12 @@ def attention_decode(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch
             _call("lily_attention_decode_mma", _p(q), _p(kv_layer), out[shift].data_ptr() if planes and not merged else _p(out),
                   _i32(block_table, "block_table"), block_table.shape[-1], _i32(seq_lens, "seq_lens"), _p(scratch), requests, splits,
                   nq, nkv, d, page_size, int(window or 0), float(scale), int(stages), cap, int(keep_first or 0) if window else 0,
-                  int(bool(sink)), shift, pages, _stream())
+                  int(bool(sink)), shift, pages, DECODE_POLLS, _stream())
             rows = requests * nkv if merged else requests
             if splits > 1 and (stages or rows * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
                 launches["count"] += 1
     elif dv == d and not values_in_keys and not flags and sinks is None and uses_tensor_cores(q.dtype, d):
-        _call("lily_attention_decode_mma", *common, int(stages), cap, int(keep_first or 0) if window else 0, 0, 0, pages, _stream())   # merges the splits itself (cluster, or combine behind)
+        _call("lily_attention_decode_mma", *common, int(stages), cap, int(keep_first or 0) if window else 0, 0, 0, pages, DECODE_POLLS, _stream())   # merges the splits itself (cluster, or combine behind)
         if splits > 1 and (stages or requests * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
             launches["count"] += 1                                   # the combine kernel, launched inside
     else:
@@ -1172,7 +1181,7 @@ def attention_decode_fused(qkv: torch.Tensor, q_gain: Optional[torch.Tensor], k_
           _dt(q_gain) if q_gain is not None else _F32, float(eps), _p(cos), _p(sin), int(rotary_dim), int(write_kv),
           _p(kv_layer), _p(out), _i32(block_table, "block_table"), block_table.shape[-1], _i32(seq_lens, "seq_lens"),
           _p(scratch), requests, splits, nq, nkv, d, page_size, int(window or 0), float(scale), int(stages),
-          float(softcap or 0.0), ld, kv_layer.shape[0], _stream())
+          float(softcap or 0.0), ld, kv_layer.shape[0], DECODE_POLLS, _stream())
     if splits > 1 and (stages or requests * nkv * -(-(nq // nkv) // 16) > decode_clusters(d, splits, nq // nkv)):
         launches["count"] += 1                                       # the combine kernel, launched inside
 

@@ -303,6 +303,14 @@ class ModelRunner:
     def free_tokens(self) -> int:
         return self.cache.free_tokens()
 
+    def check_waits(self) -> None:
+        """Raises when a kernel that the host has waited for gave up a wait of its own, so that its step's results are no results.  (A read of
+        a word in the host's memory.)"""
+        lost = getattr(self.model.ctx.ops, "attention_decode_lost", None)       # (stand-ins for the kernels wait for nothing)
+        row = lost() if lost is not None else 0
+        if row:
+            raise RuntimeError(f"decode attention: a tile of keys did not arrive in time (row {row - 1} of its step); the step's tokens are void")
+
     # ---- one step --------------------------------------------------------------------
 
     def prepare(self, entries: Sequence[StepEntry], logit_rows_in_given_order: bool = True) -> StepBatch:

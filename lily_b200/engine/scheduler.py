@@ -375,6 +375,7 @@ class Scheduler:
     def _collect(self, launched: _Launched) -> None:
         """Reads the tokens of a launched step and lets each request take its own."""
         tokens, logprobs = launched.result.read()
+        self.runner.check_waits()
         tops = launched.result.read_top()
         for i, req in enumerate(launched.sampled):
             req.pending -= 1

@@ -514,6 +514,36 @@ def test_attention_decode_by_whole_tiles(nq, nkv, d, page, window, keep, rows, s
         torch.testing.assert_close(written[at, :, :, (n - 1) % page].float(), cache[at, :, :, (n - 1) % page].float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("splits,stages", [(1, 0), (3, 0), (40, 0), (1, 3)])
+@pytest.mark.parametrize("from_projection", [False, True])
+def test_a_wait_for_a_tile_that_runs_out_is_reported(monkeypatch, from_projection, splits, stages):
+    """With no poll allowed every block gives its wait up while its copies are on their way: it waits for them, says so and leaves NaN, the
+    next call is as if nothing had been."""
+    o, nq, nkv, d, page = ops(), 16, 4, 128, 64
+    seqs = [1, 64, 129, 700, 2000]
+    cache, table, q, _, _ = _attention_case(torch.bfloat16, nq, nkv, d, page, [n - 1 for n in seqs], [1] * len(seqs), None, seed=3)
+    seq_t = torch.tensor(seqs, device=DEV, dtype=torch.int32)
+    qkv = torch.randn(1, len(seqs), (nq + 2 * nkv) * d, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4))
+    scratch = torch.empty(max(o.decode_scratch_floats(len(seqs), nq, d, splits), 1), device=DEV)
+
+    def run():
+        out = torch.zeros_like(q)
+        if from_projection:
+            o.attention_decode_fused(qkv, None, None, 1e-6, None, None, cache, table, seq_t, out, scratch, splits, nq, nkv, d, 0, page, d ** -0.5,
+                                     stages=stages)
+        else:
+            o.attention_decode(q, cache, table, seq_t, out, scratch, splits, nq, nkv, d, page, d ** -0.5, stages=stages)
+        torch.cuda.synchronize()
+        return out
+    want = run()
+    assert o.attention_decode_lost() == 0 and torch.isfinite(want).all()
+    monkeypatch.setattr(o, "DECODE_POLLS", 0)
+    assert torch.isnan(run()).all()
+    assert 1 <= o.attention_decode_lost() <= len(seqs) and o.attention_decode_lost() == 0
+    monkeypatch.undo()
+    assert torch.equal(run(), want) and o.attention_tc_status() == 0
+
+
 def test_three_stages_are_refused_where_they_do_not_fit():
     o = ops()
     nq, nkv, d, page = 2, 2, 256, 16

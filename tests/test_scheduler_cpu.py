@@ -354,3 +354,15 @@ def test_sampling_params_checks():
     assert SamplingParams(logit_bias={"3": 1}).logit_bias == {3: 1.0}
     us = [uniform_for(1, i) for i in range(1000)]
     assert all(0 <= u < 1 for u in us) and 0.45 < sum(us) / 1000 < 0.55 and uniform_for(1, 5) != uniform_for(2, 5)
+
+
+def test_a_step_whose_kernel_gave_up_a_wait_fails(setup, monkeypatch):
+    """What the kernels report of a wait that ran out reaches the caller as an error, ahead of the step's tokens."""
+    cfg, _, path = setup
+    s = scheduler(path)
+    reports = iter([0, 0, 4])
+    monkeypatch.setattr(s.runner.model.ctx.ops, "attention_decode_lost", lambda: next(reports), raising=False)
+    s.add_request("r0", prompts(cfg, [7])[0], SamplingParams(max_new_tokens=8, ignore_eos=True))
+    with pytest.raises(RuntimeError, match="row 3 of its step"):
+        s.run_to_completion()
+    assert next(reports, None) is None
