@@ -135,6 +135,10 @@ class Attention(Mixer):
             raise ValueError("the short convolution has at least one tap and comes without biases")
         self.conv_w = None
 
+    @property
+    def shares_step(self) -> bool:
+        return bool(self.spec.v_share)                # the first such layer's values of the step's tokens
+
     # ---- what it needs ----------------------------------------------------------
 
     def cache_need(self) -> CacheNeed:

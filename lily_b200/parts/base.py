@@ -117,6 +117,9 @@ class Mixer(Part):
     # True when ``forward`` reads the batch's device tensors only (never its host lists), so that a
     # decode step may be captured once in a CUDA graph and replayed with new contents.
     graph_safe: bool = False
+    # True when ``forward`` writes or reads a buffer of the step (not of the layer) that other mixers of the kind read or write: they
+    # run one after another in the order of the layers and of a block's mixers.
+    shares_step: bool = False
 
     def cache_need(self) -> Optional[CacheNeed]:
         return None

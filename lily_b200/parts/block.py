@@ -96,7 +96,10 @@ class ParallelBlock(Block):
 
     @property
     def lanes(self) -> int:
-        """Lanes a captured decode step wants: one a mixer, with the feed-forward (or the last mixer) on the step's own stream."""
+        """Lanes a captured decode step wants: one a mixer, with the feed-forward (or the last mixer) on the step's own stream.  None where two
+        mixers meet in a buffer of the step: those keep their order."""
+        if sum(getattr(m, "shares_step", False) for m in self.mixers) > 1:
+            return 0
         return len(self.mixers) - (1 if self.feed_forward is None else 0)
 
     def _side_by_side(self, h, h_ff, batch, run: RunSlots):

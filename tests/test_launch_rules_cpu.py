@@ -48,3 +48,21 @@ def test_no_block_writes_to_a_peer_that_may_not_have_started():
             assert 0 < arrive < wait < write.start(), (name, body[:200])
             assert body.count("cluster_arrive_started();") == body.count("cluster_wait_started();") == 1, name
     assert sorted(found) == ["attention_mma.cu", "combine.cu", "elementwise.cu", "elementwise.cu", "sublayer.cu"]
+
+
+@pytest.mark.parametrize("shares,ff,lanes", [((None, None), True, 2), (("first", None), True, 2), (("first", "blend"), True, 0), (("blend", "blend"), False, 0),
+                                             ((None, "blend", None), False, 2), (("first", "blend", None), True, 0)])
+def test_mixers_that_meet_in_a_buffer_of_the_step_keep_their_order(shares, ff, lanes):
+    """Attention mixers of one parallel block whose values are the first sharing layer's write and read one buffer of the step, so a captured
+    step does not run them side by side."""
+    import torch
+    import kernel_refs
+    from lily_b200.parts.attention import AttentionSpec
+    from lily_b200.parts.base import BuildContext, build_part
+    from lily_b200.parts.block import ParallelBlockSpec
+    from lily_b200.parts.mlp import SwiGLUSpec
+    from lily_b200.parts.norm import RMSNormSpec
+    mixers = tuple((f"m{i}", AttentionSpec(32, 2, 1, 16, v_share=s), f"g{i}") for i, s in enumerate(shares))
+    spec = ParallelBlockSpec("b", 32, mixers, SwiGLUSpec(32, 64) if ff else None, RMSNormSpec(32, 1e-6), 1e-6)
+    ctx = BuildContext(torch.device("cpu"), torch.float32, kernel_refs)
+    assert build_part("block", spec, "b", ctx).lanes == lanes
