@@ -1592,9 +1592,18 @@ class WkvPlan:
     fine: Optional["WkvPlan"] = None
 
 
-def wkv_plan(new_lens: Sequence[int], device) -> Optional[WkvPlan]:
-    """None when every portion runs whole whatever kernels take it.  A plan without items has a cut for the tensor-core kernels only."""
+def wkv_chunks_take(dtype: torch.dtype, d: int) -> bool:
+    """Whether the tensor-core kernels take chunks of this type and head size (of operands on whole pieces)."""
+    return dtype == torch.bfloat16 and bool(library().lily_wkv_chunk_takes(None, None, None, 8, None, None, 1, d, WKV_CHUNK))
+
+
+def wkv_plan(new_lens: Sequence[int], device, dtype: torch.dtype = torch.bfloat16, d: int = 64) -> Optional[WkvPlan]:
+    """The cut for activations of ``dtype`` and heads of ``d``; None when every portion runs whole.  A plan without items has a cut for the
+    tensor-core kernels only."""
     if not new_lens or max(new_lens) < WKV_FINE:
+        return None
+    fine = wkv_chunks_take(dtype, d)
+    if not fine and max(new_lens) <= WKV_DIRECT:
         return None
 
     def cut(direct):
@@ -1612,7 +1621,7 @@ def wkv_plan(new_lens: Sequence[int], device) -> Optional[WkvPlan]:
                 item_len.append(min(WKV_CHUNK, n - s0))
         return [item_req, item_start, item_len, long_req, long_first, long_count, short]
 
-    cuts = [cut(WKV_FINE - 1)] + ([cut(WKV_DIRECT)] if max(new_lens) > WKV_DIRECT else [])
+    cuts = ([cut(WKV_FINE - 1)] if fine else []) + ([cut(WKV_DIRECT)] if max(new_lens) > WKV_DIRECT else [])
     lists = [part for parts in cuts for part in parts]
     flat = torch.tensor([x for part in lists for x in part], dtype=torch.int32).to(device, non_blocking=True)      # one copy for all lists
     split = torch.split(flat, [len(part) for part in lists])
@@ -1620,7 +1629,7 @@ def wkv_plan(new_lens: Sequence[int], device) -> Optional[WkvPlan]:
     for i, parts in enumerate(cuts):
         p = split[7 * i:7 * i + 7]
         plan = WkvPlan(len(parts[0]), p[0], p[1], p[2], len(parts[3]), p[3], p[4], p[5], p[6] if parts[6] else None, len(parts[6]), plan)
-    return plan if len(cuts) > 1 else WkvPlan(0, None, None, None, 0, None, None, None, None, 0, plan)
+    return plan if max(new_lens) > WKV_DIRECT else WkvPlan(0, None, None, None, 0, None, None, None, None, 0, plan)
 
 
 def wkv_workspace_floats(plan: Optional[WkvPlan], heads: int, d: int) -> int:
@@ -1636,7 +1645,8 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
     ``o_t = (S + diag(u) k_t v_t^T)^T r_t``, then ``S <- diag(exp(log_decay_t)) S + k_t v_t^T``.
     ``r``, ``k``, ``v`` [tokens, heads * d] in the activation dtype (rows of equal stride), ``log_decay`` float32
     [tokens, heads * d], ``u`` float32 [heads, d].  Returns float32 [tokens, heads * d].  With a ``plan`` (``wkv_plan``)
-    and its ``workspace`` (float32, ``wkv_workspace_floats``) long portions run as chunks side by side."""
+    and its ``workspace`` (float32, ``wkv_workspace_floats``) long portions run as chunks side by side; portions up to ``WKV_DIRECT`` tokens
+    need none."""
     _dev(log_decay, u, state, cu_seqlens, slots, workspace)
     tokens = r.shape[0]
     stride = r.stride(0)
@@ -1657,6 +1667,8 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch
         return y
     tensor_cores = (plan is not None and plan.fine is not None and r.dtype == torch.bfloat16 and plan.fine.items <= 65535 and bool(
         library().lily_wkv_chunk_takes(_p(r), _p(k), _p(v), stride, _p(log_decay), _p(u), heads, d, WKV_CHUNK)))
+    if tensor_cores and not plan.items and workspace is None:
+        tensor_cores = False                      # short portions without scratch run whole
     if tensor_cores:
         plan = plan.fine
     if plan is None or not plan.items:

@@ -199,6 +199,22 @@ def test_recurrence_in_chunks_on_the_tensor_cores(lens, heads, d, strided):
 
 
 @pytest.mark.gpu
+def test_short_portions_of_the_recurrence_need_no_scratch():
+    """Portions of up to 128 tokens with a plan and without scratch run whole, as they do without a plan; longer ones ask for it."""
+    from lily_b200.csrc import ops
+    g = torch.Generator().manual_seed(11)
+    lens, heads, d = [1, 40, 128], 2, 64
+    n = sum(lens)
+    r, k, v = (torch.randn(n, heads * d, generator=g).bfloat16().cuda() for _ in range(3))
+    lw, u = -torch.rand(n, heads * d, generator=g).cuda(), torch.randn(heads, d, generator=g).cuda()
+    states = [torch.zeros(4, heads * d * d, device="cuda") for _ in range(2)]
+    run = lambda plan, state: ops.wkv_scan(r, k, v, lw, u, state, i32([0, 1, 41, n], "cuda"), i32([1, 2, 3], "cuda"), 3, heads, d, plan=plan)
+    assert torch.equal(run(ops.wkv_plan(lens, "cuda"), states[0]), run(None, states[1])) and torch.equal(*states)
+    with pytest.raises(ops.KernelError, match="workspace"):
+        run(ops.wkv_plan([1, 1, 167], "cuda"), states[0])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("token", [5, 15, 64, 100])
 @pytest.mark.parametrize("what", ["r", "k", "v", "infinite v", "decay"])
 def test_recurrence_in_chunks_keeps_what_is_not_finite_behind_its_token(token, what):

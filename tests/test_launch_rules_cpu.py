@@ -66,3 +66,22 @@ def test_mixers_that_meet_in_a_buffer_of_the_step_keep_their_order(shares, ff, l
     spec = ParallelBlockSpec("b", 32, mixers, SwiGLUSpec(32, 64) if ff else None, RMSNormSpec(32, 1e-6), 1e-6)
     ctx = BuildContext(torch.device("cpu"), torch.float32, kernel_refs)
     assert build_part("block", spec, "b", ctx).lanes == lanes
+
+
+def test_the_recurrence_is_cut_for_the_kernels_that_take_it(lib):
+    """Chunks from 33 tokens on are the tensor-core kernels': float32 and head sizes beyond theirs have the cut of before, and no scratch for
+    portions that run whole."""
+    import torch
+    from lily_b200.csrc import ops
+    for lens in ([100], [1, 33, 128], [20, 30]):
+        for dtype, d in ((torch.float32, 64), (torch.bfloat16, 80), (torch.bfloat16, 128), (torch.bfloat16, 40)):
+            plan = ops.wkv_plan(lens, "cpu", dtype, d)
+            assert plan is None and ops.wkv_workspace_floats(plan, 4, d) == 0
+    assert ops.wkv_plan([20, 30], "cpu") is None
+    fine = ops.wkv_plan([1, 33, 128], "cpu", torch.bfloat16, 48)
+    assert fine.items == 0 and fine.fine.items == 3 and fine.fine.shorts == 1
+    for dtype, chunks in ((torch.float32, None), (torch.bfloat16, 1 + 2 + 4)):
+        plan = ops.wkv_plan([1, 33, 128, 200], "cpu", dtype, 64)
+        assert plan.items == 4 and plan.shorts == 3 and (plan.fine and plan.fine.items) == chunks
+        assert plan.item_start.tolist() == [0, 64, 128, 192] and plan.item_len.tolist() == [64, 64, 64, 8] and plan.long_req.tolist() == [3]
+        assert ops.wkv_workspace_floats(plan, 4, 64) == (chunks or 4) * 4 * (64 * 64 + 64)
