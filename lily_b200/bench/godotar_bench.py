@@ -88,7 +88,7 @@ def kernel_table(z: dict, tokens: int, batch: int, context: int, reps: int = 30,
             2.0 * n * hd * wk["decay_rank"], fp32_tflops, shape=label)
         rkv = [(rnd(n, hd).to(dt), (rnd(n, hd) / 8).to(dt), rnd(n, hd).to(dt), ops.wkv_decay(a, w2t, w0)) for a in lows]
         u = rnd(heads, d)
-        plan = ops.wkv_plan([per] * reqs, dev)                                  # long portions run as chunks, as in the model
+        plan = ops.wkv_plan([per] * reqs, dev, dt, d)                                  # long portions run as chunks, as in the model
         room = torch.empty(max(1, ops.wkv_workspace_floats(plan, heads, d)), device=dev)
         add("wkv_scan", "ssd_scan", [lambda x=x, s=s: ops.wkv_scan(x[0], x[1], x[2], x[3], u, s, cu, slots, reqs, heads, d,
                                                                     plan=plan, workspace=room)

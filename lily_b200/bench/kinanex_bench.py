@@ -88,14 +88,16 @@ def kernel_table(z: dict, tokens: int, batch: int, context: int, reps: int = 30,
         projs = [rnd(n, 8 + 2 * nq).to(dt) for _ in range(copies)]
         a_log, dt_bias = rnd(nq) - 2, rnd(nq)
         states = [torch.zeros(reqs + 1, nq * dd * dd, device=dev) for _ in range(copies)]
+        dplan = ops.delta_plan([per] * reqs, dt, nq, nkv, dd, dd, dev) if per > 1 else None      # long portions run as chunks, as in the model
+        droom = torch.empty(max(1, ops.delta_workspace_floats(dplan, nq)), device=dev)
         add("delta_rule", "wkv_scan", [lambda x=x, p=p, s=s: ops.delta_rule(x, p, 8, 8 + nq, a_log, dt_bias, s, cu, slots, reqs, nq, nkv, dd, dd,
-                                                                             1e-6, dd ** -0.5)
+                                                                             1e-6, dd ** -0.5, plan=dplan, workspace=droom)
                                        for x, p, s in zip(qkvs, projs, states)],
             n * (qkv_cols * 2 + hd * 4) + 2 * reqs * nq * dd * dd * 4, 8.0 * n * hd * dd, fp32_tflops, shape=label)
         rkv = [(rnd(n, hd).to(dt), (rnd(n, hd) / 8).to(dt), rnd(n, hd).to(dt), -torch.rand(n, hd, device=dev, generator=g)) for _ in range(copies)]
         u = rnd(nq, dd)
         wstates = [torch.zeros(reqs + 1, nq * dd * dd + width, device=dev) for _ in range(copies)]
-        plan = ops.wkv_plan([per] * reqs, dev)
+        plan = ops.wkv_plan([per] * reqs, dev, dt, dd)
         room = torch.empty(max(1, ops.wkv_workspace_floats(plan, nq, dd)), device=dev)
         add("wkv_scan (like)", "-", [lambda x=x, s=s: ops.wkv_scan(x[0], x[1], x[2], x[3], u, s, cu, slots, reqs, nq, dd, plan=plan, workspace=room)
                                      for x, s in zip(rkv, wstates)],
@@ -108,7 +110,7 @@ def kernel_table(z: dict, tokens: int, batch: int, context: int, reps: int = 30,
         zs = [rnd(n, 2 * inner).to(dt) for _ in range(copies)]
         a_mat, d_skip = -torch.rand(inner, ns, device=dev, generator=g) - 0.1, rnd(inner)
         sstates = [torch.zeros(reqs + 1, inner * ns, device=dev) for _ in range(copies)]
-        cplan = ops.scan_plan([per] * reqs, dev, inner * ns)                   # long portions run as chunks, as in the model
+        cplan = ops.scan_plan([per] * reqs, dev, inner * ns, chunks=False)     # long portions run as chunks, as in the model
         croom = torch.empty(max(1, ops.selective_workspace_floats(cplan, inner, ns)), device=dev)
         add("selective_scan", "ssd_scan", [lambda x=x, lo=lo, st=st, zz=zz, s=s: ops.selective_scan(x, lo, rank, st, zz, inner, a_mat, d_skip, s, cu, slots, reqs,
                                                                                                     plan=cplan, workspace=croom)

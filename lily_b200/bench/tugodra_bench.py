@@ -141,7 +141,7 @@ def kernel_table(z: dict, tokens: int, batch: int, context: int, reps: int = 30,
         rkv = [(rnd(n, width).to(dt), (rnd(n, width) / 8).to(dt), rnd(n, width).to(dt), -torch.rand(n, width, device=dev, generator=g)) for _ in range(copies)]
         wstates = [torch.zeros(reqs + 1, wh * wd * wd, device=dev) for _ in range(copies)]
         u = rnd(wh, wd)
-        wplan = ops.wkv_plan([per] * reqs, dev)
+        wplan = ops.wkv_plan([per] * reqs, dev, dt, wd)
         wroom = torch.empty(max(1, ops.wkv_workspace_floats(wplan, wh, wd)), device=dev)
         add("wkv_scan (Godotar)", "-", [lambda x=x, s=s: ops.wkv_scan(x[0], x[1], x[2], x[3], u, s, cu, slots, reqs, wh, wd, plan=wplan, workspace=wroom)
                                         for x, s in zip(rkv, wstates)],
