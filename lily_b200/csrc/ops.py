@@ -2269,9 +2269,14 @@ def _selective_cut(plan: Optional[ScanPlan], inner: int, n_state: int) -> Option
         plan = plan.rows
     if plan is None or not plan.num_chunks:
         return None
-    if n_state > 16 and plan.num_long * -(-inner // 16) > 2.5 * sm_count():
+    if n_state > 16 and _fills_in_pieces(plan, inner):
         return None
     return plan
+
+
+def _fills_in_pieces(plan: ScanPlan, inner: int) -> bool:
+    """Whether the blocks of whole portions, 16 channels each, take most of the device's warp slots."""
+    return plan.num_long * -(-inner // 16) > 2.5 * sm_count()
 
 
 def selective_workspace_floats(plan: Optional[ScanPlan], inner: int, n_state: int) -> int:
@@ -2289,7 +2294,8 @@ def selective_scan(x: torch.Tensor, low: torch.Tensor, b_col: int, step: torch.T
     the step projection with its bias, before softplus; the gate z in ``proj[:, z_col:z_col + inner]``; ``a`` float32
     [inner, n] (negative); ``d_skip`` float32 [inner].  Returns ``(S . C + D x) * silu(z)`` in ``x``'s dtype.
     With a ``plan`` (``scan_plan``) that has chunks and a ``workspace`` of ``selective_workspace_floats``, the long
-    portions run as chunks side by side (two passes and ``selective_combine`` between them), the others in one piece."""
+    portions run as chunks side by side (two passes and ``selective_combine`` between them), the others in one piece.  Without a
+    ``workspace`` portions whose blocks fill the device (``_fills_in_pieces``) run in one piece each."""
     _dev(x, low, step, proj, a, d_skip, state, cu_seqlens, slots, workspace)
     tokens, inner = x.shape
     n = a.shape[1]
@@ -2303,7 +2309,7 @@ def selective_scan(x: torch.Tensor, low: torch.Tensor, b_col: int, step: torch.T
               _p(d_skip), _p(state), state.shape[1], _p(out), _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"))
     need = selective_workspace_floats(plan, inner, n)
     plan = _selective_cut(plan, inner, n)
-    if not need:
+    if not need or (workspace is None and _fills_in_pieces(plan, inner)):
         _call("lily_selective_scan", *common, int(requests), tokens, inner, n, _dt(x), None, None, None, 0, None, None, _stream())
         return out
     if workspace is None or workspace.dtype != torch.float32 or workspace.numel() < need:

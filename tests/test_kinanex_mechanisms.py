@@ -538,6 +538,29 @@ def test_selective_scan_a_channel_a_thread(lens, inner, state_n, dtype):
     assert float((state[:, -3:] - 7.0).abs().max()) == 0.0
 
 
+@pytest.mark.gpu
+def test_selective_scan_of_many_channels_without_scratch():
+    """Long portions whose blocks fill the device in one piece each need no scratch; of fewer channels they ask for it."""
+    from lily_b200.csrc.ops import KernelError
+    ops = ops_for("cuda")
+    g = torch.Generator().manual_seed(2)
+    n, rank, state_n = 200, 2, 4
+    for inner, refused in ((6016, False), (256, True)):
+        x, low, proj = (torch.randn(n, w, generator=g).bfloat16().cuda() for w in (inner, rank + 2 * state_n, 2 * inner))
+        step, a, d_skip = torch.randn(n, inner, generator=g).cuda(), -torch.rand(inner, state_n, generator=g).cuda(), torch.randn(inner, generator=g).cuda()
+        plan = ops.scan_plan([n], torch.device("cuda"), inner * state_n, chunks=False)
+
+        def run(**more):
+            state = torch.zeros((2, inner * state_n), device="cuda")
+            return ops.selective_scan(x, low, rank, step, proj, inner, a, d_skip, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, **more), state
+        assert ops.selective_workspace_floats(plan, inner, state_n) > 0
+        if refused:
+            with pytest.raises(KernelError, match="workspace"):
+                run(plan=plan)
+        else:
+            assert all(torch.equal(p, q) for p, q in zip(run(plan=plan), run()))
+
+
 # ------------------------------------------------------------------ feed-forward, layer scale, frequencies
 
 @pytest.mark.parametrize("device", DEVICES)
