@@ -66,21 +66,6 @@ struct Args {
     float unit_eps, q_scale;
 };
 
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 hf = __bfloat1622float2(h);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    split2(x - hf.x, y - hf.y, mid, lo);
-}
-
-template <int N>
-__device__ __forceinline__ void add(float (&total)[N][4], const float (&sum)[N][4]) {
-#pragma unroll
-    for (int j = 0; j < N; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) total[j][q] += sum[j][q];
-}
-
 __device__ __forceinline__ void stage_rows(__nv_bfloat16* dst, const __nv_bfloat16* src, size_t ld, int rows, int d) {
     const int per = d / 8;
     for (int e = threadIdx.x; e < CHUNK * per; e += THREADS) {
@@ -263,8 +248,6 @@ struct Tile {
 };
 
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
-__device__ __forceinline__ float upper(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
-__device__ __forceinline__ float lower(uint32_t pair) { return __uint_as_float(pair << 16); }
 
 // o += row i of the lower triangle's tiles times the rows of `rows`; `odd`: the rows of the tile on the diagonal hold an infinity or
 // a NaN, and are taken entry by entry so that a zero above the diagonal meets none.

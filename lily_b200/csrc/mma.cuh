@@ -1,5 +1,5 @@
 // Fragments of the warp-level tensor-core product (mma.sync m16n8k16, bfloat16 in, float32 out) and what feeds them: asynchronous
-// 16-byte copies to shared memory, ldmatrix, and the cut of a float32 number into the sum of two bfloat16 ones.
+// 16-byte copies to shared memory, ldmatrix, and the cut of a float32 number into the sum of two or three bfloat16 ones.
 #pragma once
 
 #include "common.cuh"
@@ -37,6 +37,27 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
     const __nv_bfloat162 l = __floats2bfloat162_rn(x - back.x, y - back.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// The same as three pairs, whose sum they are (an infinity becomes a NaN).
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const float2 back = __bfloat1622float2(h);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    split2(x - back.x, y - back.y, mid, lo);
+}
+
+// The second and the first number of a pair of bfloat16.
+__device__ __forceinline__ float upper(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+__device__ __forceinline__ float lower(uint32_t pair) { return __uint_as_float(pair << 16); }
+
+// Runs of 16 products' sums onto their totals by rounded additions: the tensor cores cut what they add to an accumulator off, so a total
+// kept in one would drift by half a last bit a product.
+template <int N>
+__device__ __forceinline__ void add(float (*total)[4], const float (&sum)[N][4]) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) total[j][q] += sum[j][q];
 }
 
 }  // namespace mma16

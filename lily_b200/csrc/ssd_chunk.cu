@@ -53,14 +53,6 @@ struct Args {
 
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
-// Pairs of float32 numbers as three pairs of bfloat16 whose sum they are (an infinity becomes a NaN).
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 hf = __bfloat1622float2(h);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    split2(x - hf.x, y - hf.y, mid, lo);
-}
-
 // Which of a pair of bfloat16 numbers are infinities or NaN, as a mask over the pair's bits.
 __device__ __forceinline__ uint32_t not_finite(uint32_t pair) {
     return ((pair & 0x7f80u) == 0x7f80u ? 0xffffu : 0u) | ((pair & 0x7f800000u) == 0x7f800000u ? 0xffff0000u : 0u);
@@ -109,16 +101,6 @@ __device__ __forceinline__ void stage_rows(__nv_bfloat16* dst, int stride, const
         const bool in = r < rows && c < have;
         cp_async16(smem_u32(dst + r * stride + c), src + (in ? (size_t)r * ld + c : 0), in);
     }
-}
-
-// A run of 16 products' sum onto the total by a rounded addition: the tensor cores cut what they add to an accumulator off, so a
-// total kept in one would drift by half a last bit a product.
-template <int N>
-__device__ __forceinline__ void add(float (*total)[4], const float (&sum)[N][4]) {
-#pragma unroll
-    for (int j = 0; j < N; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) total[j][q] += sum[j][q];
 }
 
 struct WriteTile {

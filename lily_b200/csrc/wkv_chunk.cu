@@ -52,15 +52,6 @@ struct Args {
     int heads, d;
 };
 
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 hf = __bfloat1622float2(h);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    split2(x - hf.x, y - hf.y, mid, lo);
-}
-__device__ __forceinline__ float upper(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
-__device__ __forceinline__ float lower(uint32_t pair) { return __uint_as_float(pair << 16); }
-
 // The three parts of a pair of columns into their planes.
 __device__ __forceinline__ void put(__nv_bfloat16 (*planes)[CHUNK][LD], int row, int col, float x, float y) {
     uint32_t p[3];
@@ -76,14 +67,6 @@ __device__ __forceinline__ void stage_values(__nv_bfloat16 (*dst)[LD], const __n
         const bool in = r < rows && c < d;
         cp_async16(smem_u32(&dst[r][c]), src + (in ? (size_t)r * ld + c : 0), in);
     }
-}
-
-template <int N>
-__device__ __forceinline__ void add(float (*total)[4], const float (&sum)[N][4]) {
-#pragma unroll
-    for (int j = 0; j < N; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) total[j][q] += sum[j][q];
 }
 
 struct WriteTile {
