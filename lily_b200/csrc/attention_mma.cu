@@ -16,8 +16,9 @@
 //    RMSNorm and the rotation, and the block whose key range holds the new position does the same
 //    for the key, copies the value, and writes both to their page before it reads them.
 //
-// Key and value tiles of 64 positions are brought in with cp.async (16-byte pieces, any page
-// size: each row's page is looked up in the block table), double buffered, into shared memory
+// Key and value tiles of 64 positions, double buffered (decode: or three buffers), come by TMA in decode where a page is a whole number of
+// tiles and the head size is 64 or 128, and with cp.async elsewhere (16-byte pieces, any page
+// size: each row's page is looked up in the block table); either way into shared memory
 // whose 16-byte pieces are XOR-swizzled by row so that ldmatrix reads without bank conflicts.
 // Scores, the running maximum and sum, and the output accumulate in float32; probabilities are
 // rounded to bfloat16 for p.v as in lily/layers/attention/triton_ops/extend_attention.py:110-112.
