@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "tcgen05.cuh"
 
+#include <atomic>
 #include <cooperative_groups.h>
 
 namespace lily {
@@ -1055,7 +1056,9 @@ LILY_API int lily_attention_decode_mma_clusters(int d, int splits, int group) {
     return 0;
 }
 
-// The host's word in which the decode kernel says that a wait for a tile ran out; made once, also while a graph is captured.
+// The host's word in which the decode kernel says that a wait for a tile ran out; made once, with the first launch that may, also while a
+// graph is captured.
+static std::atomic<int*> g_lost_word{nullptr};
 static int* lost_word() {
     static int* word = [] {
         int* p = nullptr;
@@ -1067,6 +1070,7 @@ static int* lost_word() {
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (p) *p = 0;
+        g_lost_word = p;
         return p;
     }();
     return word;
@@ -1156,7 +1160,7 @@ LILY_API int lily_attention_decode_mma_fused(const void* qkv, int qkv_planes, si
 // of the device; else as far as the host knows (the kernels it has waited for).
 LILY_API int lily_attention_decode_status(int wait) {
     if (wait && cudaDeviceSynchronize() != cudaSuccess) return -1;
-    volatile int* word = lost_word();
+    volatile int* word = g_lost_word;
     const int v = word ? *word : 0;
     if (v != 0) *word = 0;
     return v;
