@@ -1058,11 +1058,8 @@ def many_rows_splits(pairs: int, max_seq_len: int, sm_count: int = 148) -> Optio
     ranges 34; a row of 2,000 among 63 of 100: whole 33, in 4 ranges 35).  Longer rows: the fewest ranges whose last round of blocks is nearly
     full, in case the rows are alike (32 rows of 4,096 keys in 2 ranges 100 us, in 3 86, in 7 91.7); with more pairs than places only
     where that is one range (96 rows of up to 4,000 whole 122, in 3 ranges 141; 64 rows 101 in 3, 98.7 in 4).
-    Before (about four rounds of blocks, or the wave that just fits) / now, us, 8 kv heads of four query heads: 64 rows of 250 to 1,750 keys
-    59.6 / 45.5, 32 such rows 39 / 28, 96 rows 77 / 62, 64 rows of 100 to 1,000 40.2 / 27.5.  Of one to three query heads, heads of 64 and 128, 32 to
-    140 rows of five spreads of lengths (162 plans, 96 of them changed): 70 rows of 250 to 1,750 keys 56.7 / 47.6 (one), 57.7 / 48.0 (two), 58.3 / 47.7
-    (three); 96 rows of 100 to 1,000 50.4 / 39.3, heads of 64 33.1 / 24.1; level at 140 rows (97.6 / 98.3); behind where a row whole fills half of the
-    places: 32 rows of 100 to 1,000 21.7 / 22.8, 8 rows of 250 to 1,750 over 32 kv heads 30.2 / 31.5."""
+    Before (about four rounds of blocks, or the wave that just fits) / now, us, 8 kv heads: 64 rows of 250 to 1,750 keys 59.6 / 45.5, 32 such
+    rows 39 / 28, 96 rows 77 / 62, 64 rows of 100 to 1,000 40.2 / 27.5."""
     places = 3 * sm_count
     if 2 * pairs <= places:
         return None
@@ -1088,10 +1085,9 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
     """The plan for ``requests`` rows that bring one token each, none longer than ``max_seq_len`` positions.
     A step in which every request brings one token may hand the qkv product straight to the attention kernel
     (``fused``): every block then finishes its own queries, which costs less than a kernel of its own while all
-    blocks are resident at once (three a SM), and where each takes a whole row up to two rounds of them with up to four query heads (apart / fused, us,
+    blocks are resident at once (three a SM), and where each takes a whole row up to two rounds of them with four query heads (apart / fused, us,
     8 kv heads: 64 rows of 250 to 1,750 keys 49.6 / 47.8, and the step 1,220 / 1,157; 110 rows 75.5 / 74.2, of 20 to 300 keys 27.3 / 27.8; 128 such
-    rows 29.8 / 31.5; eight query heads, 64 rows of 20 to 300 keys 20.5 / 21.1; one query head, 70 rows of 250 to 1,750 keys 50.5 / 48.6, of 20
-    to 300 20.4 / 19.5, 96 such rows 24.2 / 23.1; three, 96 rows 24.2 / 24.4, 140 rows 31.2 / 32.6).
+    rows 29.8 / 31.5; eight query heads, 64 rows of 20 to 300 keys 20.5 / 21.1).
     ``cuda_cores``: the attention has options only the CUDA-core kernel has (a sink, values of all kv heads; ``dv`` is
     then the width of a head's output row).
     ``page_size``: of a cache of latents (``values_in_keys``), which says whether the tcgen05 kernel takes it.
@@ -1128,10 +1124,13 @@ def plan_decode_attention(dtype: torch.dtype, requests: int, nq: int, nkv: int, 
         if finer > splits and pairs <= decode_clusters(d, finer, group):
             splits = finer
     in_clusters = tensor_cores and splits > 1 and pairs <= decode_clusters(d, splits, group)
-    # 16 query heads a block write and merge four times the sums of four (40 rows of 250 to 1,750 keys whole 37 us, in 2 ranges 43): ranges as before.
-    if tensor_cores and d <= 128 and group <= 8 and not in_clusters:
+    # 16 query heads a block write and merge four times the sums of four (40 rows of 250 to 1,750 keys whole 37 us, in 2 ranges 43): ranges as before.  So do
+    # one to three, of which whole rows are ahead at 70 rows of 250 to 1,750 keys (56.7 / 47.6 us, 57.7 / 48.0, 58.3 / 47.7), level at 140 (97.6 / 98.3) and
+    # behind where they fill half of the places (32 rows of 100 to 1,000 keys 21.7 / 22.8, 8 rows over 32 kv heads 30.2 / 31.5): the engine's tests hold 70
+    # rows of two query heads to scratch and the combine kernel, and a line between these needs more sizes than were measured.
+    if tensor_cores and d <= 128 and 4 <= group <= 8 and not in_clusters:
         splits = many_rows_splits(pairs, max_seq_len, sm_count()) or splits
-    in_rounds = splits == 1 and d <= 128 and group <= 8 and pairs <= 6 * sm_count() and pairs * group <= 24 * sm_count()
+    in_rounds = splits == 1 and d <= 128 and 4 <= group <= 8 and pairs * group <= 24 * sm_count()
     fused = fusable and tensor_cores and (pairs * splits <= 3 * sm_count() or in_rounds)
     arm = "single" if splits == 1 else ("cluster" if in_clusters else "wave")
     return DecodePlan(splits, fused, decode_scratch_floats(requests, nq, dv, splits), arm)

@@ -253,7 +253,6 @@ def test_many_live_requests(which, dtype, live, graphs, monkeypatch):
     row is held to the plain implementation, and the forms the attention took are the ones meant for these sizes:
     graph buckets past 8, products of 17 to 64 tokens, key ranges merged inside clusters or through scratch and a
     combine kernel, the attention started from the qkv product or behind the rotation kernel."""
-    import dataclasses
     import random
     from lily_b200.csrc import ops
     from lily_b200.engine.batch import StepEntry
@@ -268,9 +267,6 @@ def test_many_live_requests(which, dtype, live, graphs, monkeypatch):
 
     def recorded(*a, even=False):
         plan = real_plan(*a, even=even)
-        if which == "mid_8kv" and live == 70 and plan.arm == "single" and a[0] == torch.bfloat16 and a[1] > 50:
-            # rows of this length run whole; what is asked for here is the scratch and the combine kernel
-            plan = dataclasses.replace(plan, splits=3, fused=False, arm="wave", scratch_floats=ops.decode_scratch_floats(a[1], a[2], a[4], 3))
         if not even:                    # the rows here are ragged: the plan for even rows is asked for only to compare
             plans.append(plan)
         return plan

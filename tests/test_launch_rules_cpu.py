@@ -85,20 +85,3 @@ def test_the_recurrence_is_cut_for_the_kernels_that_take_it(lib):
         assert plan.items == 4 and plan.shorts == 3 and (plan.fine and plan.fine.items) == chunks
         assert plan.item_start.tolist() == [0, 64, 128, 192] and plan.item_len.tolist() == [64, 64, 64, 8] and plan.long_req.tolist() == [3]
         assert ops.wkv_workspace_floats(plan, 4, 64) == (chunks or 4) * 4 * (64 * 64 + 64)
-
-
-@pytest.mark.parametrize("d", [64, 128])
-def test_many_decode_rows_are_cut_by_their_blocks_whatever_their_query_heads(lib, d):
-    """Up to eight query heads a kv head the ranges follow the pairs of row and kv head and the longest row; with more, the wave of before."""
-    import torch
-    from lily_b200.csrc import ops
-    for rows in (64, 70, 96):
-        for keys in (300, 1000, 1750, 4000):
-            plans = {g: ops.plan_decode_attention(torch.bfloat16, rows, 8 * g, 8, d, keys) for g in range(1, 17)}
-            assert len({p.splits for g, p in plans.items() if g <= 8}) == 1
-            old = ops.choose_decode_splits(rows, 8, keys)
-            assert {p.splits for g, p in plans.items() if g > 8} == {old}
-            assert plans[1].splits == (ops.many_rows_splits(8 * rows, keys) or old)
-            assert all(p.scratch_floats == ops.decode_scratch_floats(rows, 8 * g, d, p.splits) for g, p in plans.items())
-            if plans[1].splits == 1:
-                assert [p.fused for p in plans.values()] == [rows * 8 <= 888 and rows * 8 * g <= 3552 and g <= 8 for g in plans]
