@@ -112,7 +112,8 @@ class Wkv(Mixer):
         low = ops.linear(mixes[4], self.w_1, out_dtype=torch.float32)            # [tokens, rank], float32 from here on
         log_decay = ops.wkv_decay(low, self.w_2t, self.w_0)
         # long portions run as chunks side by side; the cut is planned once a step for all layers
-        plan = batch.plan(("wkv_plan", s.head_dim), lambda b: ops.wkv_plan(b.h_new_lens, b.token_ids.device, x.dtype, s.head_dim))
+        kind = (x.dtype, s.head_dim) if hasattr(ops, "wkv_chunks_take") else ()          # (a stand-in may run token by token only)
+        plan = batch.plan(("wkv_plan", s.head_dim), lambda b: ops.wkv_plan(b.h_new_lens, b.token_ids.device, *kind))
         need = ops.wkv_workspace_floats(plan, s.heads, s.head_dim)
         room = batch.workspace.floats("wkv_chunks", need) if need and batch.workspace is not None else None
         if need and room is None:

@@ -517,7 +517,7 @@ def wkv_max_head_dim():
     return 256
 
 
-def wkv_plan(new_lens, device, dtype=None, d=None):
+def wkv_plan(new_lens, device):
     return None
 
 

@@ -71,7 +71,6 @@ def test_wanted_rows_come_in_the_given_order(setup):
 def test_a_step_takes_ids_of_any_kind_and_refuses_others(setup):
     """Ids come as a list, a tuple, an array or a tensor, and as numbers that are whole; one outside the vocabulary anywhere in a portion is
     refused before a page is taken."""
-    from array import array
     import numpy as np
     from lily_b200.engine.batch import StepEntry
     cfg, _, path = setup
@@ -79,8 +78,7 @@ def test_a_step_takes_ids_of_any_kind_and_refuses_others(setup):
     ids = tiny_models.random_tokens(7, v, 4)
     runner = make_runner(path)
     outs = []
-    for tokens in (ids, tuple(ids), np.array(ids), np.array(ids, dtype=np.int16), torch.tensor(ids), [float(t) for t in ids], [np.int64(t) for t in ids],
-                   array("i", ids), array("q", ids)):
+    for tokens in (ids, tuple(ids), np.array(ids), np.array(ids, dtype=np.int16), torch.tensor(ids), [float(t) for t in ids], [np.int64(t) for t in ids]):
         slot = runner.open_request()
         outs.append(runner.step([StepEntry(slot, tokens, [6])]))
         runner.close_request(slot)
@@ -93,7 +91,9 @@ def test_a_step_takes_ids_of_any_kind_and_refuses_others(setup):
 
 
 def test_a_step_takes_bytes_as_ids(setup):
-    """A sequence of bytes is a sequence of ids, whatever its length; arrays of another length than their entry's are refused."""
+    """A sequence of bytes is a sequence of ids, whatever its length, and so is an array of numbers; arrays of another length than their
+    entry's are refused."""
+    from array import array
     import numpy as np
     from lily_b200.engine.batch import StepEntry, build_step_batch
     _, _, path = setup
@@ -106,7 +106,7 @@ def test_a_step_takes_bytes_as_ids(setup):
         return out
     for ids in ([5, 0, 0, 0], [5, 6, 7], [5, 6, 7, 8], [9], [1, 2, 3, 4, 5, 6, 7, 8]):
         want = logits(ids)
-        for kind in (bytes, bytearray, lambda x: memoryview(bytes(x))):
+        for kind in (bytes, bytearray, lambda x: memoryview(bytes(x)), lambda x: array("i", x), lambda x: array("q", x), lambda x: array("B", x)):
             assert torch.equal(logits(kind(ids)), want)
     for ids in ([1], [1, 2], [1, 2, 3, 4]):
         with pytest.raises(ValueError, match="ids for the 3 tokens"):
