@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(ROW_CHANNELS) selective_rows_kernel(const Sele
             const float4 *bp = reinterpret_cast<const float4*>(&Bs[buf][k0][0]), *cp = reinterpret_cast<const float4*>(&Cs[buf][k0][0]);
 #pragma unroll
             for (int k = 0; k < ROW_STEP; ++k) {
+                if (!OUT && k0 + k >= n_tok) break;            // a step of zero and an infinite rate make a NaN: the state that is kept meets neither
                 const float dx = dt[k] * xv[k];
                 steps += dt[k];
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};

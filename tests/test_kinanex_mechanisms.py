@@ -539,6 +539,30 @@ def test_selective_scan_a_channel_a_thread(lens, inner, state_n, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [193, 194, 195, 196, 224, 255])
+@pytest.mark.parametrize("state_n", [3, 8, 16])
+def test_selective_scan_in_chunks_with_an_infinite_rate(n, state_n):
+    """An entry whose rate is minus infinity forgets at every token: chunks that end inside a step of four tokens leave what pieces leave."""
+    ops = ops_for("cuda")
+    g = torch.Generator().manual_seed(n)
+    rank, inner = 2, 130
+    x, low, proj = (torch.randn(n, w, generator=g).cuda() for w in (inner, rank + 2 * state_n, 2 * inner))
+    step, a, d_skip = torch.randn(n, inner, generator=g).cuda(), -torch.rand(inner, state_n, generator=g).cuda(), torch.randn(inner, generator=g).cuda()
+    a[7, 1] = a[129, 2] = float("-inf")
+    plan = ops.scan_plan([n], torch.device("cuda"), inner * state_n, chunks=False)
+    need = ops.selective_workspace_floats(plan, inner, state_n)
+    assert need > 0
+
+    def run(**more):
+        state = torch.ones((2, inner * state_n), device="cuda")
+        return ops.selective_scan(x, low, rank, step, proj, inner, a, d_skip, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, **more), state
+    (y, state), (want, kept) = run(plan=plan, workspace=torch.empty(need, device="cuda")), run()
+    assert torch.isfinite(want).all() and torch.isfinite(kept).all()
+    torch.testing.assert_close(y, want, atol=1e-4, rtol=1e-4)
+    torch.testing.assert_close(state, kept, atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.gpu
 def test_selective_scan_of_many_channels_without_scratch():
     """Long portions whose blocks fill the device in one piece each need no scratch; of fewer channels they ask for it."""
     from lily_b200.csrc.ops import KernelError
