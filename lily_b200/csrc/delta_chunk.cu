@@ -80,6 +80,9 @@ __device__ __forceinline__ float exp_of(double x) {
     return fmaf(e, (float)(x - (double)hi), e);
 }
 
+// f x for a product x of two rows that may have overflowed: then one of the rows' divisors in f is zero, and so is the product of the unit vectors
+__device__ __forceinline__ float times(float f, float x) { return f == 0.f ? 0.f : f * x; }
+
 __device__ __forceinline__ int tile_of(int i, int j) { return i * (i + 1) / 2 + j; }      // the lower triangle's tiles, row by row
 
 struct Prepare {
@@ -111,8 +114,8 @@ __global__ void __launch_bounds__(THREADS) prepare_kernel(const Args a) {
         float sk = 0.f, sq = 0.f;
         for (int i = tid & 3; i < a.d; i += 4) {
             const float x = __bfloat162float(s.k[t][i]), z = __bfloat162float(s.q[t][i]);
-            sk = fmaf(x, x, sk);
-            sq = fmaf(z, z, sq);
+            sk = fmaf(x, x, sk + (x - x));                     // an infinity makes the divisor a NaN, squares that overflow a zero
+            sq = fmaf(z, z, sq + (z - z));
         }
 #pragma unroll
         for (int o = 1; o < 4; o <<= 1) {
@@ -182,8 +185,8 @@ __global__ void __launch_bounds__(THREADS) prepare_kernel(const Args a) {
             const float own = s.fk[t];
             for (int r = t; r < CHUNK; ++r) {
                 const float w = expf((s.hi[side][r] - hi) + (s.lo[side][r] - lo)) * own;
-                if (r > t) s.a[side][r][t] = s.b[side][r] * s.fk[r] * w * s.kk[r][t];
-                s.a[side][t][r] = s.fq[r] * w * s.qk[r][t];
+                if (r > t) s.a[side][r][t] = times(s.b[side][r] * s.fk[r] * w, s.kk[r][t]);
+                s.a[side][t][r] = times(s.fq[r] * w, s.qk[r][t]);
             }
         }
         __syncthreads();

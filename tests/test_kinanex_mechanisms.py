@@ -419,6 +419,29 @@ def test_delta_rule_in_chunks_keeps_what_is_not_finite_behind_its_token(monkeypa
     torch.testing.assert_close(y[~hit], clean[~hit], atol=1e-5, rtol=1e-5)
     assert bool(torch.isfinite(state).all()) == (what == "q")
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens", [(5,), (5, 6), (63, 64), (3, 70, 139)])
+def test_delta_rule_in_chunks_with_keys_whose_squares_overflow(monkeypatch, tokens):
+    """A finite key (or query) of 2^100 in every entry has a unit vector of zero: the token writes (reads) nothing, as one after another."""
+    ops = ops_for("cuda")
+    monkeypatch.setattr(ops, "delta_chunks_pay", lambda *a: True)
+    heads, kvh, d, dv, n = 4, 2, 64, 32, 140
+    qkv, proj, a_log, dt_bias = (x.cuda() for x in delta_inputs(n, heads, kvh, d, dv, 3, torch.bfloat16))
+    for t in tokens:
+        qkv[t, kvh * d:(kvh + 1) * d] = 2.0 ** 100                                             # the first key head
+        qkv[t, d:2 * d] = 2.0 ** 100                                                           # the second query head
+
+    def run(plan):
+        state = torch.zeros((2, heads * d * dv), device="cuda")
+        return ops.delta_rule(qkv, proj, 3, 3 + heads, a_log, dt_bias, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, heads, kvh, d, dv, 1e-6,
+                              d ** -0.5, plan=plan), state
+    (y, state), (want, kept) = run(ops.delta_plan([n], torch.bfloat16, heads, kvh, d, dv, torch.device("cuda"))), run(None)
+    assert torch.isfinite(want).all() and torch.isfinite(kept).all()
+    torch.testing.assert_close(y, want, atol=1e-5, rtol=1e-5)
+    torch.testing.assert_close(state, kept, atol=1e-5, rtol=1e-5)
+
+
 # ------------------------------------------------------------------ the selective scan
 
 def plain_scan(x, low, rank, step, z, a_log, d_skip):
