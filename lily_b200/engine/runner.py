@@ -76,6 +76,26 @@ def _load_library_products(device) -> None:
 _CAPTURING = threading.local()
 
 
+class _Lost:
+    """The waits that kernels of this process gave up, as the host has heard of them.  The kernels share one word, which its reader clears,
+    and it does not say whose step it was: so every runner hears of each, whichever of them read the word."""
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.count = self.row = 0
+
+    def heard(self, read) -> int:
+        with self.lock:
+            found = read()
+            if found:
+                self.count += 1
+                self.row = found
+            return self.count
+
+
+_LOST = _Lost()
+
+
 def _lane_streams(device, count: int, library: bool) -> List["torch.cuda.Stream"]:
     """The streams that a capture puts branches on, above the default priority: what runs there is a chain of short kernels beside
     products that stream weights.  A thread captures one step at a time and a replay does not use them, so a thread has one set a
@@ -242,6 +262,7 @@ class ModelRunner:
         self.future_tokens = torch.zeros(self.max_requests + 1, dtype=torch.int32, device=self.device)
         self._last_rows: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = None
         self.seq_lens: Dict[int, int] = {}
+        self._lost_heard = _LOST.count
         self._ring = _PinnedRing() if self.device.type == "cuda" else None
         self.profiler = DecodeProfiler.from_env() if self.device.type == "cuda" else None
         self.steps_run = 0
@@ -307,9 +328,10 @@ class ModelRunner:
         """Raises when a kernel that the host has waited for gave up a wait of its own, so that its step's results are no results.  (A read of
         a word in the host's memory.)"""
         lost = getattr(self.model.ctx.ops, "attention_decode_lost", None)       # (stand-ins for the kernels wait for nothing)
-        row = lost() if lost is not None else 0
-        if row:
-            raise RuntimeError(f"decode attention: a tile of keys did not arrive in time (row {row - 1} of its step); the step's tokens are void")
+        heard = _LOST.heard(lost) if lost is not None else self._lost_heard
+        if heard != self._lost_heard:
+            self._lost_heard = heard
+            raise RuntimeError(f"decode attention: a tile of keys did not arrive in time (row {_LOST.row - 1} of its step); the step's tokens are void")
 
     # ---- one step --------------------------------------------------------------------
 

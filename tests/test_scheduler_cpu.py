@@ -366,3 +366,18 @@ def test_a_step_whose_kernel_gave_up_a_wait_fails(setup, monkeypatch):
     with pytest.raises(RuntimeError, match="row 3 of its step"):
         s.run_to_completion()
     assert next(reports, None) is None
+
+
+def test_every_runner_hears_of_a_wait_that_was_given_up(setup, monkeypatch):
+    """The word in which kernels report does not say whose step it was and is cleared by its reader: each runner of the process raises
+    once, and one made afterwards does not."""
+    _, _, path = setup
+    runners = [scheduler(path).runner for _ in range(3)]
+    reports = iter([0, 6])
+    monkeypatch.setattr(runners[0].model.ctx.ops, "attention_decode_lost", lambda: next(reports, 0), raising=False)
+    runners[0].check_waits()
+    for r in (runners[1], runners[0], runners[2]):
+        with pytest.raises(RuntimeError, match="row 5 of its step"):
+            r.check_waits()
+        r.check_waits()
+    scheduler(path).runner.check_waits()
