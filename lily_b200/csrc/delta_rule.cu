@@ -255,8 +255,10 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
         const float fk = 1.f / sqrtf(kk + a.unit_eps), fq = a.q_scale / sqrtf(qq + a.unit_eps);
         const float sk = (second ? other : sum[0]) * fk, sq = (second ? sum[0] : other) * fq;
         const float u = beta * (value - decay * sk);
+        // where squares overflowed a unit vector is zero, and its product with the other too, whatever the raw one is
+        const float both = fk == 0.f || fq == 0.f ? 0.f : kq * fk * fq;
         if (lane % GROUP == 0 && j0 + mine < dv)
-            a.y[(size_t)(tok0 + t) * a.heads * dv + (size_t)head * dv + j0 + mine] = fmaf(decay, sq, kq * fk * fq * u);
+            a.y[(size_t)(tok0 + t) * a.heads * dv + (size_t)head * dv + j0 + mine] = fmaf(decay, sq, both * u);
         const float ku = u * fk;
 #pragma unroll
         for (int r = 0; r < RB; ++r) {

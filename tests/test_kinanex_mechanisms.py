@@ -442,6 +442,27 @@ def test_delta_rule_in_chunks_with_keys_whose_squares_overflow(monkeypatch, toke
     torch.testing.assert_close(state, kept, atol=1e-5, rtol=1e-5)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,q", [(2.0 ** 100, 2.0 ** 100), (2.0 ** 100, None), (None, 2.0 ** 100)])
+def test_delta_step_with_a_key_whose_squares_overflow(k, q):
+    """The same for the kernel of one token a request, held to the kernel of the prompts."""
+    ops = ops_for("cuda")
+    heads, kvh, d, dv = 4, 2, 64, 32
+    qkv, proj, a_log, dt_bias = (x.cuda() for x in delta_inputs(2, heads, kvh, d, dv, 4, torch.bfloat16))
+    if k:
+        qkv[0, kvh * d:(kvh + 1) * d] = k
+    if q:
+        qkv[0, :d] = q
+    qkv[1, kvh * d:2 * kvh * d] = 0                            # a second token that writes nothing
+    outs = []
+    for n in (1, 2):
+        state = torch.rand((2, heads * d * dv), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+        outs.append(ops.delta_rule(qkv[:n], proj[:n], 3, 3 + heads, a_log, dt_bias, state, i32([0, n], "cuda"), i32([1], "cuda"), 1, heads, kvh, d, dv,
+                                   1e-6, d ** -0.5)[0])
+    assert torch.isfinite(outs[1]).all()
+    torch.testing.assert_close(outs[0], outs[1], atol=1e-5, rtol=1e-5)
+
+
 # ------------------------------------------------------------------ the selective scan
 
 def plain_scan(x, low, rank, step, z, a_log, d_skip):
